@@ -590,6 +590,40 @@ def test_rle_fused_codec_matches_host_bytes(world, n, thr, density):
     assert float(r.abs().sum()) == 0.0
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1 << 20, (1 << 20) + 1, 592 * 2048, 592 * 2048 + 1, 3 * 592 * 2048 - 5])
+@pytest.mark.parametrize("kind", ["dense", "sparse", "one_run", "alternating"])
+def test_rle_chunks_and_run_blocks(n, kind):
+    """Several tiles per sending CTA and many blocks of runs per receiving CTA, up to runs longer
+    than a CTA's share of the output and the worst case of n runs: the bytes in the slot are the
+    host codec's, the expansion (both modes) is exact."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    e0, e1 = world.envs
+    codecs = [P.RleCodec(e, n) for e in world.envs]
+    gen = torch.Generator().manual_seed(n)
+    g = torch.randn(n, generator=gen)
+    thr = {"dense": 1.0, "sparse": 3.5, "one_run": 100.0, "alternating": 0.5}[kind]
+    if kind == "alternating":
+        g = torch.where(torch.arange(n) % 2 == 0, g.abs() + 1.0, torch.zeros(n))
+    cell = torch.full((1,), thr, dtype=torch.float32, device="cuda")
+    r = torch.zeros(n, device="cuda")
+    codecs[0].send(g.cuda(), r, cell, 1, 1)
+    status = e1.new_status("t")
+    out = torch.full((n,), 9.0, device="cuda")
+    codecs[1].recv(out, 1, False, status)
+    acc = torch.ones(n, device="cuda")
+    codecs[1].recv(acc, 1, True, status)
+    e1.flush()
+    assert status.value == 0
+    kept = torch.where(g.abs() >= thr, g, torch.zeros(n))
+    assert torch.equal(out.cpu(), kept) and torch.equal(acc.cpu(), 1 + kept)
+    assert torch.equal(r.cpu(), g - kept)
+    expect = cx.CompressorRLE.encode(g, torch.zeros(n), thr)
+    ep = codecs[1].slots[1].endpoint(e1)
+    assert e1.read_header(ep.hdr).bytes == len(expect) and e1.read_bytes(ep.pairs, len(expect)) == expect
+    world.close()
+
+
 def test_rle_fused_receive_rejects_corrupt_runs(world):
     """Host-side fault injection: run lengths that do not add up to n set BAD_HEADER and leave
     the output untouched; a payload that never arrives times out with a status."""
