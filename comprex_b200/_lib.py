@@ -65,6 +65,12 @@ class ApplyArgs(C.Structure):
 OPK_THRESHOLD, OPK_COMPRESS, OPK_APPLY, OPK_DENSE_SEND, OPK_DENSE_REDUCE, OPK_UPDATE, OPK_MM_ALLREDUCE = 1, 2, 3, 4, 5, 6, 7
 
 
+class Fold(C.Structure):
+    """A vector folded from gradient tensors (CxFold in csrc/cx_common.h)."""
+    _fields_ = [("seg_ptr", C.c_void_p), ("seg_off", C.c_void_p), ("seg_end", C.c_void_p), ("coef", C.c_void_p),
+                ("sub_seg", C.c_void_p), ("u", C.c_void_p), ("base", C.c_int64), ("nseg", C.c_int32), ("mu", C.c_float)]
+
+
 class Op(C.Structure):
     """One launch of a pre-built launch sequence (CxOp in csrc/cx_common.h)."""
     _fields_ = [("kind", C.c_int32), ("dev", C.c_int32), ("dtype", C.c_int32), ("has_ranges", C.c_int32),
@@ -74,7 +80,8 @@ class Op(C.Structure):
                 ("workspace", C.c_void_p), ("ws_bytes", C.c_int64), ("stats", C.c_void_p),
                 ("out", C.c_void_p), ("own", C.c_void_p), ("status", C.c_void_p), ("timeout_ns", C.c_uint64),
                 ("has_push", C.c_int32), ("lane", C.c_int32),
-                ("starts", C.c_int64 * MAX_PEERS), ("lens", C.c_int64 * MAX_PEERS),
+                ("starts", C.c_int64 * MAX_PEERS), ("lens", C.c_int64 * MAX_PEERS), ("fold", C.c_void_p),
+                ("chain", C.c_int32), ("pad", C.c_int32),
                 ("tg", Targets), ("src", Sources), ("apply", ApplyArgs)]
 
 
@@ -119,6 +126,8 @@ def _declare(lib) -> None:
         "cx_graph_free": (i32, [vp]),
         "cx_sizeof": (i64, [i32]),
         "cx_fold": (i32, [i32, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp, f32, f32, f32, vp]),
+        "cx_fold_coef": (i32, [i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, f32, f32, vp]),
+        "cx_fold_update": (i32, [i32, P(Fold), i64, P(ApplyArgs), vp]),
         "cx_axpy": (i32, [i32, i32, vp, i32, vp, f32, i64, vp]),
         "cx_fill_zero": (i32, [i32, vp, i64, vp]),
         "cx_rle_compress_host": (i64, [vp, vp, i64, f32, vp, i64]),
@@ -171,12 +180,36 @@ def load():
                     f"native library {path} is missing and could not be built: {exc}") from exc
         lib = C.CDLL(path)
         _declare(lib)
-        for what, mirror in enumerate((Op, Sources, Targets, ApplyArgs, None, Header)):
+        for what, mirror in enumerate((Op, Sources, Targets, ApplyArgs, None, Header, Fold)):
             if mirror is not None and lib.cx_sizeof(what) != C.sizeof(mirror):
                 raise ComprexError(f"{path} does not match this binding ({mirror.__name__} is "
                                    f"{lib.cx_sizeof(what)} bytes there, {C.sizeof(mirror)} here): rebuild it")
         _lib = lib
     return _lib
+
+
+_host_mod = None
+
+
+def host():
+    """The Python extension of csrc/python, built first when it is missing."""
+    global _host_mod
+    if _host_mod is None:
+        import importlib.machinery
+        import importlib.util
+        path = os.path.join(os.path.dirname(lib_path()), "_cxhost.so")
+        with _lock:
+            if not os.path.exists(path):
+                from . import build as _build
+                try:
+                    _build.build()
+                except Exception as exc:
+                    raise ComprexError(f"native extension {path} is missing and could not be built: {exc}") from exc
+        loader = importlib.machinery.ExtensionFileLoader("_cxhost", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_cxhost", loader))
+        loader.exec_module(mod)
+        _host_mod = mod
+    return _host_mod
 
 
 def last_error() -> str:

@@ -49,6 +49,7 @@ from .ops import primitives as P
 
 
 _log = logging.getLogger("comprex.allreduce")
+_EXACT_SAMPLES = 2 ** 31 - 128      # "sample" larger than any vector: every element is looked at
 
 
 def _chunks(size: int, nranks: int, align: int = 1):
@@ -431,12 +432,22 @@ class _ComprexAllreduceBase(_AllreduceBase):
         self.__dict__.pop("_replay_cache", None)      # the ratio is part of the recorded launches
         self.__dict__.pop("_fast_cache", None)
 
+    @property
+    def sampling(self):
+        """(default sample size, sampling factor) of the threshold estimate."""
+        return self._subsamples, self._sample_factor
+
+    @property
+    def exact_topk(self) -> bool:
+        """True when the threshold comes from the whole vector (:meth:`set_exact_topk`)."""
+        return self._subsamples >= _EXACT_SAMPLES
+
     def set_exact_topk(self, exact: bool = True) -> None:
         """Threshold from a select over the whole vector (exactly top-k) instead of the sampled
         estimate of the reference; costs a few extra passes over the vector per call."""
         if exact:
             self._sampling = getattr(self, "_sampling", (self._subsamples, self._sample_factor))
-            self._subsamples = 2 ** 31 - 128
+            self._subsamples = _EXACT_SAMPLES
         elif hasattr(self, "_sampling"):
             self._subsamples, self._sample_factor = self._sampling
         self.__dict__.pop("_replay_cache", None)
@@ -572,17 +583,35 @@ class Comprex_BigRingAllreduce(_ComprexAllreduceBase):
             got = cache[par] = (_OpSeq(env, [thr, cmp_]), _OpSeq(env, [app]))
         return got
 
-    def send_fast(self, g: torch.Tensor):
-        """Threshold + compress of ``g`` with one native call; returns (seq, parity) for recv_fast."""
+    launch_lists = _seqs
+
+    @property
+    def step(self) -> int:
+        """Number of the last exchange step."""
+        return self._step
+
+    def next_step(self):
+        """Begin the next exchange step; returns (seq, parity)."""
         self._step += 1
-        seq, par = self._step, self._step & 1
+        return self._step, self._step & 1
+
+    def send_fast(self, g: torch.Tensor, fold=None):
+        """Threshold + compress of ``g`` with one native call; returns (seq, parity) for recv_fast.
+        ``fold=(Fold, element type code)``: of a vector folded from gradient tensors instead (CUDA;
+        the struct must outlive the launch)."""
+        seq, par = self.next_step()
         if self._env.ranks == 1 and not self.consistent:
             return seq, par
         send, _ = self._seqs(par)
-        code, ptr = _lib.dtype_code(g.dtype), g.data_ptr()
         thr, cmp_ = send.arr[0], send.arr[1]
-        thr.g = cmp_.g = ptr
-        thr.dtype = cmp_.dtype = code
+        if fold is not None:
+            thr.g = cmp_.g = None
+            thr.fold = cmp_.fold = C.addressof(fold[0])
+            thr.dtype = cmp_.dtype = fold[1]
+        else:
+            thr.g = cmp_.g = g.data_ptr()
+            thr.fold = cmp_.fold = None
+            thr.dtype = cmp_.dtype = _lib.dtype_code(g.dtype)
         thr.ratio = self.compression_ratio
         send.run(seq)
         return seq, par

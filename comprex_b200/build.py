@@ -22,6 +22,7 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 OBJDIR = PKG / "build"
 LIB = LIBDIR / "libcomprex_b200.so"
+HOST = LIBDIR / "_cxhost.so"        # Python extension: host work on torch tensors (csrc/python)
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # -fmad=false: no multiply-add contraction, so that the kernels and the host
@@ -71,16 +72,37 @@ def _compile(src: Path, verbose: bool, ptxas_v: bool) -> Path:
     return obj
 
 
+def _build_host(verbose: bool) -> None:
+    """The Python extension; torch's libraries are those of the process that imports it."""
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    src = CSRC / "python" / "host.cpp"
+    if not _stale(HOST, [src, Path(__file__)]):
+        return
+    cmd = ([os.environ.get("CXX", "g++"), "-shared"] + CXX_FLAGS
+           + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+           + [f"-I{d}" for d in include_paths() + [sysconfig.get_paths()["include"]]] + [str(src), "-o", str(HOST)]
+           + [f"-L{d}" for d in library_paths()] + ["-ltorch_python", "-ltorch_cpu", "-lc10"])
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"compiling {src.name} failed:\n{res.stdout}\n{res.stderr}")
+
+
 def build(verbose: bool = False, force: bool = False, ptxas_v: bool = False) -> Path:
     """Compile every source under csrc/ for sm_100a and link the shared library."""
     LIBDIR.mkdir(exist_ok=True)
     OBJDIR.mkdir(exist_ok=True)
     if force:
-        for f in OBJDIR.glob("*.o"):
-            f.unlink()
+        for f in list(OBJDIR.glob("*.o")) + [HOST]:
+            f.unlink(missing_ok=True)
     srcs = sources()
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        host = ex.submit(_build_host, verbose)
         objs = list(ex.map(lambda s: _compile(s, verbose, ptxas_v), srcs))
+        host.result()
     if force or _stale(LIB, objs):
         cmd = [_nvcc(), "-shared", "-o", str(LIB)] + [str(o) for o in objs] + ARCH + ["-lrt", "-lpthread"]
         if verbose:

@@ -23,7 +23,7 @@
 // word and the kernel returns without touching the output.
 #include <stdlib.h>
 
-#include "cx_device.cuh"
+#include "cx_fold.cuh"
 
 namespace {
 
@@ -40,6 +40,8 @@ struct ApplyParams {
   uint32_t* status;
   uint64_t timeout_ns;
   const uint64_t* seq_cell;  // non-NULL inside a captured graph: the waits use its value
+  uint32_t chain_next;       // the kernel behind may start when this one is resident
+  uint32_t group;            // sparse ops: sub-tiles a warp takes at a time
 };
 
 __device__ __forceinline__ CxPair ld_pair(const CxPair* p) {
@@ -126,100 +128,80 @@ __device__ __forceinline__ void segment_prefix(int lane, uint32_t a, uint32_t b,
   total = __shfl_sync(0xffffffffu, incl, 31);
 }
 
+// The sparse ops: pairs go straight into the vector, source after source.  A warp takes up to 32
+// neighbouring sub-tiles at a time: lane l looks sub-tile l up, a scan lays the sub-tiles' pairs end
+// to end, and the lanes walk that sequence, kAhead x 32 pairs in flight.  So a warp is busy whatever
+// the density (10 pairs per sub-tile and source at top-k 1 %), and the chain of dependent loads
+// (table, pairs, elements) is paid once per group and source: 2^28 elements at 1 %, one source, took
+// 165 us with one sub-tile per warp at a time.
+constexpr int kAhead = 4;
+
 template <typename TO>
-__global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const ApplyParams p) {
+__global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_constant__ ApplyParams p) {
   __shared__ uint32_t s_nnz[CX_MAX_PEERS];
-  __shared__ float s_acc[kWarps][CX_SUBTILE];
+  if (p.chain_next) cx::pdl_trigger();
   if (!wait_sources(p, s_nnz)) { cx::pdl_wait(); return; }
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
   const uint32_t nwarps = gridDim.x * kWarps;
-  const float scale = p.a.op == CX_OP_SGD ? -p.a.scale : p.a.scale;
-  float* acc = s_acc[warp];
+  const bool sgd = p.a.op == CX_OP_SGD;
+  const float scale = sgd ? -p.a.scale : p.a.scale;
   uint32_t bad = 0;
-  for (uint32_t sub = blockIdx.x * kWarps + warp; sub < p.nsub; sub += nwarps) {
-    const uint32_t lo = sub * CX_SUBTILE;
-    uint32_t a = 0, b = 0;
-    if (lane < p.src.count) {
-      const uint2 entry = __ldcg(reinterpret_cast<const uint2*>(p.src.ep[lane].table) + sub);
-      a = entry.x;
-      b = min(entry.x + min(entry.y, (uint32_t)CX_SUBTILE), p.src.cap[lane]);  // never beyond the slot
-      a = min(a, b);
-    }
-    uint32_t pre, total;
-    segment_prefix(lane, a, b, pre, total);
-    if (total == 0) continue;
-    if (p.batch && total <= kBatchMax) {
-      // all pairs in one round trip, the addressed elements in a second one; the sums are formed
-      // in shared memory, source after source and rounded like the element-by-element path
-      Gathered g;
-      gather_pairs(p, lane, a, b, pre, g);
-      uint32_t d[kBatch];
-#pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
-        d[k] = (uint32_t)g.pr[k].idx - lo;
-        if (g.src[k] >= 0 && !(d[k] < CX_SUBTILE && (int64_t)g.pr[k].idx < p.n)) { bad = CX_ST_BAD_INDEX; g.src[k] = -1; }
-      }
-      if (p.a.op == CX_OP_SGD) {
-        const float* w = reinterpret_cast<const float*>(p.a.out);
-        float cur[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) cur[k] = g.src[k] >= 0 ? w[g.pr[k].idx] : 0.f;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) if (g.src[k] >= 0) acc[d[k]] = cur[k];
-      } else {
-        const TO* o = reinterpret_cast<const TO*>(p.a.out);
-        float cur[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) cur[k] = g.src[k] >= 0 ? cx::Elem<TO>::to_f(o[g.pr[k].idx]) : 0.f;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) if (g.src[k] >= 0) acc[d[k]] = cur[k];
-      }
-      __syncwarp();
-      for (int j = 0; j < p.src.count; ++j) {
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          if (g.src[k] == j) {
-            const float nv = acc[d[k]] + scale * __uint_as_float(g.pr[k].val);
-            acc[d[k]] = p.a.op == CX_OP_SGD ? nv : cx::Elem<TO>::to_f(cx::Elem<TO>::from_f(nv));
-          }
-        }
-        __syncwarp();
-      }
-#pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
-        if (g.src[k] < 0) continue;
-        const float nv = acc[d[k]];
-        if (p.a.op == CX_OP_SGD) {
-          reinterpret_cast<float*>(p.a.out)[g.pr[k].idx] = nv;
-          if (p.a.shadow) reinterpret_cast<TO*>(p.a.shadow)[g.pr[k].idx] = cx::Elem<TO>::from_f(nv);
-        } else {
-          reinterpret_cast<TO*>(p.a.out)[g.pr[k].idx] = cx::Elem<TO>::from_f(nv);
-        }
-      }
-      __syncwarp();
-      continue;
-    }
+  for (uint64_t s0 = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * p.group; s0 < p.nsub;
+       s0 += (uint64_t)nwarps * p.group) {
+    const uint32_t sub = (uint32_t)s0 + lane;
+    const bool have = lane < (int)p.group && sub < p.nsub;
+    uint2 next = have && p.src.count ? __ldcg(reinterpret_cast<const uint2*>(p.src.ep[0].table) + sub) : make_uint2(0, 0);
     for (int j = 0; j < p.src.count; ++j) {
-      const uint32_t aj = __shfl_sync(0xffffffffu, a, j);
-      const uint32_t bj = __shfl_sync(0xffffffffu, b, j);
+      const uint32_t cap = p.src.cap[j];
+      const uint32_t b = min(next.x + min(next.y, (uint32_t)CX_SUBTILE), cap);     // never beyond the slot
+      const uint32_t a = min(next.x, b);
+      if (have && j + 1 < p.src.count) next = __ldcg(reinterpret_cast<const uint2*>(p.src.ep[j + 1].table) + sub);
+      uint32_t pre, total;
+      segment_prefix(lane, a, b, pre, total);
       const CxPair* pairs = p.src.ep[j].pairs;
-      for (uint32_t i = aj + lane; i < bj; i += 32) {
-        const CxPair pr = ld_pair(pairs + i);
-        const uint32_t d = (uint32_t)pr.idx - lo;
-        if (d < CX_SUBTILE && (int64_t)pr.idx < p.n) {
-          const float val = scale * __uint_as_float(pr.val);
-          if (p.a.op == CX_OP_SGD) {
-            float* w = reinterpret_cast<float*>(p.a.out);
-            const float nw = w[pr.idx] + val;
-            w[pr.idx] = nw;
-            if (p.a.shadow) reinterpret_cast<TO*>(p.a.shadow)[pr.idx] = cx::Elem<TO>::from_f(nw);
-          } else {
-            TO* o = reinterpret_cast<TO*>(p.a.out);
-            o[pr.idx] = cx::Elem<TO>::from_f(cx::Elem<TO>::to_f(o[pr.idx]) + val);
+      for (uint32_t f0 = 0; f0 < total; f0 += 32 * kAhead) {
+        CxPair pr[kAhead];
+        uint32_t lo[kAhead];
+        bool in[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          const uint32_t f = f0 + 32 * k + lane;
+          in[k] = f < total;
+          uint32_t o = 0;          // the last sub-tile whose pairs start at or before f
+#pragma unroll
+          for (uint32_t d = 16; d > 0; d >>= 1) {
+            const uint32_t t = __shfl_sync(0xffffffffu, pre, o + d);
+            if (t <= f) o += d;
+          }
+          const uint32_t off = __shfl_sync(0xffffffffu, a, o) + (f - __shfl_sync(0xffffffffu, pre, o));
+          lo[k] = ((uint32_t)s0 + o) * CX_SUBTILE;
+          pr[k].idx = 0;
+          pr[k].val = 0;
+          if (in[k]) pr[k] = ld_pair(pairs + off);
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          if (in[k] && !((uint32_t)pr[k].idx - lo[k] < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { in[k] = false; bad = CX_ST_BAD_INDEX; }
+        }
+        // indices are unique inside one payload: the loads may all go first
+        float cur[kAhead];
+        if (sgd) {
+          float* w = reinterpret_cast<float*>(p.a.out);
+#pragma unroll
+          for (int k = 0; k < kAhead; ++k) cur[k] = in[k] ? w[pr[k].idx] : 0.f;
+#pragma unroll
+          for (int k = 0; k < kAhead; ++k) {
+            const float nw = cur[k] + scale * __uint_as_float(pr[k].val);
+            if (in[k]) w[pr[k].idx] = nw;
+            if (in[k] && p.a.shadow) reinterpret_cast<TO*>(p.a.shadow)[pr[k].idx] = cx::Elem<TO>::from_f(nw);
           }
         } else {
-          bad = CX_ST_BAD_INDEX;
+          TO* out = reinterpret_cast<TO*>(p.a.out);
+#pragma unroll
+          for (int k = 0; k < kAhead; ++k) cur[k] = in[k] ? cx::Elem<TO>::to_f(out[pr[k].idx]) : 0.f;
+#pragma unroll
+          for (int k = 0; k < kAhead; ++k)
+            if (in[k]) out[pr[k].idx] = cx::Elem<TO>::from_f(cur[k] + scale * __uint_as_float(pr[k].val));
         }
       }
       __syncwarp();  // the next source may address the same elements from other lanes
@@ -309,6 +291,24 @@ __device__ __forceinline__ void update4(const CxApplyArgs& a, const int64_t n, i
       if (a.shadow) reinterpret_cast<TO*>(a.shadow)[i + e] = cx::Elem<TO>::from_f(wv[e]);
     }
   }
+}
+
+// the update rule on one element whose state has been loaded
+template <int OP>
+__device__ __forceinline__ void load_state1(const CxApplyArgs& a, int64_t i, bool in, float& w, float& m, float& v) {
+  w = in ? reinterpret_cast<const float*>(a.out)[i] : 0.f;
+  m = OP != CX_OP_SGD && in ? a.m[i] : 0.f;
+  v = OP == CX_OP_ADAMW && in ? a.v[i] : 0.f;
+}
+template <int OP, typename TO>
+__device__ __forceinline__ void update1(const CxApplyArgs& a, int64_t i, float acc, float w, float m, float v) {
+  const float av[4] = {acc, 0.f, 0.f, 0.f};
+  float wv[4] = {w, 0.f, 0.f, 0.f}, mv[4] = {m, 0.f, 0.f, 0.f}, vv[4] = {v, 0.f, 0.f, 0.f};
+  rule4<OP>(a, av, wv, mv, vv);
+  reinterpret_cast<float*>(a.out)[i] = wv[0];
+  if (OP != CX_OP_SGD) a.m[i] = mv[0];
+  if (OP == CX_OP_ADAMW) a.v[i] = vv[0];
+  if (a.shadow) reinterpret_cast<TO*>(a.shadow)[i] = cx::Elem<TO>::from_f(wv[0]);
 }
 
 // Table look-up, zeroing of the accumulator and accumulation of all sources' pairs of one
@@ -540,9 +540,10 @@ __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(co
 }
 
 template <int OP, typename TO>
-__global__ void __launch_bounds__(kThreads) apply_dense_kernel(const ApplyParams p) {
+__global__ void __launch_bounds__(kThreads) apply_dense_kernel(const __grid_constant__ ApplyParams p) {
   __shared__ uint32_t s_nnz[CX_MAX_PEERS];
   __shared__ __align__(16) float s_acc[kWarps][CX_SUBTILE];
+  if (p.chain_next) cx::pdl_trigger();
   if (!wait_sources(p, s_nnz)) { cx::pdl_wait(); return; }
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -599,6 +600,76 @@ int launch_update(const UpdateParams& q, int grid, cudaStream_t s) {
     case CX_OP_MOMENTUM: update_dense_kernel<CX_OP_MOMENTUM, TO><<<grid, kThreads, 0, s>>>(q); return 0;
     case CX_OP_ADAMW: update_dense_kernel<CX_OP_ADAMW, TO><<<grid, kThreads, 0, s>>>(q); return 0;
     default: return cx_set_error("cx_update_dense: op must be an update rule", 0);
+  }
+}
+
+// The whole step of a rank that exchanges nothing: the folded gradient (CxFold) goes from registers
+// into the momentum and the update rule, one pass over gradient, momentum and weights.  A warp takes
+// a sub-tile; the ones at tensor borders go element by element.  25.6 M bf16 parameters with momentum:
+// 85 us for the fold and 62 us for the update as two kernels.
+struct FoldUpdateParams {
+  CxFold f;
+  CxApplyArgs a;
+  int64_t n;
+  uint32_t nsub;
+};
+
+// KEEP: 0 nothing of the folded vector is kept, 1 it is stored as the momentum, 2 read and stored
+template <int OP, typename TO, typename T, int KEEP>
+__global__ void __launch_bounds__(kThreads, OP == CX_OP_ADAMW ? 4 : 5) fold_update_kernel(const __grid_constant__ FoldUpdateParams q) {
+  cx::pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const uint32_t nwarps = gridDim.x * kWarps;
+  const uint32_t nfull = (uint32_t)(q.n / CX_SUBTILE);
+  for (uint32_t sub = blockIdx.x * kWarps + (threadIdx.x >> 5); sub < q.nsub; sub += nwarps) {
+    const int64_t lo = (int64_t)sub * CX_SUBTILE;
+    const T* g = nullptr;
+    float coef = 0.f;
+    if (sub < nfull && cx::fold_whole<T>(q.f, sub, g, coef)) {
+#pragma unroll 2
+      for (int c = 0; c < CX_SUBTILE / 128; ++c) {
+        const int e0 = c * 128 + lane * 4;
+        float x[4], y[4] = {0.f, 0.f, 0.f, 0.f};
+        cx::load4(g + e0, x);
+        if (KEEP == 2) cx::load4(q.f.u + lo + e0, y);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = q.f.mu * y[e] + coef * x[e];
+        if (KEEP) cx::store4(q.f.u + lo + e0, y);
+        update4<OP, TO>(q.a, q.n, lo + e0, y, true);
+      }
+    } else {
+      const cx::FoldBlock<T> blk = cx::fold_blocks<T>(q.f, sub, lane);
+      constexpr int kGroup = 4;      // loads in flight: none of them moves across a store
+      for (int j0 = 0; j0 < CX_SUBTILE / 32; j0 += kGroup) {
+        float x[kGroup], y[kGroup], c[kGroup], w[kGroup], m[kGroup], v[kGroup];
+        bool in[kGroup];
+#pragma unroll
+        for (int j = 0; j < kGroup; ++j) {
+          const int64_t i = lo + 32 * (j0 + j) + lane;
+          in[j] = cx::fold_element<T>(blk, j0 + j, lane, x[j], c[j]);
+          y[j] = KEEP == 2 && in[j] ? q.f.u[i] : 0.f;
+          load_state1<OP>(q.a, i, i < q.n, w[j], m[j], v[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kGroup; ++j) {
+          const int64_t i = lo + 32 * (j0 + j) + lane;
+          const float t = in[j] ? q.f.mu * y[j] + c[j] * x[j] : 0.f;
+          if (KEEP && in[j]) q.f.u[i] = t;
+          if (i < q.n) update1<OP, TO>(q.a, i, t, w[j], m[j], v[j]);
+        }
+      }
+    }
+  }
+}
+
+template <typename TO, typename T, int KEEP>
+int launch_fold_update(const FoldUpdateParams& q, int grid, cudaStream_t s) {
+  const bool cap = cx_seq_cell() != nullptr;
+  switch (q.a.op) {
+    case CX_OP_SGD: cx_launch_pdl(fold_update_kernel<CX_OP_SGD, TO, T, KEEP>, grid, kThreads, 0, s, q, cap); return 0;
+    case CX_OP_MOMENTUM: cx_launch_pdl(fold_update_kernel<CX_OP_MOMENTUM, TO, T, KEEP>, grid, kThreads, 0, s, q, cap); return 0;
+    case CX_OP_ADAMW: cx_launch_pdl(fold_update_kernel<CX_OP_ADAMW, TO, T, KEEP>, grid, kThreads, 0, s, q, cap); return 0;
+    default: return cx_set_error("cx_fold_update: op must be an update rule", 0);
   }
 }
 
@@ -762,9 +833,18 @@ int cx_apply_cuda(const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_
   if (a->op == CX_OP_ADAMW && !a->v) return cx_set_error("cx_apply: second-moment buffer missing", 0);
   p.vec = aligned16(a->out) && (!a->shadow || aligned16(a->shadow)) && (!a->m || aligned16(a->m)) &&
           (!a->v || aligned16(a->v));
+  p.chain_next = !p.seq_cell && (cx_chain_bits() & CX_CHAIN_NEXT) ? 1u : 0u;
   const int dt = update ? (a->shadow ? a->shadow_dtype : CX_F32) : a->out_dtype;
   int grid = cx_sm_count() * 6;
-  const int need = (int)((p.nsub + kWarps - 1) / kWarps);
+  p.group = 1;
+  const bool sparse = a->op == CX_OP_ADD || (a->op == CX_OP_SGD && a->wd == 0.f);
+  if (sparse) {
+    // as few sub-tiles per warp as fill one wave of warps, then as few waves as 32 per warp allow
+    const uint64_t warps = (uint64_t)grid * kWarps;
+    const uint64_t waves = (p.nsub + warps * 32 - 1) / (warps * 32);
+    p.group = (uint32_t)((p.nsub + warps * waves - 1) / (warps * waves));
+  }
+  const int need = (int)((p.nsub + (uint64_t)kWarps * p.group - 1) / ((uint64_t)kWarps * p.group));
   if (grid > need) grid = need;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int rc;
@@ -805,6 +885,42 @@ int cx_update_dense_cuda(const float* g, int64_t n, const CxApplyArgs* a, void* 
   if (rc) return rc;
   cx_note_launch();
   return cx_check_launch("update_dense_kernel");
+}
+
+// The low-precision copy of the weights has the element type of the gradients (both are the model's).
+int cx_fold_update_cuda(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream) {
+  if (!a->out) return cx_set_error("cx_fold_update: NULL vector", 0);
+  if (n < 0 || n > 0x7fffffffLL) return cx_set_error("cx_fold_update: n out of range", 0);
+  if (a->op != CX_OP_SGD && a->op != CX_OP_MOMENTUM && a->op != CX_OP_ADAMW)
+    return cx_set_error("cx_fold_update: op must be an update rule", 0);
+  if (a->op != CX_OP_SGD && !a->m) return cx_set_error("cx_fold_update: momentum buffer missing", 0);
+  if (a->op == CX_OP_ADAMW && !a->v) return cx_set_error("cx_fold_update: second-moment buffer missing", 0);
+  if (!fold->u && fold->mu != 0.f) return cx_set_error("cx_fold_update: folding with momentum needs the momentum", 0);
+  if (a->shadow && a->shadow_dtype != gdtype) return cx_set_error("cx_fold_update: gradients and weights differ in type", 0);
+  if (!(aligned16(a->out) && aligned16(fold->u) && aligned16(a->shadow) && aligned16(a->m) && aligned16(a->v)))
+    return cx_set_error("cx_fold_update: state must be 16-byte aligned", 0);
+  if (n == 0) return 0;
+  FoldUpdateParams q;
+  q.f = *fold; q.a = *a; q.n = n;
+  q.nsub = (uint32_t)((n + CX_SUBTILE - 1) / CX_SUBTILE);
+  int grid = cx_sm_count() * 8;
+  const int need = (int)((q.nsub + kWarps - 1) / kWarps);
+  if (grid > need) grid = need;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const int keep = !fold->u ? 0 : fold->mu == 0.f ? 1 : 2;
+  int rc;
+#define CX_FOLD_UPDATE(T) (keep == 0 ? launch_fold_update<T, T, 0>(q, grid, s) \
+                           : keep == 1 ? launch_fold_update<T, T, 1>(q, grid, s) : launch_fold_update<T, T, 2>(q, grid, s))
+  switch (gdtype) {
+    case CX_F32: rc = CX_FOLD_UPDATE(float); break;
+    case CX_BF16: rc = CX_FOLD_UPDATE(__nv_bfloat16); break;
+    case CX_F16: rc = CX_FOLD_UPDATE(__half); break;
+    default: return cx_set_error("cx_fold_update: unsupported dtype on CUDA", 0);
+  }
+#undef CX_FOLD_UPDATE
+  if (rc) return rc;
+  cx_note_launch();
+  return cx_check_launch("fold_update_kernel");
 }
 
 int cx_forward_cuda(const CxEndpoint* from, uint64_t expect_seq, const CxTargets* tg, uint64_t seq,

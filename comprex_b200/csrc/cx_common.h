@@ -138,6 +138,24 @@ typedef struct CxApplyArgs {
   float pad2;
 } CxApplyArgs;
 
+/* A vector that is not stored: element i of the range [base, base + n) of a flat buffer is
+ *     mu * u[i] + coef[s] * g_s[base + i - seg_off[s]]
+ * with s the gradient tensor that lies there (0 in the gaps between tensors).  All arrays are
+ * device memory.  The kernels that take a CxFold compute the sum where they need it, so that the
+ * clipped, momentum-folded gradient makes no trip through memory of its own. */
+#define CX_FOLD_ALIGN 64
+typedef struct CxFold {
+  const void* const* seg_ptr;  /* [nseg] base pointers of the gradient tensors                        */
+  const int64_t* seg_off;      /* [nseg] where the tensors start in the flat buffer: ascending multiples of CX_FOLD_ALIGN */
+  const int64_t* seg_end;      /* [nseg] and where they end                                            */
+  const float* coef;           /* [nseg] learning rate times clip factor (cx_fold_coef)                */
+  const int32_t* sub_seg;      /* per 1024 elements of the range: first tensor that ends behind their start */
+  float* u;                    /* momentum of the range, updated by the compress / update kernel; NULL: none kept */
+  int64_t base;                /* a multiple of CX_FOLD_ALIGN */
+  int32_t nseg;
+  float mu;
+} CxFold;
+
 /* ---- exported C ABI ------------------------------------------------- */
 
 const char* cx_last_error(void);
@@ -236,6 +254,16 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
             const int32_t* seg_first, int nitems, float* u, float* partial, float clip,
             float mu, float lr, void* stream);
 
+/* The first half of the fold on its own (CUDA): coef[s] = lr * clip / max(||g_s||, clip), or lr
+ * without clipping, for the tensors [seg_lo, seg_hi) whose items are [item_lo, item_hi).  Same sums,
+ * in the same order, as cx_fold; partial: scratch of 8 floats per item. */
+int cx_fold_coef(int gdtype, const void* const* seg_ptr, const int64_t* item_rel, const int32_t* item_len,
+                 const int32_t* item_seg, const int32_t* seg_first, int item_lo, int item_hi, int seg_lo, int seg_hi,
+                 float* partial, float* coef, float clip, float lr, void* stream);
+/* cx_fold and cx_update_dense in one pass over the range (CUDA): u is updated when fold->u is set,
+ * and the parameters take the folded vector as their averaged gradient. */
+int cx_fold_update(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream);
+
 /* small elementwise helpers of the engines and the optimizer */
 int cx_axpy(int dev, int ydtype, void* y, int xdtype, const void* x, float a,
             int64_t n, void* stream); /* y += a*x */
@@ -323,6 +351,11 @@ typedef struct CxOp {
   int32_t lane;                /* 0: the caller's stream; k > 0: side stream k (see cx_run_ops) */
   int64_t starts[CX_MAX_PEERS];
   int64_t lens[CX_MAX_PEERS];
+  const CxFold* fold;          /* threshold, compress: the input is this folded vector instead of g (CUDA, r and u
+                                  16-byte aligned); host memory, read when the op is issued */
+  int32_t chain;               /* 1: the op in front is of the same kind and touches nothing this one touches (other
+                                  vectors, slots, scratch): the two may run at the same time (CUDA) */
+  int32_t pad;
   CxTargets tg;                /* compress / dense send targets, dense reduce push targets */
   CxSources src;               /* apply / dense reduce sources; their seq is set per call */
   CxApplyArgs apply;
@@ -343,7 +376,7 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream);
 int cx_graph_build(CxOp* ops, int count, void** graph_out);
 int cx_graph_launch(void* graph, uint64_t seq, void* stream);
 int cx_graph_free(void* graph);
-int64_t cx_sizeof(int what); /* 0 CxOp, 1 CxSources, 2 CxTargets, 3 CxApplyArgs, 4 CxWorkCounters, 5 CxHeader */
+int64_t cx_sizeof(int what); /* 0 CxOp, 1 CxSources, 2 CxTargets, 3 CxApplyArgs, 4 CxWorkCounters, 5 CxHeader, 6 CxFold */
 
 /* bounded wait on a header from the host (status in the return value) */
 int cx_host_wait_seq(const CxHeader* hdr, uint64_t seq, uint64_t timeout_ns);

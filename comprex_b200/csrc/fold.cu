@@ -6,11 +6,13 @@
 // The tensors of a bucket are described once by a static item list (flat offset,
 // length, tensor index, offset inside the tensor; tensors larger than 65536
 // elements are cut into several items for load balance).  Per step only the table
-// of gradient pointers changes.  Two launches:
-//   1. fold_sumsq:  partial[item] = sum of squares of the item (fixed order: the
+// of gradient pointers changes.
+//   1. fold_sumsq:  partial[item][0..8) = sums of squares of the item (fixed order: the
 //      result does not depend on scheduling),
-//   2. fold_apply:  coef = clip / max(||g_tensor||, clip) from the tensor's partials,
-//                   u[off + i] = mu * u[off + i] + lr * coef * g[i].
+//   2. fold_coef:   coef = lr * clip / max(||g_tensor||, clip) from the tensor's partials,
+//   3. the kernel that consumes the vector u = mu * u + coef * g computes it where it needs it:
+//      the compress kernel (compress.cu), the dense update (apply.cu), or, for the exchanges that
+//      want it in memory, fold_apply below.
 // With mu = 0, lr = 1 this is the clipped gradient itself in fp32 (AdamW rule).
 #include "cx_device.cuh"
 
@@ -26,63 +28,122 @@ struct FoldParams {
   const int32_t* item_seg;      // [nitems]
   const int32_t* seg_first;     // [nseg + 1] first item of every tensor
   float* u;
-  float* partial;               // [nitems]
+  float* partial;               // [nitems], or [nitems * 8]: per-warp sums of squares
+  float* coef;                  // [nseg]
+  int32_t item_lo, seg_lo, seg_hi;
   float clip;                   // <= 0: no clipping
   float mu;
   float lr;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) fold_sumsq_kernel(const FoldParams p) {
-  __shared__ float s_w[kThreads / 32];
-  const int item = blockIdx.x;
+// Bound by the read of the gradients.  The sum of an item is defined by kSum = 256 strands (strand t:
+// the groups of four elements t, t + 256, ..., in that order), added up warp by warp in a fixed order,
+// so the result does not depend on how strands meet CTAs: a CTA takes 64 of them, which spreads even
+// a small model over the chip (256 strands per CTA, one load at a time: 15 us for 25.6 M bf16
+// gradients).  The per-warp sums are then left to the kernel that wants the norm (8 floats per item);
+// cx_fold, whose scratch holds one float per item, keeps an item in one CTA.
+constexpr int kSum = 256;
+constexpr int kSpread = 64;
+constexpr int kSumWarps = kSum / 32;
+constexpr int kAhead = 8;
+
+template <typename T, int kStrands>
+__global__ void __launch_bounds__(kStrands) fold_sumsq_kernel(const __grid_constant__ FoldParams p) {
+  __shared__ float s_w[kSumWarps];
+  cx::pdl_wait();
+  cx::pdl_trigger();
+  const int item = p.item_lo + blockIdx.x / (kSum / kStrands);
+  const int strand = blockIdx.x % (kSum / kStrands) * kStrands + threadIdx.x;
   const int len = p.item_len[item];
   const T* g = reinterpret_cast<const T*>(p.seg_ptr[p.item_seg[item]]) + p.item_rel[item];
   float acc = 0.f;
   if ((reinterpret_cast<uintptr_t>(g) & (4 * sizeof(T) - 1)) == 0) {
     const int nv = len / 4;
-    for (int q = threadIdx.x; q < nv; q += kThreads) {
+    int q = strand;
+    for (; q + (kAhead - 1) * kSum < nv; q += kAhead * kSum) {
+      typename cx::Raw4<T>::type x[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) x[k] = cx::Raw4<T>::load(g + 4 * (q + k * kSum));
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        float v[4];
+        cx::Raw4<T>::to_f(x[k], v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc += v[e] * v[e];
+      }
+    }
+    for (; q < nv; q += kSum) {
       float x[4];
       cx::load4(g + 4 * q, x);
-      acc += x[0] * x[0];
-      acc += x[1] * x[1];
-      acc += x[2] * x[2];
-      acc += x[3] * x[3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc += x[e] * x[e];
     }
-    for (int i = nv * 4 + threadIdx.x; i < len; i += kThreads) {
+    for (int i = nv * 4 + strand; i < len; i += kSum) {
       const float x = cx::Elem<T>::to_f(g[i]);
       acc += x * x;
     }
   } else {
-    for (int i = threadIdx.x; i < len; i += kThreads) {
+    for (int i = strand; i < len; i += kSum) {
       const float x = cx::Elem<T>::to_f(g[i]);
       acc += x * x;
     }
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = acc;
+  if (kStrands < kSum) {
+    if ((threadIdx.x & 31) == 0) p.partial[(size_t)item * kSumWarps + (strand >> 5)] = acc;
+    return;
+  }
+  if ((threadIdx.x & 31) == 0) s_w[strand >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.f;
-    for (int w = 0; w < kThreads / 32; ++w) t += s_w[w];
+    for (int w = 0; w < kSumWarps; ++w) t += s_w[w];
     p.partial[item] = t;
   }
 }
 
+// One warp: lr times the clip factor of tensor `seg`.  The partial sums are added one after the
+// other, as a single thread would, but fetched 32 at a time.
+template <int W>      // floats per item
+__device__ __forceinline__ float tensor_coef(const FoldParams& p, int seg, int lane) {
+  float coef = 1.f;
+  if (p.clip > 0.f) {
+    float ss = 0.f;
+    const int lo = p.seg_first[seg], hi = p.seg_first[seg + 1];
+    for (int i = lo; i < hi; i += 32) {
+      float x = 0.f;
+      if (i + lane < hi) {
+        const float* w = p.partial + (size_t)(i + lane) * W;
+#pragma unroll
+        for (int j = 0; j < W; ++j) x += w[j];
+      }
+      const int k = min(32, hi - i);
+      for (int j = 0; j < k; ++j) ss += __shfl_sync(0xffffffffu, x, j);
+    }
+    coef = p.clip / fmaxf(sqrtf(ss), p.clip);
+  }
+  return p.lr * coef;
+}
+
+__global__ void __launch_bounds__(kThreads) fold_coef_kernel(const __grid_constant__ FoldParams p) {
+  cx::pdl_wait();
+  cx::pdl_trigger();
+  const int seg = p.seg_lo + blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (seg >= p.seg_hi) return;
+  const float c = tensor_coef<kSumWarps>(p, seg, threadIdx.x & 31);
+  if ((threadIdx.x & 31) == 0) p.coef[seg] = c;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads) fold_apply_kernel(const FoldParams p) {
+__global__ void __launch_bounds__(kThreads) fold_apply_kernel(const __grid_constant__ FoldParams p) {
   __shared__ float s_coef;
+  cx::pdl_wait();
   const int item = blockIdx.x;
   const int seg = p.item_seg[item];
-  if (threadIdx.x == 0) {
-    float coef = 1.f;
-    if (p.clip > 0.f) {
-      float ss = 0.f;
-      for (int i = p.seg_first[seg]; i < p.seg_first[seg + 1]; ++i) ss += p.partial[i];
-      coef = p.clip / fmaxf(sqrtf(ss), p.clip);
-    }
-    s_coef = p.lr * coef;
+  if (threadIdx.x < 32) {
+    const float c = tensor_coef<1>(p, seg, threadIdx.x);
+    if (threadIdx.x == 0) s_coef = c;
   }
   __syncthreads();
   const float a = s_coef;
@@ -92,6 +153,7 @@ __global__ void __launch_bounds__(kThreads) fold_apply_kernel(const FoldParams p
   const bool vec = (reinterpret_cast<uintptr_t>(g) & (4 * sizeof(T) - 1)) == 0 &&
                    (reinterpret_cast<uintptr_t>(u) & 15) == 0;
   const int nv = vec ? len / 4 : 0;
+#pragma unroll 4
   for (int q = threadIdx.x; q < nv; q += kThreads) {
     float x[4], y[4] = {0.f, 0.f, 0.f, 0.f};
     cx::load4(g + 4 * q, x);
@@ -106,33 +168,59 @@ __global__ void __launch_bounds__(kThreads) fold_apply_kernel(const FoldParams p
   }
 }
 
+template <typename T, int kStrands>
+void launch_sumsq(const FoldParams& p, int items, cudaStream_t s) {
+  cx_launch_pdl(fold_sumsq_kernel<T, kStrands>, items * (kSum / kStrands), kStrands, 0, s, p, cx_seq_cell() != nullptr);
+  cx_note_launch();
+}
+
+template <int kStrands>
+int sumsq(int gdtype, const FoldParams& p, int items, cudaStream_t s) {
+  switch (gdtype) {
+    case CX_F32: launch_sumsq<float, kStrands>(p, items, s); return 0;
+    case CX_BF16: launch_sumsq<__nv_bfloat16, kStrands>(p, items, s); return 0;
+    case CX_F16: launch_sumsq<__half, kStrands>(p, items, s); return 0;
+    default: return cx_set_error("cx_fold: unsupported dtype on CUDA", 0);
+  }
+}
+
 }  // namespace
+
+int cx_fold_coef_cuda(int gdtype, const void* const* seg_ptr, const int64_t* item_rel, const int32_t* item_len,
+                      const int32_t* item_seg, const int32_t* seg_first, int item_lo, int item_hi, int seg_lo,
+                      int seg_hi, float* partial, float* coef, float clip, float lr, void* stream) {
+  if (seg_hi <= seg_lo) return 0;
+  FoldParams p = {};
+  p.seg_ptr = seg_ptr; p.item_rel = item_rel; p.item_len = item_len; p.item_seg = item_seg; p.seg_first = seg_first;
+  p.partial = partial; p.coef = coef; p.item_lo = item_lo; p.seg_lo = seg_lo; p.seg_hi = seg_hi;
+  p.clip = clip; p.lr = lr;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (clip > 0.f && item_hi > item_lo)
+    if (const int rc = sumsq<kSpread>(gdtype, p, item_hi - item_lo, s)) return rc;
+  const int warps = kThreads / 32;
+  cx_launch_pdl(fold_coef_kernel, (seg_hi - seg_lo + warps - 1) / warps, kThreads, 0, s, p, cx_seq_cell() != nullptr);
+  cx_note_launch();
+  return cx_check_launch("fold kernels");
+}
 
 int cx_fold_cuda(int gdtype, const void* const* seg_ptr, const int64_t* item_off,
                  const int64_t* item_rel, const int32_t* item_len, const int32_t* item_seg,
                  const int32_t* seg_first, int nitems, float* u, float* partial, float clip,
                  float mu, float lr, void* stream) {
   if (nitems <= 0) return 0;
-  FoldParams p;
+  FoldParams p = {};
   p.seg_ptr = seg_ptr; p.item_off = item_off; p.item_rel = item_rel; p.item_len = item_len;
   p.item_seg = item_seg; p.seg_first = seg_first; p.u = u; p.partial = partial;
   p.clip = clip; p.mu = mu; p.lr = lr;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (clip > 0.f)
+    if (const int rc = sumsq<kSum>(gdtype, p, nitems, s)) return rc;
+  const bool capturing = cx_seq_cell() != nullptr;
   switch (gdtype) {
-    case CX_F32:
-      if (clip > 0.f) { fold_sumsq_kernel<float><<<nitems, kThreads, 0, s>>>(p); cx_note_launch(); }
-      fold_apply_kernel<float><<<nitems, kThreads, 0, s>>>(p);
-      break;
-    case CX_BF16:
-      if (clip > 0.f) { fold_sumsq_kernel<__nv_bfloat16><<<nitems, kThreads, 0, s>>>(p); cx_note_launch(); }
-      fold_apply_kernel<__nv_bfloat16><<<nitems, kThreads, 0, s>>>(p);
-      break;
-    case CX_F16:
-      if (clip > 0.f) { fold_sumsq_kernel<__half><<<nitems, kThreads, 0, s>>>(p); cx_note_launch(); }
-      fold_apply_kernel<__half><<<nitems, kThreads, 0, s>>>(p);
-      break;
-    default:
-      return cx_set_error("cx_fold: unsupported dtype on CUDA", 0);
+    case CX_F32: cx_launch_pdl(fold_apply_kernel<float>, nitems, kThreads, 0, s, p, capturing); break;
+    case CX_BF16: cx_launch_pdl(fold_apply_kernel<__nv_bfloat16>, nitems, kThreads, 0, s, p, capturing); break;
+    case CX_F16: cx_launch_pdl(fold_apply_kernel<__half>, nitems, kThreads, 0, s, p, capturing); break;
+    default: return cx_set_error("cx_fold: unsupported dtype on CUDA", 0);
   }
   cx_note_launch();
   return cx_check_launch("fold kernels");

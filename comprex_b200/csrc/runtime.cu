@@ -19,11 +19,20 @@
 
 #include "cx_common.h"
 
+#define CX_CHAINED 1u      /* as in cx_device.cuh */
+#define CX_CHAIN_NEXT 2u
+
 // ---- forward declarations of the two back ends --------------------------------
 int cx_threshold_topk_cuda(int, const void*, const float*, int64_t, float, int, float, float*, void*, int64_t, void*);
+int cx_threshold_batch_cuda(const CxOp*, int, void*);
 int cx_threshold_topk_host(int, const void*, const float*, int64_t, float, int, float, float*);
 int cx_compress_cuda(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
                      const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
+int cx_compress_fold_cuda(int, const CxFold*, float*, int64_t, const float*, uint32_t, uint64_t,
+                          const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
+int cx_fold_coef_cuda(int, const void* const*, const int64_t*, const int32_t*, const int32_t*, const int32_t*, int, int,
+                      int, int, float*, float*, float, float, void*);
+int cx_fold_update_cuda(int, const CxFold*, int64_t, const CxApplyArgs*, void*);
 int cx_compress_host(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
                      const CxTargets*, CxStats*, uint32_t);
 int cx_apply_cuda(const CxSources*, int64_t, const CxApplyArgs*, uint32_t*, uint64_t, void*);
@@ -75,6 +84,8 @@ int cx_set_error(const char* where, int cuda_err) {
 void cx_note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static thread_local const uint64_t* g_seq_cell = nullptr;
 const uint64_t* cx_seq_cell() { return g_seq_cell; }
+static thread_local uint32_t g_chain_bits = 0;
+uint32_t cx_chain_bits() { return g_chain_bits; }
 int cx_check_launch(const char* where) {
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cx_set_error(where, (int)e);
@@ -191,6 +202,17 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
                             partial, clip, mu, lr);
 }
 
+int cx_fold_coef(int gdtype, const void* const* seg_ptr, const int64_t* item_rel, const int32_t* item_len,
+                 const int32_t* item_seg, const int32_t* seg_first, int item_lo, int item_hi, int seg_lo, int seg_hi,
+                 float* partial, float* coef, float clip, float lr, void* stream) {
+  return cx_fold_coef_cuda(gdtype, seg_ptr, item_rel, item_len, item_seg, seg_first, item_lo, item_hi, seg_lo, seg_hi,
+                           partial, coef, clip, lr, stream);
+}
+
+int cx_fold_update(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream) {
+  return cx_fold_update_cuda(gdtype, fold, n, a, stream);
+}
+
 int cx_rle_send(int dev, int gdtype, const void* g, float* r, int64_t n, const float* thr,
                 int64_t slot_bytes, uint64_t seq, const CxTargets* tg, void* workspace,
                 int64_t ws_bytes, uint32_t src_rank, void* stream) {
@@ -217,6 +239,7 @@ int64_t cx_sizeof(int what) {
     case 3: return (int64_t)sizeof(CxApplyArgs);
     case 4: return (int64_t)sizeof(CxWorkCounters);
     case 5: return (int64_t)sizeof(CxHeader);
+    case 6: return (int64_t)sizeof(CxFold);
     default: return -1;
   }
 }
@@ -227,9 +250,15 @@ namespace {
 int run_one(CxOp& o, uint64_t seq, void* stream) {
   switch (o.kind) {
     case CX_OPK_THRESHOLD:
+      if (o.fold) return cx_set_error("cx_run_ops: folded vectors are CUDA only", 0);
       return cx_threshold_select(o.dev, o.dtype, o.g, o.r, o.n, o.ratio, o.default_subsamples,
                                  o.subsample_factor, o.thr, o.workspace, o.ws_bytes, stream);
     case CX_OPK_COMPRESS:
+      if (o.fold) {
+        if (o.dev != CX_DEV_CUDA) return cx_set_error("cx_run_ops: folded vectors are CUDA only", 0);
+        return cx_compress_fold_cuda(o.dtype, o.fold, o.r, o.n, o.thr, o.cap, seq, &o.tg, o.workspace, o.ws_bytes,
+                                     o.stats, o.src_rank, stream);
+      }
       return cx_compress(o.dev, o.dtype, o.g, o.r, o.n, o.thr, o.cap, seq, &o.tg, o.workspace,
                          o.ws_bytes, o.stats, o.src_rank, stream);
     case CX_OPK_APPLY:
@@ -304,7 +333,18 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
     forked = false;
     return 0;
   };
-  for (int i = 0; i < count; ++i) {
+  // thresholds that follow one another on one lane share launches
+  auto run_some = [&](int i, void* on) -> int {      // ops taken, or a negative error
+    if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA) return cx_threshold_batch_cuda(ops + i, count - i, on);
+    auto chained = [&](int k) {
+      return k > 0 && k < count && ops[k].chain && ops[k].kind == ops[k - 1].kind && ops[k].lane == ops[k - 1].lane;
+    };
+    g_chain_bits = (chained(i) ? CX_CHAINED : 0u) | (chained(i + 1) ? CX_CHAIN_NEXT : 0u);
+    const int rc = run_one(ops[i], seq, on);
+    g_chain_bits = 0;
+    return rc ? (rc > 0 ? -rc : rc) : 1;
+  };
+  for (int i = 0, took = 0; i < count; i += took) {
     CxOp& o = ops[i];
     int rc;
     if (o.lane > 0 && o.dev == CX_DEV_CUDA) {
@@ -326,12 +366,12 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
           return cx_set_error("cx_run_ops: forking a side stream", (int)cudaGetLastError());
         open_mask |= 1u << o.lane;
       }
-      rc = run_one(o, seq, lanes->stream[o.lane]);
+      took = run_some(i, lanes->stream[o.lane]);
     } else {
       if (open_mask && (rc = join())) return rc;
-      rc = run_one(o, seq, stream);
+      took = run_some(i, stream);
     }
-    if (rc) { if (open_mask) join(); return rc; }
+    if (took < 0) { if (open_mask) join(); return took; }
   }
   if (open_mask) return join();
   return 0;

@@ -17,16 +17,23 @@
 // kernel therefore runs as a thread-block cluster of 8 CTAs: every CTA gathers one
 // eighth of the sample and stores the keys through distributed shared memory into
 // the first CTA, which then selects alone.
+//
+// The selection is a chain of dependent block-wide steps, so it takes as few as the rank
+// allows (see select_cached).  Sampling rules ask for rank 9 unless the fraction is above 1 %.
+//
+// Several vectors (the buckets of an optimizer step) share one launch, one cluster each: the
+// kernel is all latency, and one after the other they would leave the GPU idle in between.
 #include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
 
-#include "cx_device.cuh"
+#include "cx_fold.cuh"
 
 namespace {
 
 constexpr int kThreads = 1024;
-constexpr int kSmemKeys = 11264;  // 44 KB of cached sample keys
+constexpr int kSmemKeys = 11008;  // 43 KB of cached sample keys
+constexpr int kVectors = 24;      // vectors per launch: their parameters stay within 4 KB
 
 struct ThreshParams {
   const void* g;
@@ -37,9 +44,14 @@ struct ThreshParams {
   float stepsize;
   int32_t topk_pos;  // rank in descending order; <= 0 selects the sentinel
   float* thr_out;
+  CxFold fold;       // FOLD: the vector is folded from gradient tensors instead of read from g
+};
+template <int NV>
+struct ThreshBatch {
+  ThreshParams v[NV];
 };
 
-template <typename T>
+template <typename T, bool FOLD>
 __device__ __forceinline__ uint32_t sample_key(const ThreshParams& p, int i) {
   int64_t pos;
   if (p.use_all) {
@@ -50,32 +62,144 @@ __device__ __forceinline__ uint32_t sample_key(const ThreshParams& p, int i) {
   }
   float x = 0.f;
   if (p.r) x = p.r[pos];
-  if (p.g) x = x + cx::Elem<T>::to_f(reinterpret_cast<const T*>(p.g)[pos]);
+  if (FOLD) x = x + cx::fold_at<T>(p.fold, pos);
+  else if (p.g) x = x + cx::Elem<T>::to_f(reinterpret_cast<const T*>(p.g)[pos]);
   return __float_as_uint(fabsf(x));
 }
 
 constexpr int kGather = 4;  // loads of one thread that are in flight together
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) threshold_kernel(const ThreshParams p) {
+// One warp: the digit of `hist` (256 bins, walked from the top) that holds rank `rank`, and the
+// rank inside that bin.  All lanes return the same values.
+__device__ __forceinline__ uint32_t pick_digit(const uint32_t* hist, uint32_t& rank, int lane) {
+  uint32_t h[8], gsum = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { h[j] = hist[255 - 8 * lane - j]; gsum += h[j]; }
+  uint32_t incl = gsum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  const uint32_t before = incl - gsum;
+  uint32_t digit = 0, left = 0;
+  const bool mine = rank >= before && rank < incl;   // exactly one lane (rank < number of keys)
+  if (mine) {
+    uint32_t cum = before;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (rank >= cum && rank < cum + h[j]) { digit = 255 - 8 * lane - j; left = rank - cum; }
+      cum += h[j];
+    }
+  }
+  const uint32_t who = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+  digit = __shfl_sync(0xffffffffu, digit, who & 31);
+  rank = __shfl_sync(0xffffffffu, left, who & 31);
+  return digit;
+}
+
+// One warp, one key per lane (absent ones 0): the key of rank `rank` in descending order.
+__device__ __forceinline__ uint32_t warp_rank(uint32_t key, int count, int lane, uint32_t rank) {
+  uint32_t gt = 0, ge = 0;
+  for (int j = 0; j < count; ++j) {
+    const uint32_t other = __shfl_sync(0xffffffffu, key, j);
+    gt += other > key ? 1u : 0u;
+    ge += other >= key ? 1u : 0u;
+  }
+  const uint32_t who = __ballot_sync(0xffffffffu, lane < count && gt <= rank && rank < ge);
+  return __shfl_sync(0xffffffffu, key, __ffs(who) - 1);
+}
+
+// The key of rank `rank` among s_keys[0, s), for a sample that fits the block's shared memory.
+//  * rank < 32: the (rank + 1)-th largest of the 32 warps' maxima is a lower bound with at least
+//    rank + 1 keys at or above it; a handful of keys survive it, and one warp ranks those.
+//  * otherwise, up to one key per thread: bisection over the bits, one block-wide count per bit.
+//  * what is left (a large sample and a large rank): four radix passes of 8 bits.
+// 1000 samples, rank 9: 0.5 us where the radix passes took 3 us.
+__device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint32_t rank, uint32_t mymax, uint32_t* s_red,
+                                                  uint32_t* s_hist, uint32_t* s_sel) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  uint32_t key = 0, count = (uint32_t)s;
+  bool one_each = s <= kThreads;
+  if (rank < 32) {
+    if (lane == 0) s_red[w] = mymax;
+    if (tid == 0) s_sel[0] = 0;
+    __syncthreads();
+    const uint32_t bound = warp_rank(s_red[lane], 32, lane, rank);   // every warp for itself
+    for (int i = tid; i < s; i += kThreads) {
+      const uint32_t k = s_keys[i];
+      if (k >= bound) {
+        const uint32_t at = atomicAdd(&s_sel[0], 1u);
+        if (at < kThreads) s_hist[at] = k;
+      }
+    }
+    __syncthreads();
+    const uint32_t left = s_sel[0];
+    if (left <= 32) return warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank);
+    if (left <= kThreads) {
+      one_each = true;
+      count = left;
+      key = tid < (int)left ? s_hist[tid] : 0u;
+    }
+  } else if (one_each) {
+    key = tid < s ? s_keys[tid] : 0u;
+  }
+  if (one_each) {
+    // largest t with more than `rank` keys at or above it
+    uint32_t t = 0;
+    const bool have = tid < (int)count;
+    for (int bit = 30; bit >= 0; --bit) {
+      const uint32_t c = t | (1u << bit);
+      if ((uint32_t)__syncthreads_count(have && key >= c) > rank) t = c;
+    }
+    return t;
+  }
+  uint32_t prefix = 0, prefmask = 0;
+  const int s_round = (s + kThreads - 1) / kThreads * kThreads;
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    __syncthreads();
+    if (tid < 256) s_hist[tid] = 0;
+    __syncthreads();
+    for (int i = tid; i < s_round; i += kThreads) {
+      uint32_t digit = 0xffffffffu;
+      if (i < s && (s_keys[i] & prefmask) == prefix) digit = (s_keys[i] >> shift) & 255u;
+      const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+      if (digit != 0xffffffffu && lane == __ffs(peers) - 1) atomicAdd(&s_hist[digit], __popc(peers));
+    }
+    __syncthreads();
+    if (tid < 32) {
+      const uint32_t digit = pick_digit(s_hist, rank, lane);
+      if (tid == 0) { s_sel[0] = digit; s_sel[1] = rank; }
+    }
+    __syncthreads();
+    prefix |= s_sel[0] << shift;
+    prefmask |= 255u << shift;
+    rank = s_sel[1];
+  }
+  return prefix;
+}
+
+template <typename T, bool FOLD, int NV>
+__global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_constant__ ThreshBatch<NV> batch) {
   namespace cg = cooperative_groups;
   // the compress kernel queued behind this one may start its prologue now; it waits (for this
   // grid to finish) before it reads the threshold or writes the residual
-  asm volatile("griddepcontrol.launch_dependents;");
+  cx::pdl_trigger();
   __shared__ uint32_t s_keys[kSmemKeys];
-  __shared__ uint32_t s_hist[256];
-  __shared__ uint32_t s_sel[2];  // chosen digit, remaining rank
+  __shared__ uint32_t s_hist[kThreads];
+  __shared__ uint32_t s_sel[2];
   __shared__ uint32_t s_red[kThreads / 32];
   __shared__ uint32_t s_cmax[8];  // per-CTA maxima of a cluster launch (first CTA's copy is used)
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const int s = p.samples;
-  const bool cached = s <= kSmemKeys;
-  const int s_round = (s + kThreads - 1) / kThreads * kThreads;
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned ncta = cluster.num_blocks();      // 1 unless launched as a cluster (only when cached)
   const unsigned crank = cluster.block_rank();
+  const ThreshParams& p = batch.v[NV == 1 ? 0 : blockIdx.x / ncta];
+  const int s = p.samples;
+  const bool cached = s <= kSmemKeys;
   uint32_t* keys0 = ncta > 1 ? cluster.map_shared_rank(s_keys, 0) : s_keys;
+  cx::pdl_wait();     // resident early: what the kernel in front wrote may be read from here on
 
   // pass 0: gather the sample (and its maximum, for the sentinel case); CTA c of a cluster
   // takes the samples [c, c+1) * s / ncta
@@ -86,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const ThreshParams 
 #pragma unroll
     for (int u = 0; u < kGather; ++u) {
       const int i = i0 + u * kThreads;
-      k[u] = i < hi ? sample_key<T>(p, i) : 0u;
+      k[u] = i < hi ? sample_key<T, FOLD>(p, i) : 0u;
     }
 #pragma unroll
     for (int u = 0; u < kGather; ++u) {
@@ -97,39 +221,60 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const ThreshParams 
       }
     }
   }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-  if (lane == 0) s_red[tid >> 5] = mx;
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t m = 0;
-    for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_red[w]);
-    (ncta > 1 ? cluster.map_shared_rank(s_cmax, 0) : s_cmax)[crank] = m;
-  }
   if (ncta > 1) {
+    if (p.topk_pos <= 0) {
+      const uint32_t wm = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) s_red[tid >> 5] = wm;
+      __syncthreads();
+      if (tid == 0) {
+        uint32_t m = 0;
+        for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_red[w]);
+        cluster.map_shared_rank(s_cmax, 0)[crank] = m;
+      }
+    }
     cluster.sync();              // keys and maxima of all CTAs are in the first CTA's shared memory
     if (crank != 0) return;      // (no CTA touches another CTA's shared memory after this point)
-  } else {
-    __syncthreads();
+    if (p.topk_pos <= 0) {
+      if (tid == 0) {
+        uint32_t m = 0;
+        for (unsigned c = 0; c < ncta; ++c) m = max(m, s_cmax[c]);
+        *p.thr_out = __uint_as_float(m) + 1.0f;
+      }
+      return;
+    }
+    mx = 0;                      // the selection wants the maximum of this thread's keys in its own copy
+    for (int i = tid; i < s; i += kThreads) mx = max(mx, s_keys[i]);
   }
+  mx = __reduce_max_sync(0xffffffffu, mx);
   if (p.topk_pos <= 0) {
+    if (lane == 0) s_red[tid >> 5] = mx;
+    __syncthreads();
     if (tid == 0) {
       uint32_t m = 0;
-      for (unsigned c = 0; c < ncta; ++c) m = max(m, s_cmax[c]);
+      for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_red[w]);
       *p.thr_out = __uint_as_float(m) + 1.0f;
     }
     return;
   }
+  if (cached) {
+    __syncthreads();
+    const uint32_t key = select_cached(s_keys, s, (uint32_t)p.topk_pos, mx, s_red, s_hist, s_sel);
+    if (tid == 0) *p.thr_out = __uint_as_float(key);
+    return;
+  }
 
+  // a sample larger than the cache (and no workspace for the grid-wide selection below): the keys
+  // are gathered again in every radix pass
+  const int64_t s_round = ((int64_t)s + kThreads - 1) / kThreads * kThreads;
   uint32_t prefix = 0, prefmask = 0;
   uint32_t rank = (uint32_t)p.topk_pos;
   for (int shift = 24; shift >= 0; shift -= 8) {
     if (tid < 256) s_hist[tid] = 0;
     __syncthreads();
-    for (int i = tid; i < s_round; i += kThreads) {
+    for (int64_t i = tid; i < s_round; i += kThreads) {
       uint32_t digit = 0xffffffffu;
       if (i < s) {
-        const uint32_t k = cached ? s_keys[i] : sample_key<T>(p, i);
+        const uint32_t k = sample_key<T, FOLD>(p, (int)i);
         if ((k & prefmask) == prefix) digit = (k >> shift) & 255u;
       }
       const uint32_t peers = __match_any_sync(0xffffffffu, digit);
@@ -137,25 +282,8 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const ThreshParams 
     }
     __syncthreads();
     if (tid < 32) {
-      // lane L owns the 8 bins 255-8L .. 248-8L, walked from the top
-      uint32_t h[8], gsum = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { h[j] = s_hist[255 - 8 * lane - j]; gsum += h[j]; }
-      uint32_t incl = gsum;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      const uint32_t before = incl - gsum;
-      if (rank >= before && rank < incl) {  // exactly one lane
-        uint32_t cum = before;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (rank >= cum && rank < cum + h[j]) { s_sel[0] = 255 - 8 * lane - j; s_sel[1] = rank - cum; }
-          cum += h[j];
-        }
-      }
+      const uint32_t digit = pick_digit(s_hist, rank, lane);
+      if (tid == 0) { s_sel[0] = digit; s_sel[1] = rank; }
     }
     __syncthreads();
     prefix |= s_sel[0] << shift;
@@ -186,35 +314,6 @@ struct ExactParams {
   float* thr_out;
   uint32_t vec;        // 16-byte accesses are possible
 };
-
-// One warp: the digit of `hist` (256 bins, walked from the top) that holds rank `rank`, and the
-// rank inside that bin.  All lanes return the same values.
-__device__ __forceinline__ uint32_t pick_digit(const uint32_t* hist, uint32_t& rank, int lane) {
-  uint32_t h[8], gsum = 0;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) { h[j] = hist[255 - 8 * lane - j]; gsum += h[j]; }
-  uint32_t incl = gsum;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += t;
-  }
-  const uint32_t before = incl - gsum;
-  uint32_t digit = 0, left = 0;
-  const bool mine = rank >= before && rank < incl;   // exactly one lane (rank < number of keys)
-  if (mine) {
-    uint32_t cum = before;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (rank >= cum && rank < cum + h[j]) { digit = 255 - 8 * lane - j; left = rank - cum; }
-      cum += h[j];
-    }
-  }
-  const uint32_t who = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
-  digit = __shfl_sync(0xffffffffu, digit, who & 31);
-  rank = __shfl_sync(0xffffffffu, left, who & 31);
-  return digit;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kExactThreads) exact_select_kernel(const ExactParams p) {
@@ -299,17 +398,81 @@ extern "C" void cx_threshold_plan(int64_t n, float ratio, int default_subsamples
                                   float subsample_factor, int32_t* samples, int32_t* use_all,
                                   float* stepsize, int32_t* topk_pos);
 
+namespace {
+
+template <typename T, bool FOLD>
+int launch_sampled(const ThreshParams* v, int count, unsigned ncta, bool capturing, cudaStream_t s) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(ncta * (unsigned)count, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  unsigned na = 0;
+  if (ncta > 1) {      // a launch without the attribute costs the host 2 us less
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = ncta;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (!capturing && cx_pdl_enabled()) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  cudaError_t e;
+  if (count == 1) {
+    ThreshBatch<1> b;
+    b.v[0] = v[0];
+    e = cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, 1>, b);
+  } else {
+    ThreshBatch<kVectors> b;
+    memcpy(b.v, v, sizeof(ThreshParams) * (size_t)count);
+    e = cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, kVectors>, b);
+  }
+  if (e != cudaSuccess) return cx_set_error("threshold_kernel launch", (int)e);
+  cx_note_launch();
+  return cx_check_launch("threshold_kernel");
+}
+
+template <bool FOLD>
+int launch_sampled_dtype(int gdtype, const ThreshParams* v, int count, unsigned ncta, bool capturing, cudaStream_t s) {
+  switch (gdtype) {
+    case CX_F32: return launch_sampled<float, FOLD>(v, count, ncta, capturing, s);
+    case CX_BF16: return launch_sampled<__nv_bfloat16, FOLD>(v, count, ncta, capturing, s);
+    case CX_F16: return launch_sampled<__half, FOLD>(v, count, ncta, capturing, s);
+    default: return cx_set_error("cx_threshold_topk: unsupported dtype on CUDA", 0);
+  }
+}
+
+void sampled_params(ThreshParams& p, const void* g, const float* r, int64_t n, float ratio, int default_subsamples,
+                    float subsample_factor, float* thr_out) {
+  memset(&p, 0, sizeof(p));
+  p.g = g; p.r = r; p.n = n; p.thr_out = thr_out;
+  cx_threshold_plan(n, ratio, default_subsamples, subsample_factor, &p.samples, &p.use_all, &p.stepsize, &p.topk_pos);
+  if (n <= 0) { p.samples = 0; p.topk_pos = 0; }
+}
+
+// a cluster of 8 CTAs gathers large samples (their keys must fit the first CTA's shared memory)
+unsigned cluster_for(const ThreshParams& p) { return (p.samples > 2048 && p.samples <= kSmemKeys) ? 8u : 1u; }
+
+bool exact_wanted(const ThreshParams& p, const void* workspace, int64_t ws_bytes) {
+  return p.use_all && p.topk_pos > 0 && p.n > kSmemKeys && workspace && ws_bytes >= cx_threshold_workspace_bytes();
+}
+
+}  // namespace
+
 int cx_threshold_topk_cuda(int gdtype, const void* g, const float* r, int64_t n, float ratio,
                            int default_subsamples, float subsample_factor, float* thr_out,
                            void* workspace, int64_t ws_bytes, void* stream) {
   if (!g && !r) return cx_set_error("cx_threshold_topk: g and r are both NULL", 0);
   ThreshParams p;
-  p.g = g; p.r = r; p.n = n; p.thr_out = thr_out;
-  cx_threshold_plan(n, ratio, default_subsamples, subsample_factor, &p.samples, &p.use_all,
-                    &p.stepsize, &p.topk_pos);
-  if (n <= 0) { p.samples = 0; p.topk_pos = 0; }
+  sampled_params(p, g, r, n, ratio, default_subsamples, subsample_factor, thr_out);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (p.use_all && p.topk_pos > 0 && n > kSmemKeys && workspace && ws_bytes >= cx_threshold_workspace_bytes()) {
+  if (exact_wanted(p, workspace, ws_bytes)) {
     // exact selection over a vector that does not fit one CTA's shared memory: grid-wide passes
     ExactParams e;
     e.g = g; e.r = r; e.n = n; e.topk_pos = (uint32_t)p.topk_pos; e.pass = 0;
@@ -323,28 +486,40 @@ int cx_threshold_topk_cuda(int gdtype, const void* g, const float* r, int64_t n,
       default: return cx_set_error("cx_threshold_topk: unsupported dtype on CUDA", 0);
     }
   }
-  // a cluster of 8 CTAs gathers large samples (their keys must fit the first CTA's shared memory)
-  const unsigned ncta = (p.samples > 2048 && p.samples <= kSmemKeys) ? 8u : 1u;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(ncta, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = ncta;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e;
-  switch (gdtype) {
-    case CX_F32: e = cudaLaunchKernelEx(&cfg, threshold_kernel<float>, p); break;
-    case CX_BF16: e = cudaLaunchKernelEx(&cfg, threshold_kernel<__nv_bfloat16>, p); break;
-    case CX_F16: e = cudaLaunchKernelEx(&cfg, threshold_kernel<__half>, p); break;
-    default: return cx_set_error("cx_threshold_topk: unsupported dtype on CUDA", 0);
+  return launch_sampled_dtype<false>(gdtype, &p, 1, cluster_for(p), cx_seq_cell() != nullptr, s);
+}
+
+// Leading ops of the list that one launch can serve: sampled thresholds of the same element type,
+// with the same cluster size, of vectors that are all folded or all plain, into different cells.
+// Returns how many were launched (at least one), or a negative error.
+int cx_threshold_batch_cuda(const CxOp* ops, int count, void* stream) {
+  ThreshParams v[kVectors];
+  int k = 0;
+  unsigned ncta = 0;
+  for (; k < count && k < kVectors; ++k) {
+    const CxOp& o = ops[k];
+    if (o.kind != CX_OPK_THRESHOLD || o.dev != CX_DEV_CUDA || o.lane != ops[0].lane || o.dtype != ops[0].dtype ||
+        (o.fold != nullptr) != (ops[0].fold != nullptr))
+      break;
+    if (!o.g && !o.r && !o.fold) { if (k) break; return cx_set_error("cx_threshold_topk: g and r are both NULL", 0); }
+    bool same_cell = false;
+    for (int j = 0; j < k; ++j) same_cell |= v[j].thr_out == o.thr;
+    if (same_cell) break;
+    sampled_params(v[k], o.g, o.r, o.n, o.ratio, o.default_subsamples, o.subsample_factor, o.thr);
+    const bool exact = exact_wanted(v[k], o.workspace, o.ws_bytes);
+    if (exact && o.fold) { if (k) break; return cx_set_error("cx_threshold_topk: exact selection reads a plain vector", 0); }
+    if (exact || (k && cluster_for(v[k]) != ncta)) {
+      if (k) break;
+      const int rc = cx_threshold_topk_cuda(o.dtype, o.g, o.r, o.n, o.ratio, o.default_subsamples, o.subsample_factor,
+                                            o.thr, o.workspace, o.ws_bytes, stream);
+      return rc ? (rc > 0 ? -rc : rc) : 1;
+    }
+    if (k == 0) ncta = cluster_for(v[0]);
+    if (o.fold) v[k].fold = *o.fold;
   }
-  if (e != cudaSuccess) return cx_set_error("threshold_kernel launch", (int)e);
-  cx_note_launch();
-  return cx_check_launch("threshold_kernel");
+  const bool capturing = cx_seq_cell() != nullptr;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const int rc = ops[0].fold ? launch_sampled_dtype<true>(ops[0].dtype, v, k, ncta, capturing, s)
+                             : launch_sampled_dtype<false>(ops[0].dtype, v, k, ncta, capturing, s);
+  return rc ? (rc > 0 ? -rc : rc) : k;
 }

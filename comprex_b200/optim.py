@@ -46,8 +46,10 @@ into the dense update kernel.
 """
 from __future__ import annotations
 
+import ctypes as C
 import warnings
 
+import numpy as np
 import torch
 
 from . import _lib, allreduce as _ar
@@ -92,56 +94,83 @@ def _dense_layout(p: torch.Tensor) -> bool:
     return True
 
 
-def _same_layout(a: torch.Tensor, b: torch.Tensor) -> bool:
-    return all(x == y for n, x, y in zip(a.size(), a.stride(), b.stride()) if n > 1)
-
-
 class _FoldTable:
-    """Static description of a bucket's tensors for the fold kernels plus the per-step
-    table of gradient pointers (staged through a small ring of pinned buffers)."""
+    """Static description of the tensors of some buckets for the fold kernels plus the per-step
+    table of gradient pointers (staged through a small ring of pinned buffers).  Flat positions are
+    those of the optimizer's buffers; ``fold_args`` addresses one bucket's part or all of them."""
 
-    def __init__(self, env, bucket):
-        dev = env.device
-        off, rel, ln, seg, first = [], [], [], [], [0]
-        for si, (p, o) in enumerate(zip(bucket.params, bucket.offsets)):
-            k = p.numel()
-            for r in range(0, max(k, 1), _ITEM):
-                off.append(o - bucket.start + r)
-                rel.append(r)
-                ln.append(min(_ITEM, k - r))
-                seg.append(si)
-            first.append(len(off))
-        self.nitems, self.nseg = len(off), len(bucket.params)
-        self.item_off = torch.tensor(off, dtype=torch.int64, device=dev)
-        self.item_rel = torch.tensor(rel, dtype=torch.int64, device=dev)
-        self.item_len = torch.tensor(ln, dtype=torch.int32, device=dev)
-        self.item_seg = torch.tensor(seg, dtype=torch.int32, device=dev)
-        self.seg_first = torch.tensor(first, dtype=torch.int32, device=dev)
-        self.partial = torch.zeros(self.nitems, dtype=torch.float32, device=dev)
+    def __init__(self, env, buckets, dtype):
+        dev, lo = env.device, buckets[0].start
+        self.env, self.dtype, self.code = env, dtype, _lib.dtype_code(dtype)
+        self.params = [p for b in buckets for p in b.params]
+        numel = np.array([p.numel() for p in self.params], dtype=np.int64)
+        start = np.array([o for b in buckets for o in b.offsets], dtype=np.int64)
+        count = np.maximum(1, -(-numel // _ITEM))                     # items per tensor
+        first = np.concatenate(([0], np.cumsum(count)))
+        self.nseg, self.nitems = len(numel), int(first[-1])
+        seg = np.repeat(np.arange(self.nseg), count)
+        rel = (np.arange(self.nitems) - first[seg]) * _ITEM
+        wide = torch.from_numpy(np.concatenate((start[seg] + rel - lo, rel, start, start + numel))).to(dev)
+        narrow = torch.from_numpy(np.concatenate((np.minimum(_ITEM, numel[seg] - rel), seg, first)).astype(np.int32)).to(dev)
+        # cx_fold counts positions from the first bucket on
+        self.item_off, self.item_rel, self.seg_off, self.seg_end = wide.split([self.nitems] * 2 + [self.nseg] * 2)
+        self.item_len, self.item_seg, self.seg_first = narrow.split([self.nitems] * 2 + [self.nseg + 1])
+        self.partial = torch.zeros(8 * self.nitems, dtype=torch.float32, device=dev)
         self.ptrs = torch.zeros(self.nseg, dtype=torch.int64, device=dev)
-        self.last = None
+        self._collect = _lib.host().collect
+        self.scalar_type = _lib.host().scalar_type(self.params[0])
+        self.now = torch.full((self.nseg,), -1, dtype=torch.int64)
         self.cuda = dev.type == "cuda"
         if self.cuda:
             self.ring = [(torch.zeros(self.nseg, dtype=torch.int64).pin_memory(), torch.cuda.Event()) for _ in range(4)]
             self.turn = 0
+            self.coef = torch.zeros(self.nseg, dtype=torch.float32, device=dev)
+            # buckets start on sub-tile borders: one table serves them all
+            subs = torch.arange(lo, max(buckets[-1].end, lo + 1), _lib.SUBTILE, dtype=torch.int64, device=dev)
+            self.sub_seg = torch.searchsorted(self.seg_end, subs, right=True, out_int32=True)
+            self.args, self.lo = {}, lo
 
-    def stage(self, values) -> None:
-        """Upload this step's gradient pointers (async on the current stream).  The caching
-        allocator usually hands autograd the same blocks every step: an unchanged table is
-        not uploaded again."""
-        if values == self.last:
+    def refresh(self, zeros) -> None:
+        """Bring the table of gradient addresses up to this step's; ``zeros`` stands in for a missing
+        gradient.  The caching allocator usually hands autograd the same blocks every step: an
+        unchanged table is not uploaded again (otherwise: async on the current stream)."""
+        changed = self._collect(self.params, self.scalar_type, zeros.data_ptr(), self.now.data_ptr())
+        if changed == 2:                          # rare: bring the odd ones into the parameters' form first
+            for p in self.params:
+                g = p.grad
+                if g is not None and (g.dtype is not self.dtype or g.stride() != p.stride()):
+                    p.grad = torch.empty_strided(p.size(), p.stride(), dtype=self.dtype, device=p.device).copy_(g)
+            self.now.fill_(-1)
+            changed = self._collect(self.params, self.scalar_type, zeros.data_ptr(), self.now.data_ptr())
+        if not changed:
             return
-        self.last = list(values)
         if not self.cuda:
-            self.ptrs.copy_(torch.tensor(values, dtype=torch.int64))
+            self.ptrs.copy_(self.now)
             return
         host, ev = self.ring[self.turn]
         self.turn = (self.turn + 1) % len(self.ring)
         ev.synchronize()                      # the copy that last used this buffer has finished
-        host.copy_(torch.tensor(values, dtype=torch.int64))
+        host.copy_(self.now)
         self.ptrs.copy_(host, non_blocking=True)
         ev.record()
 
+    def launch_coef(self, clip: float, lr: float) -> None:
+        """Norms and clip factors of all tensors of the table (CUDA)."""
+        _lib.check(self.env.lib.cx_fold_coef(self.code, self.ptrs.data_ptr(), self.item_rel.data_ptr(),
+                                             self.item_len.data_ptr(), self.item_seg.data_ptr(),
+                                             self.seg_first.data_ptr(), 0, self.nitems, 0, self.nseg,
+                                             self.partial.data_ptr(), self.coef.data_ptr(), clip, lr,
+                                             _lib.stream_ptr(self.env.device)), "cx_fold_coef")
+
+    def fold_args(self, b, u, mu: float):
+        """The folded vector of bucket ``b`` (None: of all buckets); ``u``: its momentum, or None."""
+        f = _lib.Fold()
+        base = self.lo if b is None else b.start
+        sub = self.sub_seg.data_ptr() + 4 * ((base - self.lo) // _lib.SUBTILE)
+        f.seg_ptr, f.seg_off, f.seg_end = self.ptrs.data_ptr(), self.seg_off.data_ptr(), self.seg_end.data_ptr()
+        f.coef, f.sub_seg, f.u = self.coef.data_ptr(), sub, 0 if u is None else u.data_ptr()
+        f.base, f.nseg, f.mu = base, self.nseg, mu
+        return f
 
 
 class ComprexOptimizer(torch.optim.Optimizer):
@@ -249,6 +278,10 @@ class ComprexOptimizer(torch.optim.Optimizer):
         # backward ends, and the hooks and the side stream would only add latency
         self.overlap = bool(overlap) and dev.type == "cuda" and len(self._buckets) > 1 and not self._local
         self._armed = False
+        self._all = None
+        self._cuda = dev.type == "cuda"
+        # the folded vector is the momentum, and outlives the step, only in the reference's own rule
+        self._keeps_u = rule == "sgd" and self.local_momentum
         self._hooks = []
         if self.overlap:
             for p in self._params:
@@ -331,32 +364,118 @@ class ComprexOptimizer(torch.optim.Optimizer):
             self._mark(("origin",))             # the step's timeline starts here
 
     # ---- the step ---------------------------------------------------------------------------------
-    def _fold(self, b: _Bucket, lr: float, mu: float) -> torch.Tensor:
-        """Clip per tensor and build the vector that is exchanged for one bucket: two launches
-        that read the gradient tensors where autograd left them."""
+    def _table(self, b: _Bucket) -> _FoldTable:
         if b.fold is None:
-            b.fold = _FoldTable(self._env, b)
-        ft, ptrs = b.fold, []
-        for p in b.params:
-            g = p.grad
-            if g is None:
-                ptrs.append(self._zeros.data_ptr())
-                continue
-            if g.dtype != self._dtype or (g.stride() != p.stride() and not _same_layout(g, p)):
-                g = torch.empty_strided(p.size(), p.stride(), dtype=self._dtype, device=p.device).copy_(g)  # rare
-                p.grad = g
-            ptrs.append(g.data_ptr())
-        ft.stage(ptrs)
+            b.fold = _FoldTable(self._env, [b], self._dtype)
+        b.fold.refresh(self._zeros)
+        return b.fold
+
+    def _fold_scalars(self, lr: float, mu: float):
+        """(clip, momentum, learning rate) of the fold: the optimizers that keep their momentum in the
+        receive kernel exchange the clipped gradient itself."""
+        clip = float(self.pre_clipnorm) if self.pre_clipnorm is not None else 0.0
+        if self._keeps_u:
+            return clip, mu * self.momentum_correction, lr
+        return clip, 0.0, 1.0
+
+    def _fold(self, b: _Bucket, lr: float, mu: float) -> torch.Tensor:
+        """Clip per tensor and build the vector that is exchanged for one bucket in memory: two
+        launches that read the gradient tensors where autograd left them.  (The fused steps below
+        never store it, except as the momentum.)"""
+        ft, env = self._table(b), self._env
         u = self._update[b.start:b.end]
-        local = self.rule == "sgd" and self.local_momentum
-        env = self._env
-        _lib.check(env.lib.cx_fold(env.dev, _lib.dtype_code(self._dtype), ft.ptrs.data_ptr(), ft.item_off.data_ptr(),
+        clip, mu, lr = self._fold_scalars(lr, mu)
+        _lib.check(env.lib.cx_fold(env.dev, ft.code, ft.ptrs.data_ptr(), ft.item_off.data_ptr(),
                                    ft.item_rel.data_ptr(), ft.item_len.data_ptr(), ft.item_seg.data_ptr(),
                                    ft.seg_first.data_ptr(), ft.nitems, u.data_ptr(), ft.partial.data_ptr(),
-                                   float(self.pre_clipnorm) if self.pre_clipnorm is not None else 0.0,
-                                   mu * self.momentum_correction if local else 0.0, lr if local else 1.0,
-                                   _lib.stream_ptr(env.device)), "cx_fold")
+                                   clip, mu, lr, _lib.stream_ptr(env.device)), "cx_fold")
         return u
+
+    # ---- the fused forms (CUDA) -------------------------------------------------------------------
+    def _fusable(self, b: _Bucket) -> bool:
+        """The compress kernel can fold the bucket's gradients itself: compressed BigRing, sampled
+        threshold (an exact selection reads a stored vector)."""
+        return self._cuda and b.kind == "bigring" and not b.ar.exact_topk
+
+    def _fold_args(self, ft: _FoldTable, b: _Bucket, mu: float):
+        """The bucket's CxFold, kept with the table (the native side reads it at every launch)."""
+        f = ft.args.get(b)
+        if f is None:
+            f = ft.args[b] = ft.fold_args(b, self._update[b.start:b.end] if self._keeps_u else None, mu)
+        elif f.mu != mu:
+            f.mu = mu
+        return f
+
+    def _group(self):
+        """One table and, per parity of the exchange step, one launch list for all buckets: all norms,
+        all thresholds and all updates of a step then take one native call each."""
+        if self._all is None:
+            self._all = {"table": _FoldTable(self._env, self._buckets, self._dtype), "lists": {}}
+        return self._all
+
+    def _lists(self, g, par: int):
+        """(send ops, receive ops, views of the receive ops' arguments) for one parity."""
+        bs, k = self._buckets, len(self._buckets)
+        cfg = [(b.ar.compression_ratio, b.ar.sampling) for b in bs]
+        got = g["lists"].get(par)
+        if got is not None and got[0] == cfg:
+            return got
+        send, recv = (_lib.Op * (2 * k))(), (_lib.Op * k)()
+        for i, b in enumerate(bs):
+            s, r = b.ar.launch_lists(par)
+            send[i], send[k + i], recv[i] = s.arr[0], s.arr[1], r.arr[0]
+            send[i].ratio = b.ar.compression_ratio
+            send[i].dtype = send[k + i].dtype = g["table"].code
+            send[i].g = send[k + i].g = None
+            send[i].fold = send[k + i].fold = C.addressof(g["table"].args[b])
+            if i:                                # buckets share no vector, slot or scratch
+                send[k + i].chain = recv[i].chain = 1
+        got = g["lists"][par] = [cfg, send, recv, [recv[i].apply for i in range(k)], None]
+        return got
+
+    def _send_all(self, lr, mu) -> None:
+        """First half of the exchange of all buckets: the norms of all tensors, all thresholds, then
+        one fold-and-compress kernel per bucket."""
+        env, g, buckets = self._env, self._group(), self._buckets
+        ft = g["table"]
+        ft.refresh(self._zeros)
+        clip, mu, lr = self._fold_scalars(lr, mu)
+        ft.launch_coef(clip, lr)
+        for b in buckets:
+            self._fold_args(ft, b, mu)
+            b.seq, b.par = b.ar.next_step()
+            b.sent = True
+        seq, par = buckets[0].seq, buckets[0].par
+        send = self._lists(g, par)[1]
+        _lib.check(env.lib.cx_run_ops(send, len(send), seq, _lib.stream_ptr(env.device)), "cx_run_ops")
+
+    def _recv_all(self, lr, mu, wd) -> None:
+        """Second half: one wait-decode-update kernel per bucket."""
+        env, buckets = self._env, self._buckets
+        got = self._lists(self._group(), buckets[0].par)
+        recv, views, hyper = got[2], got[3], (lr, mu, wd, self.momentum_correction)
+        if got[4] != hyper:
+            for b, v in zip(buckets, views):
+                C.pointer(v)[0] = self._args(b.start, b.end - b.start, lr, mu, wd, 1.0 / env.ranks)
+            got[4] = hyper
+        elif self.rule == "adamw":               # the bias corrections move with every step
+            bc1, bc2 = 1.0 - self.betas[0] ** self._t, 1.0 - self.betas[1] ** self._t
+            for v in views:
+                v.bc1, v.bc2 = bc1, bc2
+        _lib.check(env.lib.cx_run_ops(recv, len(recv), buckets[0].seq, _lib.stream_ptr(env.device)), "cx_run_ops")
+
+    def _step_local(self, lr, mu, wd) -> None:
+        """The step of a rank that exchanges nothing: norms, then one fold-and-update kernel over the
+        whole flat buffer."""
+        env, g = self._env, self._group()
+        ft = g["table"]
+        ft.refresh(self._zeros)
+        args = self._args(0, self.blob_size, lr, mu, wd, 1.0)
+        clip, mu, lr = self._fold_scalars(lr, mu)
+        ft.launch_coef(clip, lr)
+        fold = ft.fold_args(None, self._update if self._keeps_u else None, mu)
+        _lib.check(env.lib.cx_fold_update(ft.code, C.byref(fold), self.blob_size, C.byref(args),
+                                          _lib.stream_ptr(env.device)), "cx_fold_update")
 
     def _hyper(self):
         """The update kernels take one learning rate, momentum and weight decay for the whole flat
@@ -413,8 +532,17 @@ class ComprexOptimizer(torch.optim.Optimizer):
         idx = self._buckets.index(b) if getattr(self, "_trace", None) is not None else -1
         self._mark(("send_start", idx))
         with nvtx_range("comprex.fold+send"):
-            u = self._fold(b, lr, mu)
-            if b.kind == "bigring":
+            fused = self._fusable(b)
+            if fused:
+                ft = self._table(b)
+                clip, mu, lr = self._fold_scalars(lr, mu)
+                ft.launch_coef(clip, lr)
+                b.seq, b.par = b.ar.send_fast(None, fold=(self._fold_args(ft, b, mu), ft.code))
+            else:
+                u = self._fold(b, lr, mu)
+            if fused:
+                pass
+            elif b.kind == "bigring":
                 b.seq, b.par = b.ar.send_fast(u)
             elif b.kind == "ring":
                 b.xbuf.copy_(u)
@@ -509,19 +637,40 @@ class ComprexOptimizer(torch.optim.Optimizer):
             import contextlib
             ctx = contextlib.nullcontext()
         with ctx:
-            for b in self._buckets:          # everything that the hooks did not send yet
-                if not b.sent:
-                    self._send(b)
-            for i, b in enumerate(self._buckets):   # then receive: all peers' payloads are on their way
-                self._mark(("recv_start", i))
-                self._recv(b, lr, mu, wd)
-                self._mark(("recv_end", i))
-                b.sent, b.ready = False, 0
+            if self._local and self._cuda:
+                with nvtx_range("comprex.update"):
+                    self._step_local(lr, mu, wd)
+            else:
+                self._exchange(lr, mu, wd)
         if use_side:
             torch.cuda.current_stream(self._env.device).wait_stream(comm)
         self._mark(("step_end",))
         self._env.maybe_check()
         return loss
+
+    def _exchange(self, lr, mu, wd) -> None:
+        pending = [b for b in self._buckets if not b.sent]     # everything that the hooks did not send yet
+        if len(pending) == len(self._buckets) and self._in_step():
+            with nvtx_range("comprex.fold+send"):
+                self._send_all(lr, mu)
+            with nvtx_range("comprex.recv+update"):
+                self._recv_all(lr, mu, wd)
+            for b in self._buckets:
+                b.sent, b.ready = False, 0
+            return
+        for b in pending:
+            self._send(b)
+        for i, b in enumerate(self._buckets):   # then receive: all peers' payloads are on their way
+            self._mark(("recv_start", i))
+            self._recv(b, lr, mu, wd)
+            self._mark(("recv_end", i))
+            b.sent, b.ready = False, 0
+
+    def _in_step(self) -> bool:
+        """All buckets are fusable and at the same exchange step (one sequence number serves the
+        launch lists); a timeline wants them one by one."""
+        return (self._trace is None and all(self._fusable(b) for b in self._buckets)
+                and len({b.ar.step for b in self._buckets}) == 1)
 
     def apply_gradients(self, grads_and_vars, *args, **kwargs):
         """Keras-style entry (keras/comprex_optimizer.py:144-145): ``(gradient, variable)`` pairs are

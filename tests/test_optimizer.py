@@ -651,3 +651,40 @@ def test_no_sync_accumulates_like_plain_accumulation():
         res.append(opt._master.clone())
         env.close()
     assert torch.equal(res[0], res[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["sgd", "sgd_no_momentum", "receive_momentum", "adamw"])
+@pytest.mark.parametrize("exchange", [True, False])
+def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange):
+    """Folding inside the compress and update kernels (register path, tensor borders, gaps, a missing
+    and an unaligned gradient, several buckets) against the vector built in memory first."""
+    sizes = [1, 63, 64, 65, 1023, 1024, 1025, 4096, 70001, 200000, 7, 2048]
+    arms = []
+    for fused in (True, False):
+        torch.manual_seed(5)
+        env = cx.GaspiEnvironment(8 << 20, device="cuda")
+        params = [torch.nn.Parameter(torch.randn(s, device="cuda").to(dtype)) for s in sizes]
+        opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.0 if kind == "sgd_no_momentum" else 0.9,
+                               compression_ratio=0.05, rule="adamw" if kind == "adamw" else "sgd", pre_clipnorm=20.0,
+                               local_momentum=kind != "receive_momentum", weight_decay=0.01, bucket_cap_mb=0.2,
+                               single_rank_bypass=not exchange)
+        assert len(opt._buckets) > 2
+        if not fused:
+            opt._fusable = lambda b: False
+            opt._step_local = lambda lr, mu, wd: opt._exchange(lr, mu, wd)
+        for step in range(4):
+            gen = torch.Generator(device="cuda").manual_seed(step)
+            for i, p in enumerate(params):
+                g = torch.randn(sizes[i] + 1, device="cuda", generator=gen).to(dtype)
+                p.grad = None if (step == 1 and i == 7) else g[1:] if i == 9 else g[:-1]     # i == 9: odd address
+            opt.step()
+        env.flush()
+        arms.append([opt._master.clone(), opt._shadow if dtype != torch.float32 else opt._master]
+                    + [t for t in (opt._m, opt._v) if t is not None] + ([opt._update] if opt._keeps_u else [])
+                    + [ar.rests for ar in opt.comprex_allreducers.values()])
+    assert len(arms[0]) == len(arms[1])
+    for a, b in zip(*arms):
+        assert torch.equal(a, b)
+    env.close()
