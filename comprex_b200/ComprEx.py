@@ -248,6 +248,10 @@ class Comprex(AbstractExchange):
         self._src = None
         self._rx_current = None
         self._held = None
+        # launch lists of the plain cases, one per parity of the message number (CUDA)
+        self._tx_ops: dict = {}
+        self._rx_ops: dict = {}
+        self._prepared = env.device.type == "cuda" and type(self) is Comprex
 
     def _nslots(self) -> int:
         return 2
@@ -388,6 +392,49 @@ class Comprex(AbstractExchange):
         self._rle.send(g, r, self._comp.thr, seq, self._dest)
         self._env.maybe_check()
 
+    def _write_prepared(self, vector) -> bool:
+        """``writeRemote`` of a plain vector with a sampled or exact top-k threshold: one call for the
+        whole launch list.  False: take the general path."""
+        thr, comp = self.threshold, self._comp
+        if (self.compressor.kind != "pairs" or type(thr) is not ThresholdTopK or self.restsVect is None
+                or getattr(self._env, "_rec", None) is not None):
+            return False
+        dest = self._dest
+        seq = self._tx_seq.get(dest, 0) + 1
+        cfg = (dest, thr.topK, thr.default_subsamples, thr.subsample_factor, self.restsVect)
+        got = self._tx_ops.get(seq & 1)
+        if got is None or got[0] != cfg[:4] or got[1] is not cfg[4]:
+            ep = self._slots[seq & 1].endpoint(self._env, dest)
+            got = self._tx_ops[seq & 1] = (cfg[:4], cfg[4], _lib.VectorOps(
+                _lib.VectorOps.SEND, comp.send_ops(self.restsVect, self.size, self.cap, P.make_targets([ep]), *cfg[1:4]),
+                self._env.device, self.size))
+        if not got[2].run(vector, seq):
+            return False
+        self._tx_seq[dest] = seq
+        thr._cell = comp.thr
+        self._env.maybe_check()
+        return True
+
+    def _read_prepared(self, vector, op: int) -> bool:
+        """``readRemote(vector)`` / ``readRemote_add`` of a plain vector.  False: take the general path."""
+        if self.compressor.kind != "pairs" or self._rx_current is not None or self._src is None:
+            return False
+        src = self._src
+        seq = self._rx_seq.get(src, 0) + 1
+        got = self._rx_ops.get((seq & 1, op))
+        if got is None:
+            o = _lib.Op()
+            o.kind, o.dev, o.n = _lib.OPK_APPLY, self._env.dev, self.size
+            o.src = P.make_sources([self._slots[seq & 1].endpoint(self._env)], [seq])
+            o.apply.op, o.apply.scale = op, 1.0
+            o.status, o.timeout_ns = self._status.dev_ptr, self._env.timeout_ns
+            got = self._rx_ops[(seq & 1, op)] = _lib.VectorOps(_lib.VectorOps.APPLY, [o], self._env.device, self.size)
+        if not got.run(vector, seq):
+            return False
+        self._rx_seq[src] = seq
+        self._env.maybe_check()
+        return True
+
     def _send(self, g, r, thr_obj, fixed_thr=None) -> None:
         if self.compressor.kind == "pairs":
             self._send_pairs(g, r, thr_obj, fixed_thr)
@@ -397,6 +444,8 @@ class Comprex(AbstractExchange):
     def writeRemote(self, vector) -> None:
         """threshold(rests + v); rests += v; send |rests| > thr; zero what was sent."""
         self._require_tx()
+        if self._prepared and self._write_prepared(vector):
+            return
         self._send(self._vec(vector), self.restsVect, self.threshold)
 
     def writeRemote_compressOnly(self, vector) -> None:
@@ -450,6 +499,8 @@ class Comprex(AbstractExchange):
         ret = vector is None
         if ret:
             vector = torch.empty(self.size, dtype=torch.float32, device=self._env.device)
+        if self._prepared and self._read_prepared(vector, _lib.OP_SET):
+            return vector if ret else None
         t, orig = to_device_vector(self._env, vector)
         if self.compressor.kind != "pairs":
             self._recv_other(t, add=False)
@@ -463,6 +514,8 @@ class Comprex(AbstractExchange):
     def readRemote_add(self, vector) -> None:
         """Wait and scatter-add into ``vector``."""
         self._require_rx()
+        if self._prepared and self._read_prepared(vector, _lib.OP_ADD):
+            return
         t, orig = to_device_vector(self._env, vector)
         if self.compressor.kind != "pairs":
             self._recv_other(t, add=True)

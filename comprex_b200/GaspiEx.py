@@ -27,6 +27,7 @@ import numpy as np
 import torch
 
 from .common import AbstractExchange, Getable  # noqa: F401  (the reference defines Getable in this module too)
+from . import _lib
 from ._lib import ComprexError
 from .ops import primitives as P
 
@@ -69,6 +70,9 @@ class GaspiEx(AbstractExchange):
         self._last_sent = None
         self._held = None       # (tensor, n) copied by forward_buffer
         self._rx_current = None  # endpoint + seq picked by readRemote_wait
+        # launch lists of the plain cases, one per parity of the message number (CUDA)
+        self._ops: dict = {}
+        self._prepared = env.device.type == "cuda"
 
     # ---- connections (src/gaspiEx.tpp:121-192) -----------------------------------
     def connectTx(self, destRank: int, tag: int = 0) -> None:
@@ -114,11 +118,40 @@ class GaspiEx(AbstractExchange):
         mc = self._slots[seqs[0] & 1].mc_endpoint(self._env) if self._src is None else None
         return P.make_targets(eps, mc=mc), seqs[0]
 
+    def _run_prepared(self, vector, role: int) -> bool:
+        """One dense message of a plain vector to or from the connected rank.  False: take the general path."""
+        if getattr(self._env, "_rec", None) is not None or self._rx_current is not None:
+            return False
+        V = _lib.VectorOps
+        peer, seqs = (self._dest, self._tx_seq) if role == V.DENSE_SEND else (self._src, self._rx_seq)
+        if peer is None:
+            return False
+        seq = seqs.get(peer, 0) + 1
+        key = (role, peer, seq & 1)
+        got = self._ops.get(key)
+        if got is None:
+            env, o = self._env, _lib.Op()
+            o.dev, o.dtype, o.src_rank, o.workspace = env.dev, _lib.dtype_code(self.dtype), env.rank, self._counters.data_ptr()
+            if role == V.DENSE_SEND:
+                o.kind, o.tg = _lib.OPK_DENSE_SEND, P.make_targets([self._slots[seq & 1].endpoint(env, peer)])
+            else:
+                o.kind, o.scale, o.src = _lib.OPK_DENSE_REDUCE, 1.0, P.make_sources([self._slots[seq & 1].endpoint(env)], [seq])
+                o.status, o.timeout_ns = self._status.dev_ptr, env.timeout_ns
+            got = self._ops[key] = V(role, [o], env.device, self.size)
+        if not got.run(vector, seq):
+            return False
+        seqs[peer] = seq
+        self._env.maybe_check()
+        return True
+
     def writeRemote(self, vector=None, size: int | None = None) -> None:
         """Send ``vector`` to the connected rank.  Without a vector, re-send the
         aliased engine's last vector (``writeRemote(size)`` of the reference)."""
         if self._dest is None:
             raise ComprexError("Send issued without connecting to Remote!")
+        if size is None and self._prepared and self._run_prepared(vector, _lib.VectorOps.DENSE_SEND):
+            self._last_sent = vector.view(-1)
+            return
         if vector is None or isinstance(vector, int):
             src = self._alias_of if self._alias_of is not None else self
             if src._last_sent is None:
@@ -166,6 +199,8 @@ class GaspiEx(AbstractExchange):
         return out
 
     def readRemote_vec(self, vector, size: int | None = None) -> None:
+        if size is None and self._prepared and self._run_prepared(vector, _lib.VectorOps.DENSE_READ):
+            return
         t, orig = to_device_vector(self._env, vector, self.dtype)
         n = t.numel() if size is None else int(size)
         if n > self.size:
@@ -176,6 +211,8 @@ class GaspiEx(AbstractExchange):
         write_back(t, orig)
 
     def readRemote_add(self, vector, size: int | None = None) -> None:
+        if size is None and self._prepared and self._run_prepared(vector, _lib.VectorOps.DENSE_ADD):
+            return
         t, orig = to_device_vector(self._env, vector, self.dtype)
         n = t.numel() if size is None else int(size)
         if n > self.size:

@@ -212,6 +212,30 @@ def host():
     return _host_mod
 
 
+class VectorOps:
+    """Launch list of one message of a prepared connection (CUDA): ``run`` hands it a vector and
+    returns False, with nothing launched, when the vector needs the caller's general path (another
+    type or device, a NumPy array, a non-contiguous tensor, another size)."""
+
+    SEND, APPLY, DENSE_SEND, DENSE_READ, DENSE_ADD = range(5)      # roles of the vector
+
+    def __init__(self, role: int, ops, device: torch.device, n: int):
+        self.ops = (Op * len(ops))(*ops)
+        self._role, self._addr, self._count = role, C.addressof(self.ops), len(ops)
+        self._device, self._n = device.index, n
+        self._run = host().run_vector
+        self._fn = C.cast(load().cx_run_ops, C.c_void_p).value
+
+    def run(self, vector, seq: int) -> bool:
+        rc = self._run(self._role, self._fn, self._addr, self._count, seq, _raw_stream(self._device), vector,
+                       self._device, self._n)
+        if rc is None:
+            return False
+        if rc:
+            check(rc, "cx_run_ops")
+        return True
+
+
 def last_error() -> str:
     return load().cx_last_error().decode("utf-8", "replace")
 

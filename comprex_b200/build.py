@@ -78,7 +78,7 @@ def _build_host(verbose: bool) -> None:
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
     src = CSRC / "python" / "host.cpp"
-    if not _stale(HOST, [src, Path(__file__)]):
+    if not _stale(HOST, [src, CSRC / "cx_common.h", Path(__file__)]):
         return
     cmd = ([os.environ.get("CXX", "g++"), "-shared"] + CXX_FLAGS
            + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]

@@ -227,6 +227,19 @@ class Compressor:
                                        self.stats.dev_ptr, env.rank, _lib.stream_ptr(env.device)),
                    "cx_compress")
 
+    def send_ops(self, r: torch.Tensor, n: int, cap: int, targets: Targets, ratio: float, default_subsamples: int,
+                 subsample_factor: float) -> list:
+        """The threshold and compress launches as ops whose input vector is filled in later."""
+        env = self.env
+        thr, cmp_ = _new_op(env, _lib.OPK_THRESHOLD, _lib.F32, n), _new_op(env, _lib.OPK_COMPRESS, _lib.F32, n)
+        thr.r = cmp_.r = r.data_ptr()
+        thr.thr = cmp_.thr = self.thr.data_ptr()
+        thr.ratio, thr.default_subsamples, thr.subsample_factor = ratio, int(default_subsamples), float(subsample_factor)
+        thr.workspace, thr.ws_bytes = self.thr_ws.data_ptr(), self.thr_ws_bytes
+        cmp_.cap, cmp_.src_rank, cmp_.stats, cmp_.tg = cap, env.rank, self.stats.dev_ptr, targets
+        cmp_.workspace, cmp_.ws_bytes = self.workspace.data_ptr(), self.ws_bytes
+        return [thr, cmp_]
+
     def last_stats(self) -> dict:
         """Statistics of the most recent compress call (synchronises)."""
         self.env.flush()
