@@ -132,9 +132,11 @@ class ThresholdTopK(_Threshold):
         ref = g if g is not None else r
         out = torch.zeros(1, dtype=torch.float32, device=ref.device)
         gd = _lib.dtype_code(g.dtype) if g is not None else _lib.F32
-        ws_bytes = int(lib.cx_threshold_workspace_bytes()) if self.exact else 0
-        if self.exact and (self._ws is None or self._ws.device != ref.device):
-            self._ws = torch.zeros(ws_bytes, dtype=torch.uint8, device=ref.device)   # grid-wide exact selection
+        ws_bytes = 0
+        if self.exact:                                # scratch of the grid-wide selection
+            ws_bytes = int(lib.cx_threshold_exact_bytes(ref.numel()) if ref.is_cuda else lib.cx_threshold_workspace_bytes())
+            if self._ws is None or self._ws.device != ref.device or self._ws.numel() < ws_bytes:
+                self._ws = torch.zeros(ws_bytes, dtype=torch.uint8, device=ref.device)
         _lib.check(lib.cx_threshold_select(_lib.dev_code(ref), gd, g.data_ptr() if g is not None else 0,
                                            r.data_ptr() if r is not None else 0, ref.numel(), self.topK,
                                            self.default_subsamples, self.subsample_factor, out.data_ptr(),

@@ -177,6 +177,8 @@ int cx_threshold_topk(int dev, int gdtype, const void* g, const float* r,
  * is switched off (every element is a sample, e.g. default_subsamples = 2^31 - 128) the CUDA
  * back end then selects over the whole vector with grid-wide radix passes instead of one CTA. */
 int64_t cx_threshold_workspace_bytes(void);
+/* Scratch (zeroed once) with which that selection makes one pass over the vector instead of four. */
+int64_t cx_threshold_exact_bytes(int64_t n);
 int cx_threshold_select(int dev, int gdtype, const void* g, const float* r, int64_t n, float ratio,
                         int default_subsamples, float subsample_factor, float* thr_out, void* workspace,
                         int64_t ws_bytes, void* stream);

@@ -374,6 +374,285 @@ __global__ void __launch_bounds__(kExactThreads) exact_select_kernel(const Exact
   if (s_hist[tid]) atomicAdd(&p.hist[256 * p.pass + tid], s_hist[tid]);
 }
 
+// ---- exact selection with one pass over the vector -----------------------------------------------
+// With scratch for candidates (cx_threshold_exact_bytes) the four passes become one:
+//   1. bracket: two keys lo <= hi from a sample of 8192 elements, one per stratum at a hashed position
+//      (a fixed stride could meet the same column of every row), between which the wanted key lies
+//      unless the sample is off by more than four standard deviations,
+//   2. collect: one pass counts the keys above hi, at hi and at lo, and appends the ones between to
+//      the candidate list (about 1 % of the vector),
+//   3. finish:  a cluster selects among the candidates by radix.  If the counts show that the bracket
+//      missed, or the candidates did not fit, it selects over the whole vector instead: always exact,
+//      only slower.
+// 10 M elements, fp32 vector and residual, top-k 1 %: 96 us with four passes.
+constexpr int kBracket = 8192;
+constexpr int kCluster = 8;
+constexpr int kBins = 2048;          // 11 bits per radix pass of the finish
+constexpr int kCollectThreads = 256;
+constexpr int kCollectEach = 16;     // elements per thread and round
+constexpr int kBuffer = 6144;        // candidates a CTA keeps before it appends them to the list
+
+struct ExactState {                  // in the workspace behind the histograms; zero between calls
+  uint32_t lo, hi;
+  uint32_t above, at_hi, at_lo;      // elements with key > hi, == hi, == lo (lo < hi)
+  uint32_t found;                    // candidates with lo < key < hi (not all of them stored when over cap)
+  uint32_t pad[58];
+};
+
+struct OnePassParams {
+  const void* g;
+  const float* r;
+  int64_t n;
+  uint32_t rank;         // in descending order
+  uint32_t cap;          // candidates that fit the list
+  uint32_t hi_rank;      // ranks of the bracket in the sample; hi_rank == ~0u: no upper bound
+  uint32_t lo_rank;      // ~0u: no lower bound
+  ExactState* st;
+  uint32_t* list;
+  float* thr_out;
+  uint32_t vec;
+};
+
+template <typename T>
+__device__ __forceinline__ uint32_t key_at(const OnePassParams& p, int64_t i) {
+  float x = p.r ? p.r[i] : 0.f;
+  if (p.g) x = x + cx::Elem<T>::to_f(reinterpret_cast<const T*>(p.g)[i]);
+  return __float_as_uint(fabsf(x));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant__ OnePassParams p) {
+  namespace cg = cooperative_groups;
+  __shared__ uint32_t s_keys[kBracket];
+  __shared__ uint32_t s_hist[kThreads];
+  __shared__ uint32_t s_sel[2];
+  __shared__ uint32_t s_red[kThreads / 32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned crank = cluster.block_rank();
+  const int tid = threadIdx.x;
+  uint32_t* k0 = cluster.map_shared_rank(s_keys, 0);
+  uint32_t* k1 = cluster.map_shared_rank(s_keys, 1);
+  cx::pdl_wait();
+  cx::pdl_trigger();
+  {
+    const uint32_t i = crank * kThreads + tid;
+    const int64_t a = (int64_t)(((uint64_t)p.n * i) / kBracket), b = (int64_t)(((uint64_t)p.n * (i + 1)) / kBracket);
+    const uint32_t h = (i + 1) * 2654435761u;
+    const uint32_t k = key_at<T>(p, a + (int64_t)(((uint64_t)(h ^ (h >> 15)) * (uint64_t)(b - a)) >> 32));
+    k0[i] = k;
+    k1[i] = k;
+  }
+  cluster.sync();                     // CTA 0 selects lo, CTA 1 hi, each in its own shared memory
+  if (crank > 1) return;
+  const uint32_t rank = crank == 0 ? p.lo_rank : p.hi_rank;
+  uint32_t key = crank == 0 ? 0u : 0xffffffffu;
+  if (rank != ~0u) {
+    uint32_t mx = 0;
+    for (int i = tid; i < kBracket; i += kThreads) mx = max(mx, s_keys[i]);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    key = select_cached(s_keys, kBracket, rank, mx, s_red, s_hist, s_sel);
+  }
+  if (tid == 0) {
+    if (crank == 0) p.st->lo = key;
+    else p.st->hi = key;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCollectThreads) collect_kernel(const __grid_constant__ OnePassParams p) {
+  __shared__ uint32_t s_buf[kBuffer];
+  __shared__ uint32_t s_fill, s_base;
+  __shared__ uint32_t s_cnt[3];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) s_fill = 0;
+  if (tid < 3) s_cnt[tid] = 0;
+  cx::pdl_wait();
+  cx::pdl_trigger();
+  const uint32_t lo = p.st->lo, hi = p.st->hi;
+  const T* g = reinterpret_cast<const T*>(p.g);
+  uint32_t above = 0, at_hi = 0, at_lo = 0;
+  __syncthreads();
+  const int64_t round = (int64_t)kCollectThreads * kCollectEach;
+  auto flush = [&]() {                // all threads
+    const uint32_t fill = s_fill;
+    if (tid == 0) s_base = atomicAdd(&p.st->found, fill);
+    __syncthreads();
+    for (uint32_t i = tid; i < fill; i += kCollectThreads)
+      if (s_base + i < p.cap) p.list[s_base + i] = s_buf[i];
+    __syncthreads();
+    if (tid == 0) s_fill = 0;
+    __syncthreads();
+  };
+  for (int64_t b = (int64_t)blockIdx.x * round; b < p.n; b += (int64_t)gridDim.x * round) {
+    float v[kCollectEach];
+    const bool whole = p.vec && b + round <= p.n;
+#pragma unroll
+    for (int k = 0; k < kCollectEach / 4; ++k) {
+      float* x = v + 4 * k;
+      const int64_t i = b + (int64_t)k * kCollectThreads * 4 + tid * 4;
+      float y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+      if (whole) {
+        if (p.r) cx::load4(p.r + i, y);
+        if (g) cx::load4(g + i, z);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (i + e < p.n && p.r) y[e] = p.r[i + e];
+          if (i + e < p.n && g) z[e] = cx::Elem<T>::to_f(g[i + e]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = g ? y[e] + z[e] : y[e];
+    }
+#pragma unroll
+    for (int k = 0; k < kCollectEach; ++k) {
+      const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
+      const bool in = whole || i < p.n;
+      const uint32_t key = __float_as_uint(fabsf(v[k]));
+      above += in && key > hi;
+      at_hi += in && key == hi;
+      at_lo += in && key == lo && lo != hi;
+      const bool cand = in && key > lo && key < hi;
+      const uint32_t who = __ballot_sync(0xffffffffu, cand);
+      if (who) {
+        uint32_t at = 0;
+        if (lane == __ffs(who) - 1) at = atomicAdd(&s_fill, (uint32_t)__popc(who));
+        at = __shfl_sync(0xffffffffu, at, __ffs(who) - 1);
+        if (cand) s_buf[at + __popc(who & ((1u << lane) - 1u))] = key;
+      }
+    }
+    __syncthreads();
+    if (s_fill > kBuffer - kCollectThreads * kCollectEach) flush();      // uniform: the next round might not fit
+    else __syncthreads();
+  }
+  if (above) atomicAdd(&s_cnt[0], above);
+  if (at_hi) atomicAdd(&s_cnt[1], at_hi);
+  if (at_lo) atomicAdd(&s_cnt[2], at_lo);
+  __syncthreads();
+  if (tid == 0) {
+    if (s_cnt[0]) atomicAdd(&p.st->above, s_cnt[0]);
+    if (s_cnt[1]) atomicAdd(&p.st->at_hi, s_cnt[1]);
+    if (s_cnt[2]) atomicAdd(&p.st->at_lo, s_cnt[2]);
+  }
+  if (s_fill) flush();
+}
+
+// the digit of a 2048-bin histogram that holds `rank`, walked from the top; block-wide, 1024 threads
+__device__ __forceinline__ uint32_t pick_bin(const uint32_t* hist, uint32_t& rank, uint32_t* s_warp, uint32_t* s_out) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const uint32_t a = hist[kBins - 1 - 2 * tid], b = hist[kBins - 2 - 2 * tid];
+  uint32_t incl = a + b;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) s_warp[w] = incl;
+  __syncthreads();
+  uint32_t before = incl - a - b;
+  for (int j = 0; j < w; ++j) before += s_warp[j];
+  if (rank >= before && rank < before + a) { s_out[0] = kBins - 1 - 2 * tid; s_out[1] = rank - before; }
+  else if (rank >= before + a && rank < before + a + b) { s_out[0] = kBins - 2 - 2 * tid; s_out[1] = rank - before - a; }
+  __syncthreads();
+  rank = s_out[1];
+  return s_out[0];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_constant__ OnePassParams p) {
+  namespace cg = cooperative_groups;
+  __shared__ uint32_t s_hist[kBins];
+  __shared__ uint32_t s_warp[kThreads / 32];
+  __shared__ uint32_t s_out[2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned crank = cluster.block_rank();
+  const int tid = threadIdx.x;
+  uint32_t* hist0 = cluster.map_shared_rank(s_hist, 0);
+  uint32_t* out0 = cluster.map_shared_rank(s_out, 0);
+  cx::pdl_wait();
+  cx::pdl_trigger();
+  const ExactState st = *p.st;
+  cluster.sync();                     // every CTA has read the state: the first one may clear it
+  if (crank == 0 && tid == 0) p.st->above = p.st->at_hi = p.st->at_lo = p.st->found = 0;
+  uint32_t rank = p.rank, base = 0, top = 0x7fffffffu;
+  bool list = false;
+  if (st.found <= p.cap && rank >= st.above) {
+    const uint32_t left = rank - st.above;
+    if (left < st.at_hi) { if (crank == 0 && tid == 0) *p.thr_out = __uint_as_float(st.hi); return; }
+    if (left - st.at_hi < st.found) {
+      list = true;
+      rank = left - st.at_hi;
+      base = st.lo + 1;
+      top = min(st.hi, 0x80000000u) - 1;
+    } else if (left - st.at_hi - st.found < st.at_lo) {
+      if (crank == 0 && tid == 0) *p.thr_out = __uint_as_float(st.lo);
+      return;
+    }
+  }
+  // radix select of key - base in [0, top - base], 11 bits at a time from the highest bit in use
+  const int bits = 32 - __clz((top - base) | 1u);
+  uint32_t prefix = 0, mask = 0;
+  const int64_t count = list ? (int64_t)st.found : p.n;
+  for (int shift = bits > 11 ? bits - 11 : 0;; shift = shift > 11 ? shift - 11 : 0) {
+    for (int i = tid; i < kBins; i += kThreads) s_hist[i] = 0;
+    cluster.sync();
+    const int64_t step = (int64_t)kCluster * kThreads;
+    for (int64_t i0 = (int64_t)crank * kThreads + tid; i0 < count; i0 += 4 * step) {
+      uint32_t k[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t i = i0 + u * step;
+        k[u] = i < count ? (list ? p.list[i] : key_at<T>(p, i)) - base : 0xffffffffu;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u * step < count && (k[u] & mask) == prefix) atomicAdd(&s_hist[(k[u] >> shift) & (kBins - 1)], 1u);
+    }
+    __syncthreads();
+    if (crank != 0)
+      for (int i = tid; i < kBins; i += kThreads) if (s_hist[i]) atomicAdd(&hist0[i], s_hist[i]);
+    cluster.sync();
+    if (crank == 0) pick_bin(s_hist, rank, s_warp, s_out);
+    cluster.sync();
+    prefix |= out0[0] << shift;
+    rank = out0[1];
+    mask = shift ? 0xffffffffu << shift : 0xffffffffu;
+    cluster.sync();
+    if (shift == 0) break;
+  }
+  if (crank == 0 && tid == 0) *p.thr_out = __uint_as_float(base + prefix);
+}
+
+template <typename T>
+int launch_one_pass(const OnePassParams& p, bool capturing, cudaStream_t s) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(kCluster, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = !capturing && cx_pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, bracket_kernel<T>, p);
+  if (e != cudaSuccess) return cx_set_error("bracket_kernel launch", (int)e);
+  const int64_t round = (int64_t)kCollectThreads * kCollectEach;
+  int grid = cx_sm_count() * 4;
+  if (grid > (p.n + round - 1) / round) grid = (int)((p.n + round - 1) / round);
+  cx_launch_pdl(collect_kernel<T>, grid, kCollectThreads, 0, s, p, capturing);
+  e = cudaLaunchKernelEx(&cfg, exact_finish_kernel<T>, p);
+  if (e != cudaSuccess) return cx_set_error("exact_finish_kernel launch", (int)e);
+  for (int k = 0; k < 3; ++k) cx_note_launch();
+  return cx_check_launch("exact selection kernels");
+}
+
+uint32_t candidate_cap(int64_t n) { return (uint32_t)(n / 16 > 65536 ? n / 16 : 65536); }
+
 template <typename T>
 int launch_exact(const ExactParams& base, cudaStream_t s) {
   int grid = cx_sm_count() * 6;
@@ -391,6 +670,10 @@ int launch_exact(const ExactParams& base, cudaStream_t s) {
 }  // namespace
 
 extern "C" int64_t cx_threshold_workspace_bytes(void) { return 4 * 256 * (int64_t)sizeof(uint32_t); }
+
+extern "C" int64_t cx_threshold_exact_bytes(int64_t n) {
+  return cx_threshold_workspace_bytes() + (int64_t)sizeof(ExactState) + 4 * (int64_t)candidate_cap(n);
+}
 
 // Host-side part of the rule, in the reference's float arithmetic.
 // sample count, stride and rank of the estimate (defined with the host back end)
@@ -472,6 +755,24 @@ int cx_threshold_topk_cuda(int gdtype, const void* g, const float* r, int64_t n,
   ThreshParams p;
   sampled_params(p, g, r, n, ratio, default_subsamples, subsample_factor, thr_out);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (exact_wanted(p, workspace, ws_bytes) && ws_bytes >= cx_threshold_exact_bytes(n)) {
+    OnePassParams q;
+    q.g = g; q.r = r; q.n = n; q.rank = (uint32_t)p.topk_pos; q.cap = candidate_cap(n); q.thr_out = thr_out;
+    q.st = reinterpret_cast<ExactState*>(reinterpret_cast<char*>(workspace) + cx_threshold_workspace_bytes());
+    q.list = reinterpret_cast<uint32_t*>(q.st + 1);
+    const double f = (double)p.topk_pos / (double)n, at = f * kBracket, slack = 4.0 * sqrt(at * (1.0 - f)) + 4.0;
+    q.hi_rank = at - slack < 0.0 ? ~0u : (uint32_t)(at - slack);
+    q.lo_rank = at + slack >= kBracket - 1 ? ~0u : (uint32_t)(at + slack + 1.0);
+    const size_t esz = gdtype == CX_F32 ? 4 : 2;
+    q.vec = (!r || (reinterpret_cast<uintptr_t>(r) & 15) == 0) && (!g || (reinterpret_cast<uintptr_t>(g) & (4 * esz - 1)) == 0);
+    const bool capturing = cx_seq_cell() != nullptr;
+    switch (gdtype) {
+      case CX_F32: return launch_one_pass<float>(q, capturing, s);
+      case CX_BF16: return launch_one_pass<__nv_bfloat16>(q, capturing, s);
+      case CX_F16: return launch_one_pass<__half>(q, capturing, s);
+      default: return cx_set_error("cx_threshold_topk: unsupported dtype on CUDA", 0);
+    }
+  }
   if (exact_wanted(p, workspace, ws_bytes)) {
     // exact selection over a vector that does not fit one CTA's shared memory: grid-wide passes
     ExactParams e;

@@ -188,6 +188,15 @@ class Compressor:
         self.thr_ws = env.scratch(self.thr_ws_bytes)
         self.stats = env.new_stats()
 
+    def threshold_ws(self, n: int, default_subsamples: int):
+        """(address, bytes) of the threshold kernels' scratch.  A selection over the whole vector gets
+        the larger one that saves it three passes, allocated on first use and kept."""
+        if default_subsamples > n and self.env.dev == _lib.DEV_CUDA:
+            need = int(self.env.lib.cx_threshold_exact_bytes(n))
+            if self.thr_ws_bytes < need:
+                self.thr_ws, self.thr_ws_bytes = self.env.scratch(need), need
+        return self.thr_ws.data_ptr(), self.thr_ws_bytes
+
     def set_threshold(self, value: float) -> None:
         if _recording(self.env):
             raise ComprexError("a constant threshold cannot be part of a recorded launch sequence")
@@ -201,12 +210,12 @@ class Compressor:
             op = _new_op(env, _lib.OPK_THRESHOLD, gd, n)
             op.g, op.r, op.thr, op.ratio = _ptr(g), _ptr(r), self.thr.data_ptr(), ratio
             op.default_subsamples, op.subsample_factor = int(default_subsamples), float(subsample_factor)
-            op.workspace, op.ws_bytes = self.thr_ws.data_ptr(), self.thr_ws_bytes
+            op.workspace, op.ws_bytes = self.threshold_ws(n, default_subsamples)
             env._rec.append(op)
             return
+        ws, ws_bytes = self.threshold_ws(n, default_subsamples)
         _lib.check(env.lib.cx_threshold_select(env.dev, gd, _ptr(g), _ptr(r), n, ratio, int(default_subsamples),
-                                               float(subsample_factor), self.thr.data_ptr(), self.thr_ws.data_ptr(),
-                                               self.thr_ws_bytes, _lib.stream_ptr(env.device)), "cx_threshold_select")
+                                               float(subsample_factor), self.thr.data_ptr(), ws, ws_bytes, _lib.stream_ptr(env.device)), "cx_threshold_select")
 
     def compress(self, g, r, n: int, cap: int, seq: int, targets: Targets) -> None:
         """r += g; emit |r| > thr into every target; zero what was emitted."""
@@ -235,7 +244,7 @@ class Compressor:
         thr.r = cmp_.r = r.data_ptr()
         thr.thr = cmp_.thr = self.thr.data_ptr()
         thr.ratio, thr.default_subsamples, thr.subsample_factor = ratio, int(default_subsamples), float(subsample_factor)
-        thr.workspace, thr.ws_bytes = self.thr_ws.data_ptr(), self.thr_ws_bytes
+        thr.workspace, thr.ws_bytes = self.threshold_ws(n, default_subsamples)
         cmp_.cap, cmp_.src_rank, cmp_.stats, cmp_.tg = cap, env.rank, self.stats.dev_ptr, targets
         cmp_.workspace, cmp_.ws_bytes = self.workspace.data_ptr(), self.ws_bytes
         return [thr, cmp_]

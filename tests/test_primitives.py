@@ -93,6 +93,43 @@ def test_exact_topk_threshold(device, n, ratio):
     env.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("data", ["normal", "columns", "ties", "few_values", "zeros", "constant", "nan"])
+@pytest.mark.parametrize("n,dtype", [(11009, torch.float32), (65536, torch.bfloat16), (1000003, torch.float32),
+                                     (1 << 21, torch.float16)])
+def test_exact_topk_one_pass(n, dtype, data):
+    """The one-pass exact selection (bracket from a sample, candidates, finish) equals a sort for all
+    ranks, where the bracket holds, where its ends are ties, and where the candidates do not fit and
+    it selects over the whole vector; the scratch is left clean."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = torch.randn(n, device="cuda", generator=gen)
+    if data == "columns":                      # every 1024th element is large
+        g[::1024] *= 1000.0
+    elif data == "ties":
+        g = g.mul(2.0).round()
+    elif data == "few_values":
+        g = torch.randint(0, 4, (n,), device="cuda", generator=gen).float() * 0.125 + 1.0
+    elif data == "zeros":
+        g[torch.rand(n, device="cuda", generator=gen) < 0.999] = 0.0
+    elif data == "constant":
+        g.fill_(-3.0)
+    elif data == "nan":
+        g[5] = float("nan")
+    g = g.to(dtype)
+    r = torch.zeros(n, device="cuda") if data == "few_values" else torch.full((n,), 0.25, device="cuda")
+    keys = (r + g.float()).abs().view(torch.int32).sort(descending=True).values
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    comp = P.Compressor(env, n)
+    for ratio in (0.0005, 0.01, 0.1, 0.5, 1.0):
+        k = int(torch.ceil(torch.tensor(float(n)) * torch.tensor(ratio)).item()) - 1
+        if k <= 0:
+            continue
+        for _ in range(2):
+            comp.threshold_topk(g, r, n, ratio, cx.ThresholdTopK.EXACT)
+            assert int(comp.thr.view(torch.int32).item()) == int(keys[k].item()), (ratio, k)
+    env.close()
+
+
 def test_threshold_reference_vector(device):
     """test/threshold.cpp:58-85: 100 ints, top 10 % -> threshold 90, 10 elements pass with >=."""
     from helpers import alt_ramp
