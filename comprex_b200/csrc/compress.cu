@@ -82,6 +82,7 @@ struct CompressParams {
   uint32_t nsub;
   uint32_t nregions;     // power of two; sub-tile s reserves in region s % nregions
   uint32_t region_size;  // cap / nregions pairs each
+  uint32_t early;        // the first sub-tile may be loaded before the kernel in front has finished
   uint32_t vec;          // g and r are aligned for 16-byte (8-byte for 16-bit g) accesses
   uint64_t seq;
   const uint64_t* seq_cell;  // non-NULL inside a captured graph: the sequence number lives there
@@ -107,62 +108,64 @@ struct FoldCompressParams {
 // One aligned, complete sub-tile, one warp, one pass: lane L holds elements {c*128 + 4L + e} in
 // registers from the loads to the write-back of the residual.
 // gl / rl: where this sub-tile's gradient and residual are read (global memory, or the copy of the
-// sub-tile that the copy engine put into shared memory); rs: the residual's sub-tile in global
-// memory, where the new residual goes.
-// up, mu, coef: folded inputs (IN != kPlain), the sub-tile's momentum and factors.
-template <typename T, bool HAS_G, bool HAS_R, bool MC, Input IN = kPlain>
-__device__ __forceinline__ void compress_subtile_regs(const CompressParams& p, const uint32_t sub,
-                                                 const int lane, const float thr,
-                                                 const T* __restrict__ gl, const float* __restrict__ rl,
-                                                 float* __restrict__ rs, CxPair* stage,
-                                                 float* __restrict__ up = nullptr, const float mu = 0.f,
-                                                 const float coef = 0.f) {
-  const int64_t sub_base = (int64_t)sub * CX_SUBTILE;
-  const T* gp = gl + lane * 4;
-  const float* rp = rl + lane * 4;
-  float* wp = rs + lane * 4;
-
-  // ---- load, add -------------------------------------------------------------
-  float v[kChunks][4];
+// sub-tile that the copy engine put into shared memory).
+template <typename T, bool HAS_G, bool HAS_R>
+__device__ __forceinline__ void load_subtile(const T* __restrict__ gl, const float* __restrict__ rl, const int lane,
+                                             float (&v)[kChunks][4]) {
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[c][e] = 0.f;
-    if (HAS_R) cx::load4(rp + c * 128, v[c]);
+    if (HAS_R) cx::load4(rl + lane * 4 + c * 128, v[c]);
   }
-  if (IN == kPlain && HAS_G) {
+  if (HAS_G) {
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       float b[4];
-      cx::load4(gp + c * 128, b);
+      cx::load4(gl + lane * 4 + c * 128, b);
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[c][e] = v[c][e] + b[e];
     }
   }
-  if (IN != kPlain) {
-    // all loads of a group are issued before its first store: the compiler must not move them across
-    constexpr int kGroup = IN == kFoldMom && sizeof(T) == 4 ? kChunks / 2 : kChunks;
+}
+
+// The same for a folded input: up, mu, coef are the sub-tile's momentum and factors.
+template <typename T, Input IN>
+__device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, const float* __restrict__ rl, float* __restrict__ up,
+                                                  const float mu, const float coef, const int lane, float (&v)[kChunks][4]) {
 #pragma unroll
-    for (int c0 = 0; c0 < kChunks; c0 += kGroup) {
-      typename cx::Raw4<T>::type x[kGroup];
-      float y[kGroup][4];
+  for (int c = 0; c < kChunks; ++c) cx::load4(rl + lane * 4 + c * 128, v[c]);
+  // all loads of a group are issued before its first store: the compiler must not move them across
+  constexpr int kGroup = IN == kFoldMom && sizeof(T) == 4 ? kChunks / 2 : kChunks;
 #pragma unroll
-      for (int c = 0; c < kGroup; ++c) {
-        x[c] = cx::Raw4<T>::load(gp + (c0 + c) * 128);
-        if (IN == kFoldMom) cx::load4(up + lane * 4 + (c0 + c) * 128, y[c]);
-      }
+  for (int c0 = 0; c0 < kChunks; c0 += kGroup) {
+    typename cx::Raw4<T>::type x[kGroup];
+    float y[kGroup][4];
 #pragma unroll
-      for (int c = 0; c < kGroup; ++c) {
-        float t[4];
-        cx::Raw4<T>::to_f(x[c], t);
+    for (int c = 0; c < kGroup; ++c) {
+      x[c] = cx::Raw4<T>::load(gl + lane * 4 + (c0 + c) * 128);
+      if (IN == kFoldMom) cx::load4(up + lane * 4 + (c0 + c) * 128, y[c]);
+    }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) t[e] = mu * (IN == kFoldMom ? y[c][e] : 0.f) + coef * t[e];
-        if (IN != kFold) cx::store4(up + lane * 4 + (c0 + c) * 128, t);
+    for (int c = 0; c < kGroup; ++c) {
+      float t[4];
+      cx::Raw4<T>::to_f(x[c], t);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[c0 + c][e] = v[c0 + c][e] + t[e];
-      }
+      for (int e = 0; e < 4; ++e) t[e] = mu * (IN == kFoldMom ? y[c][e] : 0.f) + coef * t[e];
+      if (IN != kFold) cx::store4(up + lane * 4 + (c0 + c) * 128, t);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[c0 + c][e] = v[c0 + c][e] + t[e];
     }
   }
+}
+
+// Selection, compaction and write-back of a loaded sub-tile.  rs: the residual's sub-tile in global
+// memory, where the new residual goes.
+template <bool HAS_G, bool HAS_R, bool MC>
+__device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint32_t sub, const int lane, const float thr,
+                                             float* __restrict__ rs, CxPair* stage, float (&v)[kChunks][4]) {
+  const int64_t sub_base = (int64_t)sub * CX_SUBTILE;
+  float* wp = rs + lane * 4;
 
   // ---- classify: bit c*4+e of mask, strict '>' like the reference --------------
   uint32_t mask = 0;
@@ -434,16 +437,23 @@ compress_kernel(const __grid_constant__ CompressParams p) {
   const T* __restrict__ g = reinterpret_cast<const T*>(p.g);
   float* __restrict__ r = p.r;
   CX_TRACE(0);
-  // Launched with programmatic stream serialization, this grid may be resident while the
-  // threshold kernel in front of it still runs: pull the warp's first sub-tile towards L2, then
+  const uint32_t nfull = p.vec ? (uint32_t)(p.n / CX_SUBTILE) : 0u;  // sub-tiles on the fast path
+  // Launched with programmatic stream serialization, this grid may be resident while the kernel in
+  // front of it still runs.  Behind the threshold estimate, which only reads, the warp's first
+  // sub-tile can be loaded right away (1 us off a small exchange); otherwise pull it towards L2, then
   // wait for that kernel to finish before reading its result or touching the residual.
+  float v[kChunks][4];
+  bool loaded = false;
   {
-    const uint32_t sub0 = blockIdx.x * kWarps + (tid >> 5);
-    if (sub0 < p.nsub && (tid & 31) < 2 * kChunks) {
-      const int c = (tid & 31) >> 1;
+    const uint32_t sub0 = blockIdx.x * kWarps + warp;
+    if (p.early && sub0 < nfull) {
+      load_subtile<T, HAS_G, HAS_R>(g + (int64_t)sub0 * CX_SUBTILE, r + (int64_t)sub0 * CX_SUBTILE, lane, v);
+      loaded = true;
+    } else if (sub0 < p.nsub && lane < 2 * kChunks) {
+      const int c = lane >> 1;
       const int64_t e0 = (int64_t)sub0 * CX_SUBTILE + c * 128;
       if (e0 < p.n) {
-        const void* a = (tid & 1) ? (HAS_R ? (const void*)(r + e0) : nullptr) : (HAS_G ? (const void*)(g + e0) : nullptr);
+        const void* a = (lane & 1) ? (HAS_R ? (const void*)(r + e0) : nullptr) : (HAS_G ? (const void*)(g + e0) : nullptr);
         if (a) asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
       }
     }
@@ -453,7 +463,6 @@ compress_kernel(const __grid_constant__ CompressParams p) {
   CX_TRACE(1);
   CxPair* stage = s_stage[warp];
   const uint32_t nwarps = gridDim.x * kWarps;
-  const uint32_t nfull = p.vec ? (uint32_t)(p.n / CX_SUBTILE) : 0u;  // sub-tiles on the fast path
 
   for (uint32_t sub = blockIdx.x * kWarps + warp; sub < p.nsub; sub += nwarps) {
 #if CX_COMPRESS_PREFETCH
@@ -468,7 +477,9 @@ compress_kernel(const __grid_constant__ CompressParams p) {
 #endif
     if (sub < nfull) {
       const int64_t off = (int64_t)sub * CX_SUBTILE;
-      compress_subtile_regs<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g + off, r + off, r + off, stage);
+      if (!loaded) load_subtile<T, HAS_G, HAS_R>(g + off, r + off, lane, v);
+      loaded = false;
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage, v);
     }
     else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r);
   }
@@ -503,10 +514,11 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
     const int64_t off = (int64_t)sub * CX_SUBTILE;
     const T* g = nullptr;
     float coef = 0.f;
-    if (sub < nfull && cx::fold_whole<T>(q.f, sub, g, coef))
-      compress_subtile_regs<T, true, true, MC, IN>(p, sub, lane, thr, g, r + off, r + off, s_stage[warp],
-                                                   IN == kFold ? nullptr : q.f.u + off, q.f.mu, coef);
-    else
+    if (sub < nfull && cx::fold_whole<T>(q.f, sub, g, coef)) {
+      float v[kChunks][4];
+      load_fold_subtile<T, IN>(g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, coef, lane, v);
+      emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v);
+    } else
       compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, &q.f);
   }
   compress_finish(p, tid, thr, false, s_last, s_found, s_nnz);
@@ -596,9 +608,9 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
       }
       ++consumed;
       const unsigned char* src = mine + s * kStageB;
-      compress_subtile_regs<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, reinterpret_cast<const T*>(src + kRB),
-                                                 reinterpret_cast<const float*>(src),
-                                                 r + (size_t)sub * CX_SUBTILE, stage);
+      float v[kChunks][4];
+      load_subtile<T, HAS_G, HAS_R>(reinterpret_cast<const T*>(src + kRB), reinterpret_cast<const float*>(src), lane, v);
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + (size_t)sub * CX_SUBTILE, stage, v);
       // this stage is handed back to the copy engine by a later issue()
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -721,6 +733,7 @@ void fill_params(CompressParams& p, const void* g, float* r, int64_t n, const fl
   p.region_size = cap / p.nregions;
   p.seq = seq;
   p.seq_cell = cx_seq_cell();
+  p.early = (cx_chain_bits() & CX_BEHIND_THRESHOLD) ? 1u : 0u;
   p.ctr = reinterpret_cast<CxWorkCounters*>(workspace);
   p.stats = stats; p.src_rank = src_rank;
   p.tg = *tg;

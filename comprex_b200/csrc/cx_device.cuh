@@ -37,13 +37,13 @@ __device__ __forceinline__ bool wait_seq(const uint64_t* seq_ptr, uint64_t want,
                                          uint64_t timeout_ns) {
   if (ld_acquire_sys(seq_ptr) >= want) return true;
   const uint64_t t0 = globaltimer_ns();
-  unsigned backoff = 32;
+  unsigned backoff = 20;
   // the iteration cap bounds the loop even if the timer misbehaves
   for (uint64_t it = 0; it < (1ull << 34); ++it) {
     if (ld_acquire_sys(seq_ptr) >= want) return true;
     if ((it & 15) == 15 && globaltimer_ns() - t0 > timeout_ns) return false;
     __nanosleep(backoff);
-    if (backoff < 1024) backoff <<= 1;
+    if (backoff < 160) backoff <<= 1;      // a waiting kernel is late by half a sleep on average
   }
   return false;
 }
@@ -245,6 +245,8 @@ bool cx_pdl_enabled();   // COMPREX_PDL != 0 (read once)
 // ramp of the next then share the GPU: 26 compress kernels of 13 M elements 905 us one by one.
 #define CX_CHAINED 1u      /* this kernel is chained to the one in front */
 #define CX_CHAIN_NEXT 2u   /* the kernel behind is chained to this one */
+#define CX_BEHIND_THRESHOLD 4u  /* the kernel in front is the threshold estimate of the same vector: it only reads,
+                                   and what it waited for is complete once this kernel is resident */
 uint32_t cx_chain_bits();
 
 template <typename K, typename P>

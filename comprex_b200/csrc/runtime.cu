@@ -21,6 +21,7 @@
 
 #define CX_CHAINED 1u      /* as in cx_device.cuh */
 #define CX_CHAIN_NEXT 2u
+#define CX_BEHIND_THRESHOLD 4u
 
 // ---- forward declarations of the two back ends --------------------------------
 int cx_threshold_topk_cuda(int, const void*, const float*, int64_t, float, int, float, float*, void*, int64_t, void*);
@@ -339,7 +340,9 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
     auto chained = [&](int k) {
       return k > 0 && k < count && ops[k].chain && ops[k].kind == ops[k - 1].kind && ops[k].lane == ops[k - 1].lane;
     };
-    g_chain_bits = (chained(i) ? CX_CHAINED : 0u) | (chained(i + 1) ? CX_CHAIN_NEXT : 0u);
+    const bool behind = i > 0 && ops[i].kind == CX_OPK_COMPRESS && ops[i - 1].kind == CX_OPK_THRESHOLD &&
+                        ops[i - 1].lane == ops[i].lane && ops[i - 1].dev == CX_DEV_CUDA;
+    g_chain_bits = (chained(i) ? CX_CHAINED : 0u) | (chained(i + 1) ? CX_CHAIN_NEXT : 0u) | (behind ? CX_BEHIND_THRESHOLD : 0u);
     const int rc = run_one(ops[i], seq, on);
     g_chain_bits = 0;
     return rc ? (rc > 0 ? -rc : rc) : 1;

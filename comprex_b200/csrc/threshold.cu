@@ -110,22 +110,47 @@ __device__ __forceinline__ uint32_t warp_rank(uint32_t key, int count, int lane,
   return __shfl_sync(0xffffffffu, key, __ffs(who) - 1);
 }
 
-// The key of rank `rank` among s_keys[0, s), for a sample that fits the block's shared memory.
-//  * rank < 32: the (rank + 1)-th largest of the 32 warps' maxima is a lower bound with at least
-//    rank + 1 keys at or above it; a handful of keys survive it, and one warp ranks those.
-//  * otherwise, up to one key per thread: bisection over the bits, one block-wide count per bit.
-//  * what is left (a large sample and a large rank): four radix passes of 8 bits.
-// 1000 samples, rank 9: 0.5 us where the radix passes took 3 us.
-__device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint32_t rank, uint32_t mymax, uint32_t* s_red,
+// One key per thread (threads from `count` on hold none): the largest t with more than `rank` keys at
+// or above it, which is the key of that rank.  One block-wide count per bit.
+__device__ __forceinline__ uint32_t block_rank(uint32_t key, int count, uint32_t rank) {
+  uint32_t t = 0;
+  const bool have = (int)threadIdx.x < count;
+  for (int bit = 30; bit >= 0; --bit) {
+    const uint32_t c = t | (1u << bit);
+    if ((uint32_t)__syncthreads_count(have && key >= c) > rank) t = c;
+  }
+  return t;
+}
+
+// The key of rank `rank` among s_keys[0, s), for a sample that fits the block's shared memory (valid
+// in thread 0).
+//  * A lower bound with at least rank + 1 keys at or above it leaves few keys to rank.  Up to rank 31
+//    it is the (rank + 1)-th largest of the 32 warps' maxima, and one warp finds and ranks; up to
+//    rank 767 it is that of the threads' maxima.
+//  * Up to one key per thread: bisection over the bits, no bound needed.
+//  * What is left (a large sample and a large rank, or many ties): four radix passes of 8 bits.
+// 1000 samples, rank 9: 0.5 us where the radix passes took 3 us; 8192 samples, rank 120: 3 us for 8.
+__device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint32_t rank, uint32_t* s_red,
                                                   uint32_t* s_hist, uint32_t* s_sel) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  uint32_t key = 0, count = (uint32_t)s;
-  bool one_each = s <= kThreads;
-  if (rank < 32) {
-    if (lane == 0) s_red[w] = mymax;
+  if (rank >= 32 && s <= kThreads) return block_rank(tid < s ? s_keys[tid] : 0u, s, rank);
+  if (rank < 768) {
+    uint32_t mymax = 0, bound;
+    for (int i = tid; i < s; i += kThreads) mymax = max(mymax, s_keys[i]);
     if (tid == 0) s_sel[0] = 0;
-    __syncthreads();
-    const uint32_t bound = warp_rank(s_red[lane], 32, lane, rank);   // every warp for itself
+    if (rank < 32) {
+      const uint32_t wm = __reduce_max_sync(0xffffffffu, mymax);
+      if (lane == 0) s_red[w] = wm;
+      __syncthreads();
+      if (w == 0) {
+        const uint32_t b0 = warp_rank(s_red[lane], 32, lane, rank);
+        if (lane == 0) s_sel[1] = b0;
+      }
+      __syncthreads();
+      bound = s_sel[1];
+    } else {
+      bound = block_rank(mymax, kThreads, rank);
+    }
     for (int i = tid; i < s; i += kThreads) {
       const uint32_t k = s_keys[i];
       if (k >= bound) {
@@ -135,24 +160,8 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
     }
     __syncthreads();
     const uint32_t left = s_sel[0];
-    if (left <= 32) return warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank);
-    if (left <= kThreads) {
-      one_each = true;
-      count = left;
-      key = tid < (int)left ? s_hist[tid] : 0u;
-    }
-  } else if (one_each) {
-    key = tid < s ? s_keys[tid] : 0u;
-  }
-  if (one_each) {
-    // largest t with more than `rank` keys at or above it
-    uint32_t t = 0;
-    const bool have = tid < (int)count;
-    for (int bit = 30; bit >= 0; --bit) {
-      const uint32_t c = t | (1u << bit);
-      if ((uint32_t)__syncthreads_count(have && key >= c) > rank) t = c;
-    }
-    return t;
+    if (left <= 32) return w == 0 ? warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
+    if (left <= kThreads) return block_rank(tid < (int)left ? s_hist[tid] : 0u, (int)left, rank);
   }
   uint32_t prefix = 0, prefmask = 0;
   const int s_round = (s + kThreads - 1) / kThreads * kThreads;
@@ -182,9 +191,6 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
 template <typename T, bool FOLD, int NV>
 __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_constant__ ThreshBatch<NV> batch) {
   namespace cg = cooperative_groups;
-  // the compress kernel queued behind this one may start its prologue now; it waits (for this
-  // grid to finish) before it reads the threshold or writes the residual
-  cx::pdl_trigger();
   __shared__ uint32_t s_keys[kSmemKeys];
   __shared__ uint32_t s_hist[kThreads];
   __shared__ uint32_t s_sel[2];
@@ -200,6 +206,9 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   const bool cached = s <= kSmemKeys;
   uint32_t* keys0 = ncta > 1 ? cluster.map_shared_rank(s_keys, 0) : s_keys;
   cx::pdl_wait();     // resident early: what the kernel in front wrote may be read from here on
+  // the compress kernel queued behind this one may start now: it loads what both only read, and waits
+  // for this grid to finish before it reads the threshold or writes the residual
+  cx::pdl_trigger();
 
   // pass 0: gather the sample (and its maximum, for the sentinel case); CTA c of a cluster
   // takes the samples [c, c+1) * s / ncta
@@ -242,11 +251,9 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
       }
       return;
     }
-    mx = 0;                      // the selection wants the maximum of this thread's keys in its own copy
-    for (int i = tid; i < s; i += kThreads) mx = max(mx, s_keys[i]);
   }
-  mx = __reduce_max_sync(0xffffffffu, mx);
   if (p.topk_pos <= 0) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) s_red[tid >> 5] = mx;
     __syncthreads();
     if (tid == 0) {
@@ -258,7 +265,7 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   }
   if (cached) {
     __syncthreads();
-    const uint32_t key = select_cached(s_keys, s, (uint32_t)p.topk_pos, mx, s_red, s_hist, s_sel);
+    const uint32_t key = select_cached(s_keys, s, (uint32_t)p.topk_pos, s_red, s_hist, s_sel);
     if (tid == 0) *p.thr_out = __uint_as_float(key);
     return;
   }
@@ -447,10 +454,7 @@ __global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant
   const uint32_t rank = crank == 0 ? p.lo_rank : p.hi_rank;
   uint32_t key = crank == 0 ? 0u : 0xffffffffu;
   if (rank != ~0u) {
-    uint32_t mx = 0;
-    for (int i = tid; i < kBracket; i += kThreads) mx = max(mx, s_keys[i]);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    key = select_cached(s_keys, kBracket, rank, mx, s_red, s_hist, s_sel);
+    key = select_cached(s_keys, kBracket, rank, s_red, s_hist, s_sel);
   }
   if (tid == 0) {
     if (crank == 0) p.st->lo = key;
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kCollectThreads) collect_kernel(const __grid_constant__ OnePassParams p) {
+__global__ void __launch_bounds__(kCollectThreads, 4) collect_kernel(const __grid_constant__ OnePassParams p) {
   __shared__ uint32_t s_buf[kBuffer];
   __shared__ uint32_t s_fill, s_base;
   __shared__ uint32_t s_cnt[3];
@@ -486,33 +490,44 @@ __global__ void __launch_bounds__(kCollectThreads) collect_kernel(const __grid_c
   for (int64_t b = (int64_t)blockIdx.x * round; b < p.n; b += (int64_t)gridDim.x * round) {
     float v[kCollectEach];
     const bool whole = p.vec && b + round <= p.n;
+    if (whole) {
+      constexpr int kQ = kCollectEach / 4;
+      float y[kQ][4];
+      typename cx::Raw4<T>::type z[kQ];
 #pragma unroll
-    for (int k = 0; k < kCollectEach / 4; ++k) {
-      float* x = v + 4 * k;
-      const int64_t i = b + (int64_t)k * kCollectThreads * 4 + tid * 4;
-      float y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
-      if (whole) {
-        if (p.r) cx::load4(p.r + i, y);
-        if (g) cx::load4(g + i, z);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (i + e < p.n && p.r) y[e] = p.r[i + e];
-          if (i + e < p.n && g) z[e] = cx::Elem<T>::to_f(g[i + e]);
-        }
+      for (int k = 0; k < kQ; ++k) {
+        const int64_t i = b + (int64_t)k * kCollectThreads * 4 + tid * 4;
+        if (p.r) cx::load4(p.r + i, y[k]);
+        if (g) z[k] = cx::Raw4<T>::load(g + i);
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) x[e] = g ? y[e] + z[e] : y[e];
+      for (int k = 0; k < kQ; ++k) {
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
+        if (g) cx::Raw4<T>::to_f(z[k], t);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[4 * k + e] = p.r ? (g ? y[k][e] + t[e] : y[k][e]) : t[e];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kCollectEach; ++k) {
+        const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
+        v[k] = 0.f;
+        if (i < p.n) {
+          if (p.r) v[k] = p.r[i];
+          if (g) v[k] = v[k] + cx::Elem<T>::to_f(g[i]);
+        }
+      }
     }
 #pragma unroll
     for (int k = 0; k < kCollectEach; ++k) {
       const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
-      const bool in = whole || i < p.n;
       const uint32_t key = __float_as_uint(fabsf(v[k]));
-      above += in && key > hi;
-      at_hi += in && key == hi;
-      at_lo += in && key == lo && lo != hi;
-      const bool cand = in && key > lo && key < hi;
+      const bool near = (whole || i < p.n) && key >= lo;       // few are
+      if (!__any_sync(0xffffffffu, near)) continue;
+      above += near && key > hi;
+      at_hi += near && key == hi;
+      at_lo += near && key == lo && lo != hi;
+      const bool cand = near && key > lo && key < hi;
       const uint32_t who = __ballot_sync(0xffffffffu, cand);
       if (who) {
         uint32_t at = 0;
@@ -561,18 +576,18 @@ __device__ __forceinline__ uint32_t pick_bin(const uint32_t* hist, uint32_t& ran
 template <typename T>
 __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_constant__ OnePassParams p) {
   namespace cg = cooperative_groups;
-  __shared__ uint32_t s_hist[kBins];
+  __shared__ uint32_t s_hists[3][kBins];     // one per radix pass
   __shared__ uint32_t s_warp[kThreads / 32];
   __shared__ uint32_t s_out[2];
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned crank = cluster.block_rank();
   const int tid = threadIdx.x;
-  uint32_t* hist0 = cluster.map_shared_rank(s_hist, 0);
+  for (int i = tid; i < 3 * kBins; i += kThreads) s_hists[0][i] = 0;
   uint32_t* out0 = cluster.map_shared_rank(s_out, 0);
   cx::pdl_wait();
   cx::pdl_trigger();
   const ExactState st = *p.st;
-  cluster.sync();                     // every CTA has read the state: the first one may clear it
+  cluster.sync();                     // every CTA has read the state and cleared its histograms
   if (crank == 0 && tid == 0) p.st->above = p.st->at_hi = p.st->at_lo = p.st->found = 0;
   uint32_t rank = p.rank, base = 0, top = 0x7fffffffu;
   bool list = false;
@@ -593,9 +608,10 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
   const int bits = 32 - __clz((top - base) | 1u);
   uint32_t prefix = 0, mask = 0;
   const int64_t count = list ? (int64_t)st.found : p.n;
-  for (int shift = bits > 11 ? bits - 11 : 0;; shift = shift > 11 ? shift - 11 : 0) {
-    for (int i = tid; i < kBins; i += kThreads) s_hist[i] = 0;
-    cluster.sync();
+  int pass = 0;
+  for (int shift = bits > 11 ? bits - 11 : 0;; shift = shift > 11 ? shift - 11 : 0, ++pass) {
+    uint32_t* s_hist = s_hists[pass];
+    uint32_t* hist0 = cluster.map_shared_rank(s_hist, 0);
     const int64_t step = (int64_t)kCluster * kThreads;
     for (int64_t i0 = (int64_t)crank * kThreads + tid; i0 < count; i0 += 4 * step) {
       uint32_t k[4];
@@ -616,11 +632,11 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
     cluster.sync();
     prefix |= out0[0] << shift;
     rank = out0[1];
-    mask = shift ? 0xffffffffu << shift : 0xffffffffu;
-    cluster.sync();
-    if (shift == 0) break;
+    mask = 0xffffffffu << shift;
+    if (shift == 0) break;            // (the next pass writes s_out behind its own cluster barrier)
   }
   if (crank == 0 && tid == 0) *p.thr_out = __uint_as_float(base + prefix);
+  cluster.sync();                     // the first CTA's shared memory is read until here
 }
 
 template <typename T>
