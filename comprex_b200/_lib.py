@@ -68,7 +68,8 @@ OPK_THRESHOLD, OPK_COMPRESS, OPK_APPLY, OPK_DENSE_SEND, OPK_DENSE_REDUCE, OPK_UP
 class Fold(C.Structure):
     """A vector folded from gradient tensors (CxFold in csrc/cx_common.h)."""
     _fields_ = [("seg_ptr", C.c_void_p), ("seg_off", C.c_void_p), ("seg_end", C.c_void_p), ("coef", C.c_void_p),
-                ("sub_seg", C.c_void_p), ("u", C.c_void_p), ("base", C.c_int64), ("nseg", C.c_int32), ("mu", C.c_float)]
+                ("sub_seg", C.c_void_p), ("border", C.c_void_p), ("u", C.c_void_p), ("base", C.c_int64), ("nseg", C.c_int32),
+                ("nborder", C.c_int32), ("mu", C.c_float), ("pad", C.c_int32)]
 
 
 class Op(C.Structure):

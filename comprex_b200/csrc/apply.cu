@@ -612,53 +612,87 @@ struct FoldUpdateParams {
   CxApplyArgs a;
   int64_t n;
   uint32_t nsub;
+  uint32_t nborder_ctas;
 };
 
 // KEEP: 0 nothing of the folded vector is kept, 1 it is stored as the momentum, 2 read and stored
 template <int OP, typename TO, typename T, int KEEP>
-__global__ void __launch_bounds__(kThreads, OP == CX_OP_ADAMW ? 4 : 5) fold_update_kernel(const __grid_constant__ FoldUpdateParams q) {
-  cx::pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const uint32_t nwarps = gridDim.x * kWarps;
-  const uint32_t nfull = (uint32_t)(q.n / CX_SUBTILE);
-  for (uint32_t sub = blockIdx.x * kWarps + (threadIdx.x >> 5); sub < q.nsub; sub += nwarps) {
-    const int64_t lo = (int64_t)sub * CX_SUBTILE;
-    const T* g = nullptr;
-    float coef = 0.f;
-    if (sub < nfull && cx::fold_whole<T>(q.f, sub, g, coef)) {
-#pragma unroll 2
-      for (int c = 0; c < CX_SUBTILE / 128; ++c) {
-        const int e0 = c * 128 + lane * 4;
-        float x[4], y[4] = {0.f, 0.f, 0.f, 0.f};
-        cx::load4(g + e0, x);
-        if (KEEP == 2) cx::load4(q.f.u + lo + e0, y);
+__device__ __forceinline__ void fold_update_border(const FoldUpdateParams& q, uint32_t sub, int lane) {
+  const int64_t lo = (int64_t)sub * CX_SUBTILE;
+  const cx::FoldBlock<T> blk = cx::fold_blocks<T>(q.f, sub, lane);
+  constexpr int kGroup = 4;      // loads in flight: none of them moves across a store
+#pragma unroll 1
+  for (int j0 = 0; j0 < CX_SUBTILE / 32; j0 += kGroup) {
+    float x[kGroup], y[kGroup], w[kGroup], m[kGroup], v[kGroup];
+    uint32_t in = 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = q.f.mu * y[e] + coef * x[e];
-        if (KEEP) cx::store4(q.f.u + lo + e0, y);
-        update4<OP, TO>(q.a, q.n, lo + e0, y, true);
-      }
-    } else {
-      const cx::FoldBlock<T> blk = cx::fold_blocks<T>(q.f, sub, lane);
-      constexpr int kGroup = 4;      // loads in flight: none of them moves across a store
-      for (int j0 = 0; j0 < CX_SUBTILE / 32; j0 += kGroup) {
-        float x[kGroup], y[kGroup], c[kGroup], w[kGroup], m[kGroup], v[kGroup];
-        bool in[kGroup];
-#pragma unroll
-        for (int j = 0; j < kGroup; ++j) {
-          const int64_t i = lo + 32 * (j0 + j) + lane;
-          in[j] = cx::fold_element<T>(blk, j0 + j, lane, x[j], c[j]);
-          y[j] = KEEP == 2 && in[j] ? q.f.u[i] : 0.f;
-          load_state1<OP>(q.a, i, i < q.n, w[j], m[j], v[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < kGroup; ++j) {
-          const int64_t i = lo + 32 * (j0 + j) + lane;
-          const float t = in[j] ? q.f.mu * y[j] + c[j] * x[j] : 0.f;
-          if (KEEP && in[j]) q.f.u[i] = t;
-          if (i < q.n) update1<OP, TO>(q.a, i, t, w[j], m[j], v[j]);
-        }
-      }
+    for (int j = 0; j < kGroup; ++j) {
+      const int64_t i = lo + 32 * (j0 + j) + lane;
+      const bool t = cx::fold_element<T>(blk, j0 + j, lane, x[j]);
+      in |= (t ? 1u : 0u) << j;
+      y[j] = KEEP == 2 && t ? q.f.u[i] : 0.f;
+      load_state1<OP>(q.a, i, i < q.n, w[j], m[j], v[j]);
     }
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+      const int64_t i = lo + 32 * (j0 + j) + lane;
+      const float c = __shfl_sync(0xffffffffu, blk.coef, (j0 + j) >> 1);
+      const float t = (in >> j) & 1u ? q.f.mu * y[j] + c * x[j] : 0.f;
+      if (KEEP && ((in >> j) & 1u)) q.f.u[i] = t;
+      if (i < q.n) update1<OP, TO>(q.a, i, t, w[j], m[j], v[j]);
+    }
+  }
+}
+
+template <int OP, typename TO, typename T, int KEEP>
+__global__ void __launch_bounds__(kThreads, 4) fold_update_kernel(const __grid_constant__ FoldUpdateParams q) {
+  cx::pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x < q.nborder_ctas) {
+    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kWarps)
+      fold_update_border<OP, TO, T, KEEP>(q, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane);
+    return;
+  }
+  const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kWarps;
+  uint32_t sub = (blockIdx.x - q.nborder_ctas) * kWarps + warp;
+  cx::FoldWhole<T> cur = {nullptr, 0.f, 0};
+  if (sub < q.nsub) cur = cx::fold_whole<T>(q.f, sub);
+  while (sub < q.nsub) {
+    const int64_t lo = (int64_t)sub * CX_SUBTILE;
+    const uint32_t next = sub + nwarps;
+    cx::FoldWhole<T> ahead = {nullptr, 0.f, 0};
+    if (next < q.nsub) ahead = cx::fold_whole<T>(q.f, next);
+    if (cur.kind == 2) {
+      constexpr int kGroup = OP == CX_OP_ADAMW ? 1 : 2;     // 128-element rows whose loads are in flight together
+#pragma unroll 1
+      for (int c0 = 0; c0 < CX_SUBTILE / 128; c0 += kGroup) {
+        float x[kGroup][4], y[kGroup][4], wv[kGroup][4], mv[kGroup][4], vv[kGroup][4];
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k) {
+          const int e0 = (c0 + k) * 128 + lane * 4;
+          cx::load4(cur.g + e0, x[k]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) y[k][e] = 0.f;
+          if (KEEP == 2) cx::load4(q.f.u + lo + e0, y[k]);
+          cx::load4(reinterpret_cast<const float*>(q.a.out) + lo + e0, wv[k]);
+          if (OP != CX_OP_SGD) cx::load4(q.a.m + lo + e0, mv[k]);
+          if (OP == CX_OP_ADAMW) cx::load4(q.a.v + lo + e0, vv[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k) {
+          const int e0 = (c0 + k) * 128 + lane * 4;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) y[k][e] = q.f.mu * y[k][e] + cur.coef * x[k][e];
+          if (KEEP) cx::store4(q.f.u + lo + e0, y[k]);
+          rule4<OP>(q.a, y[k], wv[k], mv[k], vv[k]);
+          store_state4<OP, TO>(q.a, lo + e0, wv[k], mv[k], vv[k]);
+        }
+      }
+    } else if (cur.kind == 1) {
+      fold_update_border<OP, TO, T, KEEP>(q, sub, lane);    // gradients at an odd address
+    }
+    cur = ahead;
+    sub = next;
   }
 }
 
@@ -903,9 +937,8 @@ int cx_fold_update_cuda(int gdtype, const CxFold* fold, int64_t n, const CxApply
   FoldUpdateParams q;
   q.f = *fold; q.a = *a; q.n = n;
   q.nsub = (uint32_t)((n + CX_SUBTILE - 1) / CX_SUBTILE);
-  int grid = cx_sm_count() * 8;
-  const int need = (int)((q.nsub + kWarps - 1) / kWarps);
-  if (grid > need) grid = need;
+  int grid;
+  q.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.nsub, kWarps, cx_sm_count() * 4, &grid);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int keep = !fold->u ? 0 : fold->mu == 0.f ? 1 : 2;
   int rc;

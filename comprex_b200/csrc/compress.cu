@@ -103,6 +103,7 @@ struct FoldCompressParams {
   CompressParams c;
   CxFold f;
   uint32_t chain;   // CX_CHAINED, CX_CHAIN_NEXT
+  uint32_t nborder_ctas;
 };
 
 // One aligned, complete sub-tile, one warp, one pass: lane L holds elements {c*128 + 4L + e} in
@@ -297,20 +298,20 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
   }
   if (IN != kPlain) {
     const cx::FoldBlock<T> blk = cx::fold_blocks<T>(*f, sub, lane);
-    constexpr int kGroup = 8;      // loads in flight: none of them moves across a store of the momentum
+    constexpr int kGroup = 16;     // loads in flight: none of them moves across a store of the momentum
 #pragma unroll
     for (int j0 = 0; j0 < kEach; j0 += kGroup) {
-      float x[kGroup], y[kGroup], coef[kGroup];
+      float x[kGroup], y[kGroup];
       uint32_t in = 0;
 #pragma unroll
       for (int j = 0; j < kGroup; ++j) {
-        const bool t = cx::fold_element<T>(blk, j0 + j, lane, x[j], coef[j]);
+        const bool t = cx::fold_element<T>(blk, j0 + j, lane, x[j]);
         in |= (t ? 1u : 0u) << j;
         y[j] = IN == kFoldMom && t ? f->u[at + 32 * (j0 + j)] : 0.f;
       }
 #pragma unroll
       for (int j = 0; j < kGroup; ++j) {
-        const float t = f->mu * y[j] + coef[j] * x[j];
+        const float t = f->mu * y[j] + __shfl_sync(0xffffffffu, blk.coef, (j0 + j) >> 1) * x[j];
         if (IN != kFold && ((in >> j) & 1u)) f->u[at + 32 * (j0 + j)] = t;
         v[j0 + j] = v[j0 + j] + ((in >> j) & 1u ? t : 0.f);
       }
@@ -508,18 +509,30 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   if (!(q.chain & CX_CHAINED)) cx::pdl_wait();
   if (q.chain & CX_CHAIN_NEXT) cx::pdl_trigger();
   const float thr = *p.thr;
-  const uint32_t nwarps = gridDim.x * kWarps;
-  const uint32_t nfull = (uint32_t)(p.n / CX_SUBTILE);
-  for (uint32_t sub = blockIdx.x * kWarps + warp; sub < p.nsub; sub += nwarps) {
-    const int64_t off = (int64_t)sub * CX_SUBTILE;
-    const T* g = nullptr;
-    float coef = 0.f;
-    if (sub < nfull && cx::fold_whole<T>(q.f, sub, g, coef)) {
-      float v[kChunks][4];
-      load_fold_subtile<T, IN>(g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, coef, lane, v);
-      emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v);
-    } else
-      compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, &q.f);
+  if (blockIdx.x < q.nborder_ctas) {
+    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kWarps)
+      compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, &q.f);
+  } else {
+    const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kWarps;
+    uint32_t sub = (blockIdx.x - q.nborder_ctas) * kWarps + warp;
+    cx::FoldWhole<T> cur = {nullptr, 0.f, 0};
+    if (sub < p.nsub) cur = cx::fold_whole<T>(q.f, sub);
+    while (sub < p.nsub) {
+      const int64_t off = (int64_t)sub * CX_SUBTILE;
+      const uint32_t next = sub + nwarps;
+      cx::FoldWhole<T> ahead = {nullptr, 0.f, 0};
+      if (cur.kind == 2) {
+        float v[kChunks][4];
+        load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v);
+        if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);     // on its way while this one is stored
+        emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v);
+      } else {
+        if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);
+        if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, &q.f);
+      }
+      cur = ahead;
+      sub = next;
+    }
   }
   compress_finish(p, tid, thr, false, s_last, s_found, s_nnz);
   if (q.chain & CX_CHAINED) cx::pdl_wait();
@@ -747,10 +760,12 @@ int grid_for(const CompressParams& p) {
 
 template <typename T, Input IN>
 void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
-  const int grid = grid_for(q.c);
+  FoldCompressParams p = q;
+  int grid;
+  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, kWarps, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS, &grid);
   const bool capturing = q.c.seq_cell != nullptr;
-  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN>, grid, kThreads, 0, s, q, capturing);
-  else cx_launch_pdl(compress_fold_kernel<T, false, IN>, grid, kThreads, 0, s, q, capturing);
+  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN>, grid, kThreads, 0, s, p, capturing);
+  else cx_launch_pdl(compress_fold_kernel<T, false, IN>, grid, kThreads, 0, s, p, capturing);
 }
 
 template <typename T>

@@ -150,10 +150,14 @@ typedef struct CxFold {
   const int64_t* seg_end;      /* [nseg] and where they end                                            */
   const float* coef;           /* [nseg] learning rate times clip factor (cx_fold_coef)                */
   const int32_t* sub_seg;      /* per 1024 elements of the range: first tensor that ends behind their start */
+  const int32_t* border;       /* [nborder] the 1024-element pieces of the flat buffer that lie in the range and are
+                                  not covered by one tensor (flat position / 1024, ascending)          */
   float* u;                    /* momentum of the range, updated by the compress / update kernel; NULL: none kept */
-  int64_t base;                /* a multiple of CX_FOLD_ALIGN */
+  int64_t base;                /* a multiple of 1024 */
   int32_t nseg;
+  int32_t nborder;
   float mu;
+  int32_t pad;
 } CxFold;
 
 /* ---- exported C ABI ------------------------------------------------- */

@@ -128,7 +128,11 @@ class _FoldTable:
             # buckets start on sub-tile borders: one table serves them all
             subs = torch.arange(lo, max(buckets[-1].end, lo + 1), _lib.SUBTILE, dtype=torch.int64, device=dev)
             self.sub_seg = torch.searchsorted(self.seg_end, subs, right=True, out_int32=True)
-            self.args, self.lo = {}, lo
+            # pieces of 1024 elements that a tensor begins or ends inside
+            cuts = np.concatenate((start, start + numel))
+            self.border = np.unique(cuts[cuts % _lib.SUBTILE != 0] // _lib.SUBTILE)
+            self.border_dev = torch.from_numpy(self.border.astype(np.int32)).to(dev)
+            self.args, self.lo, self.hi = {}, lo, buckets[-1].end
 
     def refresh(self, zeros) -> None:
         """Bring the table of gradient addresses up to this step's; ``zeros`` stands in for a missing
@@ -167,6 +171,8 @@ class _FoldTable:
         f = _lib.Fold()
         base = self.lo if b is None else b.start
         sub = self.sub_seg.data_ptr() + 4 * ((base - self.lo) // _lib.SUBTILE)
+        b0, b1 = np.searchsorted(self.border, (base // _lib.SUBTILE, -(-(self.hi if b is None else b.end) // _lib.SUBTILE)))
+        f.border, f.nborder = self.border_dev.data_ptr() + 4 * int(b0), int(b1 - b0)
         f.seg_ptr, f.seg_off, f.seg_end = self.ptrs.data_ptr(), self.seg_off.data_ptr(), self.seg_end.data_ptr()
         f.coef, f.sub_seg, f.u = self.coef.data_ptr(), sub, 0 if u is None else u.data_ptr()
         f.base, f.nseg, f.mu = base, self.nseg, mu
