@@ -36,7 +36,6 @@ struct ApplyParams {
   int64_t n;
   uint32_t nsub;
   uint32_t vec;  // every dense pointer is 16-byte aligned
-  uint32_t batch;  // sub-tiles with few pairs take the one-round-trip path
   uint32_t* status;
   uint64_t timeout_ns;
   const uint64_t* seq_cell;  // non-NULL inside a captured graph: the waits use its value
@@ -52,68 +51,31 @@ __device__ __forceinline__ CxPair ld_pair(const CxPair* p) {
   return r;
 }
 
-// Waits for all sources and validates their headers.  Returns false (uniformly
-// for the CTA) when the kernel must not touch the output.
-__device__ __forceinline__ bool wait_sources(const ApplyParams& p, uint32_t* s_nnz) {
-  __shared__ uint32_t s_bad;
-  if (threadIdx.x == 0) s_bad = 0;
-  __syncthreads();
-  if ((int)threadIdx.x < p.src.count) {
-    const int j = threadIdx.x;
-    const CxHeader* h = p.src.ep[j].hdr;
+// Waits for all sources and validates their headers: the first warp does, lane j for source j.  (Every
+// warp for itself would save the barrier, but 7000 warps polling one line cost 5 us.)  Returns false
+// (uniformly for the CTA) when the kernel must not touch the output; no table is read before, a
+// payload of another length may have a shorter one.
+__device__ __forceinline__ bool wait_sources(const ApplyParams& p) {
+  __shared__ uint32_t s_ok;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
     uint32_t bad = 0;
-    if (!cx::wait_seq(&h->seq, cx::seq_of(p.seq_cell, p.src.seq[j]), p.timeout_ns)) {
-      bad = CX_ST_TIMEOUT;
-    } else {
-      const uint32_t kind = *reinterpret_cast<const volatile uint32_t*>(&h->kind);
-      const uint32_t hn = *reinterpret_cast<const volatile uint32_t*>(&h->n);
-      if (kind != CX_KIND_PAIRS || hn != (uint32_t)p.n) bad = CX_ST_BAD_HEADER;
-      s_nnz[j] = *reinterpret_cast<const volatile uint32_t*>(&h->nnz);
+    if (lane < p.src.count) {
+      const CxHeader* h = p.src.ep[lane].hdr;
+      if (!cx::wait_seq(&h->seq, cx::seq_of(p.seq_cell, p.src.seq[lane]), p.timeout_ns)) {
+        bad = CX_ST_TIMEOUT;
+      } else {
+        const uint32_t kind = *reinterpret_cast<const volatile uint32_t*>(&h->kind);
+        const uint32_t hn = *reinterpret_cast<const volatile uint32_t*>(&h->n);
+        if (kind != CX_KIND_PAIRS || hn != (uint32_t)p.n) bad = CX_ST_BAD_HEADER;
+      }
+      if (bad && p.status) atomicOr(p.status, bad);
     }
-    if (bad) atomicOr(&s_bad, bad);
+    const bool any = __any_sync(0xffffffffu, bad != 0);
+    if (lane == 0) s_ok = any ? 0u : 1u;
   }
   __syncthreads();
-  const uint32_t bad = s_bad;
-  if (bad && threadIdx.x == 0 && p.status) atomicOr(p.status, bad);
-  return bad == 0;
-}
-
-// ---- one memory round trip for all sources of a sub-tile ------------------------------------
-// Walking the sources one after the other costs one dependent load (pairs) or two (pairs, then
-// the addressed elements) per source.  When the sub-tile's pairs of ALL sources fit four per
-// lane, they are fetched in one go instead: the segments [a_j, b_j) are laid end to end, lane l
-// takes the pairs l, l + 32, ... of that sequence, and only the cheap part (the additions, in
-// shared memory) runs source after source, which keeps the order of every sum.
-constexpr int kBatch = 4;                       // pairs per lane
-constexpr uint32_t kBatchMax = 32 * kBatch;      // pairs per sub-tile the batched path takes
-
-struct Gathered {
-  CxPair pr[kBatch];
-  int src[kBatch];   // source of the pair, -1: none
-};
-
-// a / b: lane j holds source j's segment.  total: sum of all segment lengths (<= kBatchMax).
-__device__ __forceinline__ void gather_pairs(const ApplyParams& p, int lane, uint32_t a, uint32_t b,
-                                             uint32_t pre, Gathered& g) {
-  uint32_t off[kBatch];
-#pragma unroll
-  for (int k = 0; k < kBatch; ++k) { g.src[k] = -1; off[k] = 0; }
-  for (int j = 0; j < p.src.count; ++j) {
-    const uint32_t pj = __shfl_sync(0xffffffffu, pre, j);
-    const uint32_t aj = __shfl_sync(0xffffffffu, a, j);
-    const uint32_t cj = __shfl_sync(0xffffffffu, b, j) - aj;
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-      const uint32_t f = (uint32_t)(k * 32 + lane);
-      if (f - pj < cj) { g.src[k] = j; off[k] = aj + (f - pj); }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kBatch; ++k) {
-    g.pr[k].idx = 0;
-    g.pr[k].val = 0;
-    if (g.src[k] >= 0) g.pr[k] = ld_pair(p.src.ep[g.src[k]].pairs + off[k]);
-  }
+  return s_ok != 0;
 }
 
 __device__ __forceinline__ void segment_prefix(int lane, uint32_t a, uint32_t b, uint32_t& pre, uint32_t& total) {
@@ -138,10 +100,9 @@ constexpr int kAhead = 4;
 
 template <typename TO>
 __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_constant__ ApplyParams p) {
-  __shared__ uint32_t s_nnz[CX_MAX_PEERS];
   if (p.chain_next) cx::pdl_trigger();
-  if (!wait_sources(p, s_nnz)) { cx::pdl_wait(); return; }
   const int lane = threadIdx.x & 31;
+  if (!wait_sources(p)) { cx::pdl_wait(); return; }
   const uint32_t nwarps = gridDim.x * kWarps;
   const bool sgd = p.a.op == CX_OP_SGD;
   const float scale = sgd ? -p.a.scale : p.a.scale;
@@ -311,52 +272,58 @@ __device__ __forceinline__ void update1(const CxApplyArgs& a, int64_t i, float a
   if (a.shadow) reinterpret_cast<TO*>(a.shadow)[i] = cx::Elem<TO>::from_f(wv[0]);
 }
 
-// Table look-up, zeroing of the accumulator and accumulation of all sources' pairs of one
-// sub-tile (shared by the two dense kernels).  Returns CX_ST_BAD_INDEX or 0.
-__device__ __forceinline__ uint32_t accumulate_subtile(const ApplyParams& p, uint32_t sub, int lane, float* acc) {
+// Sum of all sources' pairs of one sub-tile in shared memory (acc, cleared here).  a, b: lane j holds
+// source j's segment of its pair list.  The segments are laid end to end, lane l takes the pairs l,
+// l + 32, ... of that sequence, up to four in flight: one round trip for all sources of a sub-tile of
+// up to 128 pairs.  Sums are formed in source order: the sequence is in source order, and the few
+// sources of a row of 32 pairs take turns.  Returns CX_ST_BAD_INDEX or 0.
+constexpr int kRows = 4;
+
+__device__ __forceinline__ uint32_t accumulate_subtile(const ApplyParams& p, uint32_t sub, int lane, uint32_t a, uint32_t b,
+                                                       unsigned long long pairs, float* acc) {
   const uint32_t lo = sub * CX_SUBTILE;
-  uint32_t bad = 0, a = 0, b = 0;
-  if (lane < p.src.count) {
-    const uint2 entry = __ldcg(reinterpret_cast<const uint2*>(p.src.ep[lane].table) + sub);
-    a = entry.x;
-    b = min(entry.x + min(entry.y, (uint32_t)CX_SUBTILE), p.src.cap[lane]);  // never beyond the slot
-    a = min(a, b);
-  }
-  uint32_t pre, total;
+  uint32_t bad = 0, pre, total;
   segment_prefix(lane, a, b, pre, total);
-  Gathered g;
-  const bool batched = p.batch && total <= kBatchMax;
-  if (batched && total) gather_pairs(p, lane, a, b, pre, g);      // the loads fly while the accumulator is cleared
+  for (uint32_t f0 = 0; f0 == 0 || f0 < total; f0 += 32 * kRows) {
+    CxPair pr[kRows];
+    uint32_t src[kRows];
 #pragma unroll
-  for (int q = 0; q < CX_SUBTILE / 128; ++q)
-    *reinterpret_cast<float4*>(acc + q * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncwarp();
-  if (total == 0) return 0;
-  if (batched) {
-    for (int j = 0; j < p.src.count; ++j) {
+    for (int k = 0; k < kRows; ++k) {
+      src[k] = 0;
+      pr[k].idx = -1;
+      pr[k].val = 0;
+      if (f0 + 32 * k >= total) continue;      // warp-uniform
+      const uint32_t f = f0 + 32 * k + lane;
+      uint32_t o = 0;                          // the last source whose pairs start at or before f
 #pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
-        if (g.src[k] == j) {
-          const uint32_t d = (uint32_t)g.pr[k].idx - lo;
-          if (d < CX_SUBTILE && (int64_t)g.pr[k].idx < p.n) acc[d] += __uint_as_float(g.pr[k].val);
-          else bad = CX_ST_BAD_INDEX;
-        }
+      for (uint32_t d = CX_MAX_PEERS / 2; d > 0; d >>= 1) {
+        const uint32_t t = __shfl_sync(0xffffffffu, pre, o + d);
+        if (t <= f) o += d;
       }
+      const uint32_t off = __shfl_sync(0xffffffffu, a, o) + (f - __shfl_sync(0xffffffffu, pre, o));
+      const unsigned long long base = __shfl_sync(0xffffffffu, pairs, o);
+      src[k] = o;
+      if (f < total) {
+        pr[k] = ld_pair(reinterpret_cast<const CxPair*>(base) + off);
+        if (!((uint32_t)pr[k].idx - lo < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { bad = CX_ST_BAD_INDEX; pr[k].idx = -1; }
+      }
+    }
+    if (f0 == 0) {                             // while the pairs are on their way
+#pragma unroll
+      for (int q = 0; q < CX_SUBTILE / 128; ++q)
+        *reinterpret_cast<float4*>(acc + q * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
       __syncwarp();
     }
-    return bad;
-  }
-  for (int j = 0; j < p.src.count; ++j) {
-    const uint32_t aj = __shfl_sync(0xffffffffu, a, j);
-    const uint32_t bj = __shfl_sync(0xffffffffu, b, j);
-    const CxPair* pairs = p.src.ep[j].pairs;
-    for (uint32_t i = aj + lane; i < bj; i += 32) {
-      const CxPair pr = ld_pair(pairs + i);
-      const uint32_t d = (uint32_t)pr.idx - lo;
-      if (d < CX_SUBTILE && (int64_t)pr.idx < p.n) acc[d] += __uint_as_float(pr.val);
-      else bad = CX_ST_BAD_INDEX;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      if (f0 + 32 * k >= total) continue;
+      const uint32_t d = (uint32_t)pr[k].idx - lo;
+      const uint32_t last = __shfl_sync(0xffffffffu, src[k], 31);
+      for (uint32_t t = __shfl_sync(0xffffffffu, src[k], 0); t <= last; ++t) {     // the sources of this row
+        if (src[k] == t && pr[k].idx >= 0) acc[d] += __uint_as_float(pr[k].val);
+        __syncwarp();
+      }
     }
-    __syncwarp();
   }
   return bad;
 }
@@ -442,13 +409,12 @@ constexpr int kBulkMaxThreads = 512;
 template <int OP, typename TO, int STAGES>
 __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(const ApplyParams p) {
   extern __shared__ __align__(128) unsigned char s_dyn[];
-  __shared__ uint32_t s_nnz[CX_MAX_PEERS];
   constexpr int NARR = StateArrays<OP>::n;
   constexpr uint32_t kTileBytes = CX_SUBTILE * sizeof(float);
   constexpr uint32_t kWarpBytes = (1 + STAGES * NARR) * kTileBytes;
-  if (!wait_sources(p, s_nnz)) { cx::pdl_wait(); return; }
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
+  if (!wait_sources(p)) { cx::pdl_wait(); return; }
   const uint32_t nw = blockDim.x >> 5;
   float* acc = reinterpret_cast<float*>(s_dyn + warp * kWarpBytes);
   float* stage0 = acc + CX_SUBTILE;
@@ -539,20 +505,30 @@ __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(co
   if (bad && p.status) atomicOr(p.status, bad);
 }
 
+// CTAs of apply_dense_kernel per SM (registers)
+constexpr int dense_per_sm(int op) { return op == CX_OP_MOMENTUM || op == CX_OP_ADAMW ? 5 : 6; }
+
 template <int OP, typename TO>
-__global__ void __launch_bounds__(kThreads) apply_dense_kernel(const __grid_constant__ ApplyParams p) {
-  __shared__ uint32_t s_nnz[CX_MAX_PEERS];
+__global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel(const __grid_constant__ ApplyParams p) {
   __shared__ __align__(16) float s_acc[kWarps][CX_SUBTILE];
   if (p.chain_next) cx::pdl_trigger();
-  if (!wait_sources(p, s_nnz)) { cx::pdl_wait(); return; }
   const int lane = threadIdx.x & 31;
+  if (!wait_sources(p)) { cx::pdl_wait(); return; }
   const int warp = threadIdx.x >> 5;
   const uint32_t nwarps = gridDim.x * kWarps;
   float* acc = s_acc[warp];
   uint32_t bad = 0;
-  for (uint32_t sub = blockIdx.x * kWarps + warp; sub < p.nsub; sub += nwarps) {
+  const unsigned long long pairs = lane < p.src.count ? reinterpret_cast<unsigned long long>(p.src.ep[lane].pairs) : 0ull;
+  uint32_t sub = blockIdx.x * kWarps + warp, a, b;
+  table_entry(p, sub, lane, a, b);
+  for (; sub < p.nsub; sub += nwarps) {
     const uint32_t lo = sub * CX_SUBTILE;
-    bad |= accumulate_subtile(p, sub, lane, acc);
+    uint32_t na, nb;                          // the next sub-tile's table entries, in flight meanwhile
+    const uint64_t next = (uint64_t)sub + nwarps;
+    table_entry(p, next < p.nsub ? (uint32_t)next : p.nsub, lane, na, nb);
+    bad |= accumulate_subtile(p, sub, lane, a, b, pairs, acc);
+    a = na;
+    b = nb;
 #pragma unroll
     for (int q = 0; q < CX_SUBTILE / 128; ++q) {
       const int e0 = q * 128 + lane * 4;
@@ -858,10 +834,6 @@ int cx_apply_cuda(const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_
   p.src = *src; p.a = *a; p.n = n;
   p.nsub = (uint32_t)((n + CX_SUBTILE - 1) / CX_SUBTILE);
   p.status = status; p.timeout_ns = timeout_ns; p.seq_cell = cx_seq_cell();
-  {
-    const char* e = getenv("COMPREX_APPLY_BATCH");       // 0: always walk the sources one by one
-    p.batch = (e && e[0] == '0') ? 0u : 1u;
-  }
   const bool update = a->op != CX_OP_ADD && a->op != CX_OP_SET;
   if (update && a->op != CX_OP_SGD && !a->m) return cx_set_error("cx_apply: momentum buffer missing", 0);
   if (a->op == CX_OP_ADAMW && !a->v) return cx_set_error("cx_apply: second-moment buffer missing", 0);
@@ -869,7 +841,7 @@ int cx_apply_cuda(const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_
           (!a->v || aligned16(a->v));
   p.chain_next = !p.seq_cell && (cx_chain_bits() & CX_CHAIN_NEXT) ? 1u : 0u;
   const int dt = update ? (a->shadow ? a->shadow_dtype : CX_F32) : a->out_dtype;
-  int grid = cx_sm_count() * 6;
+  int grid = cx_sm_count() * dense_per_sm(a->op);      // the sparse ops: as many as for SET
   p.group = 1;
   const bool sparse = a->op == CX_OP_ADD || (a->op == CX_OP_SGD && a->wd == 0.f);
   if (sparse) {

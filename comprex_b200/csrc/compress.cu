@@ -106,6 +106,12 @@ struct FoldCompressParams {
   uint32_t nborder_ctas;
 };
 
+// What a warp has seen so far, for the completion.
+struct Tally {
+  uint32_t found;   // survivors
+  bool over;        // some of them did not fit the slot
+};
+
 // One aligned, complete sub-tile, one warp, one pass: lane L holds elements {c*128 + 4L + e} in
 // registers from the loads to the write-back of the residual.
 // gl / rl: where this sub-tile's gradient and residual are read (global memory, or the copy of the
@@ -164,7 +170,8 @@ __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, cons
 // memory, where the new residual goes.
 template <bool HAS_G, bool HAS_R, bool MC>
 __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint32_t sub, const int lane, const float thr,
-                                             float* __restrict__ rs, CxPair* stage, float (&v)[kChunks][4]) {
+                                             float* __restrict__ rs, CxPair* stage, float (&v)[kChunks][4],
+                                             Tally& tally) {
   const int64_t sub_base = (int64_t)sub * CX_SUBTILE;
   float* wp = rs + lane * 4;
 
@@ -201,6 +208,8 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
   }
   const uint32_t emit = base >= p.region_size ? 0u : min(count, p.region_size - base);  // pairs that fit
   base += region * p.region_size;
+  tally.found += count;
+  tally.over |= emit < count;
   {
     uint2 entry;
     entry.x = emit ? base : 0u;
@@ -284,7 +293,7 @@ template <typename T, bool HAS_G, bool HAS_R, bool MC, Input IN = kPlain>
 __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, const uint32_t sub,
                                                       const int lane, const float thr,
                                                       const T* __restrict__ g, float* __restrict__ r,
-                                                      const CxFold* f = nullptr) {
+                                                      Tally& tally, const CxFold* f = nullptr) {
   constexpr int kEach = CX_SUBTILE / 32;
   const int64_t sub_base = (int64_t)sub * CX_SUBTILE;
   const int left = (int)min((int64_t)CX_SUBTILE, p.n - sub_base) - lane;   // my elements: 32 j < left
@@ -332,6 +341,8 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
   }
   const uint32_t emit = base >= p.region_size ? 0u : min(count, p.region_size - base);
   base += region * p.region_size;
+  tally.found += count;
+  tally.over |= emit < count;
   {
     uint2 entry;
     entry.x = emit ? base : 0u;
@@ -365,34 +376,52 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
   }
 }
 
-// Completion: the CTA that arrives last adds up the regions, writes the headers and publishes the
-// notification.  `failed` (CTA-uniform or not): this CTA could not process all its sub-tiles; the
-// payload is then not published (the receivers' bounded waits run out) and the status says why.
-__device__ __forceinline__ void compress_finish(const CompressParams& p, const int tid, const float thr,
-                                                const bool failed, uint32_t& s_last, uint32_t& s_found,
-                                                uint32_t& s_nnz) {
+// Completion: every CTA adds its survivors, its arrival and its marks to one 64-bit counter with one
+// atomic, whose result tells the CTA that arrives last all it has to know; it writes the headers and
+// publishes the notification.  (Reading the 32 region counters back first was 1 us on the end of
+// every exchange; they are read only when survivors did not fit.)  `failed`: this CTA could not
+// process all its sub-tiles; the payload is then not published (the receivers' bounded waits run
+// out) and the status says why.
+constexpr int kArrived = 32, kOver = 44, kFailed = 54;     // bit positions behind the survivors; grids have < 4096 CTAs
+
+template <int MAX_WARPS>
+__device__ __forceinline__ void compress_finish(const CompressParams& p, const int tid, const float thr, const bool failed,
+                                                const Tally& tally) {
+  __shared__ uint32_t s_found[MAX_WARPS], s_mark[MAX_WARPS];
+  __shared__ unsigned long long s_all;
+  __shared__ uint32_t s_nnz;
   // the receive kernel queued behind this one may become resident now: it polls its flags
   cx::pdl_trigger();
-  // ---- completion: the CTA that arrives last publishes -------------------------------
-  if (failed) atomicOr(&p.ctr->pad[4], 1u);
+  const int nw = blockDim.x >> 5;
+  if ((tid & 31) == 0) {
+    s_found[tid >> 5] = tally.found;
+    s_mark[tid >> 5] = (tally.over ? 1u : 0u) | (failed ? 2u : 0u);
+  }
+  __syncthreads();            // all stores of the CTA are issued
   if (tid == 0) {
-    s_found = 0;
+    uint32_t found = 0, mark = 0;
+    for (int w = 0; w < nw; ++w) { found += s_found[w]; mark |= s_mark[w]; }
+    const unsigned long long mine = (unsigned long long)found | 1ull << kArrived |
+                                    (mark & 1u ? 1ull << kOver : 0ull) | (mark & 2u ? 1ull << kFailed : 0ull);
+    __threadfence();          // as in cx::cta_arrive
+    s_all = atomicAdd(reinterpret_cast<unsigned long long*>(&p.ctr->done), mine) + mine;
+    __threadfence();
     s_nnz = 0;
   }
-  const bool last = cx::cta_arrive(&p.ctr->done, gridDim.x, &s_last);
-  CX_TRACE(3);
-  if (!last) return;
-  const uint32_t any_failed = *reinterpret_cast<volatile uint32_t*>(&p.ctr->pad[4]);
-  if ((uint32_t)tid < p.nregions) {
-    const uint32_t f = *reinterpret_cast<volatile uint32_t*>(&p.ctr->region[tid][0]);
-    atomicAdd(&s_found, f);
-    atomicAdd(&s_nnz, min(f, p.region_size));
-    p.ctr->region[tid][0] = 0;
-  }
   __syncthreads();
+  CX_TRACE(3);
+  const unsigned long long all = s_all;
+  if (((all >> kArrived) & 0xfffu) != gridDim.x) return;
+  const uint32_t found = (uint32_t)all;   // survivors
+  const bool over = ((all >> kOver) & 0x3ffu) != 0, any_failed = (all >> kFailed) != 0;
+  uint32_t nnz = found;                   // pairs stored
+  if (over) {
+    if ((uint32_t)tid < p.nregions)
+      atomicAdd(&s_nnz, min(*reinterpret_cast<volatile uint32_t*>(&p.ctr->region[tid][0]), p.region_size));
+    __syncthreads();
+    nnz = s_nnz;
+  }
   CX_TRACE(4);
-  const uint32_t found = s_found;  // survivors
-  const uint32_t nnz = s_nnz;      // pairs stored
   if (tid < p.tg.count && !any_failed) {
     CxHeader* h = p.tg.ep[tid].hdr;
     h->bytes = 8ull + 8ull * nnz;
@@ -407,6 +436,7 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
     cx::st_release_sys(&h->seq, cx::seq_of(p.seq_cell, p.seq));
   }
   CX_TRACE(5);
+  if ((uint32_t)tid < p.nregions) p.ctr->region[tid][0] = 0;
   if (tid == 0) {
     if (p.stats) {
       p.stats->n = (uint32_t)p.n;
@@ -415,8 +445,7 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
       p.stats->status = (found > nnz ? CX_ST_OVERFLOW : 0u) | (any_failed ? CX_ST_TIMEOUT : 0u);
       p.stats->threshold = thr;
     }
-    p.ctr->done = 0;
-    p.ctr->pad[4] = 0;
+    *reinterpret_cast<unsigned long long*>(&p.ctr->done) = 0;
   }
   CX_TRACE(6);
 }
@@ -429,8 +458,6 @@ template <typename T, bool HAS_G, bool HAS_R, bool MC>
 __global__ void __launch_bounds__(kThreads, CX_COMPRESS_MIN_BLOCKS)
 compress_kernel(const __grid_constant__ CompressParams p) {
   __shared__ CxPair s_stage[kWarps][kStage];
-  __shared__ uint32_t s_last;
-  __shared__ uint32_t s_found, s_nnz;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -461,6 +488,7 @@ compress_kernel(const __grid_constant__ CompressParams p) {
   }
   cx::pdl_wait();
   const float thr = *p.thr;
+  Tally tally = {0, false};
   CX_TRACE(1);
   CxPair* stage = s_stage[warp];
   const uint32_t nwarps = gridDim.x * kWarps;
@@ -480,16 +508,16 @@ compress_kernel(const __grid_constant__ CompressParams p) {
       const int64_t off = (int64_t)sub * CX_SUBTILE;
       if (!loaded) load_subtile<T, HAS_G, HAS_R>(g + off, r + off, lane, v);
       loaded = false;
-      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage, v);
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage, v, tally);
     }
-    else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r);
+    else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r, tally);
   }
 
 #ifdef CX_COMPRESS_TRACE
   __syncthreads();   // the stamp marks the CTA's last warp leaving the loop
 #endif
   CX_TRACE(2);
-  compress_finish(p, tid, thr, false, s_last, s_found, s_nnz);
+  compress_finish<kWarps>(p, tid, thr, false, tally);
 }
 
 // The same for a vector that is folded from gradient tensors on the way (CxFold): what the fold
@@ -501,17 +529,16 @@ template <typename T, bool MC, Input IN>
 __global__ void __launch_bounds__(kThreads, CX_COMPRESS_MIN_BLOCKS)
 compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   __shared__ CxPair s_stage[kWarps][kStage];
-  __shared__ uint32_t s_last;
-  __shared__ uint32_t s_found, s_nnz;
   const CompressParams& p = q.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* __restrict__ r = p.r;
   if (!(q.chain & CX_CHAINED)) cx::pdl_wait();
   if (q.chain & CX_CHAIN_NEXT) cx::pdl_trigger();
   const float thr = *p.thr;
+  Tally tally = {0, false};
   if (blockIdx.x < q.nborder_ctas) {
     for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kWarps)
-      compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, &q.f);
+      compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, tally, &q.f);
   } else {
     const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kWarps;
     uint32_t sub = (blockIdx.x - q.nborder_ctas) * kWarps + warp;
@@ -525,16 +552,16 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
         float v[kChunks][4];
         load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v);
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);     // on its way while this one is stored
-        emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v);
+        emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v, tally);
       } else {
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);
-        if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, &q.f);
+        if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, tally, &q.f);
       }
       cur = ahead;
       sub = next;
     }
   }
-  compress_finish(p, tid, thr, false, s_last, s_found, s_nnz);
+  compress_finish<kWarps>(p, tid, thr, false, tally);
   if (q.chain & CX_CHAINED) cx::pdl_wait();
 }
 
@@ -558,8 +585,6 @@ template <typename T, bool HAS_G, bool HAS_R, bool MC, int STAGES>
 __global__ void __launch_bounds__(kBulkMaxWarps * 32, 1)
 compress_bulk_kernel(const __grid_constant__ CompressParams p) {
   extern __shared__ __align__(128) unsigned char s_dyn[];
-  __shared__ uint32_t s_last;
-  __shared__ uint32_t s_found, s_nnz;
   constexpr uint32_t kRB = HAS_R ? (uint32_t)(CX_SUBTILE * sizeof(float)) : 0u;
   constexpr uint32_t kGB = HAS_G ? (uint32_t)(CX_SUBTILE * sizeof(T)) : 0u;
   constexpr uint32_t kStageB = kRB + kGB;
@@ -589,6 +614,7 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
   const uint32_t first = blockIdx.x * nw + warp;
   uint32_t issued = 0, consumed = 0;
   bool failed = false;
+  Tally tally = {0, false};
 
   auto issue = [&](uint32_t sub) {   // warp-uniform call; lane 0 talks to the copy engine
     if (lane == 0) {
@@ -623,15 +649,15 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
       const unsigned char* src = mine + s * kStageB;
       float v[kChunks][4];
       load_subtile<T, HAS_G, HAS_R>(reinterpret_cast<const T*>(src + kRB), reinterpret_cast<const float*>(src), lane, v);
-      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + (size_t)sub * CX_SUBTILE, stage, v);
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + (size_t)sub * CX_SUBTILE, stage, v, tally);
       // this stage is handed back to the copy engine by a later issue()
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
     } else {
-      compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r);
+      compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r, tally);
     }
   }
-  compress_finish(p, tid, thr, failed, s_last, s_found, s_nnz);
+  compress_finish<kBulkMaxWarps>(p, tid, thr, failed, tally);
 }
 
 // n == 0: nothing to scan, only the (empty) header and the notification.

@@ -102,7 +102,7 @@ typedef struct CxSources {
 /* scratch of one sender: zero-initialised, reset by the kernel that used it */
 #define CX_MAX_REGIONS 32
 typedef struct CxWorkCounters {
-  uint32_t done;                        /* CTAs that finished                          */
+  uint32_t done;                        /* CTAs that finished (compress: one 64-bit counter with pad[0]) */
   uint32_t pad[31];
   uint32_t region[CX_MAX_REGIONS][32];  /* pairs reserved per region, one 128-byte line each */
 } CxWorkCounters;
