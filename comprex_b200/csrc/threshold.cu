@@ -387,8 +387,9 @@ __global__ void __launch_bounds__(kExactThreads) exact_select_kernel(const Exact
 //      (a fixed stride could meet the same column of every row), between which the wanted key lies
 //      unless the sample is off by more than four standard deviations,
 //   2. collect: one pass counts the keys above hi, at hi and at lo, and appends the ones between to
-//      the candidate list (about 1 % of the vector),
-//   3. finish:  a cluster selects among the candidates by radix.  If the counts show that the bracket
+//      the candidate list (about 1 % of the vector), counting them by their 11 highest bits,
+//   3. finish:  the counts name the bin; a cluster picks the few candidates in it and ranks those
+//      (more than fit: it goes on by radix).  If the counts show that the bracket
 //      missed, or the candidates did not fit, it selects over the whole vector instead: always exact,
 //      only slower.
 // 10 M elements, fp32 vector and residual, top-k 1 %: 96 us with four passes.
@@ -396,15 +397,23 @@ constexpr int kBracket = 8192;
 constexpr int kCluster = 8;
 constexpr int kBins = 2048;          // 11 bits per radix pass of the finish
 constexpr int kCollectThreads = 256;
-constexpr int kCollectEach = 16;     // elements per thread and round
-constexpr int kBuffer = 6144;        // candidates a CTA keeps before it appends them to the list
+constexpr int kCollectEach = 8;      // elements per thread and round
+constexpr int kBuffer = 4096;        // candidates a CTA keeps before it appends them to the list
+constexpr int kCollectPerSm = 6;
 
 struct ExactState {                  // in the workspace behind the histograms; zero between calls
   uint32_t lo, hi;
   uint32_t above, at_hi, at_lo;      // elements with key > hi, == hi, == lo (lo < hi)
   uint32_t found;                    // candidates with lo < key < hi (not all of them stored when over cap)
   uint32_t pad[58];
+  uint32_t hist[kBins];              // candidates by their 11 highest bits between lo and hi
 };
+
+// candidates are lo + 1 .. hi - 1; how far their distance from lo + 1 is shifted for its bin
+__device__ __forceinline__ uint32_t bracket_base(uint32_t lo) { return lo + 1; }
+__device__ __forceinline__ int bracket_bits(uint32_t lo, uint32_t hi) {
+  return 32 - __clz((min(hi, 0x80000000u) - 1 - bracket_base(lo)) | 1u);
+}
 
 struct OnePassParams {
   const void* g;
@@ -463,16 +472,19 @@ __global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kCollectThreads, 4) collect_kernel(const __grid_constant__ OnePassParams p) {
+__global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel(const __grid_constant__ OnePassParams p) {
   __shared__ uint32_t s_buf[kBuffer];
+  __shared__ uint32_t s_hist[kBins];
   __shared__ uint32_t s_fill, s_base;
   __shared__ uint32_t s_cnt[3];
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid == 0) s_fill = 0;
+  for (int i = tid; i < kBins; i += kCollectThreads) s_hist[i] = 0;
   if (tid < 3) s_cnt[tid] = 0;
   cx::pdl_wait();
   cx::pdl_trigger();
   const uint32_t lo = p.st->lo, hi = p.st->hi;
+  const int shift = max(bracket_bits(lo, hi) - 11, 0);
   const T* g = reinterpret_cast<const T*>(p.g);
   uint32_t above = 0, at_hi = 0, at_lo = 0;
   __syncthreads();
@@ -533,7 +545,10 @@ __global__ void __launch_bounds__(kCollectThreads, 4) collect_kernel(const __gri
         uint32_t at = 0;
         if (lane == __ffs(who) - 1) at = atomicAdd(&s_fill, (uint32_t)__popc(who));
         at = __shfl_sync(0xffffffffu, at, __ffs(who) - 1);
-        if (cand) s_buf[at + __popc(who & ((1u << lane) - 1u))] = key;
+        if (cand) {
+          s_buf[at + __popc(who & ((1u << lane) - 1u))] = key;
+          atomicAdd(&s_hist[(key - bracket_base(lo)) >> shift], 1u);
+        }
       }
     }
     __syncthreads();
@@ -549,6 +564,7 @@ __global__ void __launch_bounds__(kCollectThreads, 4) collect_kernel(const __gri
     if (s_cnt[1]) atomicAdd(&p.st->at_hi, s_cnt[1]);
     if (s_cnt[2]) atomicAdd(&p.st->at_lo, s_cnt[2]);
   }
+  for (int i = tid; i < kBins; i += kCollectThreads) if (s_hist[i]) atomicAdd(&p.st->hist[i], s_hist[i]);
   if (s_fill) flush();
 }
 
@@ -586,9 +602,13 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
   uint32_t* out0 = cluster.map_shared_rank(s_out, 0);
   cx::pdl_wait();
   cx::pdl_trigger();
-  const ExactState st = *p.st;
+  struct { uint32_t lo, hi, above, at_hi, at_lo, found; } st;
+  st.lo = p.st->lo; st.hi = p.st->hi; st.above = p.st->above; st.at_hi = p.st->at_hi; st.at_lo = p.st->at_lo; st.found = p.st->found;
+  s_hists[2][tid] = p.st->hist[tid];          // (the third radix pass is behind a cluster barrier that clears it again)
+  s_hists[2][tid + kThreads] = p.st->hist[tid + kThreads];
   cluster.sync();                     // every CTA has read the state and cleared its histograms
   if (crank == 0 && tid == 0) p.st->above = p.st->at_hi = p.st->at_lo = p.st->found = 0;
+  if (crank == 1) p.st->hist[tid] = p.st->hist[tid + kThreads] = 0;
   uint32_t rank = p.rank, base = 0, top = 0x7fffffffu;
   bool list = false;
   if (st.found <= p.cap && rank >= st.above) {
@@ -597,15 +617,46 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
     if (left - st.at_hi < st.found) {
       list = true;
       rank = left - st.at_hi;
-      base = st.lo + 1;
+      base = bracket_base(st.lo);
       top = min(st.hi, 0x80000000u) - 1;
     } else if (left - st.at_hi - st.found < st.at_lo) {
       if (crank == 0 && tid == 0) *p.thr_out = __uint_as_float(st.lo);
       return;
     }
   }
-  // radix select of key - base in [0, top - base], 11 bits at a time from the highest bit in use
   const int bits = 32 - __clz((top - base) | 1u);
+  if (list) {
+    const int shift = max(bits - 11, 0);
+    uint32_t in_bin = rank;
+    const uint32_t bin = pick_bin(s_hists[2], in_bin, s_warp, s_out);      // every CTA for itself
+    if (s_hists[2][bin] <= kThreads) {
+      uint32_t* few = cluster.map_shared_rank(s_hists[0], 0);              // [0]: their number
+      uint32_t* keys = cluster.map_shared_rank(s_hists[1], 0);
+      const int64_t step = (int64_t)kCluster * kThreads;
+      for (int64_t i0 = (int64_t)crank * kThreads + tid; i0 < st.found; i0 += 4 * step) {
+        uint32_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = i0 + u * step < st.found ? p.list[i0 + u * step] : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i0 + u * step < st.found && ((k[u] - base) >> shift) == bin) keys[atomicAdd(few, 1u)] = k[u];
+      }
+      cluster.sync();
+      if (crank != 0) return;
+      const uint32_t left = s_hists[0][0];
+      uint32_t key = 0;
+      if (left <= 32) {
+        if (tid < 32) key = warp_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, tid, in_bin);
+      } else {
+        key = block_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, in_bin);
+      }
+      if (tid == 0) *p.thr_out = __uint_as_float(key);
+      return;
+    }
+  }
+  for (int i = tid; i < kBins; i += kThreads) s_hists[2][i] = 0;
+  cluster.sync();
+  // radix select of key - base in [0, top - base], 11 bits at a time from the highest bit in use
   uint32_t prefix = 0, mask = 0;
   const int64_t count = list ? (int64_t)st.found : p.n;
   int pass = 0;
@@ -658,7 +709,7 @@ int launch_one_pass(const OnePassParams& p, bool capturing, cudaStream_t s) {
   cudaError_t e = cudaLaunchKernelEx(&cfg, bracket_kernel<T>, p);
   if (e != cudaSuccess) return cx_set_error("bracket_kernel launch", (int)e);
   const int64_t round = (int64_t)kCollectThreads * kCollectEach;
-  int grid = cx_sm_count() * 4;
+  int grid = cx_sm_count() * kCollectPerSm;
   if (grid > (p.n + round - 1) / round) grid = (int)((p.n + round - 1) / round);
   cx_launch_pdl(collect_kernel<T>, grid, kCollectThreads, 0, s, p, capturing);
   e = cudaLaunchKernelEx(&cfg, exact_finish_kernel<T>, p);
