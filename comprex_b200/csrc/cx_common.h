@@ -160,6 +160,19 @@ typedef struct CxFold {
   int32_t pad;
 } CxFold;
 
+/* arguments of cx_fold_coef as one object, for op lists */
+typedef struct CxFoldCoef {
+  const void* const* seg_ptr;
+  const int64_t* item_rel;
+  const int32_t* item_len;
+  const int32_t* item_seg;
+  const int32_t* seg_first;
+  float* partial;
+  float* coef;
+  int32_t items, segs;         /* all from 0 on */
+  float clip, lr;
+} CxFoldCoef;
+
 /* ---- exported C ABI ------------------------------------------------- */
 
 const char* cx_last_error(void);
@@ -327,6 +340,8 @@ int cx_host_free(void* p);
 #define CX_OPK_DENSE_SEND 4
 #define CX_OPK_DENSE_REDUCE 5
 #define CX_OPK_UPDATE 6        /* cx_update_dense: g, n, apply */
+#define CX_OPK_FOLD_COEF 8     /* cx_fold_coef (CUDA): dtype, fold = address of a CxFoldCoef */
+#define CX_OPK_FOLD_UPDATE 9   /* cx_fold_update (CUDA): dtype, fold, n, apply */
 #define CX_OPK_MM_ALLREDUCE 7  /* cx_mm_allreduce: out, own (= in), g (= stage), r (= stage_mc), starts[0] = stride,
                                   starts[1] = one_shot, starts[2] = slab bytes, lens[r] = rank r's flag block,
                                   src_rank, cap (= ranks), workspace (= counters), scale, status */

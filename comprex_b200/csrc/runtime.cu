@@ -26,6 +26,7 @@
 // ---- forward declarations of the two back ends --------------------------------
 int cx_threshold_topk_cuda(int, const void*, const float*, int64_t, float, int, float, float*, void*, int64_t, void*);
 int cx_threshold_batch_cuda(const CxOp*, int, void*);
+int cx_compress_sampled_cuda(const CxOp*, const CxOp*, uint64_t, void*);
 int cx_threshold_topk_host(int, const void*, const float*, int64_t, float, int, float, float*);
 int cx_compress_cuda(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
                      const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
@@ -281,6 +282,13 @@ int run_one(CxOp& o, uint64_t seq, void* stream) {
                              (int)o.cap, o.scale, (int)o.starts[1], o.starts[2], seq, flags, o.workspace, o.status,
                              o.timeout_ns, stream);
     }
+    case CX_OPK_FOLD_COEF: {
+      const CxFoldCoef* f = reinterpret_cast<const CxFoldCoef*>(o.fold);
+      return cx_fold_coef(o.dtype, f->seg_ptr, f->item_rel, f->item_len, f->item_seg, f->seg_first, 0, f->items, 0, f->segs,
+                          f->partial, f->coef, f->clip, f->lr, stream);
+    }
+    case CX_OPK_FOLD_UPDATE:
+      return cx_fold_update(o.dtype, o.fold, o.n, &o.apply, stream);
     case CX_OPK_UPDATE:
       return cx_update_dense(o.dev, reinterpret_cast<const float*>(o.g), o.n, &o.apply, stream);
     default:
@@ -334,8 +342,14 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
     forked = false;
     return 0;
   };
-  // thresholds that follow one another on one lane share launches
+  // thresholds that follow one another on one lane share launches, one in front of the compression of a
+  // small vector shares its kernel
   auto run_some = [&](int i, void* on) -> int {      // ops taken, or a negative error
+    if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA && i + 1 < count &&
+        ops[i + 1].kind == CX_OPK_COMPRESS && ops[i + 1].dev == CX_DEV_CUDA && ops[i + 1].lane == ops[i].lane) {
+      const int one = cx_compress_sampled_cuda(ops + i, ops + i + 1, seq, on);      // a small vector: one kernel
+      if (one) return one > 0 ? 2 : one;
+    }
     if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA) return cx_threshold_batch_cuda(ops + i, count - i, on);
     auto chained = [&](int k) {
       return k > 0 && k < count && ops[k].chain && ops[k].kind == ops[k - 1].kind && ops[k].lane == ops[k - 1].lane;

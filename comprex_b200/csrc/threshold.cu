@@ -28,6 +28,7 @@
 #include <string.h>
 
 #include "cx_fold.cuh"
+#include "cx_select.cuh"
 
 namespace {
 
@@ -53,13 +54,7 @@ struct ThreshBatch {
 
 template <typename T, bool FOLD>
 __device__ __forceinline__ uint32_t sample_key(const ThreshParams& p, int i) {
-  int64_t pos;
-  if (p.use_all) {
-    pos = i;
-  } else {
-    pos = (int64_t)(int)__fmul_rn((float)i, p.stepsize);
-    if (pos > p.n - 1) pos = p.n - 1;
-  }
+  const int64_t pos = cx::sample_position(i, p.n, p.use_all, p.stepsize);
   float x = 0.f;
   if (p.r) x = p.r[pos];
   if (FOLD) x = x + cx::fold_at<T>(p.fold, pos);
@@ -98,18 +93,6 @@ __device__ __forceinline__ uint32_t pick_digit(const uint32_t* hist, uint32_t& r
   return digit;
 }
 
-// One warp, one key per lane (absent ones 0): the key of rank `rank` in descending order.
-__device__ __forceinline__ uint32_t warp_rank(uint32_t key, int count, int lane, uint32_t rank) {
-  uint32_t gt = 0, ge = 0;
-  for (int j = 0; j < count; ++j) {
-    const uint32_t other = __shfl_sync(0xffffffffu, key, j);
-    gt += other > key ? 1u : 0u;
-    ge += other >= key ? 1u : 0u;
-  }
-  const uint32_t who = __ballot_sync(0xffffffffu, lane < count && gt <= rank && rank < ge);
-  return __shfl_sync(0xffffffffu, key, __ffs(who) - 1);
-}
-
 // One key per thread (threads from `count` on hold none): the largest t with more than `rank` keys at
 // or above it, which is the key of that rank.  One block-wide count per bit.
 __device__ __forceinline__ uint32_t block_rank(uint32_t key, int count, uint32_t rank) {
@@ -143,7 +126,7 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
       if (lane == 0) s_red[w] = wm;
       __syncthreads();
       if (w == 0) {
-        const uint32_t b0 = warp_rank(s_red[lane], 32, lane, rank);
+        const uint32_t b0 = cx::warp_rank(s_red[lane], 32, lane, rank);
         if (lane == 0) s_sel[1] = b0;
       }
       __syncthreads();
@@ -160,7 +143,7 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
     }
     __syncthreads();
     const uint32_t left = s_sel[0];
-    if (left <= 32) return w == 0 ? warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
+    if (left <= 32) return w == 0 ? cx::warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
     if (left <= kThreads) return block_rank(tid < (int)left ? s_hist[tid] : 0u, (int)left, rank);
   }
   uint32_t prefix = 0, prefmask = 0;
@@ -646,7 +629,7 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
       const uint32_t left = s_hists[0][0];
       uint32_t key = 0;
       if (left <= 32) {
-        if (tid < 32) key = warp_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, tid, in_bin);
+        if (tid < 32) key = cx::warp_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, tid, in_bin);
       } else {
         key = block_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, in_bin);
       }

@@ -46,6 +46,7 @@ into the dense update kernel.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import warnings
 
@@ -177,6 +178,48 @@ class _FoldTable:
         f.coef, f.sub_seg, f.u = self.coef.data_ptr(), sub, 0 if u is None else u.data_ptr()
         f.base, f.nseg, f.mu = base, self.nseg, mu
         return f
+
+
+class _StepPlan:
+    """See ``ComprexOptimizer._plan``."""
+
+    def __init__(self, opt, ft: _FoldTable, par, cfg):
+        self.table, self.cfg, self.hyper = ft, cfg, None
+        env, k = opt._env, len(opt._buckets)
+        self.coef = _lib.FoldCoef(*[t.data_ptr() for t in (ft.ptrs, ft.item_rel, ft.item_len, ft.item_seg, ft.seg_first,
+                                                           ft.partial, ft.coef)], ft.nitems, ft.nseg, 0.0, 0.0)
+        coef = _lib.Op()
+        coef.kind, coef.dev, coef.dtype, coef.fold = _lib.OPK_FOLD_COEF, env.dev, ft.code, C.addressof(self.coef)
+        if par is None:
+            self.folds = [ft.fold_args(None, opt._update if opt._keeps_u else None, 0.0)]
+            upd = _lib.Op()
+            upd.kind, upd.dev, upd.dtype, upd.n = _lib.OPK_FOLD_UPDATE, env.dev, ft.code, opt.blob_size
+            upd.fold = C.addressof(self.folds[0])
+            ops, self.ranges, applies = [coef, upd], [(0, opt.blob_size, 1.0)], [1]
+        else:
+            self.folds = [ft.fold_args(b, opt._update[b.start:b.end] if opt._keeps_u else None, 0.0) for b in opt._buckets]
+            self.ranges = [(b.start, b.end - b.start, 1.0 / env.ranks) for b in opt._buckets]
+            lists = [b.ar.launch_lists(par) for b in opt._buckets]
+            ops = [coef] + [s.arr[0] for s, _ in lists] + [s.arr[1] for s, _ in lists] + [r.arr[0] for _, r in lists]
+            applies = range(1 + 2 * k, 1 + 3 * k)
+        self.count = len(ops)
+        self.ops = (_lib.Op * self.count)(*ops)
+        if par is not None:
+            for i, b in enumerate(opt._buckets):
+                thr, cmp_ = self.ops[1 + i], self.ops[1 + k + i]
+                thr.ratio = b.ar.compression_ratio
+                for op in (thr, cmp_):
+                    op.g, op.dtype, op.fold = None, ft.code, C.addressof(self.folds[i])
+                if i:                            # buckets share no vector, slot or scratch
+                    cmp_.chain = self.ops[1 + 2 * k + i].chain = 1
+        self.views = [self.ops[i].apply for i in applies]
+
+    def set_hyper(self, opt, lr, mu, wd) -> None:
+        for (start, n, scale), v in zip(self.ranges, self.views):
+            C.pointer(v)[0] = opt._args(start, n, lr, mu, wd, scale)
+        self.coef.clip, mu, self.coef.lr = opt._fold_scalars(lr, mu)
+        for f in self.folds:
+            f.mu = mu
 
 
 class ComprexOptimizer(torch.optim.Optimizer):
@@ -412,76 +455,32 @@ class ComprexOptimizer(torch.optim.Optimizer):
             f.mu = mu
         return f
 
-    def _group(self):
-        """One table and, per parity of the exchange step, one launch list for all buckets: all norms,
-        all thresholds and all updates of a step then take one native call each."""
+    def _plan(self, par):
+        """The launch list of a whole step (``par``: parity of the exchange step; None: a rank that
+        exchanges nothing): norms and clip factors of all tensors, then either one fold-and-update
+        kernel over the flat buffer, or all thresholds, one fold-and-compress kernel and one
+        wait-decode-update kernel per bucket.  Issued with one native call."""
         if self._all is None:
-            self._all = {"table": _FoldTable(self._env, self._buckets, self._dtype), "lists": {}}
-        return self._all
+            self._all = (_FoldTable(self._env, self._buckets, self._dtype), {})
+        ft, plans = self._all
+        cfg = None if par is None else [(b.ar.compression_ratio, b.ar.sampling) for b in self._buckets]
+        plan = plans.get(par)
+        if plan is None or plan.cfg != cfg:
+            plan = plans[par] = _StepPlan(self, ft, par, cfg)
+        return plan
 
-    def _lists(self, g, par: int):
-        """(send ops, receive ops, views of the receive ops' arguments) for one parity."""
-        bs, k = self._buckets, len(self._buckets)
-        cfg = [(b.ar.compression_ratio, b.ar.sampling) for b in bs]
-        got = g["lists"].get(par)
-        if got is not None and got[0] == cfg:
-            return got
-        send, recv = (_lib.Op * (2 * k))(), (_lib.Op * k)()
-        for i, b in enumerate(bs):
-            s, r = b.ar.launch_lists(par)
-            send[i], send[k + i], recv[i] = s.arr[0], s.arr[1], r.arr[0]
-            send[i].ratio = b.ar.compression_ratio
-            send[i].dtype = send[k + i].dtype = g["table"].code
-            send[i].g = send[k + i].g = None
-            send[i].fold = send[k + i].fold = C.addressof(g["table"].args[b])
-            if i:                                # buckets share no vector, slot or scratch
-                send[k + i].chain = recv[i].chain = 1
-        got = g["lists"][par] = [cfg, send, recv, [recv[i].apply for i in range(k)], None]
-        return got
-
-    def _send_all(self, lr, mu) -> None:
-        """First half of the exchange of all buckets: the norms of all tensors, all thresholds, then
-        one fold-and-compress kernel per bucket."""
-        env, g, buckets = self._env, self._group(), self._buckets
-        ft = g["table"]
-        ft.refresh(self._zeros)
-        clip, mu, lr = self._fold_scalars(lr, mu)
-        ft.launch_coef(clip, lr)
-        for b in buckets:
-            self._fold_args(ft, b, mu)
-            b.seq, b.par = b.ar.next_step()
-            b.sent = True
-        seq, par = buckets[0].seq, buckets[0].par
-        send = self._lists(g, par)[1]
-        _lib.check(env.lib.cx_run_ops(send, len(send), seq, _lib.stream_ptr(env.device)), "cx_run_ops")
-
-    def _recv_all(self, lr, mu, wd) -> None:
-        """Second half: one wait-decode-update kernel per bucket."""
-        env, buckets = self._env, self._buckets
-        got = self._lists(self._group(), buckets[0].par)
-        recv, views, hyper = got[2], got[3], (lr, mu, wd, self.momentum_correction)
-        if got[4] != hyper:
-            for b, v in zip(buckets, views):
-                C.pointer(v)[0] = self._args(b.start, b.end - b.start, lr, mu, wd, 1.0 / env.ranks)
-            got[4] = hyper
+    def _run_plan(self, par, seq: int, lr, mu, wd) -> None:
+        plan = self._plan(par)
+        plan.table.refresh(self._zeros)
+        hyper = (lr, mu, wd, self.momentum_correction, self.pre_clipnorm)
+        if plan.hyper != hyper:
+            plan.set_hyper(self, lr, mu, wd)
+            plan.hyper = hyper
         elif self.rule == "adamw":               # the bias corrections move with every step
             bc1, bc2 = 1.0 - self.betas[0] ** self._t, 1.0 - self.betas[1] ** self._t
-            for v in views:
+            for v in plan.views:
                 v.bc1, v.bc2 = bc1, bc2
-        _lib.check(env.lib.cx_run_ops(recv, len(recv), buckets[0].seq, _lib.stream_ptr(env.device)), "cx_run_ops")
-
-    def _step_local(self, lr, mu, wd) -> None:
-        """The step of a rank that exchanges nothing: norms, then one fold-and-update kernel over the
-        whole flat buffer."""
-        env, g = self._env, self._group()
-        ft = g["table"]
-        ft.refresh(self._zeros)
-        args = self._args(0, self.blob_size, lr, mu, wd, 1.0)
-        clip, mu, lr = self._fold_scalars(lr, mu)
-        ft.launch_coef(clip, lr)
-        fold = ft.fold_args(None, self._update if self._keeps_u else None, mu)
-        _lib.check(env.lib.cx_fold_update(ft.code, C.byref(fold), self.blob_size, C.byref(args),
-                                          _lib.stream_ptr(env.device)), "cx_fold_update")
+        _lib.check(self._env.lib.cx_run_ops(plan.ops, plan.count, seq, _lib.stream_ptr(self._env.device)), "cx_run_ops")
 
     def _hyper(self):
         """The update kernels take one learning rate, momentum and weight decay for the whole flat
@@ -585,8 +584,6 @@ class ComprexOptimizer(torch.optim.Optimizer):
         """Context for gradient accumulation with ``overlap=True``: backward passes inside it
         only accumulate; the buckets go out during the first backward pass after it (or in
         ``step``)."""
-        import contextlib
-
         @contextlib.contextmanager
         def ctx():
             armed, self._armed = self._armed, False
@@ -640,12 +637,11 @@ class ComprexOptimizer(torch.optim.Optimizer):
             comm.wait_stream(torch.cuda.current_stream(self._env.device))
             ctx = torch.cuda.stream(comm)
         else:
-            import contextlib
             ctx = contextlib.nullcontext()
         with ctx:
             if self._local and self._cuda:
                 with nvtx_range("comprex.update"):
-                    self._step_local(lr, mu, wd)
+                    self._run_plan(None, 0, lr, mu, wd)
             else:
                 self._exchange(lr, mu, wd)
         if use_side:
@@ -657,12 +653,11 @@ class ComprexOptimizer(torch.optim.Optimizer):
     def _exchange(self, lr, mu, wd) -> None:
         pending = [b for b in self._buckets if not b.sent]     # everything that the hooks did not send yet
         if len(pending) == len(self._buckets) and self._in_step():
-            with nvtx_range("comprex.fold+send"):
-                self._send_all(lr, mu)
-            with nvtx_range("comprex.recv+update"):
-                self._recv_all(lr, mu, wd)
             for b in self._buckets:
-                b.sent, b.ready = False, 0
+                b.seq, b.par = b.ar.next_step()
+                b.ready = 0
+            with nvtx_range("comprex.exchange"):
+                self._run_plan(self._buckets[0].par, self._buckets[0].seq, lr, mu, wd)
             return
         for b in pending:
             self._send(b)

@@ -29,11 +29,15 @@ def nvtx_enabled() -> bool:
     return _nvtx_on and torch.cuda.is_available()
 
 
-@contextlib.contextmanager
+_no_range = contextlib.nullcontext()
+
+
 def nvtx_range(name: str):
-    if not nvtx_enabled():
-        yield
-        return
+    return _nvtx_range(name) if _nvtx_on and nvtx_enabled() else _no_range
+
+
+@contextlib.contextmanager
+def _nvtx_range(name: str):
     torch.cuda.nvtx.range_push(name)
     try:
         yield

@@ -673,7 +673,7 @@ def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange):
         assert len(opt._buckets) > 2
         if not fused:
             opt._fusable = lambda b: False
-            opt._step_local = lambda lr, mu, wd: opt._exchange(lr, mu, wd)
+            opt._cuda = False
         for step in range(4):
             gen = torch.Generator(device="cuda").manual_seed(step)
             for i, p in enumerate(params):

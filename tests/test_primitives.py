@@ -696,6 +696,46 @@ def test_rle_fused_receive_rejects_corrupt_runs(world):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 1000, 1023, 8 * 1024, 8 * 1024 + 1, 100003, 296 * 8 * 1024, 296 * 8 * 1024 + 1])
+@pytest.mark.parametrize("ratio", [0.001, 0.01, 0.1, 0.7])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_threshold_and_compress_as_one_list(n, ratio, dtype):
+    """The op list [threshold, compress] (one kernel up to a grid that is resident as a whole) gives
+    threshold, payload and residual of the two launches issued one by one, call after call; views at
+    odd addresses too."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    e0, e1 = world.envs
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    slots = [[P.SparseSlot.create(e, n, n) for e in world.envs][1] for _ in range(2)]
+    comps = [P.Compressor(e0, n) for _ in range(2)]
+    for shift in (0, 1):
+        rs = [torch.randn(n + 1, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))[shift:shift + n].mul(0.5)
+              for _ in range(2)]
+        if shift:
+            rs = [torch.cat((torch.zeros(1, device="cuda"), r))[1:] for r in rs]
+        for seq in (1, 2, 3):
+            g = torch.randn(n + 1, device="cuda", generator=gen).to(dtype)[shift:shift + n]
+            comps[0].threshold_topk(g, rs[0], n, ratio)
+            comps[0].compress(g, rs[0], n, n, seq, P.make_targets([slots[0].endpoint(e0, 1)]))
+            ops = (_lib.Op * 2)(*comps[1].send_ops(rs[1], n, n, P.make_targets([slots[1].endpoint(e0, 1)]), ratio, 1000, 10.0))
+            for o in ops:
+                o.g, o.dtype = g.data_ptr(), _lib.dtype_code(dtype)
+            before = _lib.launch_count()
+            _lib.check(e0.lib.cx_run_ops(ops, 2, seq, _lib.stream_ptr(e0.device)))
+            launches = _lib.launch_count() - before
+            e0.flush()
+            small = n <= 296 * 8 * 1024 and min(n, max(1000, int(10 / ratio))) <= 1024
+            assert launches == (1 if small else 2), launches
+            assert torch.equal(comps[0].thr, comps[1].thr)
+            a, b = (read_pairs(e1, s) for s in slots)
+            assert a[0].seq == b[0].seq == seq and a[0].nnz == b[0].nnz and a[0].nnz_found == b[0].nnz_found
+            for x, y in zip(a[1:], b[1:]):
+                assert torch.equal(x, y)
+            assert torch.equal(rs[0], rs[1])
+    world.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [1000, 4096, 100003, (1 << 22) + 5])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_cuda_kernels_match_host_bitwise(n, dtype):
