@@ -33,7 +33,6 @@
 #include <string.h>
 
 #include "cx_fold.cuh"
-#include "cx_select.cuh"
 
 namespace {
 
@@ -385,8 +384,6 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
 // out) and the status says why.
 constexpr int kArrived = 32, kOver = 44, kFailed = 54;     // bit positions behind the survivors; grids have < 4096 CTAs
 
-constexpr int kGathered = 8;   // CxWorkCounters::pad: CTAs that have read their sample (compress_sampled_kernel)
-
 template <int MAX_WARPS>
 __device__ __forceinline__ void compress_finish(const CompressParams& p, const int tid, const float thr, const bool failed,
                                                 const Tally& tally) {
@@ -406,9 +403,7 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
     for (int w = 0; w < nw; ++w) { found += s_found[w]; mark |= s_mark[w]; }
     const unsigned long long mine = (unsigned long long)found | 1ull << kArrived |
                                     (mark & 1u ? 1ull << kOver : 0ull) | (mark & 2u ? 1ull << kFailed : 0ull);
-    __threadfence();          // as in cx::cta_arrive
-    s_all = atomicAdd(reinterpret_cast<unsigned long long*>(&p.ctr->done), mine) + mine;
-    __threadfence();
+    s_all = cx::arrive_u64(reinterpret_cast<unsigned long long*>(&p.ctr->done), mine) + mine;   // as in cx::cta_arrive
     s_nnz = 0;
   }
   __syncthreads();
@@ -449,7 +444,6 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
       p.stats->threshold = thr;
     }
     *reinterpret_cast<unsigned long long*>(&p.ctr->done) = 0;
-    p.ctr->pad[kGathered] = 0;
   }
   CX_TRACE(6);
 }
@@ -522,93 +516,6 @@ compress_kernel(const __grid_constant__ CompressParams p) {
 #endif
   CX_TRACE(2);
   compress_finish<kWarps>(p, tid, thr, false, tally);
-}
-
-// Threshold estimate and compression of a small vector in one kernel.  Two kernels cost a launch more
-// on the host and, on the GPU, the end of the first and the look-up of its result by the second.  Here
-// every CTA gathers the whole sample (at most 1024 elements, all in L2) and selects the threshold for
-// itself while its sub-tiles are on their way to registers.  The residual is sampled and updated in the
-// same kernel, so no CTA writes before all have gathered: they count themselves in and the count is
-// watched while the selection runs.  The launch is cooperative, so all CTAs are resident and the wait
-// ends; it is bounded all the same (a failed one publishes nothing and leaves the residual alone).
-struct SampledParams {
-  CompressParams c;
-  int32_t samples, use_all;
-  float stepsize;
-  int32_t topk_pos;
-  float* thr_out;
-};
-constexpr int kMaxSample = 1024;
-
-template <typename T, bool MC>
-__global__ void __launch_bounds__(kThreads, CX_COMPRESS_MIN_BLOCKS)
-compress_sampled_kernel(const __grid_constant__ SampledParams q) {
-  __shared__ CxPair s_stage[kWarps][kStage];     // first the selection's scratch
-  __shared__ uint32_t s_keys[kMaxSample];
-  __shared__ float s_thr;
-  __shared__ uint32_t s_ok;
-  static_assert(sizeof(CxPair) * kStage * kWarps >= 4 * kMaxSample, "selection scratch");
-  const CompressParams& p = q.c;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const T* __restrict__ g = reinterpret_cast<const T*>(p.g);
-  float* __restrict__ r = p.r;
-  cx::pdl_wait();
-  const uint32_t nfull = p.vec ? (uint32_t)(p.n / CX_SUBTILE) : 0u;
-  const uint32_t sub = blockIdx.x * kWarps + warp;          // one per warp: the grid covers the vector
-  const int64_t off = (int64_t)sub * CX_SUBTILE;
-  float a[kMaxSample / kThreads], b[kMaxSample / kThreads];
-#pragma unroll
-  for (int u = 0; u < kMaxSample / kThreads; ++u) {
-    const int i = tid + u * kThreads;
-    a[u] = b[u] = 0.f;
-    if (i < q.samples) {
-      const int64_t pos = cx::sample_position(i, p.n, q.use_all, q.stepsize);
-      a[u] = r[pos];
-      b[u] = cx::Elem<T>::to_f(g[pos]);
-    }
-  }
-  float v[kChunks][4];
-  if (sub < nfull) load_subtile<T, true, true>(g + off, r + off, lane, v);
-#pragma unroll
-  for (int u = 0; u < kMaxSample / kThreads; ++u)
-    s_keys[tid + u * kThreads] = __float_as_uint(fabsf(a[u] + b[u]));
-  __syncthreads();
-  if (tid == 32) {
-    bool ok = gridDim.x == 1;
-    if (!ok) {
-      const uint32_t seen = atomicAdd(&p.ctr->pad[kGathered], 1u) + 1u;
-      ok = seen == gridDim.x;
-      const uint64_t t0 = cx::globaltimer_ns();
-      for (uint32_t it = 0; !ok && it < (1u << 24); ++it) {
-        ok = *reinterpret_cast<volatile uint32_t*>(&p.ctr->pad[kGathered]) == gridDim.x;
-        if (!ok && (it & 63) == 63 && cx::globaltimer_ns() - t0 > 1000000000ull) break;
-      }
-    }
-    s_ok = ok ? 1u : 0u;
-  }
-  if (warp == 0) {
-    float thr;
-    if (q.topk_pos <= 0) {                                   // the estimate says: send nothing
-      uint32_t mx = 0;
-      for (int j = 0; j < kMaxSample / 32; ++j) mx = max(mx, s_keys[32 * j + lane]);
-      thr = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) + 1.0f;
-    } else {
-      thr = __uint_as_float(cx::warp_select(s_keys, q.samples, (uint32_t)q.topk_pos, lane, reinterpret_cast<uint32_t*>(s_stage)));
-    }
-    if (lane == 0) {
-      s_thr = thr;
-      if (blockIdx.x == 0) *q.thr_out = thr;
-    }
-  }
-  __syncthreads();
-  const float thr = s_thr;
-  const bool ok = s_ok != 0;
-  Tally tally = {0, false};
-  if (ok) {
-    if (sub < nfull) emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v, tally);
-    else if (sub < p.nsub) compress_subtile_edge<T, true, true, MC>(p, sub, lane, thr, g, r, tally);
-  }
-  compress_finish<kWarps>(p, tid, thr, !ok, tally);
 }
 
 // The same for a vector that is folded from gradient tensors on the way (CxFold): what the fold
@@ -894,66 +801,6 @@ void launch_fold_input(const FoldCompressParams& q, cudaStream_t s) {
 
 }  // namespace
 
-extern "C" void cx_threshold_plan(int64_t n, float ratio, int default_subsamples, float subsample_factor,
-                                  int32_t* samples, int32_t* use_all, float* stepsize, int32_t* topk_pos);
-
-namespace {
-
-template <typename T, bool MC>
-int launch_sampled_mc(const SampledParams& q, int grid, cudaStream_t s) {
-  auto kern = compress_sampled_kernel<T, MC>;
-  static int per_sm[64] = {0};                // resident CTAs per SM, asked once per device
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (!per_sm[dev]) {
-    int k = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kThreads, 0) != cudaSuccess) return 0;
-    per_sm[dev] = k > 0 ? k : -1;
-  }
-  if (per_sm[dev] < 0 || grid > per_sm[dev] * cx_sm_count()) return 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, q);
-  if (e != cudaSuccess) return cx_set_error("compress_sampled_kernel launch", (int)e);
-  cx_note_launch();
-  return 1;
-}
-
-}  // namespace
-
-// Threshold and compress ops of one vector as one launch, where it pays: a sample of at most 1024
-// elements and one sub-tile per warp of a grid that is resident as a whole.  Returns 1 when launched,
-// 0 when the two ops have to be launched one by one, or a negative error.
-int cx_compress_sampled_cuda(const CxOp* t, const CxOp* c, uint64_t seq, void* stream) {
-  if (t->n != c->n || t->g != c->g || t->r != c->r || t->dtype != c->dtype || t->thr != c->thr || t->fold || c->fold ||
-      !c->g || !c->r || c->n <= 0 || c->n > (int64_t)CX_SUBTILE * kWarps * 1024 || cx_seq_cell() != nullptr ||
-      c->ws_bytes < cx_workspace_bytes(c->n) || c->tg.count < 0 || c->tg.count >= CX_MAX_PEERS || bulk_wanted())
-    return 0;
-  SampledParams q;
-  cx_threshold_plan(t->n, t->ratio, t->default_subsamples, t->subsample_factor, &q.samples, &q.use_all, &q.stepsize, &q.topk_pos);
-  if (q.samples > kMaxSample) return 0;
-  q.thr_out = t->thr;
-  fill_params(q.c, c->g, c->r, c->n, c->thr, c->cap, seq, &c->tg, c->workspace, c->stats, c->src_rank);
-  const size_t esz = c->dtype == CX_F32 ? 4 : 2;
-  q.c.vec = (reinterpret_cast<uintptr_t>(c->r) & 15) == 0 && (reinterpret_cast<uintptr_t>(c->g) & (4 * esz - 1)) == 0;
-  const int grid = (int)((q.c.nsub + kWarps - 1) / kWarps);
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const bool mc = (c->tg.pad & CX_TG_MULTICAST) != 0;
-  switch (c->dtype) {
-    case CX_F32: return mc ? launch_sampled_mc<float, true>(q, grid, s) : launch_sampled_mc<float, false>(q, grid, s);
-    case CX_BF16: return mc ? launch_sampled_mc<__nv_bfloat16, true>(q, grid, s) : launch_sampled_mc<__nv_bfloat16, false>(q, grid, s);
-    case CX_F16: return mc ? launch_sampled_mc<__half, true>(q, grid, s) : launch_sampled_mc<__half, false>(q, grid, s);
-    default: return 0;
-  }
-}
-
 int cx_compress_fold_cuda(int gdtype, const CxFold* fold, float* r, int64_t n, const float* thr, uint32_t cap,
                           uint64_t seq, const CxTargets* tg, void* workspace, int64_t ws_bytes, CxStats* stats,
                           uint32_t src_rank, void* stream) {
@@ -977,6 +824,7 @@ int cx_compress_fold_cuda(int gdtype, const CxFold* fold, float* r, int64_t n, c
     case CX_F16: launch_fold_input<__half>(q, s); break;
     default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
   }
+  cx_note_stream(stream, false);
   cx_note_launch();
   return cx_check_launch("compress_fold_kernel");
 }
@@ -995,6 +843,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (n == 0) {
     compress_empty_kernel<<<1, 32, 0, s>>>(p);
+    cx_note_stream(stream, false);
     cx_note_launch();
     return cx_check_launch("compress_empty_kernel");
   }
@@ -1012,6 +861,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
       default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
     }
     if (rc) return rc;
+    cx_note_stream(stream, false);
     cx_note_launch();
     return cx_check_launch("compress_bulk_kernel");
   }
@@ -1022,6 +872,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
     case CX_F16: launch_mode<__half>(p, grid, s); break;
     default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
   }
+  cx_note_stream(stream, false);
   cx_note_launch();
   return cx_check_launch("compress_kernel");
 }

@@ -164,13 +164,21 @@ const uint64_t* cx_seq_cell();
 // one thread per CTA at system scope 9.8 us, one thread per CTA at GPU scope 3.7 us (1.3 us for
 // the arrival, 1.9 us for the release of the headers).
 namespace cx {
+// count in: everything ordered before by this thread is visible before the count, everything after it
+// sees what the earlier arrivals published (one instruction instead of fence, atomic, fence)
+__device__ __forceinline__ uint32_t arrive_u32(uint32_t* p, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ unsigned long long arrive_u64(unsigned long long* p, unsigned long long v) {
+  unsigned long long old;
+  asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
+  return old;
+}
 __device__ __forceinline__ bool cta_arrive(uint32_t* counter, uint32_t group, uint32_t* s_last) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    *s_last = (atomicAdd(counter, 1u) == group - 1u) ? 1u : 0u;
-    __threadfence();
-  }
+  if (threadIdx.x == 0) *s_last = arrive_u32(counter, 1u) == group - 1u ? 1u : 0u;
   __syncthreads();
   return *s_last != 0u;
 }
@@ -236,6 +244,14 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 }  // namespace cx
 
 bool cx_pdl_enabled();   // COMPREX_PDL != 0 (read once)
+
+// The kernels that end a message or a step call pdl_trigger at their start: the kernel behind (the
+// threshold of the next message, the norms of the next step) waits at its own start, and its launch
+// is over when it may go on.  A receive kernel, however, does not wait at its start when its sender is
+// in front of it, so it has to know what is: senders note "not early", kernels that trigger at their
+// start note "early", and cx_front_wait says whether the kernel about to be launched must wait first.
+void cx_note_stream(const void* stream, bool early);
+bool cx_front_wait(const void* stream);
 
 // Launches of one op list that may overlap (CxOp::chain), for the op this thread issues right now.
 // A chained kernel does not wait for the one in front before it starts, only before it ends, so that

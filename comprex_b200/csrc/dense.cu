@@ -110,6 +110,7 @@ __device__ __forceinline__ void mc_store4(__half* mc, const float (&v)[4]) {
 
 template <typename T, bool HAS_R>
 __global__ void __launch_bounds__(kThreads, 4) dense_send_kernel(const __grid_constant__ SendParams p) {
+  cx::pdl_wait();
   __shared__ uint32_t s_last;
   const T* __restrict__ g = reinterpret_cast<const T*>(p.g);
   const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -216,6 +217,7 @@ struct ReduceParams {
   uint64_t timeout_ns;
   Ranges rg;           // gather mode: source j lands at out[start_j .. start_j+len_j)
   int32_t gather;
+  int32_t front_wait;  // the kernel in front may be at work on the same vectors
   int32_t vec16;       // every operand and target takes 16-byte accesses
 };
 
@@ -438,6 +440,8 @@ __device__ __forceinline__ void dense_reduce_body(const ReduceParams& p) {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 4) dense_reduce_kernel(const __grid_constant__ ReduceParams p) {
+  if (!p.has_push) cx::pdl_trigger();      // (a pushing reduce is a sender too: receivers behind it do not wait)
+  if (p.front_wait) cx::pdl_wait();
   dense_reduce_body<T>(p);
   cx::pdl_wait();   // launched early behind the sending kernel: do not complete before that grid has
 }
@@ -502,18 +506,20 @@ int cx_dense_send_cuda(int dtype, const void* g, float* r, int64_t n, uint64_t s
   }
   const int grid = grid_for(work, starts || r ? 8 : 4);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const bool capturing = p.seq_cell != nullptr;
+  cx_note_stream(stream, false);
   switch (dtype) {
     case CX_F32:
-      if (r) dense_send_kernel<float, true><<<grid, kThreads, 0, s>>>(p);
-      else dense_send_kernel<float, false><<<grid, kThreads, 0, s>>>(p);
+      if (r) cx_launch_pdl(dense_send_kernel<float, true>, grid, kThreads, 0, s, p, capturing);
+      else cx_launch_pdl(dense_send_kernel<float, false>, grid, kThreads, 0, s, p, capturing);
       break;
     case CX_BF16:
-      if (r) dense_send_kernel<__nv_bfloat16, true><<<grid, kThreads, 0, s>>>(p);
-      else dense_send_kernel<__nv_bfloat16, false><<<grid, kThreads, 0, s>>>(p);
+      if (r) cx_launch_pdl(dense_send_kernel<__nv_bfloat16, true>, grid, kThreads, 0, s, p, capturing);
+      else cx_launch_pdl(dense_send_kernel<__nv_bfloat16, false>, grid, kThreads, 0, s, p, capturing);
       break;
     case CX_F16:
-      if (r) dense_send_kernel<__half, true><<<grid, kThreads, 0, s>>>(p);
-      else dense_send_kernel<__half, false><<<grid, kThreads, 0, s>>>(p);
+      if (r) cx_launch_pdl(dense_send_kernel<__half, true>, grid, kThreads, 0, s, p, capturing);
+      else cx_launch_pdl(dense_send_kernel<__half, false>, grid, kThreads, 0, s, p, capturing);
       break;
     default: return cx_set_error("cx_dense_send: unsupported dtype on CUDA", 0);
   }
@@ -535,6 +541,8 @@ int cx_dense_reduce_cuda(int dtype, void* out, const void* own, int64_t n, const
   p.ctr = reinterpret_cast<CxWorkCounters*>(counters);
   p.status = status; p.timeout_ns = timeout_ns;
   p.gather = starts != nullptr;
+  p.front_wait = cx_front_wait(stream) ? 1 : 0;
+  cx_note_stream(stream, !p.has_push);
   {
     uintptr_t bits = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(own);
     for (int j = 0; j < src->count; ++j) bits |= reinterpret_cast<uintptr_t>(src->ep[j].pairs);

@@ -26,7 +26,6 @@
 // ---- forward declarations of the two back ends --------------------------------
 int cx_threshold_topk_cuda(int, const void*, const float*, int64_t, float, int, float, float*, void*, int64_t, void*);
 int cx_threshold_batch_cuda(const CxOp*, int, void*);
-int cx_compress_sampled_cuda(const CxOp*, const CxOp*, uint64_t, void*);
 int cx_threshold_topk_host(int, const void*, const float*, int64_t, float, int, float, float*);
 int cx_compress_cuda(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
                      const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
@@ -86,6 +85,19 @@ int cx_set_error(const char* where, int cuda_err) {
 void cx_note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static thread_local const uint64_t* g_seq_cell = nullptr;
 const uint64_t* cx_seq_cell() { return g_seq_cell; }
+// Whether the kernel this library launched last on a stream lets the kernel behind it in before it has
+// finished (cx_device.cuh).  A slot per stream (hashed); what is not known counts as one that does.
+static std::atomic<uint64_t> g_last[64];
+static std::atomic<uint64_t>& last_slot(const void* stream) {
+  const uint64_t s = reinterpret_cast<uint64_t>(stream);
+  return g_last[(s >> 4 ^ s >> 10 ^ s >> 16) & 63];
+}
+void cx_note_stream(const void* stream, bool early) {
+  last_slot(stream).store(reinterpret_cast<uint64_t>(stream) << 2 | 2u | (early ? 1u : 0u), std::memory_order_relaxed);
+}
+bool cx_front_wait(const void* stream) {
+  return last_slot(stream).load(std::memory_order_relaxed) != (reinterpret_cast<uint64_t>(stream) << 2 | 2u);
+}
 static thread_local uint32_t g_chain_bits = 0;
 uint32_t cx_chain_bits() { return g_chain_bits; }
 int cx_check_launch(const char* where) {
@@ -342,14 +354,8 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
     forked = false;
     return 0;
   };
-  // thresholds that follow one another on one lane share launches, one in front of the compression of a
-  // small vector shares its kernel
+  // thresholds that follow one another on one lane share launches
   auto run_some = [&](int i, void* on) -> int {      // ops taken, or a negative error
-    if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA && i + 1 < count &&
-        ops[i + 1].kind == CX_OPK_COMPRESS && ops[i + 1].dev == CX_DEV_CUDA && ops[i + 1].lane == ops[i].lane) {
-      const int one = cx_compress_sampled_cuda(ops + i, ops + i + 1, seq, on);      // a small vector: one kernel
-      if (one) return one > 0 ? 2 : one;
-    }
     if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA) return cx_threshold_batch_cuda(ops + i, count - i, on);
     auto chained = [&](int k) {
       return k > 0 && k < count && ops[k].chain && ops[k].kind == ops[k - 1].kind && ops[k].lane == ops[k - 1].lane;

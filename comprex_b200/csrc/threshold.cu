@@ -28,7 +28,6 @@
 #include <string.h>
 
 #include "cx_fold.cuh"
-#include "cx_select.cuh"
 
 namespace {
 
@@ -52,9 +51,28 @@ struct ThreshBatch {
   ThreshParams v[NV];
 };
 
+// element that sample i looks at (the reference's float arithmetic)
+__device__ __forceinline__ int64_t sample_position(int i, int64_t n, int use_all, float stepsize) {
+  if (use_all) return i;
+  const int64_t pos = (int64_t)(int)__fmul_rn((float)i, stepsize);
+  return pos > n - 1 ? n - 1 : pos;
+}
+
+// One warp, one key per lane, the first `count` lanes: the key of rank `rank` in descending order.
+__device__ __forceinline__ uint32_t warp_rank(uint32_t key, int count, int lane, uint32_t rank) {
+  uint32_t gt = 0, ge = 0;
+  for (int j = 0; j < count; ++j) {
+    const uint32_t other = __shfl_sync(0xffffffffu, key, j);
+    gt += other > key ? 1u : 0u;
+    ge += other >= key ? 1u : 0u;
+  }
+  const uint32_t who = __ballot_sync(0xffffffffu, lane < count && gt <= rank && rank < ge);
+  return __shfl_sync(0xffffffffu, key, __ffs(who) - 1);
+}
+
 template <typename T, bool FOLD>
 __device__ __forceinline__ uint32_t sample_key(const ThreshParams& p, int i) {
-  const int64_t pos = cx::sample_position(i, p.n, p.use_all, p.stepsize);
+  const int64_t pos = sample_position(i, p.n, p.use_all, p.stepsize);
   float x = 0.f;
   if (p.r) x = p.r[pos];
   if (FOLD) x = x + cx::fold_at<T>(p.fold, pos);
@@ -126,7 +144,7 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
       if (lane == 0) s_red[w] = wm;
       __syncthreads();
       if (w == 0) {
-        const uint32_t b0 = cx::warp_rank(s_red[lane], 32, lane, rank);
+        const uint32_t b0 = warp_rank(s_red[lane], 32, lane, rank);
         if (lane == 0) s_sel[1] = b0;
       }
       __syncthreads();
@@ -143,7 +161,7 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
     }
     __syncthreads();
     const uint32_t left = s_sel[0];
-    if (left <= 32) return w == 0 ? cx::warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
+    if (left <= 32) return w == 0 ? warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
     if (left <= kThreads) return block_rank(tid < (int)left ? s_hist[tid] : 0u, (int)left, rank);
   }
   uint32_t prefix = 0, prefmask = 0;
@@ -189,9 +207,6 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   const bool cached = s <= kSmemKeys;
   uint32_t* keys0 = ncta > 1 ? cluster.map_shared_rank(s_keys, 0) : s_keys;
   cx::pdl_wait();     // resident early: what the kernel in front wrote may be read from here on
-  // the compress kernel queued behind this one may start now: it loads what both only read, and waits
-  // for this grid to finish before it reads the threshold or writes the residual
-  cx::pdl_trigger();
 
   // pass 0: gather the sample (and its maximum, for the sentinel case); CTA c of a cluster
   // takes the samples [c, c+1) * s / ncta
@@ -213,6 +228,10 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
       }
     }
   }
+  // the compress kernel queued behind this one may start now: it loads what both only read, and waits
+  // for this grid to finish before it reads the threshold or writes the residual.  (Let in before the
+  // gather, its 20 MB of loads were in front of the sample's.)
+  cx::pdl_trigger();
   if (ncta > 1) {
     if (p.topk_pos <= 0) {
       const uint32_t wm = __reduce_max_sync(0xffffffffu, mx);
@@ -378,10 +397,11 @@ __global__ void __launch_bounds__(kExactThreads) exact_select_kernel(const Exact
 // 10 M elements, fp32 vector and residual, top-k 1 %: 96 us with four passes.
 constexpr int kBracket = 8192;
 constexpr int kCluster = 8;
+constexpr int kBracketThreads = 512;   // fits next to a receive kernel's CTAs
 constexpr int kBins = 2048;          // 11 bits per radix pass of the finish
 constexpr int kCollectThreads = 256;
 constexpr int kCollectEach = 8;      // elements per thread and round
-constexpr int kBuffer = 4096;        // candidates a CTA keeps before it appends them to the list
+constexpr int kBuffer = 3072;        // candidates a CTA keeps before it appends them to the list
 constexpr int kCollectPerSm = 6;
 
 struct ExactState {                  // in the workspace behind the histograms; zero between calls
@@ -419,13 +439,63 @@ __device__ __forceinline__ uint32_t key_at(const OnePassParams& p, int64_t i) {
   return __float_as_uint(fabsf(x));
 }
 
+// The digit of a 2048-bin histogram that holds `rank`, walked from the top; all THREADS threads.
+template <int THREADS>
+__device__ __forceinline__ uint32_t pick_bin(const uint32_t* hist, uint32_t& rank, uint32_t* s_warp, uint32_t* s_out) {
+  constexpr int kEach = kBins / THREADS;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  uint32_t h[kEach], sum = 0;
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) { h[j] = hist[kBins - 1 - kEach * tid - j]; sum += h[j]; }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) s_warp[w] = incl;
+  __syncthreads();
+  // lane j holds warp j's sum: the warps before mine
+  uint32_t before = __reduce_add_sync(0xffffffffu, lane < w ? s_warp[lane] : 0u) + incl - sum;
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    if (rank >= before && rank < before + h[j]) { s_out[0] = kBins - 1 - kEach * tid - j; s_out[1] = rank - before; }
+    before += h[j];
+  }
+  __syncthreads();
+  rank = s_out[1];
+  return s_out[0];
+}
+
+// The key of rank `rank` among s_keys[0, count): three radix passes (11, 11, 9 bits).
+template <int THREADS>
+__device__ __forceinline__ uint32_t radix_rank(const uint32_t* s_keys, int count, uint32_t rank, uint32_t* s_hist,
+                                               uint32_t* s_warp, uint32_t* s_out) {
+  uint32_t prefix = 0, mask = 0;
+#pragma unroll
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = pass == 0 ? 20 : pass == 1 ? 9 : 0;
+    const uint32_t low = pass == 2 ? 511u : 2047u;
+    for (int i = threadIdx.x; i < kBins; i += THREADS) s_hist[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < count; i += THREADS) {
+      const uint32_t k = s_keys[i];
+      if ((k & mask) == prefix) atomicAdd(&s_hist[(k >> shift) & low], 1u);
+    }
+    __syncthreads();
+    prefix |= pick_bin<THREADS>(s_hist, rank, s_warp, s_out) << shift;
+    mask |= low << shift;
+  }
+  return prefix;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant__ OnePassParams p) {
+__global__ void __launch_bounds__(kBracketThreads) bracket_kernel(const __grid_constant__ OnePassParams p) {
   namespace cg = cooperative_groups;
   __shared__ uint32_t s_keys[kBracket];
-  __shared__ uint32_t s_hist[kThreads];
-  __shared__ uint32_t s_sel[2];
-  __shared__ uint32_t s_red[kThreads / 32];
+  __shared__ uint32_t s_hist[kBins];
+  __shared__ uint32_t s_out[2];
+  __shared__ uint32_t s_warp[kBracketThreads / 32];
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned crank = cluster.block_rank();
   const int tid = threadIdx.x;
@@ -434,20 +504,23 @@ __global__ void __launch_bounds__(kThreads) bracket_kernel(const __grid_constant
   cx::pdl_wait();
   cx::pdl_trigger();
   {
-    const uint32_t i = crank * kThreads + tid;
-    const int64_t a = (int64_t)(((uint64_t)p.n * i) / kBracket), b = (int64_t)(((uint64_t)p.n * (i + 1)) / kBracket);
-    const uint32_t h = (i + 1) * 2654435761u;
-    const uint32_t k = key_at<T>(p, a + (int64_t)(((uint64_t)(h ^ (h >> 15)) * (uint64_t)(b - a)) >> 32));
-    k0[i] = k;
-    k1[i] = k;
+    constexpr int kEach = kBracket / kCluster / kBracketThreads;
+    uint32_t k[kEach];
+#pragma unroll
+    for (int u = 0; u < kEach; ++u) {
+      const uint32_t i = (crank * kEach + u) * kBracketThreads + tid;
+      const int64_t a = (int64_t)(((uint64_t)p.n * i) / kBracket), b = (int64_t)(((uint64_t)p.n * (i + 1)) / kBracket);
+      const uint32_t h = (i + 1) * 2654435761u;
+      k[u] = key_at<T>(p, a + (int64_t)(((uint64_t)(h ^ (h >> 15)) * (uint64_t)(b - a)) >> 32));
+    }
+#pragma unroll
+    for (int u = 0; u < kEach; ++u) k0[(crank * kEach + u) * kBracketThreads + tid] = k1[(crank * kEach + u) * kBracketThreads + tid] = k[u];
   }
   cluster.sync();                     // CTA 0 selects lo, CTA 1 hi, each in its own shared memory
   if (crank > 1) return;
   const uint32_t rank = crank == 0 ? p.lo_rank : p.hi_rank;
   uint32_t key = crank == 0 ? 0u : 0xffffffffu;
-  if (rank != ~0u) {
-    key = select_cached(s_keys, kBracket, rank, s_red, s_hist, s_sel);
-  }
+  if (rank != ~0u) key = radix_rank<kBracketThreads>(s_keys, kBracket, rank, s_hist, s_warp, s_out);
   if (tid == 0) {
     if (crank == 0) p.st->lo = key;
     else p.st->hi = key;
@@ -551,27 +624,6 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
   if (s_fill) flush();
 }
 
-// the digit of a 2048-bin histogram that holds `rank`, walked from the top; block-wide, 1024 threads
-__device__ __forceinline__ uint32_t pick_bin(const uint32_t* hist, uint32_t& rank, uint32_t* s_warp, uint32_t* s_out) {
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const uint32_t a = hist[kBins - 1 - 2 * tid], b = hist[kBins - 2 - 2 * tid];
-  uint32_t incl = a + b;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += t;
-  }
-  if (lane == 31) s_warp[w] = incl;
-  __syncthreads();
-  uint32_t before = incl - a - b;
-  for (int j = 0; j < w; ++j) before += s_warp[j];
-  if (rank >= before && rank < before + a) { s_out[0] = kBins - 1 - 2 * tid; s_out[1] = rank - before; }
-  else if (rank >= before + a && rank < before + a + b) { s_out[0] = kBins - 2 - 2 * tid; s_out[1] = rank - before - a; }
-  __syncthreads();
-  rank = s_out[1];
-  return s_out[0];
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_constant__ OnePassParams p) {
   namespace cg = cooperative_groups;
@@ -611,7 +663,7 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
   if (list) {
     const int shift = max(bits - 11, 0);
     uint32_t in_bin = rank;
-    const uint32_t bin = pick_bin(s_hists[2], in_bin, s_warp, s_out);      // every CTA for itself
+    const uint32_t bin = pick_bin<kThreads>(s_hists[2], in_bin, s_warp, s_out);      // every CTA for itself
     if (s_hists[2][bin] <= kThreads) {
       uint32_t* few = cluster.map_shared_rank(s_hists[0], 0);              // [0]: their number
       uint32_t* keys = cluster.map_shared_rank(s_hists[1], 0);
@@ -627,13 +679,15 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
       cluster.sync();
       if (crank != 0) return;
       const uint32_t left = s_hists[0][0];
-      uint32_t key = 0;
-      if (left <= 32) {
-        if (tid < 32) key = cx::warp_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, tid, in_bin);
-      } else {
-        key = block_rank(tid < (int)left ? s_hists[1][tid] : 0u, (int)left, in_bin);
+      if (tid < (int)left) {              // every key counts the ones above it
+        const uint32_t key = s_hists[1][tid];
+        uint32_t gt = 0, ge = 0;
+        for (uint32_t j = 0; j < left; ++j) {
+          gt += s_hists[1][j] > key ? 1u : 0u;
+          ge += s_hists[1][j] >= key ? 1u : 0u;
+        }
+        if (gt <= in_bin && in_bin < ge) *p.thr_out = __uint_as_float(key);    // equal keys write the same
       }
-      if (tid == 0) *p.thr_out = __uint_as_float(key);
       return;
     }
   }
@@ -662,7 +716,7 @@ __global__ void __launch_bounds__(kThreads) exact_finish_kernel(const __grid_con
     if (crank != 0)
       for (int i = tid; i < kBins; i += kThreads) if (s_hist[i]) atomicAdd(&hist0[i], s_hist[i]);
     cluster.sync();
-    if (crank == 0) pick_bin(s_hist, rank, s_warp, s_out);
+    if (crank == 0) pick_bin<kThreads>(s_hist, rank, s_warp, s_out);
     cluster.sync();
     prefix |= out0[0] << shift;
     rank = out0[1];
@@ -689,7 +743,9 @@ int launch_one_pass(const OnePassParams& p, bool capturing, cudaStream_t s) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = !capturing && cx_pdl_enabled() ? 2 : 1;
+  cfg.blockDim = dim3(kBracketThreads, 1, 1);
   cudaError_t e = cudaLaunchKernelEx(&cfg, bracket_kernel<T>, p);
+  cfg.blockDim = dim3(kThreads, 1, 1);
   if (e != cudaSuccess) return cx_set_error("bracket_kernel launch", (int)e);
   const int64_t round = (int64_t)kCollectThreads * kCollectEach;
   int grid = cx_sm_count() * kCollectPerSm;

@@ -700,7 +700,7 @@ def test_rle_fused_receive_rejects_corrupt_runs(world):
 @pytest.mark.parametrize("ratio", [0.001, 0.01, 0.1, 0.7])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_threshold_and_compress_as_one_list(n, ratio, dtype):
-    """The op list [threshold, compress] (one kernel up to a grid that is resident as a whole) gives
+    """The op list [threshold, compress] (the compress kernel loads ahead of the threshold) gives
     threshold, payload and residual of the two launches issued one by one, call after call; views at
     odd addresses too."""
     world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
@@ -720,12 +720,8 @@ def test_threshold_and_compress_as_one_list(n, ratio, dtype):
             ops = (_lib.Op * 2)(*comps[1].send_ops(rs[1], n, n, P.make_targets([slots[1].endpoint(e0, 1)]), ratio, 1000, 10.0))
             for o in ops:
                 o.g, o.dtype = g.data_ptr(), _lib.dtype_code(dtype)
-            before = _lib.launch_count()
             _lib.check(e0.lib.cx_run_ops(ops, 2, seq, _lib.stream_ptr(e0.device)))
-            launches = _lib.launch_count() - before
             e0.flush()
-            small = n <= 296 * 8 * 1024 and min(n, max(1000, int(10 / ratio))) <= 1024
-            assert launches == (1 if small else 2), launches
             assert torch.equal(comps[0].thr, comps[1].thr)
             a, b = (read_pairs(e1, s) for s in slots)
             assert a[0].seq == b[0].seq == seq and a[0].nnz == b[0].nnz and a[0].nnz_found == b[0].nnz_found
