@@ -76,7 +76,7 @@ class Fold(C.Structure):
 class FoldCoef(C.Structure):
     """Arguments of cx_fold_coef (CxFoldCoef in csrc/cx_common.h)."""
     _fields_ = [("seg_ptr", C.c_void_p), ("item_rel", C.c_void_p), ("item_len", C.c_void_p), ("item_seg", C.c_void_p),
-                ("seg_first", C.c_void_p), ("partial", C.c_void_p), ("coef", C.c_void_p), ("items", C.c_int32),
+                ("seg_first", C.c_void_p), ("partial", C.c_void_p), ("coef", C.c_void_p), ("count", C.c_void_p), ("items", C.c_int32),
                 ("segs", C.c_int32), ("clip", C.c_float), ("lr", C.c_float)]
 
 
@@ -136,7 +136,7 @@ def _declare(lib) -> None:
         "cx_graph_free": (i32, [vp]),
         "cx_sizeof": (i64, [i32]),
         "cx_fold": (i32, [i32, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp, f32, f32, f32, vp]),
-        "cx_fold_coef": (i32, [i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, f32, f32, vp]),
+        "cx_fold_coef": (i32, [i32, P(FoldCoef), vp]),
         "cx_fold_update": (i32, [i32, P(Fold), i64, P(ApplyArgs), vp]),
         "cx_axpy": (i32, [i32, i32, vp, i32, vp, f32, i64, vp]),
         "cx_fill_zero": (i32, [i32, vp, i64, vp]),

@@ -160,16 +160,17 @@ typedef struct CxFold {
   int32_t pad;
 } CxFold;
 
-/* arguments of cx_fold_coef as one object, for op lists */
+/* arguments of cx_fold_coef; the item arrays as for cx_fold, every tensor with at least one item */
 typedef struct CxFoldCoef {
   const void* const* seg_ptr;
   const int64_t* item_rel;
   const int32_t* item_len;
   const int32_t* item_seg;
   const int32_t* seg_first;
-  float* partial;
-  float* coef;
-  int32_t items, segs;         /* all from 0 on */
+  float* partial;              /* scratch: 8 floats per item                                         */
+  float* coef;                 /* out: one factor per tensor                                          */
+  uint32_t* count;             /* scratch: one counter per tensor, zeroed once, left zeroed           */
+  int32_t items, segs;
   float clip, lr;
 } CxFoldCoef;
 
@@ -274,11 +275,8 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
             float mu, float lr, void* stream);
 
 /* The first half of the fold on its own (CUDA): coef[s] = lr * clip / max(||g_s||, clip), or lr
- * without clipping, for the tensors [seg_lo, seg_hi) whose items are [item_lo, item_hi).  Same sums,
- * in the same order, as cx_fold; partial: scratch of 8 floats per item. */
-int cx_fold_coef(int gdtype, const void* const* seg_ptr, const int64_t* item_rel, const int32_t* item_len,
-                 const int32_t* item_seg, const int32_t* seg_first, int item_lo, int item_hi, int seg_lo, int seg_hi,
-                 float* partial, float* coef, float clip, float lr, void* stream);
+ * without clipping.  Same sums, in the same order, as cx_fold. */
+int cx_fold_coef(int gdtype, const CxFoldCoef* f, void* stream);
 /* cx_fold and cx_update_dense in one pass over the range (CUDA): u is updated when fold->u is set,
  * and the parameters take the folded vector as their averaged gradient. */
 int cx_fold_update(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream);

@@ -116,6 +116,39 @@ PyObject* run_vector(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return PyLong_FromLong(rc);
 }
 
+// install(pairs): `v.grad = g` for every (g, v); the checks of the attribute are left to it whenever
+// the pair is not plainly two tensors of the same kind.
+PyObject* install(PyObject*, PyObject* pairs) {
+  PyObject* it = PyObject_GetIter(pairs);
+  if (!it) return nullptr;
+  while (PyObject* pair = PyIter_Next(it)) {
+    PyObject* two = PySequence_Fast(pair, "install: (gradient, variable) pairs");
+    Py_DECREF(pair);
+    bool ok = two && PySequence_Fast_GET_SIZE(two) == 2;
+    if (two && !ok) PyErr_SetString(PyExc_ValueError, "install: (gradient, variable) pairs");
+    if (ok) {
+      PyObject* g = PySequence_Fast_GET_ITEM(two, 0);
+      PyObject* v = PySequence_Fast_GET_ITEM(two, 1);
+      bool done = false;
+      if (THPVariable_Check(g) && THPVariable_Check(v) && g != v) {
+        const at::Tensor& gt = THPVariable_Unpack(g);
+        const at::Tensor& vt = THPVariable_Unpack(v);
+        if (gt.defined() && vt.defined() && vt.is_leaf() && gt.layout() == at::kStrided && vt.layout() == at::kStrided &&
+            gt.scalar_type() == vt.scalar_type() && gt.device() == vt.device() && gt.sizes() == vt.sizes()) {
+          vt.mutable_grad() = gt;
+          done = true;
+        }
+      }
+      ok = done || PyObject_SetAttrString(v, "grad", g) == 0;
+    }
+    Py_XDECREF(two);
+    if (!ok) break;
+  }
+  Py_DECREF(it);
+  if (PyErr_Occurred()) return nullptr;
+  Py_RETURN_NONE;
+}
+
 // the value `collect` wants for a dtype, from a tensor of that dtype
 PyObject* scalar_type(PyObject*, PyObject* o) {
   if (!THPVariable_Check(o)) {
@@ -128,6 +161,7 @@ PyObject* scalar_type(PyObject*, PyObject* o) {
 PyMethodDef methods[] = {{"collect", collect, METH_VARARGS, nullptr},
                          {"run_vector", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(run_vector)),
                           METH_FASTCALL, nullptr},
+                         {"install", install, METH_O, nullptr},
                          {"scalar_type", scalar_type, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_cxhost", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -31,8 +31,7 @@ int cx_compress_cuda(int, const void*, float*, int64_t, const float*, uint32_t, 
                      const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
 int cx_compress_fold_cuda(int, const CxFold*, float*, int64_t, const float*, uint32_t, uint64_t,
                           const CxTargets*, void*, int64_t, CxStats*, uint32_t, void*);
-int cx_fold_coef_cuda(int, const void* const*, const int64_t*, const int32_t*, const int32_t*, const int32_t*, int, int,
-                      int, int, float*, float*, float, float, void*);
+int cx_fold_coef_cuda(int, const CxFoldCoef*, void*);
 int cx_fold_update_cuda(int, const CxFold*, int64_t, const CxApplyArgs*, void*);
 int cx_compress_host(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
                      const CxTargets*, CxStats*, uint32_t);
@@ -216,12 +215,7 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
                             partial, clip, mu, lr);
 }
 
-int cx_fold_coef(int gdtype, const void* const* seg_ptr, const int64_t* item_rel, const int32_t* item_len,
-                 const int32_t* item_seg, const int32_t* seg_first, int item_lo, int item_hi, int seg_lo, int seg_hi,
-                 float* partial, float* coef, float clip, float lr, void* stream) {
-  return cx_fold_coef_cuda(gdtype, seg_ptr, item_rel, item_len, item_seg, seg_first, item_lo, item_hi, seg_lo, seg_hi,
-                           partial, coef, clip, lr, stream);
-}
+int cx_fold_coef(int gdtype, const CxFoldCoef* f, void* stream) { return cx_fold_coef_cuda(gdtype, f, stream); }
 
 int cx_fold_update(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream) {
   return cx_fold_update_cuda(gdtype, fold, n, a, stream);
@@ -294,11 +288,8 @@ int run_one(CxOp& o, uint64_t seq, void* stream) {
                              (int)o.cap, o.scale, (int)o.starts[1], o.starts[2], seq, flags, o.workspace, o.status,
                              o.timeout_ns, stream);
     }
-    case CX_OPK_FOLD_COEF: {
-      const CxFoldCoef* f = reinterpret_cast<const CxFoldCoef*>(o.fold);
-      return cx_fold_coef(o.dtype, f->seg_ptr, f->item_rel, f->item_len, f->item_seg, f->seg_first, 0, f->items, 0, f->segs,
-                          f->partial, f->coef, f->clip, f->lr, stream);
-    }
+    case CX_OPK_FOLD_COEF:
+      return cx_fold_coef(o.dtype, reinterpret_cast<const CxFoldCoef*>(o.fold), stream);
     case CX_OPK_FOLD_UPDATE:
       return cx_fold_update(o.dtype, o.fold, o.n, &o.apply, stream);
     case CX_OPK_UPDATE:

@@ -52,6 +52,7 @@ import warnings
 
 import numpy as np
 import torch
+from torch.optim import optimizer as _torch_optimizer
 
 from . import _lib, allreduce as _ar
 from ._lib import ComprexError
@@ -76,7 +77,7 @@ class _Bucket:
         self.kind, self.xbuf, self.plan, self.u = None, None, None, None
 
 
-_ITEM = 65536     # elements per fold work item
+_ITEM = 16384     # elements per fold work item: one round of loads for 256 threads
 _ALIGN = 64       # tensors start on 128-byte (bf16) / 256-byte (fp32) boundaries of the flat buffers
 
 
@@ -126,6 +127,7 @@ class _FoldTable:
             self.ring = [(torch.zeros(self.nseg, dtype=torch.int64).pin_memory(), torch.cuda.Event()) for _ in range(4)]
             self.turn = 0
             self.coef = torch.zeros(self.nseg, dtype=torch.float32, device=dev)
+            self.count = torch.zeros(self.nseg, dtype=torch.int32, device=dev)
             # buckets start on sub-tile borders: one table serves them all
             subs = torch.arange(lo, max(buckets[-1].end, lo + 1), _lib.SUBTILE, dtype=torch.int64, device=dev)
             self.sub_seg = torch.searchsorted(self.seg_end, subs, right=True, out_int32=True)
@@ -161,11 +163,13 @@ class _FoldTable:
 
     def launch_coef(self, clip: float, lr: float) -> None:
         """Norms and clip factors of all tensors of the table (CUDA)."""
-        _lib.check(self.env.lib.cx_fold_coef(self.code, self.ptrs.data_ptr(), self.item_rel.data_ptr(),
-                                             self.item_len.data_ptr(), self.item_seg.data_ptr(),
-                                             self.seg_first.data_ptr(), 0, self.nitems, 0, self.nseg,
-                                             self.partial.data_ptr(), self.coef.data_ptr(), clip, lr,
-                                             _lib.stream_ptr(self.env.device)), "cx_fold_coef")
+        f = self.coef_args(clip, lr)
+        _lib.check(self.env.lib.cx_fold_coef(self.code, C.byref(f), _lib.stream_ptr(self.env.device)), "cx_fold_coef")
+
+    def coef_args(self, clip: float, lr: float):
+        return _lib.FoldCoef(*[t.data_ptr() for t in (self.ptrs, self.item_rel, self.item_len, self.item_seg, self.seg_first,
+                                                      self.partial, self.coef, self.count)],
+                             self.nitems, self.nseg, clip, lr)
 
     def fold_args(self, b, u, mu: float):
         """The folded vector of bucket ``b`` (None: of all buckets); ``u``: its momentum, or None."""
@@ -186,8 +190,7 @@ class _StepPlan:
     def __init__(self, opt, ft: _FoldTable, par, cfg):
         self.table, self.cfg, self.hyper = ft, cfg, None
         env, k = opt._env, len(opt._buckets)
-        self.coef = _lib.FoldCoef(*[t.data_ptr() for t in (ft.ptrs, ft.item_rel, ft.item_len, ft.item_seg, ft.seg_first,
-                                                           ft.partial, ft.coef)], ft.nitems, ft.nseg, 0.0, 0.0)
+        self.coef = ft.coef_args(0.0, 0.0)
         coef = _lib.Op()
         coef.kind, coef.dev, coef.dtype, coef.fold = _lib.OPK_FOLD_COEF, env.dev, ft.code, C.addressof(self.coef)
         if par is None:
@@ -622,6 +625,9 @@ class ComprexOptimizer(torch.optim.Optimizer):
 
     @torch.no_grad()
     def step(self, closure=None):
+        return self._step(closure)
+
+    def _step(self, closure=None):
         loss = None
         if closure is not None:
             with torch.enable_grad():
@@ -676,9 +682,19 @@ class ComprexOptimizer(torch.optim.Optimizer):
     def apply_gradients(self, grads_and_vars, *args, **kwargs):
         """Keras-style entry (keras/comprex_optimizer.py:144-145): ``(gradient, variable)`` pairs are
         installed as the variables' ``.grad`` and one step is taken."""
-        for g, v in grads_and_vars:
-            v.grad = g
-        return self.step()
+        _lib.host().install(grads_and_vars)
+        # torch wraps `step` of every optimizer (hooks, a profiler range, schedulers that count): 8 us
+        # that nobody sees when none of these is in use
+        if (type(self) is not ComprexOptimizer or "step" in self.__dict__ or self._optimizer_step_pre_hooks
+                or self._optimizer_step_post_hooks or _torch_optimizer._global_optimizer_pre_hooks
+                or _torch_optimizer._global_optimizer_post_hooks or torch._C._autograd._profiler_enabled()):
+            return self.step()
+        grad_mode = torch.is_grad_enabled()
+        torch._C._set_grad_enabled(False)
+        try:
+            return self._step()
+        finally:
+            torch._C._set_grad_enabled(grad_mode)
 
     def refresh_master(self) -> None:
         """Take the model's current tensors as the master weights: call it after the parameters
