@@ -527,43 +527,9 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_kernel(const __grid_c
   }
 }
 
-// a warp's tile of kTile elements: lane L holds elements 128 k + 4 L + e
-template <typename T>
-__device__ __forceinline__ void load_tile(const OnePassParams& p, int64_t b, int lane, float (&v)[kTile / 32]) {
-  const T* g = reinterpret_cast<const T*>(p.g);
-  if (p.vec && b + kTile <= p.n) {
-    constexpr int kQ = kTile / 128;
-    float y[kQ][4];
-    typename cx::Raw4<T>::type z[kQ];
-#pragma unroll
-    for (int k = 0; k < kQ; ++k) {
-      const int64_t i = b + k * 128 + lane * 4;
-      if (p.r) cx::load4(p.r + i, y[k]);
-      if (g) z[k] = cx::Raw4<T>::load(g + i);
-    }
-#pragma unroll
-    for (int k = 0; k < kQ; ++k) {
-      float t[4] = {0.f, 0.f, 0.f, 0.f};
-      if (g) cx::Raw4<T>::to_f(z[k], t);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[4 * k + e] = p.r ? (g ? y[k][e] + t[e] : y[k][e]) : t[e];
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kTile / 32; ++k) {
-      const int64_t i = b + (k / 4) * 128 + lane * 4 + (k & 3);
-      v[k] = 0.f;
-      if (i < p.n) {
-        if (p.r) v[k] = p.r[i];
-        if (g) v[k] = v[k] + cx::Elem<T>::to_f(g[i]);
-      }
-    }
-  }
-}
-
 // Bound by the read of the vector.  A warp takes kTile elements at a time and keeps its candidates in a
-// buffer of its own, so no warp waits for another before the end; the first tile is loaded while the
-// bracket is still being found (both only read).
+// buffer of its own, so no warp waits for another before the end (with a buffer per CTA and its two
+// barriers per round: 22 us for 10 M elements, 3.6 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel(const __grid_constant__ OnePassParams p) {
   constexpr int kCWarps = kCollectThreads / 32;
@@ -572,43 +538,60 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
   __shared__ uint32_t s_fill[kCWarps];
   __shared__ uint32_t s_base, s_cnt[3];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int64_t stride = (int64_t)gridDim.x * kCWarps * kTile;
-  int64_t b = ((int64_t)blockIdx.x * kCWarps + w) * kTile;
-  float v[kTile / 32];
-  load_tile<T>(p, b, lane, v);
   for (int i = tid; i < kBins; i += kCollectThreads) s_hist[i] = 0;
   if (tid < 3) s_cnt[tid] = 0;
   cx::pdl_wait();
   cx::pdl_trigger();
   const uint32_t lo = p.st->lo, hi = p.st->hi;
   const int shift = max(bracket_bits(lo, hi) - 11, 0);
+  const T* g = reinterpret_cast<const T*>(p.g);
   uint32_t above = 0, at_hi = 0, at_lo = 0, fill = 0;
   uint32_t* buf = s_buf[w];
   __syncthreads();
-  for (; b < p.n; b += stride) {
-    // bit k of near: element k at or above lo (few are), of cand: inside the bracket
-    uint32_t near = 0, cand = 0;
+  const int64_t stride = (int64_t)gridDim.x * kCWarps * kTile;
+  for (int64_t b = ((int64_t)blockIdx.x * kCWarps + w) * kTile; b < p.n; b += stride) {
+    float v[kTile / 32];
+    const bool whole = p.vec && b + kTile <= p.n;
+    if (whole) {
+      constexpr int kQ = kTile / 128;
+      float y[kQ][4];
+      typename cx::Raw4<T>::type z[kQ];
 #pragma unroll
-    for (int k = 0; k < kTile / 32; ++k) near |= (__float_as_uint(fabsf(v[k])) >= lo ? 1u : 0u) << k;
-    if (b + kTile > p.n) {
+      for (int k = 0; k < kQ; ++k) {
+        const int64_t i = b + k * 128 + lane * 4;
+        if (p.r) cx::load4(p.r + i, y[k]);
+        if (g) z[k] = cx::Raw4<T>::load(g + i);
+      }
 #pragma unroll
-      for (int k = 0; k < kTile / 32; ++k)
-        if (b + (k / 4) * 128 + lane * 4 + (k & 3) >= p.n) near &= ~(1u << k);
-    }
-    if (near) {
+      for (int k = 0; k < kQ; ++k) {
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
+        if (g) cx::Raw4<T>::to_f(z[k], t);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[4 * k + e] = p.r ? (g ? y[k][e] + t[e] : y[k][e]) : t[e];
+      }
+    } else {
 #pragma unroll
       for (int k = 0; k < kTile / 32; ++k) {
-        if ((near >> k) & 1u) {
-          const uint32_t key = __float_as_uint(fabsf(v[k]));
-          above += key > hi ? 1u : 0u;
-          at_hi += key == hi ? 1u : 0u;
-          at_lo += key == lo && lo != hi ? 1u : 0u;
-          cand |= (key > lo && key < hi ? 1u : 0u) << k;
+        const int64_t i = b + (k / 4) * 128 + lane * 4 + (k & 3);
+        v[k] = 0.f;
+        if (i < p.n) {
+          if (p.r) v[k] = p.r[i];
+          if (g) v[k] = v[k] + cx::Elem<T>::to_f(g[i]);
         }
       }
     }
-    __syncwarp();
-    for (uint32_t who; (who = __ballot_sync(0xffffffffu, cand != 0)) != 0;) {
+#pragma unroll
+    for (int k = 0; k < kTile / 32; ++k) {
+      const int64_t i = b + (k / 4) * 128 + lane * 4 + (k & 3);
+      const uint32_t key = __float_as_uint(fabsf(v[k]));
+      const bool near = (whole || i < p.n) && key >= lo;       // few are
+      if (!__any_sync(0xffffffffu, near)) continue;
+      above += near && key > hi;
+      at_hi += near && key == hi;
+      at_lo += near && key == lo && lo != hi;
+      const bool cand = near && key > lo && key < hi;
+      const uint32_t who = __ballot_sync(0xffffffffu, cand);
+      if (!who) continue;
       if (fill + 32 > kBuffer) {                               // rare: a dense bracket
         uint32_t at = 0;
         if (lane == 0) at = atomicAdd(&p.st->found, fill);
@@ -619,18 +602,11 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
         fill = 0;
       }
       if (cand) {
-        const int k = __ffs(cand) - 1;
-        cand &= cand - 1;
-        float x = v[0];
-#pragma unroll
-        for (int j = 1; j < kTile / 32; ++j) x = k == j ? v[j] : x;
-        const uint32_t key = __float_as_uint(fabsf(x));
         buf[fill + __popc(who & ((1u << lane) - 1u))] = key;
         atomicAdd(&s_hist[(key - bracket_base(lo)) >> shift], 1u);
       }
       fill += __popc(who);
     }
-    if (b + stride < p.n) load_tile<T>(p, b + stride, lane, v);
   }
   above = __reduce_add_sync(0xffffffffu, above);
   at_hi = __reduce_add_sync(0xffffffffu, at_hi);
