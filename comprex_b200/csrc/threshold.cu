@@ -400,8 +400,8 @@ constexpr int kCluster = 8;
 constexpr int kBracketThreads = 512;   // fits next to a receive kernel's CTAs
 constexpr int kBins = 2048;          // 11 bits per radix pass of the finish
 constexpr int kCollectThreads = 256;
-constexpr int kTile = 256;           // elements a warp takes at a time
-constexpr int kBuffer = 256;         // candidates a warp keeps before it appends them to the list
+constexpr int kCollectEach = 8;      // elements per thread and round
+constexpr int kBuffer = 3072;        // candidates a CTA keeps before it appends them to the list
 constexpr int kCollectPerSm = 6;
 
 struct ExactState {                  // in the workspace behind the histograms; zero between calls
@@ -527,17 +527,14 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_kernel(const __grid_c
   }
 }
 
-// Bound by the read of the vector.  A warp takes kTile elements at a time and keeps its candidates in a
-// buffer of its own, so no warp waits for another before the end (with a buffer per CTA and its two
-// barriers per round: 22 us for 10 M elements, 3.6 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel(const __grid_constant__ OnePassParams p) {
-  constexpr int kCWarps = kCollectThreads / 32;
-  __shared__ uint32_t s_buf[kCWarps][kBuffer];
+  __shared__ uint32_t s_buf[kBuffer];
   __shared__ uint32_t s_hist[kBins];
-  __shared__ uint32_t s_fill[kCWarps];
-  __shared__ uint32_t s_base, s_cnt[3];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  __shared__ uint32_t s_fill, s_base;
+  __shared__ uint32_t s_cnt[3];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) s_fill = 0;
   for (int i = tid; i < kBins; i += kCollectThreads) s_hist[i] = 0;
   if (tid < 3) s_cnt[tid] = 0;
   cx::pdl_wait();
@@ -545,20 +542,29 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
   const uint32_t lo = p.st->lo, hi = p.st->hi;
   const int shift = max(bracket_bits(lo, hi) - 11, 0);
   const T* g = reinterpret_cast<const T*>(p.g);
-  uint32_t above = 0, at_hi = 0, at_lo = 0, fill = 0;
-  uint32_t* buf = s_buf[w];
+  uint32_t above = 0, at_hi = 0, at_lo = 0;
   __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * kCWarps * kTile;
-  for (int64_t b = ((int64_t)blockIdx.x * kCWarps + w) * kTile; b < p.n; b += stride) {
-    float v[kTile / 32];
-    const bool whole = p.vec && b + kTile <= p.n;
+  const int64_t round = (int64_t)kCollectThreads * kCollectEach;
+  auto flush = [&]() {                // all threads
+    const uint32_t fill = s_fill;
+    if (tid == 0) s_base = atomicAdd(&p.st->found, fill);
+    __syncthreads();
+    for (uint32_t i = tid; i < fill; i += kCollectThreads)
+      if (s_base + i < p.cap) p.list[s_base + i] = s_buf[i];
+    __syncthreads();
+    if (tid == 0) s_fill = 0;
+    __syncthreads();
+  };
+  for (int64_t b = (int64_t)blockIdx.x * round; b < p.n; b += (int64_t)gridDim.x * round) {
+    float v[kCollectEach];
+    const bool whole = p.vec && b + round <= p.n;
     if (whole) {
-      constexpr int kQ = kTile / 128;
+      constexpr int kQ = kCollectEach / 4;
       float y[kQ][4];
       typename cx::Raw4<T>::type z[kQ];
 #pragma unroll
       for (int k = 0; k < kQ; ++k) {
-        const int64_t i = b + k * 128 + lane * 4;
+        const int64_t i = b + (int64_t)k * kCollectThreads * 4 + tid * 4;
         if (p.r) cx::load4(p.r + i, y[k]);
         if (g) z[k] = cx::Raw4<T>::load(g + i);
       }
@@ -571,8 +577,8 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
       }
     } else {
 #pragma unroll
-      for (int k = 0; k < kTile / 32; ++k) {
-        const int64_t i = b + (k / 4) * 128 + lane * 4 + (k & 3);
+      for (int k = 0; k < kCollectEach; ++k) {
+        const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
         v[k] = 0.f;
         if (i < p.n) {
           if (p.r) v[k] = p.r[i];
@@ -581,8 +587,8 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
       }
     }
 #pragma unroll
-    for (int k = 0; k < kTile / 32; ++k) {
-      const int64_t i = b + (k / 4) * 128 + lane * 4 + (k & 3);
+    for (int k = 0; k < kCollectEach; ++k) {
+      const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
       const uint32_t key = __float_as_uint(fabsf(v[k]));
       const bool near = (whole || i < p.n) && key >= lo;       // few are
       if (!__any_sync(0xffffffffu, near)) continue;
@@ -591,48 +597,31 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
       at_lo += near && key == lo && lo != hi;
       const bool cand = near && key > lo && key < hi;
       const uint32_t who = __ballot_sync(0xffffffffu, cand);
-      if (!who) continue;
-      if (fill + 32 > kBuffer) {                               // rare: a dense bracket
+      if (who) {
         uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(&p.st->found, fill);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        for (uint32_t j = lane; j < fill; j += 32)
-          if (at + j < p.cap) p.list[at + j] = buf[j];
-        __syncwarp();
-        fill = 0;
+        if (lane == __ffs(who) - 1) at = atomicAdd(&s_fill, (uint32_t)__popc(who));
+        at = __shfl_sync(0xffffffffu, at, __ffs(who) - 1);
+        if (cand) {
+          s_buf[at + __popc(who & ((1u << lane) - 1u))] = key;
+          atomicAdd(&s_hist[(key - bracket_base(lo)) >> shift], 1u);
+        }
       }
-      if (cand) {
-        buf[fill + __popc(who & ((1u << lane) - 1u))] = key;
-        atomicAdd(&s_hist[(key - bracket_base(lo)) >> shift], 1u);
-      }
-      fill += __popc(who);
     }
+    __syncthreads();
+    if (s_fill > kBuffer - kCollectThreads * kCollectEach) flush();      // uniform: the next round might not fit
+    else __syncthreads();
   }
-  above = __reduce_add_sync(0xffffffffu, above);
-  at_hi = __reduce_add_sync(0xffffffffu, at_hi);
-  at_lo = __reduce_add_sync(0xffffffffu, at_lo);
-  if (lane == 0) {
-    s_fill[w] = fill;
-    if (above) atomicAdd(&s_cnt[0], above);
-    if (at_hi) atomicAdd(&s_cnt[1], at_hi);
-    if (at_lo) atomicAdd(&s_cnt[2], at_lo);
-  }
+  if (above) atomicAdd(&s_cnt[0], above);
+  if (at_hi) atomicAdd(&s_cnt[1], at_hi);
+  if (at_lo) atomicAdd(&s_cnt[2], at_lo);
   __syncthreads();
   if (tid == 0) {
-    uint32_t all = 0;
-    for (int j = 0; j < kCWarps; ++j) all += s_fill[j];
-    s_base = all ? atomicAdd(&p.st->found, all) : 0u;
-  } else if (tid == 32) {
     if (s_cnt[0]) atomicAdd(&p.st->above, s_cnt[0]);
     if (s_cnt[1]) atomicAdd(&p.st->at_hi, s_cnt[1]);
     if (s_cnt[2]) atomicAdd(&p.st->at_lo, s_cnt[2]);
   }
   for (int i = tid; i < kBins; i += kCollectThreads) if (s_hist[i]) atomicAdd(&p.st->hist[i], s_hist[i]);
-  __syncthreads();
-  uint32_t at = s_base;
-  for (int j = 0; j < w; ++j) at += s_fill[j];
-  for (uint32_t j = lane; j < fill; j += 32)
-    if (at + j < p.cap) p.list[at + j] = buf[j];
+  if (s_fill) flush();
 }
 
 template <typename T>
@@ -758,7 +747,7 @@ int launch_one_pass(const OnePassParams& p, bool capturing, cudaStream_t s) {
   cudaError_t e = cudaLaunchKernelEx(&cfg, bracket_kernel<T>, p);
   cfg.blockDim = dim3(kThreads, 1, 1);
   if (e != cudaSuccess) return cx_set_error("bracket_kernel launch", (int)e);
-  const int64_t round = (int64_t)kCollectThreads / 32 * kTile;
+  const int64_t round = (int64_t)kCollectThreads * kCollectEach;
   int grid = cx_sm_count() * kCollectPerSm;
   if (grid > (p.n + round - 1) / round) grid = (int)((p.n + round - 1) / round);
   cx_launch_pdl(collect_kernel<T>, grid, kCollectThreads, 0, s, p, capturing);
