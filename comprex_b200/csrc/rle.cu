@@ -41,12 +41,9 @@ constexpr int kPer = 8;
 constexpr int kSeg = 32 * kPer;          // elements a warp takes at a time
 constexpr int kSendPerSm = 4;            // resident CTAs of the emit kernel
 constexpr int kMaxSend = 1024;           // sending CTAs
-constexpr int kExpand = 128;             // threads of an expanding CTA: many small ones overlap their look-ups
-constexpr int kExpandWarps = kExpand / 32;
-constexpr int kExpandPerSm = 8;
-constexpr int kGroups = kExpand;         // groups of run blocks, one per thread of an expanding CTA
+constexpr int kGroups = 256;             // groups of run blocks, one per thread of a receiving CTA
 constexpr int kRunBlock = 1024;          // runs per block: one warp sums it, one CTA scans it
-constexpr int kWindow = 32 * kExpand;    // outputs per window: one mask word per thread
+constexpr int kWindow = 32 * kThreads;   // outputs per window: one mask word per thread
 
 struct ChunkTotals {       // of one warp's chunk, or of a CTA's eight
   int32_t nnz;             // selected elements
@@ -456,7 +453,7 @@ __device__ __forceinline__ V block_prefix(V x, V& tot, V* sm) {
   V pre = 0;
   tot = 0;
 #pragma unroll
-  for (int j = 0; j < kExpandWarps; ++j) {
+  for (int j = 0; j < kWarps; ++j) {
     if (j < w) pre += sm[j];
     tot += sm[j];
   }
@@ -466,12 +463,12 @@ __device__ __forceinline__ V block_prefix(V x, V& tot, V* sm) {
 // Bound by the output (read and written for `add`).  Looking every output's run up by bisection in
 // the scanned block took 40 us for 2^22 elements at top-k 10 %; the mask needs one shared-memory
 // atomic per run and two shared-memory reads per four outputs.
-__global__ void __launch_bounds__(kExpand, kExpandPerSm) rle_expand_kernel(const __grid_constant__ RecvParams p) {
-  __shared__ long long s_l[kExpandWarps];
-  __shared__ int s_a[kExpandWarps], s_b[kExpandWarps];
+__global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_constant__ RecvParams p) {
+  __shared__ long long s_l[kWarps];
+  __shared__ int s_a[kWarps], s_b[kWarps];
   __shared__ int s_pick[3];
-  __shared__ uint32_t s_mask[kExpand];    // run starts of the window, then its selected outputs
-  __shared__ int s_base[kExpand];         // index of the word's first value
+  __shared__ uint32_t s_mask[kThreads];    // run starts of the window, then its selected outputs
+  __shared__ int s_base[kThreads];         // index of the word's first value
   cx::pdl_wait();
   cx::pdl_trigger();
   if (!p.meta->ok) return;
@@ -505,7 +502,7 @@ __global__ void __launch_bounds__(kExpand, kExpandPerSm) rle_expand_kernel(const
     const int count = (int)min(bpg, nblocks - b0);
     const int gs = s_pick[1], gy = s_pick[2];
     __syncthreads();
-    for (int i = tid; i < count; i += kExpand) {
+    for (int i = tid; i < count; i += kThreads) {
       const RunSums x = p.block[b0 + i];
       const int64_t next = i + 1 < count ? (int64_t)gs + p.block[b0 + i + 1].len : (int64_t)p.n;
       if (gs + (int64_t)x.len <= e0 && (i + 1 == count || next > e0)) { s_pick[0] = i; s_pick[1] = gs + x.len; s_pick[2] = gy + x.yes; }
@@ -524,19 +521,18 @@ __global__ void __launch_bounds__(kExpand, kExpandPerSm) rle_expand_kernel(const
     s_mask[tid] = 0;
     // blocks of runs that reach into the window; a run that began earlier counts at its first bit
     for (;;) {
-      constexpr int kEach = kRunBlock / kExpand;
-      int len[kEach], mine = 0, part = 0;
+      int len[4], mine = 0, part = 0;
 #pragma unroll
-      for (int k = 0; k < kEach; ++k) {
-        const int64_t q = blk * kRunBlock + kEach * tid + k;
+      for (int k = 0; k < 4; ++k) {
+        const int64_t q = blk * kRunBlock + 4 * tid + k;
         len[k] = q < nruns ? runs[q] : 0;
         mine += len[k];
       }
       int tot;
       int pos = at + block_prefix<int>(mine, tot, s_a);
 #pragma unroll
-      for (int k = 0; k < kEach; ++k) {
-        if (blk * kRunBlock + kEach * tid + k < nruns && pos < w1) {
+      for (int k = 0; k < 4; ++k) {
+        if (blk * kRunBlock + 4 * tid + k < nruns && pos < w1) {
           const int bit = pos > w0 ? (int)(pos - w0) : 0;
           atomicXor(&s_mask[bit >> 5], 1u << (bit & 31));
           const bool yes = ((k & 1) == 0) == (first != 0);
@@ -564,7 +560,7 @@ __global__ void __launch_bounds__(kExpand, kExpandPerSm) rle_expand_kernel(const
     __syncthreads();
     int carry = __popc(odd & ((1u << lane) - 1u)) & 1;
 #pragma unroll
-    for (int j = 0; j < kExpandWarps; ++j) if (j < w) carry ^= s_b[j];
+    for (int j = 0; j < kWarps; ++j) if (j < w) carry ^= s_b[j];
     if (carry ^ (first ? 0 : 1)) x = ~x;
     const int64_t left = w1 - w0 - 32 * (int64_t)tid;
     if (left < 32) x &= left <= 0 ? 0u : (1u << left) - 1u;
@@ -575,8 +571,8 @@ __global__ void __launch_bounds__(kExpand, kExpandPerSm) rle_expand_kernel(const
     vbase += total;
     __syncthreads();
 #pragma unroll 4
-    for (int it = 0; it < kWindow / (4 * kExpand); ++it) {
-      const int o = it * 4 * kExpand + 4 * tid;
+    for (int it = 0; it < kWindow / (4 * kThreads); ++it) {
+      const int o = it * 4 * kThreads + 4 * tid;
       const int64_t i0 = w0 + o;
       if (i0 >= w1) continue;
       const uint32_t word = s_mask[o >> 5];
@@ -673,9 +669,9 @@ int cx_rle_recv_cuda(const CxEndpoint* src, uint64_t expect_seq, float* out, int
   int64_t groups = n / (kRunBlock * kWarps) + 1;
   if (groups > kGroups) groups = kGroups;
   p.groups = (int)groups;
-  // expand: an equal number of windows per CTA, at most one wave of CTAs
+  // expand: an equal number of windows per CTA, at most four CTAs per SM
   const int64_t windows = (n + kWindow - 1) / kWindow;
-  const int64_t wave = kExpandPerSm * (int64_t)cx_sm_count();
+  const int64_t wave = 4 * (int64_t)cx_sm_count();
   p.per_cta = (windows + wave - 1) / wave * kWindow;
   char* ws = reinterpret_cast<char*>(workspace);
   p.meta = reinterpret_cast<RleRxMeta*>(ws);
@@ -689,7 +685,7 @@ int cx_rle_recv_cuda(const CxEndpoint* src, uint64_t expect_seq, float* out, int
   cx_note_launch();
   if (n > 0) {
     const int64_t blocks = (n + p.per_cta - 1) / p.per_cta;
-    cx_launch_pdl(rle_expand_kernel, (int)blocks, kExpand, 0, s, p, false);
+    cx_launch_pdl(rle_expand_kernel, (int)blocks, kThreads, 0, s, p, false);
     cx_note_launch();
   }
   return cx_check_launch("rle receive kernels");
