@@ -32,6 +32,7 @@
 namespace {
 
 constexpr int kThreads = 1024;
+constexpr int kWarps = kThreads / 32;
 constexpr int kSmemKeys = 11008;  // 43 KB of cached sample keys
 constexpr int kVectors = 24;      // vectors per launch: their parameters stay within 4 KB
 
@@ -58,16 +59,14 @@ __device__ __forceinline__ int64_t sample_position(int i, int64_t n, int use_all
   return pos > n - 1 ? n - 1 : pos;
 }
 
-// One warp, one key per lane, the first `count` lanes: the key of rank `rank` in descending order.
-__device__ __forceinline__ uint32_t warp_rank(uint32_t key, int count, int lane, uint32_t rank) {
-  uint32_t gt = 0, ge = 0;
-  for (int j = 0; j < count; ++j) {
-    const uint32_t other = __shfl_sync(0xffffffffu, key, j);
-    gt += other > key ? 1u : 0u;
-    ge += other >= key ? 1u : 0u;
-  }
-  const uint32_t who = __ballot_sync(0xffffffffu, lane < count && gt <= rank && rank < ge);
-  return __shfl_sync(0xffffffffu, key, __ffs(who) - 1);
+// Up to 32 keys, one per lane (the same in every warp), of which warp w looks at key w: true if that is
+// the key of rank `rank` in descending order.  Two ballots where one warp that ranks them all takes a
+// chain of 32 shuffles (1 us behind the barrier).
+__device__ __forceinline__ bool has_rank(uint32_t key, uint32_t valid, int w, uint32_t rank) {
+  const uint32_t mine = __shfl_sync(0xffffffffu, key, w);
+  const uint32_t gt = __popc(__ballot_sync(0xffffffffu, key > mine) & valid);
+  const uint32_t ge = __popc(__ballot_sync(0xffffffffu, key >= mine) & valid);
+  return ((valid >> w) & 1u) && gt <= rank && rank < ge;
 }
 
 template <typename T, bool FOLD>
@@ -112,45 +111,60 @@ __device__ __forceinline__ uint32_t pick_digit(const uint32_t* hist, uint32_t& r
 }
 
 // One key per thread (threads from `count` on hold none): the largest t with more than `rank` keys at
-// or above it, which is the key of that rank.  One block-wide count per bit.
-__device__ __forceinline__ uint32_t block_rank(uint32_t key, int count, uint32_t rank) {
-  uint32_t t = 0;
+// or above it, which is the key of that rank, in every thread.  One block-wide count per bit until the
+// keys that agree with t so far are few enough to be ranked together.  s_few: 32 words, s_two: two.
+__device__ __forceinline__ uint32_t block_rank(uint32_t key, int count, uint32_t rank, uint32_t* s_few, uint32_t* s_two) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool have = (int)threadIdx.x < count;
-  for (int bit = 30; bit >= 0; --bit) {
+  uint32_t t = 0, at_t = count, above = 0;    // keys at or above t; keys at or above the end of its interval
+  if (threadIdx.x == 0) s_two[0] = 0;
+  int bit = 30;
+  do {
     const uint32_t c = t | (1u << bit);
-    if ((uint32_t)__syncthreads_count(have && key >= c) > rank) t = c;
-  }
-  return t;
+    const uint32_t m = __syncthreads_count(have && key >= c);
+    if (m > rank) { t = c; at_t = m; } else above = m;
+    --bit;
+  } while (bit >= 0 && at_t - above > 32);
+  if (bit < 0) return t;
+  if (have && key >= t && (key >> (bit + 1)) == (t >> (bit + 1))) s_few[atomicAdd(&s_two[0], 1u)] = key;
+  __syncthreads();
+  const uint32_t k = s_few[lane];
+  if (has_rank(k, 0xffffffffu >> (32 - (at_t - above)), w, rank - above) && lane == w) s_two[1] = k;
+  __syncthreads();
+  return s_two[1];
 }
 
-// The key of rank `rank` among s_keys[0, s), for a sample that fits the block's shared memory (valid
-// in thread 0).
+// The key of rank `rank` among s_keys[0, s), for a sample that fits the block's shared memory, to *out.
+// s_max: the largest keys of `maxima` (a multiple of 32) disjoint parts that cover the sample.
 //  * A lower bound with at least rank + 1 keys at or above it leaves few keys to rank.  Up to rank 31
-//    it is the (rank + 1)-th largest of the 32 warps' maxima, and one warp finds and ranks; up to
-//    rank 767 it is that of the threads' maxima.
+//    it is the (rank + 1)-th largest of 32 parts' maxima, and the warps rank what is left together;
+//    up to rank 767 it is that of the threads' maxima.
 //  * Up to one key per thread: bisection over the bits, no bound needed.
 //  * What is left (a large sample and a large rank, or many ties): four radix passes of 8 bits.
-// 1000 samples, rank 9: 0.5 us where the radix passes took 3 us; 8192 samples, rank 120: 3 us for 8.
-__device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint32_t rank, uint32_t* s_red,
-                                                  uint32_t* s_hist, uint32_t* s_sel) {
+// One warp ranking by shuffles and one count per bit to the last one: the 64 Ki exchange (1000 samples,
+// rank 9) took 12.7 us instead of 12.3, 25 M elements (10 000 samples) 57.7 for 57.2, 4 M at 10 %
+// (rank 99) 57.0 for 56.7.
+__device__ __forceinline__ void select_cached(uint32_t* s_keys, int s, uint32_t rank, const uint32_t* s_max, int maxima,
+                                              uint32_t* s_hist, uint32_t* s_sel, float* out) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (rank >= 32 && s <= kThreads) return block_rank(tid < s ? s_keys[tid] : 0u, s, rank);
+  if (rank >= 32 && s <= kThreads) {
+    const uint32_t key = block_rank(tid < s ? s_keys[tid] : 0u, s, rank, s_hist, s_sel + 2);
+    if (tid == 0) *out = __uint_as_float(key);
+    return;
+  }
   if (rank < 768) {
-    uint32_t mymax = 0, bound;
-    for (int i = tid; i < s; i += kThreads) mymax = max(mymax, s_keys[i]);
+    uint32_t bound;
     if (tid == 0) s_sel[0] = 0;
     if (rank < 32) {
-      const uint32_t wm = __reduce_max_sync(0xffffffffu, mymax);
-      if (lane == 0) s_red[w] = wm;
-      __syncthreads();
-      if (w == 0) {
-        const uint32_t b0 = warp_rank(s_red[lane], 32, lane, rank);
-        if (lane == 0) s_sel[1] = b0;
-      }
+      uint32_t m = 0;
+      for (int i = lane; i < maxima; i += 32) m = max(m, s_max[i]);
+      if (has_rank(m, 0xffffffffu, w, rank) && lane == w) s_sel[1] = m;
       __syncthreads();
       bound = s_sel[1];
     } else {
-      bound = block_rank(mymax, kThreads, rank);
+      uint32_t mymax = 0;
+      for (int i = tid; i < s; i += kThreads) mymax = max(mymax, s_keys[i]);
+      bound = block_rank(mymax, kThreads, rank, s_hist, s_sel + 2);
     }
     for (int i = tid; i < s; i += kThreads) {
       const uint32_t k = s_keys[i];
@@ -161,8 +175,16 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
     }
     __syncthreads();
     const uint32_t left = s_sel[0];
-    if (left <= 32) return w == 0 ? warp_rank(lane < (int)left ? s_hist[lane] : 0u, (int)left, lane, rank) : 0u;
-    if (left <= kThreads) return block_rank(tid < (int)left ? s_hist[tid] : 0u, (int)left, rank);
+    if (left <= 32) {
+      const uint32_t key = s_hist[lane];        // (what lies behind `left` is not counted)
+      if (has_rank(key, 0xffffffffu >> (32 - left), w, rank) && lane == w) *out = __uint_as_float(key);
+      return;
+    }
+    if (left <= kThreads) {
+      const uint32_t key = block_rank(tid < (int)left ? s_hist[tid] : 0u, (int)left, rank, s_hist, s_sel + 2);
+      if (tid == 0) *out = __uint_as_float(key);
+      return;
+    }
   }
   uint32_t prefix = 0, prefmask = 0;
   const int s_round = (s + kThreads - 1) / kThreads * kThreads;
@@ -186,7 +208,7 @@ __device__ __forceinline__ uint32_t select_cached(uint32_t* s_keys, int s, uint3
     prefmask |= 255u << shift;
     rank = s_sel[1];
   }
-  return prefix;
+  if (tid == 0) *out = __uint_as_float(prefix);
 }
 
 template <typename T, bool FOLD, int NV>
@@ -194,9 +216,8 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   namespace cg = cooperative_groups;
   __shared__ uint32_t s_keys[kSmemKeys];
   __shared__ uint32_t s_hist[kThreads];
-  __shared__ uint32_t s_sel[2];
-  __shared__ uint32_t s_red[kThreads / 32];
-  __shared__ uint32_t s_cmax[8];  // per-CTA maxima of a cluster launch (first CTA's copy is used)
+  __shared__ uint32_t s_sel[4];
+  uint32_t* s_max = s_hist;  // the warps' maxima (of a cluster launch in the first CTA's copy), until it selects
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   cg::cluster_group cluster = cg::this_cluster();
@@ -206,7 +227,9 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   const int s = p.samples;
   const bool cached = s <= kSmemKeys;
   uint32_t* keys0 = ncta > 1 ? cluster.map_shared_rank(s_keys, 0) : s_keys;
+  if (ncta > 1) cluster.barrier_arrive();
   cx::pdl_wait();     // resident early: what the kernel in front wrote may be read from here on
+  if (ncta > 1) cluster.barrier_wait();   // every CTA runs: its shared memory may be written
 
   // pass 0: gather the sample (and its maximum, for the sentinel case); CTA c of a cluster
   // takes the samples [c, c+1) * s / ncta
@@ -232,43 +255,25 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
   // for this grid to finish before it reads the threshold or writes the residual.  (Let in before the
   // gather, its 20 MB of loads were in front of the sample's.)
   cx::pdl_trigger();
+  const uint32_t wm = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) (ncta > 1 ? cluster.map_shared_rank(s_max, 0) : s_max)[crank * kWarps + (tid >> 5)] = wm;
   if (ncta > 1) {
-    if (p.topk_pos <= 0) {
-      const uint32_t wm = __reduce_max_sync(0xffffffffu, mx);
-      if (lane == 0) s_red[tid >> 5] = wm;
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t m = 0;
-        for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_red[w]);
-        cluster.map_shared_rank(s_cmax, 0)[crank] = m;
-      }
-    }
     cluster.sync();              // keys and maxima of all CTAs are in the first CTA's shared memory
     if (crank != 0) return;      // (no CTA touches another CTA's shared memory after this point)
-    if (p.topk_pos <= 0) {
-      if (tid == 0) {
-        uint32_t m = 0;
-        for (unsigned c = 0; c < ncta; ++c) m = max(m, s_cmax[c]);
-        *p.thr_out = __uint_as_float(m) + 1.0f;
-      }
-      return;
-    }
+  } else {
+    __syncthreads();
   }
   if (p.topk_pos <= 0) {
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane == 0) s_red[tid >> 5] = mx;
-    __syncthreads();
-    if (tid == 0) {
+    if (tid < 32) {
       uint32_t m = 0;
-      for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_red[w]);
-      *p.thr_out = __uint_as_float(m) + 1.0f;
+      for (unsigned i = lane; i < ncta * kWarps; i += 32) m = max(m, s_max[i]);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (tid == 0) *p.thr_out = __uint_as_float(m) + 1.0f;
     }
     return;
   }
   if (cached) {
-    __syncthreads();
-    const uint32_t key = select_cached(s_keys, s, (uint32_t)p.topk_pos, s_red, s_hist, s_sel);
-    if (tid == 0) *p.thr_out = __uint_as_float(key);
+    select_cached(s_keys, s, (uint32_t)p.topk_pos, s_max, (int)(ncta * kWarps), s_hist, s_sel, p.thr_out);
     return;
   }
 

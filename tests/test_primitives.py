@@ -130,6 +130,31 @@ def test_exact_topk_one_pass(n, dtype, data):
     env.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("data", ["normal", "ties", "constant", "ends"])
+@pytest.mark.parametrize("n", [33, 1000, 1024, 1025, 2049, 11008])
+def test_threshold_selection_ranks(n, data):
+    """The block-wide selection at the edges of its ranges: ranks around 32 and 768, samples around one
+    key per thread and the cluster's first size, few distinct keys."""
+    torch.manual_seed(n)
+    g = torch.randn(n)
+    if data == "ties":
+        g = g.mul(2.0).round()
+    elif data == "constant":
+        g.fill_(-3.0)
+    elif data == "ends":                       # only zeros and infinities
+        g = torch.where(g > 0.5, torch.inf, 0.0)
+    keys = g.abs().sort(descending=True).values
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    comp, dev = P.Compressor(env, n), g.cuda()
+    for rank in (1, 9, 31, 32, 99, 767, 768, n // 2, n - 1):
+        ratio = (rank + 0.5) / n               # ceil(n * ratio) - 1 == rank
+        if rank < n and ratio < 1.0:
+            comp.threshold_topk(dev, None, n, ratio, n, 1.0)
+            assert comp.thr.item() == float(keys[rank]), rank
+    env.close()
+
+
 def test_threshold_reference_vector(device):
     """test/threshold.cpp:58-85: 100 ints, top 10 % -> threshold 90, 10 elements pass with >=."""
     from helpers import alt_ramp
