@@ -345,6 +345,32 @@ def test_apply_add_and_set(world, n, out_dtype):
     assert st.value == 0
 
 
+@pytest.mark.parametrize("counts", [[0], [1024], [0, 0, 33], [31, 32, 33, 0, 1, 1024, 0, 64, 65, 0], [257] * 3 + [0] * 9])
+def test_apply_set_segment_lengths(world, counts):
+    """Segments of a sub-tile at the edges of the decode's rows of 32 pairs and batches of rows."""
+    e0, dev, n = world.envs[0], world.device, 3 * 1024 + 100
+    torch.manual_seed(len(counts))
+    eps, want = [], torch.zeros(n)
+    for c in counts:
+        x = torch.zeros(n)
+        for k, base in enumerate((0, 1024, 2048, 3072)):     # the second sub-tile is full, the third empty
+            tile = min(1024, n - base)
+            m = min(tile, (c, 1024 if c else 0, 0, c)[k])
+            x[base + torch.randperm(tile)[:m]] = torch.randn(m)
+        slot = P.SparseSlot.create(e0, n, n)
+        for e in world.envs[1:]:
+            P.SparseSlot.create(e, n, n)
+        comp = P.Compressor(e0, n)
+        comp.set_threshold(0.0)
+        comp.compress(x.to(dev), None, n, n, 3, P.make_targets([slot.endpoint(e0, 0)]))
+        eps.append(slot.endpoint(e0, 0))
+        want += x
+    st, out = e0.new_status("t"), torch.full((n,), 7.0, device=dev)
+    P.apply_sparse(e0, P.make_sources(eps, [3] * len(eps)), n, P.args_set(out, 1.0), st)
+    e0.flush()
+    assert st.value == 0 and torch.equal(out.cpu(), want)
+
+
 @pytest.mark.parametrize("op", ["sgd", "sgd_wd", "momentum", "adamw"])
 @pytest.mark.parametrize("shadow", [False, True])
 def test_apply_fused_updates(world, op, shadow):
