@@ -93,13 +93,15 @@ __device__ __forceinline__ void segment_prefix(int lane, uint32_t a, uint32_t b,
 
 // The sparse ops: pairs go straight into the vector, source after source.  A warp takes up to 32
 // neighbouring sub-tiles at a time: lane l looks sub-tile l up, a scan lays the sub-tiles' pairs end
-// to end, and the lanes walk that sequence, kAhead x 32 pairs in flight.  So a warp is busy whatever
+// to end, and the lanes walk that sequence, AHEAD x 32 pairs in flight.  So a warp is busy whatever
 // the density (10 pairs per sub-tile and source at top-k 1 %), and the chain of dependent loads
 // (table, pairs, elements) is paid once per group and source: 2^28 elements at 1 %, one source, took
 // 165 us with one sub-tile per warp at a time.
-constexpr int kAhead = 4;
+// Large groups (many sub-tiles per warp, two rounds or more) take eight rows at a time: 2^28 elements at 1 %
+// 653 -> 646 us; the registers that this costs leave fewer warps, 25 M elements at 0.1 % 57 -> 59 us with it.
+constexpr int kAhead = 4, kAheadLarge = 8, kLargeGroup = 16;
 
-template <typename TO>
+template <typename TO, int AHEAD>
 __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_constant__ ApplyParams p) {
   cx::pdl_trigger();
   if (p.front_wait) cx::pdl_wait();
@@ -122,14 +124,18 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
       uint32_t pre, total;
       segment_prefix(lane, a, b, pre, total);
       const CxPair* pairs = p.src.ep[j].pairs;
-      for (uint32_t f0 = 0; f0 < total; f0 += 32 * kAhead) {
-        CxPair pr[kAhead];
-        uint32_t lo[kAhead];
-        bool in[kAhead];
+      for (uint32_t f0 = 0; f0 < total; f0 += 32 * AHEAD) {
+        CxPair pr[AHEAD];
+        uint32_t lo[AHEAD];
+        bool in[AHEAD];
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
           const uint32_t f = f0 + 32 * k + lane;
           in[k] = f < total;
+          lo[k] = 0;
+          pr[k].idx = 0;
+          pr[k].val = 0;
+          if (f0 + 32 * k >= total) continue;      // warp-uniform
           uint32_t o = 0;          // the last sub-tile whose pairs start at or before f
 #pragma unroll
           for (uint32_t d = 16; d > 0; d >>= 1) {
@@ -138,22 +144,20 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
           }
           const uint32_t off = __shfl_sync(0xffffffffu, a, o) + (f - __shfl_sync(0xffffffffu, pre, o));
           lo[k] = ((uint32_t)s0 + o) * CX_SUBTILE;
-          pr[k].idx = 0;
-          pr[k].val = 0;
           if (in[k]) pr[k] = ld_pair(pairs + off);
         }
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
           if (in[k] && !((uint32_t)pr[k].idx - lo[k] < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { in[k] = false; bad = CX_ST_BAD_INDEX; }
         }
         // indices are unique inside one payload: the loads may all go first
-        float cur[kAhead];
+        float cur[AHEAD];
         if (sgd) {
           float* w = reinterpret_cast<float*>(p.a.out);
 #pragma unroll
-          for (int k = 0; k < kAhead; ++k) cur[k] = in[k] ? w[pr[k].idx] : 0.f;
+          for (int k = 0; k < AHEAD; ++k) cur[k] = in[k] ? w[pr[k].idx] : 0.f;
 #pragma unroll
-          for (int k = 0; k < kAhead; ++k) {
+          for (int k = 0; k < AHEAD; ++k) {
             const float nw = cur[k] + scale * __uint_as_float(pr[k].val);
             if (in[k]) w[pr[k].idx] = nw;
             if (in[k] && p.a.shadow) reinterpret_cast<TO*>(p.a.shadow)[pr[k].idx] = cx::Elem<TO>::from_f(nw);
@@ -161,9 +165,9 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
         } else {
           TO* out = reinterpret_cast<TO*>(p.a.out);
 #pragma unroll
-          for (int k = 0; k < kAhead; ++k) cur[k] = in[k] ? cx::Elem<TO>::to_f(out[pr[k].idx]) : 0.f;
+          for (int k = 0; k < AHEAD; ++k) cur[k] = in[k] ? cx::Elem<TO>::to_f(out[pr[k].idx]) : 0.f;
 #pragma unroll
-          for (int k = 0; k < kAhead; ++k)
+          for (int k = 0; k < AHEAD; ++k)
             if (in[k]) out[pr[k].idx] = cx::Elem<TO>::from_f(cur[k] + scale * __uint_as_float(pr[k].val));
         }
       }
@@ -813,7 +817,8 @@ int launch_apply(const ApplyParams& p, int grid, cudaStream_t s) {
     if (op == CX_OP_ADAMW) return launch_bulk<CX_OP_ADAMW, TO>(p, s);
   }
   const bool cap = p.seq_cell != nullptr;
-  if (sparse) cx_launch_pdl(apply_sparse_kernel<TO>, grid, kThreads, 0, s, p, cap);
+  if (sparse && p.group >= kLargeGroup) cx_launch_pdl(apply_sparse_kernel<TO, kAheadLarge>, grid, kThreads, 0, s, p, cap);
+  else if (sparse) cx_launch_pdl(apply_sparse_kernel<TO, kAhead>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_SET) cx_launch_pdl(apply_dense_kernel<CX_OP_SET, TO>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_SGD) cx_launch_pdl(apply_dense_kernel<CX_OP_SGD, TO>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_MOMENTUM) cx_launch_pdl(apply_dense_kernel<CX_OP_MOMENTUM, TO>, grid, kThreads, 0, s, p, cap);

@@ -36,10 +36,10 @@
 
 namespace {
 
-// Two CTAs (16 warps) per SM: each lane keeps a whole sub-tile share of 32 values in registers
-// with all its loads in flight, which needs ~100 registers; squeezing the kernel into three or
-// more CTAs per SM makes it spill and measured slower at every size (2^24 elements, 1 %: 55 us
-// with two, 69 us with three), and so did an L2 prefetch of the warp's next sub-tile.
+// Two CTAs of 256 threads or their like (16 warps) per SM: each lane keeps a whole sub-tile share of 32
+// values in registers with all its loads in flight, which needs ~100 registers; squeezing more warps onto
+// an SM makes it spill and measured slower at every size (2^24 elements, 1 %: 55 us with 16 warps, 69 us
+// with 24), and so did an L2 prefetch of the warp's next sub-tile.
 #ifndef CX_COMPRESS_MIN_BLOCKS
 #define CX_COMPRESS_MIN_BLOCKS 2
 #endif
@@ -50,8 +50,15 @@ namespace {
 #define CX_COMPRESS_BULK_DEFAULT 0
 #endif
 
-constexpr int kThreads = 256;
+// Warps of one CTA wait for one another only at its end, so small CTAs spread a short vector over more
+// SMs and let each go as soon as it is done: 65 536 elements 12.3 us with 256 threads, 12.0 with 128 and
+// 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference, and the kernel that
+// folds (below) is 0.5 us slower with them.
+constexpr int kThreads = 64;
 constexpr int kWarps = kThreads / 32;
+constexpr int kFoldThreads = 256;
+constexpr int kPerSm = CX_COMPRESS_MIN_BLOCKS * kFoldThreads / kThreads;
+constexpr int kFoldWarps = kFoldThreads / 32;
 constexpr int kChunks = CX_SUBTILE / 128;  // 128 elements = 32 lanes x 4
 constexpr int kStage = 128;                // pairs staged per warp and pass
 
@@ -453,7 +460,7 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
 // the multicast endpoint tg.ep[tg.count] (multimem.st) instead of once per target; headers and
 // notifications are still written target by target.
 template <typename T, bool HAS_G, bool HAS_R, bool MC>
-__global__ void __launch_bounds__(kThreads, CX_COMPRESS_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, kPerSm)
 compress_kernel(const __grid_constant__ CompressParams p) {
   __shared__ CxPair s_stage[kWarps][kStage];
 
@@ -524,9 +531,9 @@ compress_kernel(const __grid_constant__ CompressParams p) {
 // 13.1 M bf16 gradients with momentum: 44 us for the fold and 34 us for the compression as two
 // kernels.
 template <typename T, bool MC, Input IN>
-__global__ void __launch_bounds__(kThreads, CX_COMPRESS_MIN_BLOCKS)
+__global__ void __launch_bounds__(kFoldThreads, CX_COMPRESS_MIN_BLOCKS)
 compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
-  __shared__ CxPair s_stage[kWarps][kStage];
+  __shared__ CxPair s_stage[kFoldWarps][kStage];
   const CompressParams& p = q.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* __restrict__ r = p.r;
@@ -535,11 +542,11 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   const float thr = *p.thr;
   Tally tally = {0, false};
   if (blockIdx.x < q.nborder_ctas) {
-    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kWarps)
+    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kFoldWarps)
       compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, tally, &q.f);
   } else {
-    const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kWarps;
-    uint32_t sub = (blockIdx.x - q.nborder_ctas) * kWarps + warp;
+    const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kFoldWarps;
+    uint32_t sub = (blockIdx.x - q.nborder_ctas) * kFoldWarps + warp;
     cx::FoldWhole<T> cur = {nullptr, 0.f, 0};
     if (sub < p.nsub) cur = cx::fold_whole<T>(q.f, sub);
     while (sub < p.nsub) {
@@ -559,7 +566,7 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
       sub = next;
     }
   }
-  compress_finish<kWarps>(p, tid, thr, false, tally);
+  compress_finish<kFoldWarps>(p, tid, thr, false, tally);
   if (q.chain & CX_CHAINED) cx::pdl_wait();
 }
 
@@ -777,7 +784,7 @@ void fill_params(CompressParams& p, const void* g, float* r, int64_t n, const fl
 }
 
 int grid_for(const CompressParams& p) {
-  const int grid = cx_sm_count() * CX_COMPRESS_MIN_BLOCKS;
+  const int grid = cx_sm_count() * kPerSm;
   const int need = (int)((p.nsub + kWarps - 1) / kWarps);
   return grid < need ? grid : need;
 }
@@ -786,10 +793,10 @@ template <typename T, Input IN>
 void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
   FoldCompressParams p = q;
   int grid;
-  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, kWarps, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS, &grid);
+  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, kFoldWarps, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS, &grid);
   const bool capturing = q.c.seq_cell != nullptr;
-  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN>, grid, kThreads, 0, s, p, capturing);
-  else cx_launch_pdl(compress_fold_kernel<T, false, IN>, grid, kThreads, 0, s, p, capturing);
+  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN>, grid, kFoldThreads, 0, s, p, capturing);
+  else cx_launch_pdl(compress_fold_kernel<T, false, IN>, grid, kFoldThreads, 0, s, p, capturing);
 }
 
 template <typename T>

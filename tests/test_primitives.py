@@ -371,6 +371,30 @@ def test_apply_set_segment_lengths(world, counts):
     assert st.value == 0 and torch.equal(out.cpu(), want)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", ["add", "sgd"])
+def test_apply_sparse_large_groups(op):
+    """Vectors so long that a warp of the sparse decode takes 16 sub-tiles or more at a time."""
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    n = (1 << 27) + 5
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.zeros(n, device="cuda")
+    at = torch.randint(0, n, (1 << 20,), device="cuda", generator=gen)
+    x[at] = torch.randn(at.numel(), device="cuda", generator=gen)
+    x[5 * 1024:7 * 1024] = 1.5                     # two full sub-tiles
+    cap = 1 << 21
+    slot, comp, st = P.SparseSlot.create(env, n, cap), P.Compressor(env, n), env.new_status("t")
+    comp.set_threshold(0.0)
+    comp.compress(x, None, n, cap, 3, P.make_targets([slot.endpoint(env, 0)]))
+    src = P.make_sources([slot.endpoint(env, 0)], [3])
+    out = torch.ones(n, device="cuda")
+    args = P.args_add(out, 0.5) if op == "add" else P.args_update(_lib.OP_SGD, out, 0.25)
+    P.apply_sparse(env, src, n, args, st)
+    env.flush()
+    assert st.value == 0 and torch.equal(out, 1 + 0.5 * x if op == "add" else 1 - 0.25 * x)
+    env.close()
+
+
 @pytest.mark.parametrize("op", ["sgd", "sgd_wd", "momentum", "adamw"])
 @pytest.mark.parametrize("shadow", [False, True])
 def test_apply_fused_updates(world, op, shadow):
