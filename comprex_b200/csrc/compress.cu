@@ -53,7 +53,7 @@ namespace {
 // Warps of one CTA wait for one another only at its end, so small CTAs spread a short vector over more
 // SMs and let each go as soon as it is done: 65 536 elements 12.3 us with 256 threads, 12.0 with 128 and
 // 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference, and the kernel that
-// folds (below) is 0.5 us slower with them.
+// folds (below) is slower with them.
 constexpr int kThreads = 64;
 constexpr int kWarps = kThreads / 32;
 constexpr int kFoldThreads = 256;
@@ -530,10 +530,11 @@ compress_kernel(const __grid_constant__ CompressParams p) {
 // that one tensor covers take the register path, the ones at tensor borders the edge path.
 // 13.1 M bf16 gradients with momentum: 44 us for the fold and 34 us for the compression as two
 // kernels.
-template <typename T, bool MC, Input IN>
-__global__ void __launch_bounds__(kFoldThreads, CX_COMPRESS_MIN_BLOCKS)
+template <typename T, bool MC, Input IN, int THREADS>
+__global__ void __launch_bounds__(THREADS, CX_COMPRESS_MIN_BLOCKS * kFoldThreads / THREADS)
 compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
-  __shared__ CxPair s_stage[kFoldWarps][kStage];
+  constexpr int WARPS = THREADS / 32;
+  __shared__ CxPair s_stage[WARPS][kStage];
   const CompressParams& p = q.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* __restrict__ r = p.r;
@@ -542,11 +543,11 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   const float thr = *p.thr;
   Tally tally = {0, false};
   if (blockIdx.x < q.nborder_ctas) {
-    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * kFoldWarps)
+    for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * WARPS)
       compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, tally, &q.f);
   } else {
-    const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kFoldWarps;
-    uint32_t sub = (blockIdx.x - q.nborder_ctas) * kFoldWarps + warp;
+    const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * WARPS;
+    uint32_t sub = (blockIdx.x - q.nborder_ctas) * WARPS + warp;
     cx::FoldWhole<T> cur = {nullptr, 0.f, 0};
     if (sub < p.nsub) cur = cx::fold_whole<T>(q.f, sub);
     while (sub < p.nsub) {
@@ -566,7 +567,7 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
       sub = next;
     }
   }
-  compress_finish<kFoldWarps>(p, tid, thr, false, tally);
+  compress_finish<WARPS>(p, tid, thr, false, tally);
   if (q.chain & CX_CHAINED) cx::pdl_wait();
 }
 
@@ -789,14 +790,22 @@ int grid_for(const CompressParams& p) {
   return grid < need ? grid : need;
 }
 
-template <typename T, Input IN>
-void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
+template <typename T, Input IN, int THREADS>
+void launch_fold_threads(const FoldCompressParams& q, cudaStream_t s) {
   FoldCompressParams p = q;
   int grid;
-  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, kFoldWarps, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS, &grid);
+  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, THREADS / 32, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS * (kFoldThreads / THREADS), &grid);
   const bool capturing = q.c.seq_cell != nullptr;
-  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN>, grid, kFoldThreads, 0, s, p, capturing);
-  else cx_launch_pdl(compress_fold_kernel<T, false, IN>, grid, kFoldThreads, 0, s, p, capturing);
+  if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
+  else cx_launch_pdl(compress_fold_kernel<T, false, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
+}
+
+// small CTAs for a vector too short for a large one on every SM (LeNet step 22.1 -> 21.8 us; the 13 M
+// element buckets of a ResNet-50 step are 0.6 us faster with the large ones)
+template <typename T, Input IN>
+void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
+  if (q.c.nsub <= (uint32_t)(cx_sm_count() * kFoldWarps)) launch_fold_threads<T, IN, kThreads>(q, s);
+  else launch_fold_threads<T, IN, kFoldThreads>(q, s);
 }
 
 template <typename T>
