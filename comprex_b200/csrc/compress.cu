@@ -389,7 +389,14 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
 // every exchange; they are read only when survivors did not fit.)  `failed`: this CTA could not
 // process all its sub-tiles; the payload is then not published (the receivers' bounded waits run
 // out) and the status says why.
-constexpr int kArrived = 32, kOver = 44, kFailed = 54;     // bit positions behind the survivors; grids have < 4096 CTAs
+//
+// The fields: 31 bits for the survivors (a vector has fewer than 2^31 elements), 12 for the CTAs that arrived,
+// 12 for those whose survivors did not all fit (all of them may say so: a dense residual that is flushed does
+// that), 9 for those that failed (only the bulk variant's can, one CTA per SM).  No field may carry into the
+// next one: the launches below keep their grids within kMaxGrid and kMaxBulkGrid.
+constexpr int kArrived = 31, kOver = 43, kFailed = 55;
+constexpr int kMaxGrid = (1 << (kOver - kArrived)) - 1, kMaxBulkGrid = (1 << (64 - kFailed)) - 1;
+static_assert(kFailed - kOver >= kOver - kArrived, "every CTA that arrives may have overflowed");
 
 template <int MAX_WARPS>
 __device__ __forceinline__ void compress_finish(const CompressParams& p, const int tid, const float thr, const bool failed,
@@ -416,9 +423,9 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
   __syncthreads();
   CX_TRACE(3);
   const unsigned long long all = s_all;
-  if (((all >> kArrived) & 0xfffu) != gridDim.x) return;
-  const uint32_t found = (uint32_t)all;   // survivors
-  const bool over = ((all >> kOver) & 0x3ffu) != 0, any_failed = (all >> kFailed) != 0;
+  if (((all >> kArrived) & (uint32_t)kMaxGrid) != gridDim.x) return;
+  const uint32_t found = (uint32_t)(all & ((1ull << kArrived) - 1));   // survivors
+  const bool over = ((all >> kOver) & ((1u << (kFailed - kOver)) - 1)) != 0, any_failed = (all >> kFailed) != 0;
   uint32_t nnz = found;                   // pairs stored
   if (over) {
     if ((uint32_t)tid < p.nregions)
@@ -731,6 +738,7 @@ int launch_bulk_one(const CompressParams& p, cudaStream_t s) {
     configured[dev] = true;
   }
   int grid = cx_sm_count();
+  if (grid > kMaxBulkGrid) grid = kMaxBulkGrid;
   const int need = (int)((p.nsub + nw - 1) / nw);
   if (grid > need) grid = need;
   cx_launch_pdl(kern, grid, nw * 32, smem, s, p, p.seq_cell != nullptr);
@@ -784,8 +792,14 @@ void fill_params(CompressParams& p, const void* g, float* r, int64_t n, const fl
   p.tg = *tg;
 }
 
+// one wave of CTAs, no more than the completion counter's fields hold
+int wave(int per_sm) {
+  const int grid = cx_sm_count() * per_sm;
+  return grid < kMaxGrid ? grid : kMaxGrid;
+}
+
 int grid_for(const CompressParams& p) {
-  const int grid = cx_sm_count() * kPerSm;
+  const int grid = wave(kPerSm);
   const int need = (int)((p.nsub + kWarps - 1) / kWarps);
   return grid < need ? grid : need;
 }
@@ -794,7 +808,7 @@ template <typename T, Input IN, int THREADS>
 void launch_fold_threads(const FoldCompressParams& q, cudaStream_t s) {
   FoldCompressParams p = q;
   int grid;
-  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, THREADS / 32, cx_sm_count() * CX_COMPRESS_MIN_BLOCKS * (kFoldThreads / THREADS), &grid);
+  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, THREADS / 32, wave(CX_COMPRESS_MIN_BLOCKS * (kFoldThreads / THREADS)), &grid);
   const bool capturing = q.c.seq_cell != nullptr;
   if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
   else cx_launch_pdl(compress_fold_kernel<T, false, IN, THREADS>, grid, THREADS, 0, s, p, capturing);

@@ -689,3 +689,22 @@ def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange, l
     for a, b in zip(*arms):
         assert torch.equal(a, b)
     env.close()
+
+
+@pytest.mark.gpu
+def test_flush_of_a_dense_residual_of_a_large_bucket():
+    """The flush sends a dense residual through slots of half its size, several rounds in which every CTA
+    finds its region full: all of it arrives, nothing is left."""
+    env = cx.GaspiEnvironment(256 << 20, device="cuda", timeout_ms=2000)
+    n = 13_000_003
+    opt = ComprexOptimizer([torch.nn.Parameter(torch.zeros(n, device="cuda"))], env, lr=1.0, momentum=0.0,
+                           pre_clipnorm=None, single_rank_bypass=False)
+    opt.describe()                                   # sets the exchange up
+    rests = next(iter(opt.comprex_allreducers.values())).rests
+    rests.normal_(generator=torch.Generator(device="cuda").manual_seed(1)).abs_().add_(0.25)
+    want = -rests
+    opt.flush()
+    env.flush()
+    env.check()
+    assert torch.equal(opt._master[:n], want[:n]) and not rests.any()
+    env.close()

@@ -283,6 +283,36 @@ def test_compress_capacity_overflow_keeps_residual(world):
     e0.check()  # overflow is soft: no exception
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", [2, 64])
+@pytest.mark.parametrize("has_g", [False, True])
+def test_compress_overflow_in_every_cta(share, has_g):
+    """A dense vector through a slot of n / share pairs: the survivors of every CTA of a full grid do not
+    fit.  The payload is published all the same, every region is full, and what was not sent stays."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    e0, e1 = world.envs
+    n = (1 << 24) + 5
+    cap = n // share
+    slot = [P.SparseSlot.create(e, n, cap) for e in world.envs][1]
+    gen = torch.Generator(device="cuda").manual_seed(share)
+    r = torch.randn(n, device="cuda", generator=gen).abs_().add_(0.25)
+    g = torch.randn(n, device="cuda", generator=gen).abs_() if has_g else None
+    x = r + g if has_g else r.clone()
+    comp = P.Compressor(e0, n)
+    comp.set_threshold(0.0)
+    comp.compress(g, r, n, cap, 1, P.make_targets([slot.endpoint(e0, 1)]))
+    e0.flush()
+    st = comp.last_stats()
+    assert st["status"] == _lib.ST_OVERFLOW
+    regions, region_size = P.compress_regions(n, cap)
+    hdr, idx, val, _ = read_pairs(e1, slot)
+    assert hdr.seq == 1 and hdr.nnz_found == n and hdr.nnz == st["nnz"] == regions * region_size
+    sent = torch.zeros(n)
+    sent[idx.long()] = val
+    assert idx.unique().numel() == hdr.nnz and torch.equal(sent + r.cpu(), x.cpu())
+    world.close()
+
+
 @pytest.mark.parametrize("mode", ["update", "plain"])
 def test_compress_modes(world, mode):
     e0, e1 = world.envs
