@@ -117,6 +117,7 @@ def _declare(lib) -> None:
         "cx_threshold_topk": (i32, [i32, i32, vp, vp, i64, f32, i32, f32, vp, vp]),
         "cx_threshold_workspace_bytes": (i64, []),
         "cx_threshold_exact_bytes": (i64, [i64]),
+        "cx_threshold_whole": (i32, [i64, f32, i32, f32]),
         "cx_threshold_select": (i32, [i32, i32, vp, vp, i64, f32, i32, f32, vp, vp, i64, vp]),
         "cx_compress": (i32, [i32, i32, vp, vp, i64, vp, u32, u64, P(Targets), vp, i64, vp, u32, vp]),
         "cx_apply": (i32, [i32, P(Sources), i64, P(ApplyArgs), vp, u64, vp]),

@@ -439,8 +439,13 @@ class _ComprexAllreduceBase(_AllreduceBase):
 
     @property
     def exact_topk(self) -> bool:
-        """True when the threshold comes from the whole vector (:meth:`set_exact_topk`)."""
-        return self._subsamples >= _EXACT_SAMPLES
+        """True when the threshold comes from a select over the whole vector: :meth:`set_exact_topk`, or
+        a fraction so small that the sampling rule asks for every element."""
+        rule = (self.size, self.compression_ratio, self._subsamples, self._sample_factor)
+        got = self.__dict__.get("_whole")
+        if got is None or got[0] != rule:
+            got = self._whole = (rule, bool(self._env.lib.cx_threshold_whole(*rule)))
+        return self._subsamples >= _EXACT_SAMPLES or got[1]
 
     def set_exact_topk(self, exact: bool = True) -> None:
         """Threshold from a select over the whole vector (exactly top-k) instead of the sampled

@@ -197,6 +197,9 @@ int cx_threshold_topk(int dev, int gdtype, const void* g, const float* r,
 int64_t cx_threshold_workspace_bytes(void);
 /* Scratch (zeroed once) with which that selection makes one pass over the vector instead of four. */
 int64_t cx_threshold_exact_bytes(int64_t n);
+/* 1 if the CUDA back end selects over the whole vector under this sampling rule: the sample is every element,
+ * and they do not fit one CTA.  That selection reads a stored vector (CxOp::fold is refused). */
+int cx_threshold_whole(int64_t n, float ratio, int default_subsamples, float subsample_factor);
 int cx_threshold_select(int dev, int gdtype, const void* g, const float* r, int64_t n, float ratio,
                         int default_subsamples, float subsample_factor, float* thr_out, void* workspace,
                         int64_t ws_bytes, void* stream);

@@ -853,11 +853,19 @@ void sampled_params(ThreshParams& p, const void* g, const float* r, int64_t n, f
 // a cluster of 8 CTAs gathers large samples (their keys must fit the first CTA's shared memory)
 unsigned cluster_for(const ThreshParams& p) { return (p.samples > 2048 && p.samples <= kSmemKeys) ? 8u : 1u; }
 
+bool whole_vector(const ThreshParams& p) { return p.use_all && p.topk_pos > 0 && p.n > kSmemKeys; }
+
 bool exact_wanted(const ThreshParams& p, const void* workspace, int64_t ws_bytes) {
-  return p.use_all && p.topk_pos > 0 && p.n > kSmemKeys && workspace && ws_bytes >= cx_threshold_workspace_bytes();
+  return whole_vector(p) && workspace && ws_bytes >= cx_threshold_workspace_bytes();
 }
 
 }  // namespace
+
+extern "C" int cx_threshold_whole(int64_t n, float ratio, int default_subsamples, float subsample_factor) {
+  ThreshParams p;
+  sampled_params(p, nullptr, nullptr, n, ratio, default_subsamples, subsample_factor, nullptr);
+  return whole_vector(p) ? 1 : 0;
+}
 
 int cx_threshold_topk_cuda(int gdtype, const void* g, const float* r, int64_t n, float ratio,
                            int default_subsamples, float subsample_factor, float* thr_out,

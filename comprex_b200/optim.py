@@ -453,7 +453,7 @@ class ComprexOptimizer(torch.optim.Optimizer):
     # ---- the fused forms (CUDA) -------------------------------------------------------------------
     def _fusable(self, b: _Bucket) -> bool:
         """The compress kernel can fold the bucket's gradients itself: compressed BigRing, sampled
-        threshold (an exact selection reads a stored vector)."""
+        threshold (a selection over the whole vector reads a stored one)."""
         return self._cuda and b.kind == "bigring" and not b.ar.exact_topk
 
     def _fold_args(self, ft: _FoldTable, b: _Bucket, mu: float):

@@ -708,3 +708,46 @@ def test_flush_of_a_dense_residual_of_a_large_bucket():
     env.check()
     assert torch.equal(opt._master[:n], want[:n]) and not rests.any()
     env.close()
+
+
+@pytest.mark.parametrize("n,ratio,whole", [(11008, 1e-4, False), (11009, 1e-4, True), (39999, 1e-4, True), (40000, 1e-4, False),
+                                           (62000, 5e-5, True), (20000, 1e-2, False)])
+def test_whole_vector_selection_is_named(n, ratio, whole):
+    """A fraction so small that the sample is the whole vector, which does not fit one CTA."""
+    env = cx.GaspiEnvironment(1 << 20, device="cpu")
+    ar = cx.Comprex_BigRingAllreduce(env)
+    ar.setup_connections(n, 1, ratio, 1.0, consistent=True)
+    assert ar.exact_topk is whole
+    ar.set_compression_ratio(1e-2)
+    assert ar.exact_topk is False
+    ar.set_exact_topk(True)
+    assert ar.exact_topk is True
+    env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[11009, 20000], [11008, 39999, 40000], [200000, 20000], [62000]])
+@pytest.mark.parametrize("ratio", [1e-4, 5e-5])
+def test_step_whose_sample_is_the_whole_bucket(sizes, ratio):
+    """Fractions below 1 / 2750: buckets whose sample is every element, buckets whose sample exceeds one
+    CTA's shared memory, and both in one step, against the vector built in memory first."""
+    arms = []
+    for fused in (True, False):
+        torch.manual_seed(5)
+        env = cx.GaspiEnvironment(8 << 20, device="cuda")
+        params = [torch.nn.Parameter(torch.randn(s, device="cuda")) for s in sizes]
+        opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.9, compression_ratio=ratio, pre_clipnorm=20.0,
+                               aggregate_blob=False, single_rank_bypass=False)
+        assert len(opt._buckets) == len(sizes)
+        if not fused:
+            opt._fusable = lambda b: False
+        for step in range(3):
+            gen = torch.Generator(device="cuda").manual_seed(step)
+            for p in params:
+                p.grad = torch.randn(p.numel(), device="cuda", generator=gen)
+            opt.step()
+        env.flush()
+        arms.append([opt._master.clone(), opt._update.clone()] + [ar.rests.clone() for ar in opt.comprex_allreducers.values()])
+        env.close()
+    for a, b in zip(*arms):
+        assert torch.equal(a, b)
