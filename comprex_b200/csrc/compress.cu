@@ -404,14 +404,16 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
   __shared__ uint32_t s_found[MAX_WARPS], s_mark[MAX_WARPS];
   __shared__ unsigned long long s_all;
   __shared__ uint32_t s_nnz;
-  // the receive kernel queued behind this one may become resident now: it polls its flags
-  cx::pdl_trigger();
   const int nw = blockDim.x >> 5;
   if ((tid & 31) == 0) {
     s_found[tid >> 5] = tally.found;
     s_mark[tid >> 5] = (tally.over ? 1u : 0u) | (failed ? 2u : 0u);
   }
   __syncthreads();            // all stores of the CTA are issued
+  // The receive kernel queued behind this one may become resident now: it polls its flags.  Not before the
+  // barrier: one thread's trigger counts for its CTA, and a receiver whose payloads are all there already
+  // may write the vector that the CTA's other warps still read.
+  cx::pdl_trigger();
   if (tid == 0) {
     uint32_t found = 0, mark = 0;
     for (int w = 0; w < nw; ++w) { found += s_found[w]; mark |= s_mark[w]; }

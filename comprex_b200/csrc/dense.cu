@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 4) dense_send_kernel(const __grid_co
       }
     }
   }
+  __syncthreads();     // one thread's trigger counts for its CTA: every thread has read its part of g
   cx::pdl_trigger();   // the reducing kernel queued behind this one may become resident and poll
   if (!cx::cta_arrive(&p.ctr->done, gridDim.x, &s_last)) return;
   if ((int)threadIdx.x < p.tg.count)

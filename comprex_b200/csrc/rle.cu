@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(kThreads, kSendPerSm) rle_emit_kernel(const __
   }
   if (lo < hi && hi == p.n && lane < p.tg.count)     // the warp that holds the last element closes the last run
     reinterpret_cast<int32_t*>(reinterpret_cast<char*>(p.tg.ep[lane].pairs) + runs_off)[q0 - 1] = (int)(p.n - prev);
+  __syncthreads();       // one thread's trigger counts for its CTA: every warp has read its chunk of g
   cx::pdl_trigger();
   if (!cx::cta_arrive(&p.meta->done, gridDim.x, &s_lastblock)) return;
   if (tid < p.tg.count) {

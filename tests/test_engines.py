@@ -249,3 +249,44 @@ def test_fastcomprex_is_one_step_stale_and_conserves(world):
         ra, rb = a[1].readRemote(), b[2].readRemote()
         assert torch.equal(ra, rb)
     assert float(ra.abs().sum()) > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [5003, (1 << 24) + 3])
+@pytest.mark.parametrize("kind", ["pairs", "exact", "rle", "dense"])
+@pytest.mark.parametrize("add", [True, False])
+def test_receive_into_the_vector_just_sent(n, kind, add):
+    """writeRemote(v) and then a receive into the same v, while the peer's message is already there: the
+    receive kernel has nothing to wait for but the sender in front of it, which must have read all of v."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    ex = [cx.GaspiEx(e, n) if kind == "dense" else cx.Comprex(e, n) for e in world.envs]
+    for r, e in enumerate(ex):
+        if kind != "dense":
+            e.setThreshold(cx.ThresholdTopK(0.1, exact=kind == "exact"))
+            e.setCompressor(cx.CompressorRLE() if kind == "rle" else cx.CompressorIndexPairs())
+        e.connectTo(1 - r, 1 - r)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    kept = [torch.zeros(n, device="cuda") for _ in ex]
+    for _ in range(3):
+        v, peer = (torch.randn(n, device="cuda", generator=gen) for _ in range(2))
+        before = v.clone()
+        torch.cuda.synchronize()
+        ex[1].writeRemote(peer)
+        ex[0].writeRemote(v)
+        if add:
+            ex[0].readRemote_add(v)
+        else:
+            (ex[0].readRemote_vec if kind == "dense" else ex[0].readRemote)(v)
+        got = torch.empty(n, device="cuda")
+        (ex[1].readRemote_vec if kind == "dense" else ex[1].readRemote)(got)
+        if kind == "dense":
+            sent, here = before, peer
+        else:
+            # an element is either sent or kept: both sums are exact
+            sent = before + kept[0] - ex[0].getRests()
+            here = peer + kept[1] - ex[1].getRests()
+            kept = [e.getRests() for e in ex]
+        assert torch.equal(got, sent) and torch.equal(v, before + here if add else here)
+        for e in world.envs:
+            e.check()
+    world.close()
