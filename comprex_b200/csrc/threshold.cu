@@ -506,8 +506,10 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_kernel(const __grid_c
   const int tid = threadIdx.x;
   uint32_t* k0 = cluster.map_shared_rank(s_keys, 0);
   uint32_t* k1 = cluster.map_shared_rank(s_keys, 1);
+  cluster.barrier_arrive();
   cx::pdl_wait();
   cx::pdl_trigger();
+  cluster.barrier_wait();             // every CTA runs: the first two's shared memory may be written
   {
     constexpr int kEach = kBracket / kCluster / kBracketThreads;
     uint32_t k[kEach];
