@@ -248,8 +248,9 @@ bool cx_pdl_enabled();   // COMPREX_PDL != 0 (read once)
 // The kernels that end a message or a step call pdl_trigger at their start: the kernel behind (the
 // threshold of the next message, the norms of the next step) waits at its own start, and its launch
 // is over when it may go on.  A receive kernel, however, does not wait at its start when its sender is
-// in front of it, so it has to know what is: senders note "not early", kernels that trigger at their
-// start note "early", and cx_front_wait says whether the kernel about to be launched must wait first.
+// in front of it, so it has to know what is: senders note "not early"; every other kernel that triggers
+// before it is done with its operands notes "early" (receive kernels, thresholds, norms, dense updates),
+// and cx_front_wait says whether the kernel about to be launched must wait first.
 void cx_note_stream(const void* stream, bool early);
 bool cx_front_wait(const void* stream);
 

@@ -204,6 +204,7 @@ int cx_fold_coef_cuda(int gdtype, const CxFoldCoef* f, void* stream) {
     cx_launch_pdl(fold_coef_kernel, (f->segs + kThreads - 1) / kThreads, kThreads, 0, s, p, cx_seq_cell() != nullptr);
     cx_note_launch();
   }
+  cx_note_stream(stream, true);  // the norms read the gradients behind their trigger
   return cx_check_launch("fold kernels");
 }
 

@@ -760,6 +760,7 @@ int launch_one_pass(const OnePassParams& p, bool capturing, cudaStream_t s) {
   cx_launch_pdl(collect_kernel<T>, grid, kCollectThreads, 0, s, p, capturing);
   e = cudaLaunchKernelEx(&cfg, exact_finish_kernel<T>, p);
   if (e != cudaSuccess) return cx_set_error("exact_finish_kernel launch", (int)e);
+  cx_note_stream(s, true);       // it may read the whole vector behind its trigger
   for (int k = 0; k < 3; ++k) cx_note_launch();
   return cx_check_launch("exact selection kernels");
 }
@@ -830,6 +831,7 @@ int launch_sampled(const ThreshParams* v, int count, unsigned ncta, bool capturi
     e = cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, kVectors>, b);
   }
   if (e != cudaSuccess) return cx_set_error("threshold_kernel launch", (int)e);
+  cx_note_stream(s, true);       // a sample larger than the cache is gathered again behind the trigger
   cx_note_launch();
   return cx_check_launch("threshold_kernel");
 }

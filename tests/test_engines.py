@@ -4,13 +4,15 @@ Scenarios follow the reference's own checks: test/comprex.cpp (3 x writeRemote +
 flushRests, receiver accumulates with readRemote_add, result == 3 * values),
 examples/comprEx.cpp, examples/gaspiEx.py.
 """
+import math
+
 import numpy as np
 import pytest
 import torch
 
 import comprex_b200 as cx
 
-from helpers import alt_ramp
+from helpers import alt_ramp, ref_threshold_topk
 
 
 @pytest.fixture
@@ -287,6 +289,50 @@ def test_receive_into_the_vector_just_sent(n, kind, add):
             here = peer + kept[1] - ex[1].getRests()
             kept = [e.getRests() for e in ex]
         assert torch.equal(got, sent) and torch.equal(v, before + here if add else here)
+        for e in world.envs:
+            e.check()
+    world.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["exact", "exact_ties", "sample", "large_sample"])
+@pytest.mark.parametrize("kind", ["pairs", "rle", "dense"])
+def test_receive_behind_a_threshold_of_the_same_vector(how, kind):
+    """writeRemote(x), a threshold of y, then a receive into y whose message is already there: the threshold
+    kernels let the receive kernel in early, and may read y again after that (candidates that do not fit,
+    a sample that exceeds one CTA)."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    n = (1 << 22) + 3
+    ex = [cx.GaspiEx(e, n) if kind == "dense" else cx.Comprex(e, n) for e in world.envs]
+    for r, e in enumerate(ex):
+        if kind != "dense":
+            e.setThreshold(cx.ThresholdTopK(0.1))
+            e.setCompressor(cx.CompressorRLE() if kind == "rle" else cx.CompressorIndexPairs())
+        e.connectTo(1 - r, 1 - r)
+    ratio = {"sample": 0.01, "large_sample": 0.0004}.get(how, 0.3)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    for _ in range(3):
+        x, y, peer = (torch.randn(n, device="cuda", generator=gen) for _ in range(3))
+        if how == "exact_ties":
+            y = torch.randint(0, 4, (n,), device="cuda", generator=gen).float()
+        if how.startswith("exact"):
+            want = float(y.abs().sort(descending=True).values[math.ceil(np.float32(n) * np.float32(ratio)) - 1])
+        else:
+            want = ref_threshold_topk(y, ratio)
+        before = y.clone()
+        thr = cx.ThresholdTopK(ratio, exact=how.startswith("exact"))
+        torch.cuda.synchronize()
+        ex[1].writeRemote(peer)
+        ex[0].writeRemote(x)
+        thr.prepare(y)
+        ex[0].readRemote_add(y)
+        assert thr.getThreshold() == want
+        here = peer
+        if kind != "dense":
+            here = peer - ex[1].getRests()
+            ex[1].resetRests()
+        assert torch.equal(y, before + here)
+        (ex[1].readRemote_vec if kind == "dense" else ex[1].readRemote)(x)
         for e in world.envs:
             e.check()
     world.close()
