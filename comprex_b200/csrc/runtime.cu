@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "cx_common.h"
+#include "cx_notes.h"
 
 #define CX_CHAINED 1u      /* as in cx_device.cuh */
 #define CX_CHAIN_NEXT 2u
@@ -85,18 +86,14 @@ void cx_note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static thread_local const uint64_t* g_seq_cell = nullptr;
 const uint64_t* cx_seq_cell() { return g_seq_cell; }
 // Whether the kernel this library launched last on a stream lets the kernel behind it in before it has
-// finished (cx_device.cuh).  A slot per stream (hashed); what is not known counts as one that does.
-static std::atomic<uint64_t> g_last[64];
-static std::atomic<uint64_t>& last_slot(const void* stream) {
-  const uint64_t s = reinterpret_cast<uint64_t>(stream);
-  return g_last[(s >> 4 ^ s >> 10 ^ s >> 16) & 63];
+// finished (cx_device.cuh).
+static CxStreamNotes g_notes;
+static int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
-void cx_note_stream(const void* stream, bool early) {
-  last_slot(stream).store(reinterpret_cast<uint64_t>(stream) << 2 | 2u | (early ? 1u : 0u), std::memory_order_relaxed);
-}
-bool cx_front_wait(const void* stream) {
-  return last_slot(stream).load(std::memory_order_relaxed) != (reinterpret_cast<uint64_t>(stream) << 2 | 2u);
-}
+void cx_note_stream(const void* stream, bool early) { g_notes.note(current_device(), stream, early); }
+bool cx_front_wait(const void* stream) { return g_notes.front_wait(current_device(), stream); }
 static thread_local uint32_t g_chain_bits = 0;
 uint32_t cx_chain_bits() { return g_chain_bits; }
 int cx_check_launch(const char* where) {

@@ -7,7 +7,8 @@
 //     no survivor, exactly `capacity` survivors, more survivors than capacity,
 //   * canary words before and after every slot region, checked after every case,
 //   * the two-parity slot protocol between two threads that play two ranks
-//     (send(s) -> recv(s) on both sides, slots alternating by the parity of s).
+//     (send(s) -> recv(s) on both sides, slots alternating by the parity of s),
+//   * the notes on streams that decide whether a receive kernel waits for the kernel in front.
 // Exit code 0 = all checks passed.
 #include <math.h>
 #include <stdint.h>
@@ -19,6 +20,7 @@
 #include <vector>
 
 #include "../cx_common.h"
+#include "../cx_notes.h"
 
 int cx_threshold_topk_host(int, const void*, const float*, int64_t, float, int, float, float*);
 int cx_compress_host(int, const void*, float*, int64_t, const float*, uint32_t, uint64_t,
@@ -232,6 +234,35 @@ static void protocol_case() {
   CHECK(status == CX_ST_TIMEOUT && out[0] == 3.f && out[(size_t)n - 1] == 3.f);
 }
 
+// Only the last note of the very stream lets a receive kernel go without waiting.
+static void notes_case() {
+  static CxStreamNotes notes;
+  const void *zero = nullptr, *a = (const void*)0x5000, *b = (const void*)0x9000;
+  CHECK(notes.front_wait(0, a));                       // nothing is known
+  notes.note(0, a, false);
+  CHECK(!notes.front_wait(0, a) && notes.front_wait(0, b));
+  notes.note(0, a, true);
+  CHECK(notes.front_wait(0, a));
+  notes.note(0, zero, true);                           // the default streams of two devices
+  notes.note(1, zero, false);
+  CHECK(notes.front_wait(0, zero) && !notes.front_wait(1, zero));
+  notes.note(1, (const void*)1, true);                 // the default stream by its other name
+  CHECK(notes.front_wait(1, zero));
+  notes.note(0, (const void*)2, false);                // another stream in every thread
+  CHECK(notes.front_wait(0, (const void*)2));
+  notes.note(-1, a, false);
+  notes.note(CxStreamNotes::kDevices, a, false);
+  CHECK(notes.front_wait(-1, a) && notes.front_wait(CxStreamNotes::kDevices, a));
+  for (uintptr_t k = 0; k < 4096; ++k) {               // streams that share a slot
+    notes.note(0, a, false);
+    const void* other = (const void*)(0x100000 + 16 * k);
+    notes.note(0, other, false);
+    CHECK(!notes.front_wait(0, other));
+    notes.note(0, other, true);
+    CHECK(notes.front_wait(0, other));
+  }
+}
+
 int main(int argc, char** argv) {
   const bool only_protocol = argc > 1 && !strcmp(argv[1], "--protocol");
   if (!only_protocol) {
@@ -258,6 +289,7 @@ int main(int argc, char** argv) {
       rle_case(n, 5.f);
     }
   }
+  notes_case();
   protocol_case();
   if (g_fail) { fprintf(stderr, "%d checks failed (%s)\n", g_fail, g_err); return 1; }
   printf("host selftest passed\n");
