@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 class CxStreamNotes {
  public:
@@ -11,6 +12,11 @@ class CxStreamNotes {
 
   void note(int dev, const void* stream, bool early) {
     if (known(dev, stream)) slot(dev, stream).store(word(stream, early), std::memory_order_relaxed);
+  }
+  // Held from the question or the note to the launch it is about: the notes of a stream are in the order of
+  // its kernels then, also where several threads share the stream.
+  std::mutex& order(int dev, const void* stream) {
+    return known(dev, stream) ? order_[dev][index(stream)] : order_of_others_;
   }
   // true unless the last note of this very stream says "not early"
   bool front_wait(int dev, const void* stream) const {
@@ -30,8 +36,12 @@ class CxStreamNotes {
   static uint64_t word(const void* stream, bool early) { return handle(stream) << 2 | 2u | (early ? 1u : 0u); }
   // hashed: what another stream has overwritten counts as early
   std::atomic<uint64_t>& slot(int dev, const void* stream) const {
+    return last_[dev][index(stream)];
+  }
+  static unsigned index(const void* stream) {
     const uint64_t s = handle(stream);
-    return last_[dev][(s >> 4 ^ s >> 10 ^ s >> 16) % kSlots];
+    return (unsigned)((s >> 4 ^ s >> 10 ^ s >> 16) % kSlots);
   }
   mutable std::atomic<uint64_t> last_[kDevices][kSlots] = {};
+  std::mutex order_[kDevices][kSlots], order_of_others_;
 };

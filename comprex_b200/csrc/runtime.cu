@@ -94,6 +94,25 @@ static int current_device() {
 }
 void cx_note_stream(const void* stream, bool early) { g_notes.note(current_device(), stream, early); }
 bool cx_front_wait(const void* stream) { return g_notes.front_wait(current_device(), stream); }
+namespace {
+// A thread's turn on a stream: launches that take part in the notes are made inside one.  (Ops of a list on
+// a side stream need none of their own, one list at a time uses those.)
+thread_local int g_turns = 0;
+class Turn {
+ public:
+  Turn(int dev, const void* stream) : mine_(dev == CX_DEV_CUDA) {
+    if (mine_ && g_turns++ == 0) held_ = std::unique_lock<std::mutex>(g_notes.order(current_device(), stream));
+  }
+  ~Turn() {
+    if (mine_) --g_turns;
+  }
+  Turn(const Turn&) = delete;
+
+ private:
+  const bool mine_;
+  std::unique_lock<std::mutex> held_;
+};
+}  // namespace
 static thread_local uint32_t g_chain_bits = 0;
 uint32_t cx_chain_bits() { return g_chain_bits; }
 int cx_check_launch(const char* where) {
@@ -126,6 +145,7 @@ int cx_version(void) { return 1; }
 int cx_threshold_select(int dev, int gdtype, const void* g, const float* r, int64_t n, float ratio,
                         int default_subsamples, float subsample_factor, float* thr_out, void* workspace,
                         int64_t ws_bytes, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_threshold_topk_cuda(gdtype, g, r, n, ratio, default_subsamples, subsample_factor, thr_out,
                                       workspace, ws_bytes, stream)
@@ -141,6 +161,7 @@ int cx_threshold_topk(int dev, int gdtype, const void* g, const float* r, int64_
 int cx_compress(int dev, int gdtype, const void* g, float* r, int64_t n, const float* thr,
                 uint32_t cap, uint64_t seq, const CxTargets* tg, void* workspace, int64_t ws_bytes,
                 CxStats* stats, uint32_t src_rank, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_compress_cuda(gdtype, g, r, n, thr, cap, seq, tg, workspace, ws_bytes, stats, src_rank, stream)
              : cx_compress_host(gdtype, g, r, n, thr, cap, seq, tg, stats, src_rank);
@@ -148,6 +169,7 @@ int cx_compress(int dev, int gdtype, const void* g, float* r, int64_t n, const f
 
 int cx_apply(int dev, const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_t* status,
              uint64_t timeout_ns, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA ? cx_apply_cuda(src, n, a, status, timeout_ns, stream)
                             : cx_apply_host(src, n, a, status, timeout_ns);
 }
@@ -172,6 +194,7 @@ int cx_mm_allreduce(int dtype, void* out, const void* in, void* stage, void* sta
 int cx_forward(int dev, const CxEndpoint* from, uint64_t expect_seq, const CxTargets* tg,
                uint64_t seq, uint32_t cap, void* counters, uint32_t* status, uint64_t timeout_ns,
                void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_forward_cuda(from, expect_seq, tg, seq, cap, counters, status, timeout_ns, stream)
              : cx_forward_host(from, expect_seq, tg, seq, cap, status, timeout_ns);
@@ -180,6 +203,7 @@ int cx_forward(int dev, const CxEndpoint* from, uint64_t expect_seq, const CxTar
 int cx_dense_send(int dev, int dtype, const void* g, float* r, int64_t n, uint64_t seq,
                   const CxTargets* tg, const int64_t* starts, const int64_t* lens, void* counters,
                   uint32_t src_rank, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_dense_send_cuda(dtype, g, r, n, seq, tg, starts, lens, counters, src_rank, stream)
              : cx_dense_send_host(dtype, g, r, n, seq, tg, starts, lens, src_rank);
@@ -189,6 +213,7 @@ int cx_dense_reduce(int dev, int dtype, void* out, const void* own, int64_t n, c
                     float scale, const CxTargets* push, uint64_t push_seq, const int64_t* starts,
                     const int64_t* lens, void* counters, uint32_t src_rank, uint32_t* status,
                     uint64_t timeout_ns, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_dense_reduce_cuda(dtype, out, own, n, src, scale, push, push_seq, starts, lens,
                                     counters, src_rank, status, timeout_ns, stream)
@@ -205,6 +230,7 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
             const int64_t* item_rel, const int32_t* item_len, const int32_t* item_seg,
             const int32_t* seg_first, int nitems, float* u, float* partial, float clip, float mu,
             float lr, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_fold_cuda(gdtype, seg_ptr, item_off, item_rel, item_len, item_seg, seg_first, nitems, u,
                             partial, clip, mu, lr, stream)
@@ -212,15 +238,20 @@ int cx_fold(int dev, int gdtype, const void* const* seg_ptr, const int64_t* item
                             partial, clip, mu, lr);
 }
 
-int cx_fold_coef(int gdtype, const CxFoldCoef* f, void* stream) { return cx_fold_coef_cuda(gdtype, f, stream); }
+int cx_fold_coef(int gdtype, const CxFoldCoef* f, void* stream) {
+  Turn turn(CX_DEV_CUDA, stream);
+  return cx_fold_coef_cuda(gdtype, f, stream);
+}
 
 int cx_fold_update(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream) {
+  Turn turn(CX_DEV_CUDA, stream);
   return cx_fold_update_cuda(gdtype, fold, n, a, stream);
 }
 
 int cx_rle_send(int dev, int gdtype, const void* g, float* r, int64_t n, const float* thr,
                 int64_t slot_bytes, uint64_t seq, const CxTargets* tg, void* workspace,
                 int64_t ws_bytes, uint32_t src_rank, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_rle_send_cuda(gdtype, g, r, n, thr, slot_bytes, seq, tg, workspace, ws_bytes, src_rank, stream)
              : cx_rle_send_host(gdtype, g, r, n, thr, slot_bytes, seq, tg, src_rank);
@@ -229,6 +260,7 @@ int cx_rle_send(int dev, int gdtype, const void* g, float* r, int64_t n, const f
 int cx_rle_recv(int dev, const CxEndpoint* src, uint64_t expect_seq, float* out, int64_t n, int add,
                 int64_t slot_bytes, void* workspace, int64_t ws_bytes, uint32_t* status,
                 uint64_t timeout_ns, void* stream) {
+  Turn turn(dev, stream);
   return dev == CX_DEV_CUDA
              ? cx_rle_recv_cuda(src, expect_seq, out, n, add, slot_bytes, workspace, ws_bytes, status,
                                 timeout_ns, stream)
@@ -326,6 +358,9 @@ Lanes* lanes_for_current_device() {
 }  // namespace
 
 int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
+  bool cuda = false;           // (host ops wait for other threads' messages: no turn)
+  for (int i = 0; i < count; ++i) cuda |= ops[i].dev == CX_DEV_CUDA;
+  Turn turn(cuda ? CX_DEV_CUDA : CX_DEV_HOST, stream);
   cudaStream_t main_stream = reinterpret_cast<cudaStream_t>(stream);
   Lanes* lanes = nullptr;
   std::unique_lock<std::mutex> lanes_held;   // taken with the first side-stream op, released on return

@@ -263,6 +263,33 @@ static void notes_case() {
   }
 }
 
+// Two threads share a stream: whoever is told not to wait has a kernel in front that is not early.
+static void notes_threads_case() {
+  static CxStreamNotes notes;
+  const void* stream = (const void*)0x5000;
+  bool front_early = false;                            // the kernel launched last; the stream's, not the notes'
+  int wrong[2] = {0, 0}, free_to_go = 0;
+  auto launches = [&](int me) {
+    for (int k = 0; k < 20000; ++k) {
+      std::lock_guard<std::mutex> turn(notes.order(0, stream));
+      if (k % 3 == me) {                               // a sender
+        front_early = false;
+        notes.note(0, stream, false);
+      } else {                                         // a receive kernel
+        const bool wait = notes.front_wait(0, stream);
+        notes.note(0, stream, true);
+        if (!wait && front_early) ++wrong[me];
+        if (!wait) ++free_to_go;
+        front_early = true;
+      }
+    }
+  };
+  std::thread a(launches, 0), b(launches, 1);
+  a.join();
+  b.join();
+  CHECK(wrong[0] == 0 && wrong[1] == 0 && free_to_go > 0);
+}
+
 int main(int argc, char** argv) {
   const bool only_protocol = argc > 1 && !strcmp(argv[1], "--protocol");
   if (!only_protocol) {
@@ -290,6 +317,7 @@ int main(int argc, char** argv) {
     }
   }
   notes_case();
+  notes_threads_case();
   protocol_case();
   if (g_fail) { fprintf(stderr, "%d checks failed (%s)\n", g_fail, g_err); return 1; }
   printf("host selftest passed\n");

@@ -5,6 +5,7 @@ flushRests, receiver accumulates with readRemote_add, result == 3 * values),
 examples/comprEx.cpp, examples/gaspiEx.py.
 """
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -336,3 +337,52 @@ def test_receive_behind_a_threshold_of_the_same_vector(how, kind):
         for e in world.envs:
             e.check()
     world.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["pairs", "dense"])
+def test_two_threads_on_one_stream(kind):
+    """Two threads, each with engines of its own, on the default stream: a receive kernel lets the next one in
+    early, so the next receive into the same vector has to know that it is in front, whatever the other
+    thread launches in between.  Whole numbers: all sums are exact."""
+    n, rounds = (1 << 20) + 7, 60
+    worlds = [cx.LoopbackWorld(2, device="cuda", timeout_ms=2000) for _ in range(2)]
+    pairs = []
+    for w in worlds:
+        ex = [cx.GaspiEx(e, n) if kind == "dense" else cx.Comprex(e, n) for e in w.envs]
+        for r, e in enumerate(ex):
+            if kind != "dense":
+                e.setThreshold(cx.ThresholdTopK(0.1))
+                e.setCompressor(cx.CompressorIndexPairs())
+            e.connectTo(1 - r, 1 - r)
+        pairs.append(ex)
+    out, err = [None, None], []
+
+    def work(t):
+        try:
+            tx, rx = pairs[t]
+            gen = torch.Generator(device="cuda").manual_seed(t)
+            acc, total = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+            for _ in range(rounds):
+                for _ in range(2):
+                    v = torch.randint(-9, 10, (n,), device="cuda", generator=gen).float()
+                    total += v
+                    tx.writeRemote(v)
+                rx.readRemote_add(acc)
+                rx.readRemote_add(acc)
+            out[t] = (acc if kind == "dense" else acc + tx.getRests(), total)
+        except BaseException as e:       # noqa: BLE001 - reported by the main thread
+            err.append(e)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not err, err
+    for got, want in out:
+        assert torch.equal(got, want)
+    for w in worlds:
+        for e in w.envs:
+            e.check()
+        w.close()
