@@ -339,8 +339,6 @@ class ComprexOptimizer(torch.optim.Optimizer):
         self._armed = False
         self._all = None
         self._cuda = dev.type == "cuda"
-        # the folded vector is the momentum, and outlives the step, only in the reference's own rule
-        self._keeps_u = rule == "sgd" and self.local_momentum
         self._hooks = []
         if self.overlap:
             for p in self._params:
@@ -429,6 +427,11 @@ class ComprexOptimizer(torch.optim.Optimizer):
         b.fold.refresh(self._zeros)
         return b.fold
 
+    @property
+    def _keeps_u(self) -> bool:
+        """The folded vector is the momentum, and outlives the step, only in the reference's own rule."""
+        return self.rule == "sgd" and self.local_momentum
+
     def _fold_scalars(self, lr: float, mu: float):
         """(clip, momentum, learning rate) of the fold: the optimizers that keep their momentum in the
         receive kernel exchange the clipped gradient itself."""
@@ -458,9 +461,10 @@ class ComprexOptimizer(torch.optim.Optimizer):
 
     def _fold_args(self, ft: _FoldTable, b: _Bucket, mu: float):
         """The bucket's CxFold, kept with the table (the native side reads it at every launch)."""
-        f = ft.args.get(b)
+        keeps = self._keeps_u
+        f = ft.args.get((b, keeps))
         if f is None:
-            f = ft.args[b] = ft.fold_args(b, self._update[b.start:b.end] if self._keeps_u else None, mu)
+            f = ft.args[(b, keeps)] = ft.fold_args(b, self._update[b.start:b.end] if keeps else None, mu)
         elif f.mu != mu:
             f.mu = mu
         return f
@@ -473,7 +477,7 @@ class ComprexOptimizer(torch.optim.Optimizer):
         if self._all is None:
             self._all = (_FoldTable(self._env, self._buckets, self._dtype), {})
         ft, plans = self._all
-        cfg = None if par is None else [(b.ar.compression_ratio, b.ar.sampling) for b in self._buckets]
+        cfg = (self._keeps_u, None if par is None else [(b.ar.compression_ratio, b.ar.sampling) for b in self._buckets])
         plan = plans.get(par)
         if plan is None or plan.cfg != cfg:
             plan = plans[par] = _StepPlan(self, ft, par, cfg)
@@ -482,7 +486,8 @@ class ComprexOptimizer(torch.optim.Optimizer):
     def _run_plan(self, par, seq: int, lr, mu, wd) -> None:
         plan = self._plan(par)
         plan.table.refresh(self._zeros)
-        hyper = (lr, mu, wd, self.momentum_correction, self.pre_clipnorm)
+        # everything the descriptors hold that a program may change between steps
+        hyper = (lr, mu, wd, self.momentum_correction, self.pre_clipnorm, *self.betas, self.eps)
         if plan.hyper != hyper:
             plan.set_hyper(self, lr, mu, wd)
             plan.hyper = hyper

@@ -751,3 +751,44 @@ def test_step_whose_sample_is_the_whole_bucket(sizes, ratio):
         env.close()
     for a, b in zip(*arms):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["adamw", "receive_momentum"])
+@pytest.mark.parametrize("exchange", [True, False])
+def test_settings_changed_between_steps(kind, exchange):
+    """Everything a program may change between steps reaches the next one: the launch list of the whole step
+    against the kernels issued bucket by bucket."""
+    sizes, arms = [70001, 200, 4096], []
+    for fused in (True, False):
+        torch.manual_seed(5)
+        env = cx.GaspiEnvironment(8 << 20, device="cuda")
+        params = [torch.nn.Parameter(torch.randn(s, device="cuda")) for s in sizes]
+        opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.9, compression_ratio=0.05, pre_clipnorm=20.0,
+                               rule="adamw" if kind == "adamw" else "sgd", local_momentum=False, weight_decay=0.01,
+                               bucket_cap_mb=0.2, single_rank_bypass=not exchange)
+        assert len(opt._buckets) > 1
+        if not fused:
+            opt._fusable = lambda b: False
+            opt._cuda = False
+        changes = [{}, {}, dict(betas=(0.5, 0.6)), dict(eps=1e-2), {}, dict(betas=[0.8, 0.9], eps=1e-4),
+                   dict(pre_clipnorm=None), dict(momentum_correction=0.5), dict(local_momentum=True), {}, {}]
+        for step, change in enumerate(changes):
+            for k, v in change.items():
+                if k != "local_momentum" or kind == "receive_momentum":
+                    setattr(opt, k, v)
+                    if k == "local_momentum":
+                        opt._update.zero_()          # the momentum starts here
+            if step == 4:
+                opt.set_compression_ratio(0.02)
+                opt.param_groups[0]["lr"] = 0.02
+            gen = torch.Generator(device="cuda").manual_seed(step)
+            for p in params:
+                p.grad = torch.randn(p.numel(), device="cuda", generator=gen)
+            opt.step()
+        env.flush()
+        arms.append([opt._master.clone(), opt._m.clone(), (opt._v if kind == "adamw" else opt._update).clone()]
+                    + [ar.rests.clone() for ar in opt.comprex_allreducers.values()])
+        env.close()
+    for a, b in zip(*arms):
+        assert torch.equal(a, b)
