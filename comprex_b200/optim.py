@@ -483,7 +483,9 @@ class ComprexOptimizer(torch.optim.Optimizer):
             plan = plans[par] = _StepPlan(self, ft, par, cfg)
         return plan
 
-    def _run_plan(self, par, seq: int, lr, mu, wd) -> None:
+    def _prepare_plan(self, par, lr, mu, wd):
+        """The launch list with this step's gradients and settings; launches nothing, so a step that
+        raises here has not begun."""
         plan = self._plan(par)
         plan.table.refresh(self._zeros)
         # everything the descriptors hold that a program may change between steps
@@ -495,6 +497,9 @@ class ComprexOptimizer(torch.optim.Optimizer):
             bc1, bc2 = 1.0 - self.betas[0] ** self._t, 1.0 - self.betas[1] ** self._t
             for v in plan.views:
                 v.bc1, v.bc2 = bc1, bc2
+        return plan
+
+    def _launch_plan(self, plan, seq: int) -> None:
         _lib.check(self._env.lib.cx_run_ops(plan.ops, plan.count, seq, _lib.stream_ptr(self._env.device)), "cx_run_ops")
 
     def _hyper(self):
@@ -659,7 +664,7 @@ class ComprexOptimizer(torch.optim.Optimizer):
         with ctx:
             if self._local and self._cuda:
                 with nvtx_range("comprex.update"):
-                    self._run_plan(None, 0, lr, mu, wd)
+                    self._launch_plan(self._prepare_plan(None, lr, mu, wd), 0)
             else:
                 self._exchange(lr, mu, wd)
         if use_side:
@@ -671,11 +676,12 @@ class ComprexOptimizer(torch.optim.Optimizer):
     def _exchange(self, lr, mu, wd) -> None:
         pending = [b for b in self._buckets if not b.sent]     # everything that the hooks did not send yet
         if len(pending) == len(self._buckets) and self._in_step():
-            for b in self._buckets:
-                b.seq, b.par = b.ar.next_step()
-                b.ready = 0
             with nvtx_range("comprex.exchange"):
-                self._run_plan(self._buckets[0].par, self._buckets[0].seq, lr, mu, wd)
+                plan = self._prepare_plan((self._buckets[0].ar.step + 1) & 1, lr, mu, wd)
+                for b in self._buckets:
+                    b.seq, b.par = b.ar.next_step()
+                    b.ready = 0
+                self._launch_plan(plan, self._buckets[0].seq)
             return
         for b in pending:
             self._send(b)

@@ -792,3 +792,28 @@ def test_settings_changed_between_steps(kind, exchange):
         env.close()
     for a, b in zip(*arms):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_step_that_raises_has_not_begun():
+    """A gradient that cannot be taken (a sparse one) raises before the exchange moves on: the peers have seen
+    nothing of that step, so the next one must carry its number."""
+    env = cx.GaspiEnvironment(8 << 20, device="cuda")
+    params = [torch.nn.Parameter(torch.zeros(s, device="cuda")) for s in (3000, 500)]
+    opt = ComprexOptimizer(params, env, lr=1.0, momentum=0.0, compression_ratio=1.0, pre_clipnorm=None,
+                           aggregate_blob=False, single_rank_bypass=False)
+    for p in params:
+        p.grad = torch.ones_like(p)
+    opt.step()
+    ars = list(opt.comprex_allreducers.values())
+    before = [ar.step for ar in ars]
+    params[0].grad = torch.sparse_coo_tensor([[1]], [1.0], (3000,), device="cuda")
+    with pytest.raises(RuntimeError):
+        opt.step()
+    assert [ar.step for ar in ars] == before
+    params[0].grad = torch.ones_like(params[0])
+    opt.step()
+    assert [ar.step for ar in ars] == [s + 1 for s in before]
+    env.flush()
+    env.check()
+    env.close()
