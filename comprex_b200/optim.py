@@ -150,12 +150,15 @@ class _FoldTable:
         unchanged table is not uploaded again (otherwise: async on the current stream)."""
         changed = self._collect(self.params, self.scalar_type, zeros.data_ptr(), self.now.data_ptr())
         if changed == 2:                          # rare: bring the odd ones into the parameters' form first
+            self.now.fill_(-1)                    # incomplete, and not what the device holds, should this raise
             for p in self.params:
                 g = p.grad
                 if g is not None and (g.dtype is not self.dtype or g.stride() != p.stride()):
                     p.grad = torch.empty_strided(p.size(), p.stride(), dtype=self.dtype, device=p.device).copy_(g)
-            self.now.fill_(-1)
             changed = self._collect(self.params, self.scalar_type, zeros.data_ptr(), self.now.data_ptr())
+            if changed == 2:
+                self.now.fill_(-1)
+                raise ComprexError("a gradient does not have its parameter's shape")
         if not changed:
             return
         if not self.cuda:

@@ -817,3 +817,42 @@ def test_step_that_raises_has_not_begun():
     env.flush()
     env.check()
     env.close()
+
+
+def test_gradients_after_a_step_that_raised(device):
+    """The table of gradient addresses after a step that raised half-way through it: the next step reads the
+    gradients that are installed then, not those of the step before."""
+    env = cx.GaspiEnvironment(1 << 20, device=device)
+    params = [torch.nn.Parameter(torch.zeros(100, device=device)) for _ in range(2)]
+    opt = ComprexOptimizer(params, env, lr=1.0, momentum=0.0, pre_clipnorm=None)
+    old = [torch.ones(100, device=device) for _ in params]
+    for p, g in zip(params, old):
+        p.grad = g
+    opt.step()
+    params[1].grad = torch.full((100,), 2.0, device=device)       # (the table starts with the last parameter)
+    params[0].grad = torch.sparse_coo_tensor([[1]], [1.0], (100,), device=device)
+    with pytest.raises(RuntimeError):
+        opt.step()
+    params[0].grad = old[0]
+    opt.step()
+    env.flush()
+    assert torch.equal(params[0].detach().cpu(), torch.full((100,), -2.0))
+    assert torch.equal(params[1].detach().cpu(), torch.full((100,), -3.0))
+    env.close()
+
+
+def test_gradient_of_another_size_raises(device):
+    env = cx.GaspiEnvironment(1 << 20, device=device)
+    params = [torch.nn.Parameter(torch.zeros(100, device=device)) for _ in range(2)]
+    opt = ComprexOptimizer(params, env, lr=1.0, momentum=0.0, pre_clipnorm=None)
+    for p in params:
+        p.grad = torch.ones(100, device=device)
+    params[0].grad.resize_(60)
+    with pytest.raises(cx.ComprexError, match="shape"):
+        opt.step()
+    params[0].grad = torch.ones(100, device=device)
+    opt.step()
+    env.flush()
+    for p in params:
+        assert torch.equal(p.detach().cpu(), torch.full((100,), -1.0))
+    env.close()
