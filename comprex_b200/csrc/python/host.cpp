@@ -5,6 +5,9 @@
 //  * run_vector: the launches of one message of a prepared connection.  Checks of the vector,
 //    descriptors and native calls took 20 us per exchange in Python, the kernels of a 64 k-element
 //    exchange take 15 us.
+// Tensors of unusual kinds (nested, sparse, wrapped by a transform) throw at the questions asked here.  No
+// exception may leave these functions: such a tensor is not the plain case, and the caller's general path
+// says what is wrong with it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -40,13 +43,17 @@ PyObject* collect(PyObject*, PyObject* args) {
       PyErr_SetString(PyExc_TypeError, "collect: not a tensor");
       return nullptr;
     }
-    const at::Tensor& p = THPVariable_Unpack(o);
-    const at::Tensor& g = p.grad();
     int64_t a = static_cast<int64_t>(zeros);
-    if (g.defined()) {
-      if (static_cast<int>(g.scalar_type()) != scalar_type || g.layout() != at::kStrided || !same_layout(g, p))
-        return PyLong_FromLong(2);
-      a = reinterpret_cast<int64_t>(g.data_ptr());
+    try {
+      const at::Tensor& p = THPVariable_Unpack(o);
+      const at::Tensor& g = p.grad();
+      if (g.defined()) {
+        if (static_cast<int>(g.scalar_type()) != scalar_type || g.layout() != at::kStrided || !same_layout(g, p))
+          return PyLong_FromLong(2);
+        a = reinterpret_cast<int64_t>(g.data_ptr());
+      }
+    } catch (const std::exception&) {
+      return PyLong_FromLong(2);
     }
     changed |= table[i] != a;
     table[i] = a;
@@ -86,12 +93,19 @@ PyObject* run_vector(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int64_t n = PyLong_AsLongLong(a[8]);
   if (PyErr_Occurred()) return nullptr;
   if (!THPVariable_CheckExact(a[6])) Py_RETURN_NONE;
-  const at::Tensor& t = THPVariable_Unpack(a[6]);
-  if (!t.is_cuda() || t.device().index() != device || !t.is_contiguous()) Py_RETURN_NONE;
-  const int code = element_code(t);
-  if (code < 0) Py_RETURN_NONE;
-  const int64_t len = t.numel();
-  void* ptr = t.data_ptr();
+  int code;
+  int64_t len;
+  void* ptr;
+  try {
+    const at::Tensor& t = THPVariable_Unpack(a[6]);
+    if (!t.is_cuda() || t.device().index() != device || t.layout() != at::kStrided || !t.is_contiguous()) Py_RETURN_NONE;
+    code = element_code(t);
+    if (code < 0) Py_RETURN_NONE;
+    len = t.numel();
+    ptr = t.data_ptr();
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;
+  }
   if (role == kSend) {
     if (len != n) Py_RETURN_NONE;
     for (long i = 0; i < count; ++i) {
@@ -131,12 +145,16 @@ PyObject* install(PyObject*, PyObject* pairs) {
       PyObject* v = PySequence_Fast_GET_ITEM(two, 1);
       bool done = false;
       if (THPVariable_Check(g) && THPVariable_Check(v) && g != v) {
-        const at::Tensor& gt = THPVariable_Unpack(g);
-        const at::Tensor& vt = THPVariable_Unpack(v);
-        if (gt.defined() && vt.defined() && vt.is_leaf() && gt.layout() == at::kStrided && vt.layout() == at::kStrided &&
-            gt.scalar_type() == vt.scalar_type() && gt.device() == vt.device() && gt.sizes() == vt.sizes()) {
-          vt.mutable_grad() = gt;
-          done = true;
+        try {
+          const at::Tensor& gt = THPVariable_Unpack(g);
+          const at::Tensor& vt = THPVariable_Unpack(v);
+          if (gt.defined() && vt.defined() && vt.is_leaf() && gt.layout() == at::kStrided && vt.layout() == at::kStrided &&
+              gt.scalar_type() == vt.scalar_type() && gt.device() == vt.device() && gt.sizes() == vt.sizes()) {
+            vt.mutable_grad() = gt;
+            done = true;
+          }
+        } catch (const std::exception&) {
+          done = false;
         }
       }
       ok = done || PyObject_SetAttrString(v, "grad", g) == 0;
@@ -155,7 +173,7 @@ PyObject* scalar_type(PyObject*, PyObject* o) {
     PyErr_SetString(PyExc_TypeError, "scalar_type: not a tensor");
     return nullptr;
   }
-  return PyLong_FromLong(static_cast<long>(THPVariable_Unpack(o).scalar_type()));
+  return PyLong_FromLong(static_cast<long>(THPVariable_Unpack(o).scalar_type()));      // (does not throw)
 }
 
 PyMethodDef methods[] = {{"collect", collect, METH_VARARGS, nullptr},

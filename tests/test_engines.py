@@ -386,3 +386,28 @@ def test_two_threads_on_one_stream(kind):
         for e in w.envs:
             e.check()
         w.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cls", ["Comprex", "GaspiEx"])
+def test_unusual_vectors_raise(cls):
+    """Vectors that have no address (sparse, wrapped by a transform) raise and leave the connection usable."""
+    env = cx.GaspiEnvironment(1 << 20, device="cuda")
+    n = 100
+    ex = getattr(cx, cls)(env, n)
+    if cls == "Comprex":
+        ex.setThreshold(cx.ThresholdTopK(1.0))
+        ex.setCompressor(cx.CompressorIndexPairs())
+    ex.connectTo(0, 0)
+    sparse = torch.sparse_coo_tensor([[1]], [1.0], (n,), device="cuda", check_invariants=True)
+    for call in (ex.writeRemote, ex.readRemote_add):
+        with pytest.raises(Exception):
+            call(sparse)
+        with pytest.raises(Exception):
+            torch.func.vmap(lambda x: call(x) or x)(torch.zeros(3, n, device="cuda"))
+    v, out = torch.randn(n, device="cuda"), torch.zeros(n, device="cuda")
+    ex.writeRemote(v)
+    ex.readRemote_add(out)
+    assert torch.equal(out + (ex.getRests() if cls == "Comprex" else 0), v)
+    env.check()
+    env.close()

@@ -3,6 +3,9 @@ keras/comprex_optimizer.py:97-133,150-163, conservation through flush,
 bucketed layout, checkpoint/resume, replica consistency across real ranks.
 """
 import copy
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -856,3 +859,41 @@ def test_gradient_of_another_size_raises(device):
     for p in params:
         assert torch.equal(p.detach().cpu(), torch.full((100,), -1.0))
     env.close()
+
+
+def test_unusual_tensors_raise_instead_of_ending_the_process():
+    """Nested tensors throw at every question about their sizes: installing them as gradients does what the
+    attribute does.  In a process of its own, an exception that left the native code would end it."""
+    code = """
+import torch
+from comprex_b200 import _lib
+nt = lambda: torch.nested.nested_tensor([torch.ones(2), torch.ones(3)])
+def kind(f):
+    try:
+        f()
+    except Exception as e:
+        return type(e).__name__
+    return "ok"
+v, w = nt(), nt()
+def attribute():
+    v.grad = nt()
+assert kind(attribute) == kind(lambda: _lib.host().install([(nt(), w)]))
+p = torch.nn.Parameter(torch.zeros(5))
+table = torch.zeros(1, dtype=torch.int64)
+code = _lib.host().scalar_type(p)
+def under_vmap(x):
+    p.grad = None
+    try:
+        p.grad = x
+    except Exception:
+        return x
+    assert _lib.host().collect([p], code, 0, table.data_ptr()) == 2
+    return x
+torch.func.vmap(under_vmap)(torch.zeros(3, 5))
+_lib.host().install([(torch.ones(5), p)])
+assert p.grad.sum() == 5
+print("done")
+"""
+    res = subprocess.run([sys.executable, "-W", "ignore", "-c", code], capture_output=True, text=True, timeout=300,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert res.returncode == 0 and "done" in res.stdout, res.stdout + res.stderr
