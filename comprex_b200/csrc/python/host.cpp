@@ -149,7 +149,7 @@ PyObject* install(PyObject*, PyObject* pairs) {
           const at::Tensor& gt = THPVariable_Unpack(g);
           const at::Tensor& vt = THPVariable_Unpack(v);
           if (gt.defined() && vt.defined() && vt.is_leaf() && gt.layout() == at::kStrided && vt.layout() == at::kStrided &&
-              gt.scalar_type() == vt.scalar_type() && gt.device() == vt.device() && gt.sizes() == vt.sizes()) {
+              gt.scalar_type() == vt.scalar_type() && vt.grad_dtype() == vt.scalar_type() && gt.device() == vt.device() && gt.sizes() == vt.sizes()) {
             vt.mutable_grad() = gt;
             done = true;
           }

@@ -897,3 +897,19 @@ print("done")
     res = subprocess.run([sys.executable, "-W", "ignore", "-c", code], capture_output=True, text=True, timeout=300,
                          cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert res.returncode == 0 and "done" in res.stdout, res.stdout + res.stderr
+
+
+def test_apply_gradients_honours_grad_dtype():
+    """What the attribute refuses stays refused: a gradient of another type than the parameter's grad_dtype."""
+    p = torch.nn.Parameter(torch.zeros(100, dtype=torch.bfloat16))
+    env = cx.GaspiEnvironment(1 << 20, device="cpu")
+    opt = ComprexOptimizer([p], env, lr=1.0, momentum=0.0, pre_clipnorm=None)
+    if not hasattr(p, "grad_dtype"):
+        pytest.skip("this torch has no grad_dtype")
+    p.grad_dtype = torch.float32
+    with pytest.raises(RuntimeError, match="grad_dtype"):
+        opt.apply_gradients([(torch.ones(100, dtype=torch.bfloat16), p)])
+    p.grad_dtype = None
+    opt.apply_gradients([(torch.ones(100, dtype=torch.bfloat16), p)])
+    assert torch.equal(p.detach().float(), torch.full((100,), -1.0))
+    env.close()
