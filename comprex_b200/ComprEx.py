@@ -423,14 +423,14 @@ class Comprex(AbstractExchange):
             return False
         src = self._src
         seq = self._rx_seq.get(src, 0) + 1
-        got = self._rx_ops.get((seq & 1, op))
+        got = self._rx_ops.get((seq & 1, op, self._env.timeout_ns))
         if got is None:
             o = _lib.Op()
             o.kind, o.dev, o.n = _lib.OPK_APPLY, self._env.dev, self.size
             o.src = P.make_sources([self._slots[seq & 1].endpoint(self._env)], [seq])
             o.apply.op, o.apply.scale = op, 1.0
             o.status, o.timeout_ns = self._status.dev_ptr, self._env.timeout_ns
-            got = self._rx_ops[(seq & 1, op)] = _lib.VectorOps(_lib.VectorOps.APPLY, [o], self._env.device, self.size)
+            got = self._rx_ops[(seq & 1, op, o.timeout_ns)] = _lib.VectorOps(_lib.VectorOps.APPLY, [o], self._env.device, self.size)
         if not got.run(vector, seq):
             return False
         self._rx_seq[src] = seq

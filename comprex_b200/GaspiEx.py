@@ -127,7 +127,7 @@ class GaspiEx(AbstractExchange):
         if peer is None:
             return False
         seq = seqs.get(peer, 0) + 1
-        key = (role, peer, seq & 1)
+        key = (role, peer, seq & 1, self._env.timeout_ns)
         got = self._ops.get(key)
         if got is None:
             env, o = self._env, _lib.Op()

@@ -6,6 +6,7 @@ examples/comprEx.cpp, examples/gaspiEx.py.
 """
 import math
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -410,4 +411,31 @@ def test_unusual_vectors_raise(cls):
     ex.readRemote_add(out)
     assert torch.equal(out + (ex.getRests() if cls == "Comprex" else 0), v)
     env.check()
+    env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cls", ["Comprex", "GaspiEx"])
+def test_time_budget_changed_between_reads(cls):
+    """A read waits as long as the environment says when it is issued, also behind earlier reads."""
+    env = cx.GaspiEnvironment(1 << 20, device="cuda", timeout_ms=8000)
+    n = 100
+    ex = getattr(cx, cls)(env, n)
+    if cls == "Comprex":
+        ex.setThreshold(cx.ThresholdTopK(1.0))
+        ex.setCompressor(cx.CompressorIndexPairs())
+    ex.connectTo(0, 0)
+    out = torch.zeros(n, device="cuda")
+    for _ in range(4):
+        ex.writeRemote(torch.ones(n, device="cuda"))
+        ex.readRemote_add(out)
+    env.flush()
+    env.check()
+    env.timeout_ns = 50_000_000
+    start = time.perf_counter()
+    ex.readRemote_add(out)                   # nothing was sent
+    torch.cuda.synchronize()
+    assert time.perf_counter() - start < 4.0
+    with pytest.raises(cx.ComprexError, match="TIMEOUT"):
+        env.check()
     env.close()
