@@ -910,7 +910,8 @@ int cx_update_dense_cuda(const float* g, int64_t n, const CxApplyArgs* a, void* 
 // The low-precision copy of the weights has the element type of the gradients (both are the model's).
 int cx_fold_update_cuda(int gdtype, const CxFold* fold, int64_t n, const CxApplyArgs* a, void* stream) {
   if (!a->out) return cx_set_error("cx_fold_update: NULL vector", 0);
-  if (n < 0 || n > 0x7fffffffLL) return cx_set_error("cx_fold_update: n out of range", 0);
+  // all buckets of a model at once: only their sub-tiles are counted in 32 bits
+  if (n < 0 || n > (1LL << 40)) return cx_set_error("cx_fold_update: n out of range", 0);
   if (a->op != CX_OP_SGD && a->op != CX_OP_MOMENTUM && a->op != CX_OP_ADAMW)
     return cx_set_error("cx_fold_update: op must be an update rule", 0);
   if (a->op != CX_OP_SGD && !a->m) return cx_set_error("cx_fold_update: momentum buffer missing", 0);

@@ -913,3 +913,28 @@ def test_apply_gradients_honours_grad_dtype():
     opt.apply_gradients([(torch.ones(100, dtype=torch.bfloat16), p)])
     assert torch.equal(p.detach().float(), torch.full((100,), -1.0))
     env.close()
+
+
+@pytest.mark.gpu
+def test_local_step_of_more_than_2_31_parameters():
+    """One rank, nothing to exchange: all buckets are updated in one pass, which may be longer than any one
+    bucket can be."""
+    n = (1 << 30) + 8
+    env = cx.GaspiEnvironment(1 << 20, device="cuda")
+    params = [torch.nn.Parameter(torch.zeros(n, device="cuda", dtype=torch.bfloat16)) for _ in range(2)]
+    opt = ComprexOptimizer(params, env, lr=0.5, momentum=0.9, pre_clipnorm=None, bucket_cap_mb=1024)
+    assert opt.blob_size > 2 ** 31 and len(opt._buckets) == 2
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    grads = [torch.empty(n, device="cuda", dtype=torch.bfloat16).normal_(generator=gen) for _ in params]
+    opt.apply_gradients(list(zip(grads, params)))
+    env.flush()
+    for p, g in zip(params, grads):
+        assert torch.equal(p.detach(), -0.5 * g)       # half of a bf16 number is one
+    opt.apply_gradients(list(zip(grads, params)))      # momentum 1.9, in all 2.9 times the first update
+    env.flush()
+    for p, g in zip(params, grads):
+        for k in range(0, n, 1 << 28):
+            want = -1.45 * g[k:k + (1 << 28)].float()
+            # fp32 sums rounded to bf16 once
+            assert ((p.detach()[k:k + (1 << 28)].float() - want).abs() <= want.abs() * 2.0 ** -8 * 1.001).all()
+    env.close()
