@@ -2,8 +2,8 @@
 examples/tictocTimer.hxx, and nothing inside the library).
 
 * ``nvtx_range(name)``: an NVTX range when ``COMPREX_NVTX=1`` (or ``enable_nvtx()``) and a
-  CUDA device is present, otherwise a no-op; the optimizer wraps fold / send / receive of
-  every bucket in one.
+  CUDA device is present, otherwise a no-op; the optimizer wraps the launches of a whole step in
+  one, or, where it goes bucket by bucket, fold / send and receive of every bucket.
 * ``PhaseTimer``: device time of named phases with CUDA events on the current stream
   (host monotonic clock on the CPU), read after a synchronise; ``summary()`` gives count,
   total and mean per phase.
@@ -29,20 +29,25 @@ def nvtx_enabled() -> bool:
     return _nvtx_on and torch.cuda.is_available()
 
 
-_no_range = contextlib.nullcontext()
+class nvtx_range(contextlib.ContextDecorator):
+    """``with nvtx_range("name"):`` or ``@nvtx_range("name")``; a decorated function asks at every call
+    whether ranges are on."""
 
+    def __init__(self, name: str):
+        self._name, self._pushed = name, False
 
-def nvtx_range(name: str):
-    return _nvtx_range(name) if _nvtx_on and nvtx_enabled() else _no_range
+    def _recreate_cm(self):
+        return type(self)(self._name)          # one per call of a decorated function: it may call itself
 
+    def __enter__(self):
+        if _nvtx_on and nvtx_enabled():
+            torch.cuda.nvtx.range_push(self._name)
+            self._pushed = True
 
-@contextlib.contextmanager
-def _nvtx_range(name: str):
-    torch.cuda.nvtx.range_push(name)
-    try:
-        yield
-    finally:
-        torch.cuda.nvtx.range_pop()
+    def __exit__(self, *exc):
+        if self._pushed:
+            self._pushed = False
+            torch.cuda.nvtx.range_pop()
 
 
 class PhaseTimer:

@@ -99,3 +99,29 @@ def test_prefetcher_and_async_scalar(device):
     assert len(single) == 2 and float(single[0].sum()) == 2.0
     if pin:
         assert feed.h2d_bytes == 5 * (12 * 4 + 8)
+
+
+def test_nvtx_range_as_context_and_decorator(monkeypatch):
+    """A range is asked for when it is entered, also by a function that was decorated before ranges were on;
+    what is pushed is popped, whatever happens inside."""
+    from comprex_b200.utils import trace
+    log = []
+    monkeypatch.setattr(trace.torch.cuda.nvtx, "range_push", lambda name: log.append(name))
+    monkeypatch.setattr(trace.torch.cuda.nvtx, "range_pop", lambda: log.append("pop"))
+    monkeypatch.setattr(trace.torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(trace, "_nvtx_on", False)
+
+    @nvtx_range("f")
+    def f(k):
+        if k < 0:
+            raise ValueError
+        return f(k - 1) + 1 if k else 0
+
+    assert f(2) == 2 and log == []
+    trace.enable_nvtx()
+    assert f(1) == 1 and log == ["f", "f", "pop", "pop"]
+    with pytest.raises(ValueError):
+        f(-1)
+    with nvtx_range("g"):
+        trace.enable_nvtx(False)
+    assert log == ["f", "f", "pop", "pop", "f", "pop", "g", "pop"]
