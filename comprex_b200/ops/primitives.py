@@ -192,8 +192,9 @@ class Compressor:
         """(address, bytes) of the threshold kernels' scratch.  A selection over the whole vector gets
         the larger one that saves it three passes, allocated on first use and kept."""
         if default_subsamples > n and self.env.dev == _lib.DEV_CUDA:
-            need = int(self.env.lib.cx_threshold_exact_bytes(n))
+            need = int(self.env.lib.cx_threshold_exact_bytes(max(n, self.n)))
             if self.thr_ws_bytes < need:
+                self._thr_ws_small = self.thr_ws          # prepared launch lists go on using it
                 self.thr_ws, self.thr_ws_bytes = self.env.scratch(need), need
         return self.thr_ws.data_ptr(), self.thr_ws_bytes
 

@@ -439,3 +439,31 @@ def test_time_budget_changed_between_reads(cls):
     with pytest.raises(cx.ComprexError, match="TIMEOUT"):
         env.check()
     env.close()
+
+
+@pytest.mark.gpu
+def test_prepared_sends_survive_a_change_to_exact_and_back():
+    """A fraction so small that every element is sampled uses the small scratch; one message with exact top-k in
+    between brings a larger one.  The launch list that was prepared before must not use memory that has
+    become somebody else's."""
+    env = cx.GaspiEnvironment(1 << 20, device="cuda")
+    n = 30000
+    ex = cx.Comprex(env, n)
+    ex.setCompressor(cx.CompressorIndexPairs())
+    ex.connectTo(0, 0)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    out, total, others = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda"), []
+    for k, exact in enumerate((False, False, True, False, False, False)):
+        ex.setThreshold(cx.ThresholdTopK(1e-4, exact=exact))
+        v = torch.randint(-1000, 1000, (n,), device="cuda", generator=gen).float()
+        held = ex.getRests() + v
+        want = held.abs().sort(descending=True).values[2]      # ceil(n * 1e-4) - 1
+        total += v
+        ex.writeRemote(v)
+        ex.readRemote_add(out)
+        assert ex.threshold.getThreshold() == float(want)
+        assert torch.equal(out + ex.getRests(), total)
+        others += [torch.full((1024,), 7, dtype=torch.int32, device="cuda") for _ in range(32)]
+        assert all(bool((t == 7).all()) for t in others), k
+    env.check()
+    env.close()
