@@ -6,7 +6,7 @@ Needs the library built with the stamps compiled in (they are off by default):
     python bench/compress_phases.py [--log2-sizes 20 22 24 26] [--ratio 0.01] [--no-flush]
 
 Thread 0 of every CTA stamps: entry, start of the sub-tile loop, end of the loop, arrival at the
-completion counter, and (in the CTA that arrives last) regions summed, headers published, end.
+completion counter, and (in the CTA that arrives last) the totals known, headers published, end.
 Printed per size: the CUDA-event time of the launch and the stamps in nanoseconds since the first
 CTA's entry (median over the timed launches; L2 flushed before every launch unless --no-flush).
 """
@@ -49,7 +49,8 @@ def main():
         r = torch.randn(n, device=dev) * 0.5
         flush = torch.zeros(256 << 20, dtype=torch.uint8, device=dev)
         res = []
-        nb = min(2 * torch.cuda.get_device_properties(dev).multi_processor_count, (n // 1024 + 7) // 8)
+        # the stamps' rows are zero where no CTA ran: the grid follows from them
+        rows = 2048
         for it in range(args.iters):
             comp.threshold_topk(g, r, n, args.ratio)
             torch.cuda.synchronize()
@@ -60,19 +61,22 @@ def main():
             comp.compress(g, r, n, cap, it + 1, tg)
             b.record()
             torch.cuda.synchronize()
-            buf = (C.c_ulonglong * (8 * nb))()
-            if lib.cx_compress_trace(buf, 8 * nb) != 0:
+            buf = (C.c_ulonglong * (8 * rows))()
+            if lib.cx_compress_trace(buf, 8 * rows) != 0:
                 raise SystemExit("reading the stamps failed")
-            t = [[buf[8 * i + k] for i in range(nb)] for k in range(8)]
+            begin = max(buf[8 * i] for i in range(rows)) - 2_000_000         # (rows of an earlier, larger launch)
+            cta = [i for i in range(rows) if buf[8 * i] > begin]
+            nb = len(cta)
+            t = [[buf[8 * i + k] for i in cta] for k in range(8)]
             t0 = min(t[0])
-            last = max(range(nb), key=lambda i: t[3][i])        # the CTA that arrived last
+            last = max(range(nb), key=lambda i: t[6][i])        # only the CTA that arrived last stamps the end
             if it >= 3:
                 res.append((a.elapsed_time(b) * 1e3, statistics.median(t[1]) - t0, min(t[2]) - t0, max(t[2]) - t0,
                             statistics.median(t[3]) - t0, t[3][last] - t0, t[4][last] - t0, t[5][last] - t0,
                             t[6][last] - t0))
         m = [statistics.median(x[i] for x in res) for i in range(9)]
         print(f"n=2^{lg} ctas={nb} event_us={m[0]:.1f} | ns since the first entry: loop start {m[1]:.0f}, loop end "
-              f"{m[2]:.0f}..{m[3]:.0f}, arrived median {m[4]:.0f} last {m[5]:.0f}, regions summed {m[6]:.0f}, "
+              f"{m[2]:.0f}..{m[3]:.0f}, arrived median {m[4]:.0f} last {m[5]:.0f}, totals known {m[6]:.0f}, "
               f"published {m[7]:.0f}, end {m[8]:.0f}", flush=True)
         env.close()
 

@@ -14,7 +14,7 @@
 // keeps data-parallel replicas bit-identical.
 //
 //  * sparse ops (ADD; SGD without weight decay) touch only the addressed
-//    elements in global memory;
+//    elements in global memory, source after source, each rounded on its own;
 //  * dense ops (SET, SGD with decay, momentum, AdamW) accumulate the sub-tile
 //    in shared memory and then walk it once with 16-byte accesses, so the
 //    averaged gradient never exists in global memory.
@@ -55,12 +55,14 @@ __device__ __forceinline__ CxPair ld_pair(const CxPair* p) {
 // Waits for all sources and validates their headers: the first warp does, lane j for source j.  (Every
 // warp for itself would save the barrier, but 7000 warps polling one line cost 5 us.)  Returns false
 // (uniformly for the CTA) when the kernel must not touch the output; no table is read before, a
-// payload of another length may have a shorter one.
-__device__ __forceinline__ bool wait_sources(const ApplyParams& p) {
+// payload of another length may have a shorter one.  PAIRS: `pairs` is the number of all sources together.
+template <bool PAIRS = false>
+__device__ __forceinline__ bool wait_sources(const ApplyParams& p, uint64_t* pairs = nullptr) {
   __shared__ uint32_t s_ok;
+  __shared__ uint32_t s_pairs[2];
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    uint32_t bad = 0;
+    uint32_t bad = 0, nnz = 0;
     if (lane < p.src.count) {
       const CxHeader* h = p.src.ep[lane].hdr;
       if (!cx::wait_seq(&h->seq, cx::seq_of(p.seq_cell, p.src.seq[lane]), p.timeout_ns)) {
@@ -69,13 +71,19 @@ __device__ __forceinline__ bool wait_sources(const ApplyParams& p) {
         const uint32_t kind = *reinterpret_cast<const volatile uint32_t*>(&h->kind);
         const uint32_t hn = *reinterpret_cast<const volatile uint32_t*>(&h->n);
         if (kind != CX_KIND_PAIRS || hn != (uint32_t)p.n) bad = CX_ST_BAD_HEADER;
+        if (PAIRS) nnz = *reinterpret_cast<const volatile uint32_t*>(&h->nnz);
       }
       if (bad && p.status) atomicOr(p.status, bad);
     }
     const bool any = __any_sync(0xffffffffu, bad != 0);
+    if (PAIRS) {               // in halves: sixteen 32-bit counts
+      const uint32_t high = __reduce_add_sync(0xffffffffu, nnz >> 16), low = __reduce_add_sync(0xffffffffu, nnz & 0xffffu);
+      if (lane == 0) { s_pairs[0] = low; s_pairs[1] = high; }
+    }
     if (lane == 0) s_ok = any ? 0u : 1u;
   }
   __syncthreads();
+  if (PAIRS) *pairs = ((uint64_t)s_pairs[1] << 16) + s_pairs[0];
   return s_ok != 0;
 }
 
@@ -91,6 +99,17 @@ __device__ __forceinline__ void segment_prefix(int lane, uint32_t a, uint32_t b,
   total = __shfl_sync(0xffffffffu, incl, 31);
 }
 
+__device__ __forceinline__ void table_entry(const ApplyParams& p, uint32_t sub, int lane, uint32_t& a, uint32_t& b) {
+  a = 0;
+  b = 0;
+  if (lane < p.src.count && sub < p.nsub) {
+    const uint2 entry = __ldcg(reinterpret_cast<const uint2*>(p.src.ep[lane].table) + sub);
+    a = entry.x;
+    b = min(entry.x + min(entry.y, (uint32_t)CX_SUBTILE), p.src.cap[lane]);  // never beyond the slot
+    a = min(a, b);
+  }
+}
+
 // The sparse ops: pairs go straight into the vector, source after source.  A warp takes up to 32
 // neighbouring sub-tiles at a time: lane l looks sub-tile l up, a scan lays the sub-tiles' pairs end
 // to end, and the lanes walk that sequence, AHEAD x 32 pairs in flight.  So a warp is busy whatever
@@ -101,20 +120,37 @@ __device__ __forceinline__ void segment_prefix(int lane, uint32_t a, uint32_t b,
 // 653 -> 646 us; the registers that this costs leave fewer warps, 25 M elements at 0.1 % 57 -> 59 us with it.
 constexpr int kAhead = 4, kAheadLarge = 8, kLargeGroup = 16;
 
-template <typename TO, int AHEAD>
+// What several sources touch has to stay in L2 until the last of them has come to it, so a warp takes fewer
+// sub-tiles at a time then: as many as keep the 64-byte pieces that all warps touch within half of L2 (126 MB).
+// A vector whose touched pieces fit there anyway is not bound by that; where every source fills a row of
+// 32 pairs in every sub-tile, one at a time is best.  2^28 elements, 7 sources, 1 / 2 / 4 / 8 / 19 sub-tiles:
+// 0.1 % 344 / 211 / 129 / 98 / 98 us, 1 % 504 / 396 / 488 / 650 / 739, 10 % 1192 / 1479 / 2266 / 2667 / 2641.
+// (One sub-tile at a time with all its sources in one round trip, as the batches below do: 166 / 438 / 1729.)
+constexpr uint64_t kInL2 = 96ull << 20, kHalfL2 = 63ull << 20;
+__device__ __forceinline__ uint32_t group_of_several(const ApplyParams& p, uint64_t pairs, int esize) {
+  if (pairs >= (uint64_t)p.nsub * 32 * p.src.count) return 1;
+  const uint64_t touched = min((uint64_t)CX_SUBTILE * esize * p.nsub, 64 * pairs);     // of the whole vector
+  if (touched <= kInL2) return p.group;
+  const uint64_t fit = kHalfL2 * p.nsub / touched / ((uint64_t)gridDim.x * kWarps);
+  return max(1u, (uint32_t)min((uint64_t)p.group, fit));
+}
+
+template <typename TO, int AHEAD, bool SEVERAL>
 __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_constant__ ApplyParams p) {
   cx::pdl_trigger();
   if (p.front_wait) cx::pdl_wait();
   const int lane = threadIdx.x & 31;
-  if (!wait_sources(p)) { cx::pdl_wait(); return; }
+  uint64_t all = 0;
+  if (!wait_sources<SEVERAL>(p, &all)) { cx::pdl_wait(); return; }
+  const uint32_t group = SEVERAL ? group_of_several(p, all, p.a.op == CX_OP_SGD ? 4 : (int)sizeof(TO)) : p.group;
   const uint32_t nwarps = gridDim.x * kWarps;
   const bool sgd = p.a.op == CX_OP_SGD;
   const float scale = sgd ? -p.a.scale : p.a.scale;
   uint32_t bad = 0;
-  for (uint64_t s0 = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * p.group; s0 < p.nsub;
-       s0 += (uint64_t)nwarps * p.group) {
+  for (uint64_t s0 = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * group; s0 < p.nsub;
+       s0 += (uint64_t)nwarps * group) {
     const uint32_t sub = (uint32_t)s0 + lane;
-    const bool have = lane < (int)p.group && sub < p.nsub;
+    const bool have = lane < (int)group && sub < p.nsub;
     uint2 next = have && p.src.count ? __ldcg(reinterpret_cast<const uint2*>(p.src.ep[0].table) + sub) : make_uint2(0, 0);
     for (int j = 0; j < p.src.count; ++j) {
       const uint32_t cap = p.src.cap[j];
@@ -173,6 +209,120 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
       }
       __syncwarp();  // the next source may address the same elements from other lanes
     }
+  }
+  if (bad && p.status) atomicOr(p.status, bad);
+  cx::pdl_wait();   // launched early behind its sender: do not complete before that grid has
+}
+
+// Several sources and few sub-tiles per warp: one chain of dependent loads per source would be most of the
+// kernel's time, so the pairs of all sources of a sub-tile are laid end to end and 128 of them at a time are
+// fetched in one round trip, the elements they address in a second one.  The additions go source after
+// source in shared memory: pairs that address the same element share the slot of one of them.
+// ADD, fp32, 7 sources, a group of sub-tiles source after source against this: 2^20 elements at 0.1 / 1 / 10 %
+// 16.4 / 18.4 / 21.5 -> 10.3 / 11.3 / 20.5 us, 2^22 18.4 / 20.5 / 27.5 -> 12.3 / 14.5 / 28.7.
+constexpr int kBatch = 4;                     // pairs per lane
+constexpr uint32_t kBatchPairs = 32 * kBatch;
+// Up to one sub-tile per warp (7.2 M elements), and up to two with more than four sources: 12 M elements, 0.1 / 1 %,
+// 2 sources 14.3 / 16.4 us in batches and 12.3 / 16.4 in groups, 7 sources 18.5 / 24.6 and 18.5 / 28.7.
+inline bool in_batches(uint32_t group, int sources) { return sources > 1 && group <= (sources > 4 ? 2u : 1u); }
+
+template <typename TO>
+__global__ void __launch_bounds__(kThreads, 6) apply_sparse_batch_kernel(const __grid_constant__ ApplyParams p) {
+  __shared__ uint8_t s_slot[kWarps][CX_SUBTILE];
+  __shared__ float s_acc[kWarps][kBatchPairs];
+  cx::pdl_trigger();
+  if (p.front_wait) cx::pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!wait_sources(p)) { cx::pdl_wait(); return; }
+  const uint32_t nwarps = gridDim.x * kWarps;
+  const bool sgd = p.a.op == CX_OP_SGD;
+  const float scale = sgd ? -p.a.scale : p.a.scale;
+  uint8_t* slot = s_slot[warp];
+  float* acc = s_acc[warp];
+  uint32_t bad = 0;
+  uint32_t sub = blockIdx.x * kWarps + warp, a, b;
+  table_entry(p, sub, lane, a, b);
+  for (; sub < p.nsub; sub += nwarps) {
+    const uint32_t lo = sub * CX_SUBTILE;
+    uint32_t na, nb, pre, total;              // the next sub-tile's table entries, in flight meanwhile
+    const uint64_t next = (uint64_t)sub + nwarps;
+    table_entry(p, next < p.nsub ? (uint32_t)next : p.nsub, lane, na, nb);
+    segment_prefix(lane, a, b, pre, total);
+    int j0 = 0, j1 = 0;                       // the batch's pairs are of the sources [j0, j1) (warp-uniform)
+    for (uint32_t f0 = 0; f0 < total; f0 += kBatchPairs) {
+      int src[kBatch];                        // source of the pair, -1: none
+      uint32_t off[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) { src[k] = -1; off[k] = 0; }
+      j0 = max(j1 - 1, 0);                    // the last source of the batch before may have more
+      for (j1 = j0; j1 < p.src.count; ++j1) {
+        const int j = j1;
+        const uint32_t pj = __shfl_sync(0xffffffffu, pre, j), aj = __shfl_sync(0xffffffffu, a, j);
+        const uint32_t cj = __shfl_sync(0xffffffffu, b, j) - aj;
+        if (pj >= f0 + kBatchPairs) break;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const uint32_t f = f0 + 32 * k + lane;
+          if (f - pj < cj) { src[k] = j; off[k] = aj + (f - pj); }
+        }
+      }
+      CxPair pr[kBatch];
+      uint32_t d[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        pr[k].idx = 0;
+        pr[k].val = 0;
+        if (src[k] >= 0) pr[k] = ld_pair(p.src.ep[src[k]].pairs + off[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        d[k] = (uint32_t)pr[k].idx - lo;
+        if (src[k] >= 0 && !(d[k] < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { bad = CX_ST_BAD_INDEX; src[k] = -1; }
+        if (src[k] >= 0) slot[d[k]] = (uint8_t)(32 * k + lane);
+      }
+      float cur[kBatch];
+      if (sgd) {
+        const float* w = reinterpret_cast<const float*>(p.a.out);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) cur[k] = src[k] >= 0 ? w[pr[k].idx] : 0.f;
+      } else {
+        const TO* out = reinterpret_cast<const TO*>(p.a.out);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) cur[k] = src[k] >= 0 ? cx::Elem<TO>::to_f(out[pr[k].idx]) : 0.f;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (src[k] < 0) continue;
+        d[k] = slot[d[k]];
+        acc[d[k]] = cur[k];                   // the same value from every pair of the element
+      }
+      __syncwarp();
+      for (int j = j0; j < j1; ++j) {         // rounded like the element-by-element path
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          if (src[k] == j) {
+            const float nv = acc[d[k]] + scale * __uint_as_float(pr[k].val);
+            acc[d[k]] = sgd ? nv : cx::Elem<TO>::to_f(cx::Elem<TO>::from_f(nv));
+          }
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (src[k] < 0) continue;
+        const float nv = acc[d[k]];
+        if (sgd) {
+          reinterpret_cast<float*>(p.a.out)[pr[k].idx] = nv;
+          if (p.a.shadow) reinterpret_cast<TO*>(p.a.shadow)[pr[k].idx] = cx::Elem<TO>::from_f(nv);
+        } else {
+          reinterpret_cast<TO*>(p.a.out)[pr[k].idx] = cx::Elem<TO>::from_f(nv);
+        }
+      }
+      __syncwarp();                           // the next batch may address the same elements from other lanes
+    }
+    a = na;
+    b = nb;
   }
   if (bad && p.status) atomicOr(p.status, bad);
   cx::pdl_wait();   // launched early behind its sender: do not complete before that grid has
@@ -378,17 +528,6 @@ __device__ __forceinline__ uint32_t accumulate_subtile_ahead(const ApplyParams& 
     __syncwarp();
   }
   return bad;
-}
-
-__device__ __forceinline__ void table_entry(const ApplyParams& p, uint32_t sub, int lane, uint32_t& a, uint32_t& b) {
-  a = 0;
-  b = 0;
-  if (lane < p.src.count && sub < p.nsub) {
-    const uint2 entry = __ldcg(reinterpret_cast<const uint2*>(p.src.ep[lane].table) + sub);
-    a = entry.x;
-    b = min(entry.x + min(entry.y, (uint32_t)CX_SUBTILE), p.src.cap[lane]);  // never beyond the slot
-    a = min(a, b);
-  }
 }
 
 // ---- bulk-copy (TMA) pipeline for the optimizer state ---------------------------------------
@@ -817,8 +956,11 @@ int launch_apply(const ApplyParams& p, int grid, cudaStream_t s) {
     if (op == CX_OP_ADAMW) return launch_bulk<CX_OP_ADAMW, TO>(p, s);
   }
   const bool cap = p.seq_cell != nullptr;
-  if (sparse && p.group >= kLargeGroup) cx_launch_pdl(apply_sparse_kernel<TO, kAheadLarge>, grid, kThreads, 0, s, p, cap);
-  else if (sparse) cx_launch_pdl(apply_sparse_kernel<TO, kAhead>, grid, kThreads, 0, s, p, cap);
+  const bool several = p.src.count > 1;
+  if (sparse && in_batches(p.group, p.src.count)) cx_launch_pdl(apply_sparse_batch_kernel<TO>, grid, kThreads, 0, s, p, cap);
+  else if (sparse && several) cx_launch_pdl(apply_sparse_kernel<TO, kAhead, true>, grid, kThreads, 0, s, p, cap);
+  else if (sparse && p.group >= kLargeGroup) cx_launch_pdl(apply_sparse_kernel<TO, kAheadLarge, false>, grid, kThreads, 0, s, p, cap);
+  else if (sparse) cx_launch_pdl(apply_sparse_kernel<TO, kAhead, false>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_SET) cx_launch_pdl(apply_dense_kernel<CX_OP_SET, TO>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_SGD) cx_launch_pdl(apply_dense_kernel<CX_OP_SGD, TO>, grid, kThreads, 0, s, p, cap);
   else if (op == CX_OP_MOMENTUM) cx_launch_pdl(apply_dense_kernel<CX_OP_MOMENTUM, TO>, grid, kThreads, 0, s, p, cap);
@@ -857,7 +999,9 @@ int cx_apply_cuda(const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_
     const uint64_t waves = (p.nsub + warps * 32 - 1) / (warps * 32);
     p.group = (uint32_t)((p.nsub + warps * waves - 1) / (warps * waves));
   }
-  const int need = (int)((p.nsub + (uint64_t)kWarps * p.group - 1) / ((uint64_t)kWarps * p.group));
+  // (the kernels for several sources may take fewer sub-tiles at a time)
+  const uint64_t per_cta = (uint64_t)kWarps * (src->count > 1 ? 1u : p.group);
+  const int need = (int)((p.nsub + per_cta - 1) / per_cta);
   if (grid > need) grid = need;
   // A dense kernel lets the next one in early when that one is chained to it, or when it leaves most of
   // the GPU free.  Otherwise early CTAs of the next kernel fill the gaps of this one unevenly, and SMs

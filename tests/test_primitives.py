@@ -425,6 +425,51 @@ def test_apply_sparse_large_groups(op):
     env.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1000, 70001, 148 * 48 * 1024, 148 * 48 * 3 * 1024 + 1, 148 * 48 * 3 * 1024 + 1025, 50_000_003])
+@pytest.mark.parametrize("nsrc", [2, 7, 15])
+@pytest.mark.parametrize("density", [0.0005, 0.01, 0.2])
+@pytest.mark.parametrize("what", ["add", "add_bf16", "sgd_shadow"])
+def test_apply_sparse_several_sources(n, nsrc, density, what):
+    """The sparse decode of several sources at the edges of its walks (batches of 128 pairs per sub-tile, groups
+    of sub-tiles by the sources' pair counts): every element takes the sources one after the other, rounded
+    after each; elements that several sources address, sub-tiles that are full in all of them, empty ones."""
+    if n > 10_000_000 and (nsrc == 15 or (nsrc == 2 and what != "add")):
+        pytest.skip("large vectors with seven sources, and with two where the result is fp32")
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(nsrc)
+    dt = torch.bfloat16 if what == "add_bf16" else torch.float32
+    out = torch.randn(n, device="cuda", generator=gen).to(dt)
+    shadow = torch.zeros(n, dtype=torch.bfloat16, device="cuda") if what == "sgd_shadow" else None
+    want = out.clone()
+    slots, st = [], env.new_status("t")
+    touched = torch.zeros(n, dtype=torch.bool, device="cuda")
+    for j in range(nsrc):
+        x = torch.randn(n, device="cuda", generator=gen)
+        x[torch.rand(n, device="cuda", generator=gen) >= density] = 0
+        x[: min(n, 40)] = 1.0 + j                                    # elements of every source
+        if n > 8192:
+            x[2048:3072] = 0.5 + j                                   # a full sub-tile
+            x[4096:5120] = 0
+        cap = 32 * ((int((x != 0).sum()) // 16) + 1024 + 256)        # regions fill unevenly
+        slot, comp = P.SparseSlot.create(env, n, cap), P.Compressor(env, n)
+        comp.set_threshold(0.0)
+        comp.compress(x, None, n, cap, 5, P.make_targets([slot.endpoint(env, 0)]))
+        assert comp.last_stats()["status"] == 0
+        slots.append(slot)
+        touched |= x != 0
+        scale = torch.tensor(0.3, dtype=torch.float32, device="cuda")
+        want = torch.where(x != 0, (want.float() + (-scale if what == "sgd_shadow" else scale) * x).to(dt), want)
+    src = P.make_sources([s.endpoint(env, 0) for s in slots], [5] * nsrc)
+    args = (P.args_update(_lib.OP_SGD, out, 0.3, shadow=shadow) if what == "sgd_shadow" else P.args_add(out, 0.3))
+    P.apply_sparse(env, src, n, args, st)
+    env.flush()
+    assert st.value == 0 and torch.equal(out, want)
+    if shadow is not None:
+        assert torch.equal(shadow, torch.where(touched, want.to(torch.bfloat16), torch.zeros_like(shadow)))
+    env.close()
+
+
 @pytest.mark.parametrize("op", ["sgd", "sgd_wd", "momentum", "adamw"])
 @pytest.mark.parametrize("shadow", [False, True])
 def test_apply_fused_updates(world, op, shadow):
