@@ -8,7 +8,7 @@ after warm-up and with an L2 flush between iterations:
                    ``--targets`` slots (local memory stands in for peers),
 * ``residual_add_torch`` - ``torch.add(r, g, out=r)``: the same dense traffic through torch's own
                    elementwise kernel, as the size-matched reference for the compress rows,
-* ``apply_add``  - wait + scatter-add of ``--sources`` payloads,
+* ``apply_add``  - wait + scatter-add of ``--sources`` payloads, each of a vector of its own,
 * ``apply_set``  - wait + dense result (sum of the payloads, zero elsewhere): the receive side of
                    the replica-consistent allreduce,
 * ``apply_sgd`` / ``apply_adamw`` - the same fused with the parameter update.
@@ -145,24 +145,30 @@ def main():
                     "apply_sgd": (k_sgd, args.sources * nnz * (8 + 64)),
                     "apply_adamw": (k_adamw, args.sources * nnz * 8 + 24 * n),
                 }
-                r0 = r.clone()
-                for name, (fn, nbytes) in kernels.items():
+                filled = False
+                for name in kernels:
+                    fn, nbytes = kernels[name]
                     if name not in ("compress", "residual_add_torch") and dname != args.dtypes[0]:
                         continue   # only the compress kernel reads the gradient dtype
                     if args.kernels and name not in args.kernels:
                         continue
-                    if name == "apply_add":
-                        # the receive kernels see a payload of the nominal density again: the timed
-                        # compress calls above fed the same gradient into a growing residual
-                        r.copy_(r0)
-                        k_thr()
-                        k_comp()
-                        nnz = comp.last_stats()["nnz"]
+                    if name.startswith("apply") and not filled:
+                        # every source sends a vector of its own at the nominal density: payloads that
+                        # address the same elements would be decoded from the cache
+                        filled = True
+                        nnz = 0
+                        for s_ in slots[: args.sources]:
+                            out.normal_(0.0, 1.25 ** 0.5)
+                            comp.threshold_topk(out, None, n, ratio)
+                            comp.compress(out, None, n, cap, 1, P.make_targets([s_.endpoint(env)]))
+                            nnz += comp.last_stats()["nnz"]
+                        out.zero_()
                         for key in ("apply_add", "apply_sgd"):
-                            kernels[key] = (kernels[key][0], args.sources * nnz * (8 + 64))
-                        kernels["apply_set"] = (kernels["apply_set"][0], args.sources * nnz * 8 + 4 * n)
-                        kernels["apply_adamw"] = (kernels["apply_adamw"][0], args.sources * nnz * 8 + 24 * n)
-                        nbytes = kernels[name][1]
+                            kernels[key] = (kernels[key][0], nnz * (8 + 64))
+                        kernels["apply_set"] = (kernels["apply_set"][0], nnz * 8 + 4 * n)
+                        kernels["apply_adamw"] = (kernels["apply_adamw"][0], nnz * 8 + 24 * n)
+                        nnz //= args.sources
+                        fn, nbytes = kernels[name]
                     for _ in range(args.warmup):
                         fn()
                     reps = 10 if n * 12 < (100 << 20) else 1

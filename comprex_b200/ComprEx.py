@@ -186,9 +186,9 @@ class CompressorRLE(_Compressor):
     The byte layout follows the reference (``n | nnz | values | nRuns |
     firstIsYes | runs``) but values are stored at their packed position, which
     the reference's codec gets wrong for thresholds above zero.  Engines use the
-    fused codec of ``csrc/rle.cu`` (count / scan / emit kernels that store the
-    payload straight into the receiver's slot, bounded wait + run check + expand on
-    the other side); ``encode`` / ``decode`` below are the host codec on byte strings,
+    fused codec of ``csrc/rle.cu`` (count and emit kernels that store the
+    payload straight into the receiver's slot; index and expand kernels with a bounded
+    wait and the checks of the runs on the other side); ``encode`` / ``decode`` below are the host codec on byte strings,
     the oracle of the tests.
     """
     kind = "rle"

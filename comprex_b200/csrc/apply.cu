@@ -900,9 +900,8 @@ __global__ void __launch_bounds__(kThreads) forward_kernel(const ForwardParams p
 #endif
 
 // COMPREX_APPLY_BULK=1 routes the dense updates through the bulk-copy kernel.  It is off by
-// default: on B200 it is 3 % faster than the register kernel for AdamW at 2^28 elements and
-// 1 % survivors (1336 vs 1385 us) and slower everywhere else (2^24: 179 vs 136 us; 10 %
-// survivors: 2784 vs 1787 us), because its shared-memory footprint leaves 14 warps per SM to
+// default: AdamW at 2^28 elements and 1 % survivors takes 1336 us in it and 1098 in the register
+// kernel (2^24: 179 and 79 us; 10 % survivors: 2784 and 1275 us), because its shared-memory footprint leaves 14 warps per SM to
 // cover an instruction-issue-bound update.  The variable is read at every call.
 bool bulk_enabled() {
   const char* e = getenv("COMPREX_APPLY_BULK");

@@ -27,8 +27,9 @@
 //
 // Survivors that do not fit into the slot are not emitted and stay in the
 // residual, which error feedback makes safe; the count is reported.  The CTA
-// that finishes last writes the header and publishes the notification
-// (st.release.sys) after every CTA's stores were fenced at system scope.
+// that finishes last writes the header and publishes the notification: its
+// st.release.sys covers the stores of all CTAs, which were ordered before their
+// arrivals at GPU scope (cx::cta_arrive).
 #include <stdlib.h>
 #include <string.h>
 
@@ -36,9 +37,9 @@
 
 namespace {
 
-// Two CTAs of 256 threads or their like (16 warps) per SM: each lane keeps a whole sub-tile share of 32
-// values in registers with all its loads in flight, which needs ~100 registers; squeezing more warps onto
-// an SM makes it spill and measured slower at every size (2^24 elements, 1 %: 55 us with 16 warps, 69 us
+// 16 warps per SM: each lane keeps a whole sub-tile share of 32 values in registers with all its loads in
+// flight, which takes the 128 registers that leaves a thread (no spills without multicast; the folding
+// kernel spills 126 bytes a thread with fp32 momentum and 78 to 198 with 16-bit gradients).  Squeezing more warps onto an SM makes it spill and measured slower at every size (2^24 elements, 1 %: 55 us with 16 warps, 69 us
 // with 24), and so did an L2 prefetch of the warp's next sub-tile.
 #ifndef CX_COMPRESS_MIN_BLOCKS
 #define CX_COMPRESS_MIN_BLOCKS 2

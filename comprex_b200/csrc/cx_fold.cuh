@@ -101,7 +101,7 @@ __device__ __forceinline__ FoldWhole<T> fold_whole(const CxFold& f, uint32_t sub
 // Sub-tiles at tensor borders take several times as long as whole ones (more dependent loads); met
 // late in a warp's share they were a tail of 25 us.  The first CTAs of the grid do nothing else, the
 // others skip them.  Returns how many: all that are needed while the grid has room, else their share
-// of the work at four times the cost.
+// of the work, a border sub-tile counted as four whole ones (by its dependent loads; not swept).
 inline int cx_border_ctas(const CxFold& f, int64_t nsub, int warps, int room, int* grid) {
   const int64_t nat = (nsub + warps - 1) / warps, bor = (f.nborder + warps - 1) / warps;
   if (nat + bor <= room) { *grid = (int)(nat + bor); return (int)bor; }

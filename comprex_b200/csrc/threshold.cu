@@ -6,8 +6,8 @@
 // vector is shorter), and takes the element of rank ceil(samples*topK)-1 in
 // descending |x| order; when that rank is <= 0 the threshold is max|x| + 1
 // so that nothing is sent.  This kernel reproduces that rule bit for bit: the
-// sample keys are the bit patterns of |x| (monotonic for non-negative floats)
-// and a 4-pass 8-bit radix select over one CTA finds the element of that rank.
+// sample keys are the bit patterns of |x| (monotonic for non-negative floats),
+// and one CTA finds the element of that rank (select_cached; by radix where that does not apply).
 // The result stays in device memory, where the compress kernel reads it, so
 // no host round trip sits between the two.
 //

@@ -6,22 +6,28 @@ momentum buffer scaled by the learning rate (``mom = m*mom + lr*g``),
 concatenates everything into one blob, allreduces the blob with one of six
 collectives (default ``comprex_bigring``), divides by the number of ranks and
 applies ``var = (1-wd)*var - update``.  This class keeps those semantics for
-PyTorch and maps a step onto five kernel launches per bucket:
+PyTorch and maps a step onto these launches:
 
-1. per-tensor sums of squares and 2. clip + momentum fold, read straight from
-   the gradient tensors autograd produced into the flat fp32 update vector,
-3. threshold estimate of ``residual + update`` (device resident),
-4. fused ``residual += update`` / select / store pairs into every peer's slot,
-5. fused wait / scatter-add in rank order / average / parameter update, which
+1. per-tensor sums of squares, read straight from the gradient tensors autograd
+   produced; they leave every tensor's clip factor,
+2. threshold estimate of ``residual + update`` (device resident),
+3. fused clip / momentum / ``residual += update`` / select / store pairs into every
+   peer's slot,
+4. fused wait / scatter-add in rank order / average / parameter update, which
    also refreshes the low-precision copy of the weights when the model is held
    in bf16 or fp16.
+
+A step that finds all buckets unsent issues them as one list: 1 once, 2 once per 24
+buckets, 3 and 4 once per bucket.  Buckets that an exchange takes in memory (the other
+collectives, a threshold selected over the whole vector) are folded into the flat
+vector first.
 
 The parameters live in one flat fp32 master buffer (the model's tensors are
 views of it, or of its low-precision shadow, in their own memory order, so
 channels-last weights stay channels-last); there is no flat gradient buffer,
 no concatenation and no slicing copy.  The flat
 buffers are laid out in reverse parameter order and cut into buckets of
-``bucket_cap_mb``; with ``overlap=True`` (and more than one bucket) a bucket's steps 1-4 are launched on a
+``bucket_cap_mb``; with ``overlap=True`` (and more than one bucket) a bucket's steps 1-3 are launched on a
 side stream from a post-accumulate-grad hook as soon as its last gradient is
 produced, i.e. while backward is still running for earlier layers, and
 ``step()`` only launches the receive/update kernels.  Every rank, the sender
@@ -77,11 +83,15 @@ class _Bucket:
         self.kind, self.xbuf, self.plan, self.u = None, None, None, None
 
 
+_SMS = 148        # of a B200
+
+
 def _item_size(total: int) -> int:
     """Elements per fold work item.  Every item ends with an arrival at its tensor's counter (1 us), so
-    items are long where there are enough of them for every SM, and one round of loads of 256 threads
-    otherwise (ResNet-50, single rank: 98.4 us with 65536, 101.8 with 16384; LeNet-5: 22.2 and 21.5)."""
-    return 65536 if total >= 65536 * 148 else 16384
+    items are long where there is one for every SM, and one round of loads of 256 threads otherwise
+    (a step of 62 k parameters 22.2 us with 65536 and 21.5 with 16384, of 25.6 M 98.4 and 101.8, of 355 M
+    2195 and 2211; between those sizes the line was not measured)."""
+    return 65536 if total >= 65536 * _SMS else 16384
 
 
 _ALIGN = 64       # tensors start on 128-byte (bf16) / 256-byte (fp32) boundaries of the flat buffers
