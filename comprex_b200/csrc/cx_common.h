@@ -302,6 +302,7 @@ int cx_rle_decode_host(const void* in, int64_t in_bytes, float* out, int64_t n,
  * as it was. */
 int64_t cx_rle_slot_bytes(int64_t n);
 int64_t cx_rle_workspace_bytes(int64_t n);
+int64_t cx_rle_recv_workspace_bytes(int64_t n);     /* enough where the workspace only receives */
 int cx_rle_send(int dev, int gdtype, const void* g, float* r, int64_t n, const float* thr,
                 int64_t slot_bytes, uint64_t seq, const CxTargets* tg, void* workspace,
                 int64_t ws_bytes, uint32_t src_rank, void* stream);

@@ -7,17 +7,20 @@
 //   nRuns x i32 run lengths, alternating selected / not selected.
 // Selection: |r + g| >= thr, except that zeros are never selected at thr == 0.
 //
-// Send = two launches on one stream, both over the same partition of the vector into one
-// contiguous chunk per warp (a CTA's eight chunks are neighbours; one wave of CTAs, so the totals
+// Send = two launches on one stream over the same partition of the vector, one contiguous chunk of whole
+// 1024-element sub-tiles per warp (a CTA's eight chunks are neighbours; one wave of CTAs, so the totals
 // are few):
-//   1. rle_count:  per chunk: selected elements, run starts, and whether its first element
-//                  starts a run.  Only sums leave the warp, no scan is needed,
-//   2. rle_emit:   every CTA adds up the totals of the CTAs before it (a few hundred numbers),
-//                  then every warp walks its chunk on its own, 256 elements at a time with running
-//                  offsets: values and run starts are compacted in shared memory and stored
-//                  coalesced at their final position in every target, the residual is updated from
-//                  the same registers.  The last CTA writes the two small headers and releases the
-//                  sequence number.
+//   1. rle_scan:   the only pass over the vector.  Lane l looks at element 32 j + l, so a ballot is 32
+//                  bits of the selection in order: the words go to scratch, the selected values, compacted
+//                  per chunk, too, the residual is updated.  Totals of every chunk: selected elements, run
+//                  starts, the last of them.
+//   2. rle_emit:   every CTA adds up the totals of the CTAs before it (a few hundred numbers); then every
+//                  warp copies its chunk's values and turns its words into run lengths, coalesced at their
+//                  final position in every target.  (The runs lie behind the values, so nobody can write a
+//                  run before all values are counted.)  The last CTA writes the two small headers and
+//                  releases the sequence number.
+// With two passes over the vector (count, then load again and emit, a lane per 8 elements) 2^22 fp32 elements
+// at 10 % took 10 + 17 us, 177 and 495 instructions per 256 elements at half of the issue rate.
 // Receive = two launches:
 //   1. rle_index:  waits (bounded), checks the headers, sums the run lengths of every block of
 //                  kRunBlock runs (one warp per block) and leaves prefixes inside groups of blocks,
@@ -25,6 +28,7 @@
 //                  starts in, and takes windows of kWindow outputs: the start of every run flips
 //                  one bit of a mask in shared memory, the prefix parity of the mask says which
 //                  outputs are selected, and counting selected bits gives the index of every value.
+//                  The first window of `out` is on its way to L2 while the index is made.
 //                  The checks (lengths add up to n and nnz) happen before the first store, in every
 //                  CTA alike.
 // A payload that fails a check sets BAD_HEADER in the status word and leaves `out` untouched.
@@ -37,20 +41,22 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kPer = 8;
-constexpr int kSeg = 32 * kPer;          // elements a warp takes at a time
-constexpr int kSendPerSm = 4;            // resident CTAs of the emit kernel
+constexpr int kSendPerSm = 4;            // resident CTAs of the scan kernel
+constexpr int kRows = 16;                // rows of 32 elements whose loads are in flight together
 constexpr int kMaxSend = 1024;           // sending CTAs
 constexpr int kGroups = 256;             // groups of run blocks, one per thread of a receiving CTA
 constexpr int kRunBlock = 1024;          // runs per block: one warp sums it, one CTA scans it
 constexpr int kWindow = 32 * kThreads;   // outputs per window: one mask word per thread
+constexpr int kRunsEach = 2 * kRunBlock / kThreads;   // runs a thread takes at a time
+constexpr int kRowsOut = 8;              // rows of 32 outputs in flight together
 
-struct ChunkTotals {       // of one warp's chunk, or of a CTA's eight
-  int32_t nnz;             // selected elements
-  int32_t starts;          // elements that start a run
-  int32_t last;            // position of the last run start (-1: none)
-  int32_t first;           // 1 if the chunk's first element starts a run
+struct ChunkTotals {       // of one warp's chunk, or of a CTA's eight.  Whether the first element starts a run is
+  int32_t nnz;             // selected elements                        the element's in front to say: not counted
+  int32_t starts;          // elements but the first that start a run
+  int32_t last;            // position of the last of these (-1: none)
+  int32_t ends;            // kFirstYes, kLastYes: the first / last element is selected; kEmpty: no elements
 };
+constexpr int kFirstYes = 1, kLastYes = 2, kEmpty = 4;
 
 struct RleMeta {           // first 256 bytes of the sender's workspace
   uint32_t done;
@@ -75,155 +81,145 @@ struct SendParams {
   RleMeta* meta;
   ChunkTotals* cta;      // [gridDim.x]
   ChunkTotals* chunk;    // [gridDim.x * kWarps]
-  int32_t segs;          // segments per chunk
+  uint32_t* bits;        // [sub-tiles * 32] selected elements
+  float* vals;           // [n] selected values, every chunk's from its first element's place on
+  int32_t subs;          // sub-tiles per chunk
   uint32_t src_rank;
 };
 
-__device__ __forceinline__ bool selected(float v, float thr) {
-  return fabsf(v) >= thr && !(thr == 0.f && v == 0.f);
+// |v| >= cut selects: like the reference, except that zeros are never selected
+__device__ __forceinline__ float cut_of(float thr) { return thr == 0.f ? __uint_as_float(1u) : thr; }
+
+// totals of a, with what follows it; `start`: position of b's first element
+__device__ __forceinline__ ChunkTotals append(const ChunkTotals& a, const ChunkTotals& b, int64_t start) {
+  if (b.ends & kEmpty) return a;
+  ChunkTotals t;
+  const bool edge = ((a.ends & kLastYes) != 0) != ((b.ends & kFirstYes) != 0);
+  t.nnz = a.nnz + b.nnz;
+  t.starts = a.starts + b.starts + (edge ? 1 : 0);
+  t.last = b.last >= 0 ? b.last : edge ? (int32_t)start : a.last;
+  t.ends = (a.ends & kFirstYes) | (b.ends & kLastYes);
+  return t;
 }
 
-template <typename T>
-__device__ __forceinline__ float value_at(const SendParams& p, int64_t i) {
-  float v = p.g ? cx::Elem<T>::to_f(reinterpret_cast<const T*>(p.g)[i]) : 0.f;
-  if (p.r) v += p.r[i];
-  return v;
-}
-
-__device__ __forceinline__ int valid_at(int64_t n, int64_t base) {
-  const int64_t left = n - base;
-  return left >= kPer ? kPer : (left > 0 ? (int)left : 0);
-}
-
-// the thread's 8 consecutive values (zero beyond the vector's end)
-template <typename T>
-__device__ __forceinline__ void load_values(const SendParams& p, int64_t base, float (&v)[kPer]) {
-  const int valid = valid_at(p.n, base);
-  const T* g = reinterpret_cast<const T*>(p.g);
-  const bool gvec = !g || (reinterpret_cast<uintptr_t>(g) & (4 * sizeof(T) - 1)) == 0;
-  const bool rvec = !p.r || (reinterpret_cast<uintptr_t>(p.r) & 15) == 0;
-  if (valid == kPer && gvec && rvec) {
-    float a[4], b[4];
-    if (g) { cx::load4(g + base, a); cx::load4(g + base + 4, b); }
-    else { for (int e = 0; e < 4; ++e) a[e] = b[e] = 0.f; }
-    if (p.r) {
-      float c[4], d[4];
-      cx::load4(p.r + base, c); cx::load4(p.r + base + 4, d);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { a[e] += c[e]; b[e] += d[e]; }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { v[e] = a[e]; v[4 + e] = b[e]; }
-  } else {
-#pragma unroll
-    for (int e = 0; e < kPer; ++e) v[e] = e < valid ? value_at<T>(p, base + e) : 0.f;
-  }
-}
-
-__device__ __forceinline__ uint32_t yes_mask(const float (&v)[kPer], int valid, float thr) {
-  uint32_t yes = 0;
-#pragma unroll
-  for (int e = 0; e < kPer; ++e)
-    if (e < valid && selected(v[e], thr)) yes |= 1u << e;
-  return yes;
-}
-
-// bits of the run starts among the thread's valid elements, given the element in front of them
-__device__ __forceinline__ uint32_t start_mask(uint32_t yes, int valid, bool prev_yes) {
-  const uint32_t vm = valid >= kPer ? 0xffu : ((1u << valid) - 1u);
-  return (yes ^ ((yes << 1) | (prev_yes ? 1u : 0u))) & vm;
-}
-
-// Bound by the read of g and r.  The element in front of a lane's share comes from the lane to the
-// left; only the first one of a chunk is read from memory (nothing writes r in this kernel).
-template <typename T>
-__global__ void __launch_bounds__(kThreads) rle_count_kernel(const __grid_constant__ SendParams p) {
+// One pass: g and r are read, r and the words are written.  A lane holds every 32nd element, so no access
+// needs an alignment and the selection of a row is one ballot.
+template <typename T, bool HAS_G, bool HAS_R>
+__global__ void __launch_bounds__(kThreads, kSendPerSm) rle_scan_kernel(const __grid_constant__ SendParams p) {
   __shared__ ChunkTotals s_chunk[kWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t chunk = (int64_t)blockIdx.x * kWarps + w;
+  const int64_t lo = chunk * p.subs * CX_SUBTILE, hi = min(lo + (int64_t)p.subs * CX_SUBTILE, p.n);
+  const T* __restrict__ g = reinterpret_cast<const T*>(p.g);
+  if (lo + 32 * lane < hi) {           // the first sub-tile starts its way to L2 behind the kernel in front
+    if (HAS_R) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.r + lo + 32 * lane));
+    if (HAS_G) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + lo + 32 * lane));
+  }
   cx::pdl_wait();
   cx::pdl_trigger();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float thr = *p.thr;
-  const int64_t chunk = (int64_t)blockIdx.x * kWarps + w;
-  const int64_t lo = chunk * p.segs * kSeg;
-  const int64_t hi = min(lo + (int64_t)p.segs * kSeg, p.n);
-  uint32_t tail = 0;
-  if (lane == 0 && lo > 0 && lo < hi) tail = selected(value_at<T>(p, lo - 1), thr) ? 1u : 0u;
-  int nnz = 0, st = 0, last = -1, first = 0;
-#pragma unroll 2
-  for (int64_t seg = lo; seg < hi; seg += kSeg) {
-    const int64_t base = seg + lane * kPer;
-    float v[kPer];
-    load_values<T>(p, base, v);
-    const int valid = valid_at(p.n, base);
-    const uint32_t yes = yes_mask(v, valid, thr);
-    const uint32_t edge = yes >> (kPer - 1);
-    uint32_t prev = __shfl_up_sync(0xffffffffu, edge, 1);
-    if (lane == 0) prev = tail;
-    tail = __shfl_sync(0xffffffffu, edge, 31);
-    uint32_t starts = start_mask(yes, valid, prev != 0);
-    if (base == 0 && valid > 0) {                     // element 0 always starts a run
-      starts |= 1u;
-      p.meta->first_yes = (int)(yes & 1u);
-    }
-    if (base == lo) first = (int)(starts & 1u);
-    nnz += __popc(yes);
-    st += __popc(starts);
-    if (starts) last = (int)(base + 31 - __clz(starts));
-  }
-  if (p.n == 0 && threadIdx.x == 0) p.meta->first_yes = 0;
+  const float cut = cut_of(*p.thr);
+  float* vals = p.vals + lo;
+  const uint32_t below = (1u << lane) - 1u;
+  uint32_t nnz = 0, tail = 0;          // selected so far (the same in all lanes), bit of the element in front
+  int st = 0, last = -1, ends = lo < hi ? 0 : kEmpty;
+  for (int64_t sub = lo; sub < hi; sub += CX_SUBTILE) {
+    const int left = (int)min((int64_t)CX_SUBTILE, hi - sub);
+    uint32_t word = 0;                 // elements 32 lane ... of the sub-tile
+#pragma unroll 1
+    for (int j0 = 0; j0 < CX_SUBTILE / 32; j0 += kRows) {
+      const int64_t at = sub + 32 * j0 + lane;
+      const int here = left - 32 * j0 - lane;          // my elements: 32 j < here
+      float v[kRows], b[kRows];
+      if (here > 32 * (kRows - 1)) {
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    nnz += __shfl_xor_sync(0xffffffffu, nnz, d);
-    st += __shfl_xor_sync(0xffffffffu, st, d);
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, d));
+        for (int j = 0; j < kRows; ++j) {
+          v[j] = HAS_R ? p.r[at + 32 * j] : 0.f;
+          b[j] = HAS_G ? cx::Elem<T>::to_f(g[at + 32 * j]) : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+          v[j] = HAS_R && 32 * j < here ? p.r[at + 32 * j] : 0.f;
+          b[j] = HAS_G && 32 * j < here ? cx::Elem<T>::to_f(g[at + 32 * j]) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) {
+        if (HAS_R && HAS_G) v[j] = b[j] + v[j];
+        else if (HAS_G) v[j] = b[j];
+        const bool yes = 32 * j < here && fabsf(v[j]) >= cut;
+        const uint32_t row = __ballot_sync(0xffffffffu, yes);
+        if (lane == j0 + j) word = row;
+        if (yes) vals[nnz + __popc(row & below)] = v[j];
+        nnz += __popc(row);
+        if (HAS_R && 32 * j < here) p.r[at + 32 * j] = yes ? 0.f : v[j];
+      }
+    }
+    p.bits[(sub >> 5) + lane] = word;
+    uint32_t prev = __shfl_up_sync(0xffffffffu, word >> 31, 1);
+    if (lane == 0) prev = sub == lo ? word & 1u : tail;          // the chunk's first element: as if it went on
+    tail = __shfl_sync(0xffffffffu, word >> 31, 31);
+    if (sub == lo) ends |= __shfl_sync(0xffffffffu, word, 0) & 1u ? kFirstYes : 0;
+    const int valid = left - 32 * lane;
+    uint32_t starts = word ^ (word << 1 | prev);
+    if (valid < 32) starts &= valid <= 0 ? 0u : (1u << valid) - 1u;
+    st += __popc(starts);
+    if (starts) last = (int)(sub + 32 * lane + 31 - __clz(starts));
+    if (sub + CX_SUBTILE >= hi) {
+      const int end = left - 1;
+      ends |= (__shfl_sync(0xffffffffu, word, end >> 5) >> (end & 31)) & 1u ? kLastYes : 0;
+    }
   }
+  st = __reduce_add_sync(0xffffffffu, st);
+  last = __reduce_max_sync(0xffffffffu, last);
   if (lane == 0) {
-    s_chunk[w] = ChunkTotals{nnz, st, last, first};
+    s_chunk[w] = ChunkTotals{(int32_t)nnz, st, last, ends};
     p.chunk[chunk] = s_chunk[w];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     ChunkTotals t = s_chunk[0];
-    for (int j = 1; j < kWarps; ++j) { t.nnz += s_chunk[j].nnz; t.starts += s_chunk[j].starts; t.last = max(t.last, s_chunk[j].last); }
+    for (int j = 1; j < kWarps; ++j) t = append(t, s_chunk[j], (chunk + j) * p.subs * CX_SUBTILE);
     p.cta[blockIdx.x] = t;
+    if (blockIdx.x == 0) p.meta->first_yes = p.n > 0 && (t.ends & kFirstYes) ? 1 : 0;
   }
 }
 
-template <typename T>
+// Bound by latency: totals, words, then the stores of the payload (2^22 elements at 10 %: 4.7 MB).
 __global__ void __launch_bounds__(kThreads, kSendPerSm) rle_emit_kernel(const __grid_constant__ SendParams p) {
-  __shared__ float s_val[kWarps][kSeg];
-  __shared__ int s_start[kWarps][kSeg];
+  __shared__ uint16_t s_start[kWarps][CX_SUBTILE];
   __shared__ int s_pre[kWarps][5];
+  __shared__ ChunkTotals s_chunk[kWarps];
   __shared__ uint32_t s_lastblock;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int64_t chunk = (int64_t)blockIdx.x * kWarps + w;
-  const int64_t lo = chunk * p.segs * kSeg;
-  const int64_t hi = min(lo + (int64_t)p.segs * kSeg, p.n);
-  // resident early: the count kernel only reads, so the first segment may be fetched before it ends
-  float v[kPer];
-  load_values<T>(p, lo + lane * kPer, v);
+  const int64_t chunk = (int64_t)blockIdx.x * kWarps + w, span = (int64_t)p.subs * CX_SUBTILE;
+  const int64_t lo = chunk * span, hi = min(lo + span, p.n);
   cx::pdl_wait();
   const float thr = *p.thr;
-  // offsets of this chunk and the totals of all
+  // my chunk's first words, and the element in front of it
+  uint32_t word = lo < hi ? p.bits[(lo >> 5) + lane] : 0u;
+  uint32_t tail = lo > 0 && lo < hi ? p.bits[(lo >> 5) - 1] >> 31 : 0u;
+  // where this chunk's values and runs go, and the totals of all: CTA c's first element starts a run when the
+  // one in front of it differs
   int k0 = 0, q0 = 0, prev = -1, nnz_total = 0, nruns = 0;
   for (int c = tid; c < (int)gridDim.x; c += kThreads) {
     const ChunkTotals t = p.cta[c];
+    const bool edge = c == 0 ? p.n > 0 : ((p.cta[c - 1].ends & kLastYes) != 0) != ((t.ends & kFirstYes) != 0);
+    const int starts = t.starts + (edge ? 1 : 0);
     nnz_total += t.nnz;
-    nruns += t.starts;
-    if (c < (int)blockIdx.x) { k0 += t.nnz; q0 += t.starts; prev = max(prev, t.last); }
+    nruns += starts;
+    if (c < (int)blockIdx.x) {
+      k0 += t.nnz;
+      q0 += starts;
+      prev = max(prev, t.last >= 0 ? t.last : edge ? (int)(c * kWarps * span) : -1);
+    }
   }
-  if (tid < kWarps) {                      // the chunks of this CTA, one per thread
-    const ChunkTotals t = p.chunk[(int64_t)blockIdx.x * kWarps + tid];
-    s_start[0][4 * tid] = t.nnz; s_start[0][4 * tid + 1] = t.starts; s_start[0][4 * tid + 2] = t.last; s_start[0][4 * tid + 3] = t.first;
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    k0 += __shfl_xor_sync(0xffffffffu, k0, d);
-    q0 += __shfl_xor_sync(0xffffffffu, q0, d);
-    prev = max(prev, __shfl_xor_sync(0xffffffffu, prev, d));
-    nnz_total += __shfl_xor_sync(0xffffffffu, nnz_total, d);
-    nruns += __shfl_xor_sync(0xffffffffu, nruns, d);
-  }
+  if (tid < kWarps) s_chunk[tid] = p.chunk[(int64_t)blockIdx.x * kWarps + tid];
+  k0 = __reduce_add_sync(0xffffffffu, k0);
+  q0 = __reduce_add_sync(0xffffffffu, q0);
+  prev = __reduce_max_sync(0xffffffffu, prev);
+  nnz_total = __reduce_add_sync(0xffffffffu, nnz_total);
+  nruns = __reduce_add_sync(0xffffffffu, nruns);
   if (lane == 0) { s_pre[w][0] = k0; s_pre[w][1] = q0; s_pre[w][2] = prev; s_pre[w][3] = nnz_total; s_pre[w][4] = nruns; }
   __syncthreads();
   k0 = q0 = nnz_total = nruns = 0;
@@ -232,72 +228,65 @@ __global__ void __launch_bounds__(kThreads, kSendPerSm) rle_emit_kernel(const __
   for (int j = 0; j < kWarps; ++j) {
     k0 += s_pre[j][0]; q0 += s_pre[j][1]; prev = max(prev, s_pre[j][2]); nnz_total += s_pre[j][3]; nruns += s_pre[j][4];
   }
-  for (int j = 0; j < w; ++j) { k0 += s_start[0][4 * j]; q0 += s_start[0][4 * j + 1]; prev = max(prev, s_start[0][4 * j + 2]); }
-  const bool first_start = s_start[0][4 * w + 3] != 0;
-  __syncthreads();
+  {
+    // the chunks of this CTA in front of mine; the first one's first element is seen against the CTA before
+    uint32_t front = (uint32_t)__shfl_sync(0xffffffffu, tail, 0);
+    const int64_t first = (int64_t)blockIdx.x * kWarps * span;
+    if (w > 0) front = first > 0 ? p.bits[(first >> 5) - 1] >> 31 : 0u;
+    for (int j = 0; j < w; ++j) {
+      const ChunkTotals t = s_chunk[j];
+      if (t.ends & kEmpty) break;
+      const int64_t start = first + j * span;
+      const bool edge = start == 0 || (front != 0) != ((t.ends & kFirstYes) != 0);
+      k0 += t.nnz;
+      q0 += t.starts + (edge ? 1 : 0);
+      prev = t.last >= 0 ? t.last : edge ? (int)start : prev;
+      front = t.ends & kLastYes ? 1u : 0u;
+    }
+  }
+  const int mine = s_chunk[w].ends & kEmpty ? 0 : s_chunk[w].nnz;
   const size_t runs_off = 8 + 4 * (size_t)nnz_total + 8;
-  float* sv = s_val[w];
-  int* ss = s_start[w];
-  uint32_t tail = 0;           // the last element of the segment before
-  for (int64_t seg = lo; seg < hi; seg += kSeg) {
-    const int64_t base = seg + lane * kPer;
-    const int valid = valid_at(p.n, base);
-    const uint32_t yes = yes_mask(v, valid, thr);
-    const uint32_t edge = yes >> (kPer - 1);
-    uint32_t before = __shfl_up_sync(0xffffffffu, edge, 1);
-    if (lane == 0) before = tail;
-    tail = __shfl_sync(0xffffffffu, edge, 31);
-    uint32_t starts = start_mask(yes, valid, before != 0);
-    if (seg == lo && lane == 0) starts = (starts & ~1u) | (first_start ? 1u : 0u);
-    // one scan for both counts (at most 256 each)
-    const uint32_t mine = (uint32_t)__popc(yes) | ((uint32_t)__popc(starts) << 16);
-    uint32_t incl = mine;
+  // the chunk's values
+  for (int k = 0; k < p.tg.count; ++k) {
+    float* out = reinterpret_cast<float*>(reinterpret_cast<char*>(p.tg.ep[k].pairs) + 8) + k0;
+    const float* in = p.vals + lo;
+#pragma unroll 4
+    for (int i = lane; i < mine; i += 32) out[i] = in[i];
+  }
+  uint16_t* ss = s_start[w];
+  for (int64_t sub = lo; sub < hi; sub += CX_SUBTILE) {
+    const int valid = (int)min((int64_t)32, max((int64_t)0, hi - sub - 32 * lane));
+    uint32_t front = __shfl_up_sync(0xffffffffu, word >> 31, 1);
+    if (lane == 0) front = tail;
+    tail = __shfl_sync(0xffffffffu, word >> 31, 31);
+    uint32_t starts = word ^ (word << 1 | front);
+    if (sub == 0 && lane == 0) starts |= 1u;                    // element 0 always starts a run
+    if (valid < 32) starts &= (1u << valid) - 1u;
+    if (sub + CX_SUBTILE < hi) word = p.bits[(sub >> 5) + 32 + lane];      // under way during the stores
+    const uint32_t number = __popc(starts);
+    uint32_t incl = number;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += t;
     }
-    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t kv = (incl - mine) & 0xffffu, ks = (incl - mine) >> 16;
-#pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-      if ((yes >> e) & 1u) sv[kv++] = v[e];
-      if ((starts >> e) & 1u) ss[ks++] = (int)(base + e);
-    }
-    if (p.r && valid > 0) {
-      if (valid == kPer && (reinterpret_cast<uintptr_t>(p.r) & 15) == 0) {
-        float a[4], b[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          a[e] = (yes >> e) & 1u ? 0.f : v[e];
-          b[e] = (yes >> (4 + e)) & 1u ? 0.f : v[4 + e];
-        }
-        cx::store4(p.r + base, a);
-        cx::store4(p.r + base + 4, b);
-      } else {
-#pragma unroll
-        for (int e = 0; e < kPer; ++e) if (e < valid) p.r[base + e] = (yes >> e) & 1u ? 0.f : v[e];
-      }
-    }
-    if (seg + kSeg < hi) load_values<T>(p, base + kSeg, v);    // the next segment, in flight during the stores
+    const int ns = (int)__shfl_sync(0xffffffffu, incl, 31);
+    uint16_t* list = ss + (incl - number);
+    for (uint32_t bits = starts; bits; bits &= bits - 1) *list++ = (uint16_t)(32 * lane + __ffs(bits) - 1);
     __syncwarp();
-    const int nv = (int)(tot & 0xffffu), ns = (int)(tot >> 16);
     for (int k = 0; k < p.tg.count; ++k) {
-      char* pay = reinterpret_cast<char*>(p.tg.ep[k].pairs);
-      float* vals = reinterpret_cast<float*>(pay + 8) + k0;
-      for (int i = lane; i < nv; i += 32) vals[i] = sv[i];
-      int32_t* runs = reinterpret_cast<int32_t*>(pay + runs_off) + q0 - 1;   // start q closes run q - 1
+      // start q closes run q - 1
+      int32_t* runs = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(p.tg.ep[k].pairs) + runs_off) + q0 - 1;
       for (int i = lane; i < ns; i += 32)
-        if (q0 + i > 0) runs[i] = ss[i] - (i ? ss[i - 1] : prev);
+        if (q0 + i > 0) runs[i] = i ? (int)ss[i] - (int)ss[i - 1] : (int)(sub + ss[0] - prev);
     }
-    if (ns) prev = ss[ns - 1];
-    k0 += nv;
+    if (ns) prev = (int)(sub + ss[ns - 1]);
     q0 += ns;
     __syncwarp();
   }
   if (lo < hi && hi == p.n && lane < p.tg.count)     // the warp that holds the last element closes the last run
     reinterpret_cast<int32_t*>(reinterpret_cast<char*>(p.tg.ep[lane].pairs) + runs_off)[q0 - 1] = (int)(p.n - prev);
-  __syncthreads();       // one thread's trigger counts for its CTA: every warp has read its chunk of g
+  __syncthreads();
   cx::pdl_trigger();
   if (!cx::cta_arrive(&p.meta->done, gridDim.x, &s_lastblock)) return;
   if (tid < p.tg.count) {
@@ -349,34 +338,40 @@ __device__ __forceinline__ int64_t blocks_per_group(int64_t nruns, int groups) {
 }
 
 __global__ void __launch_bounds__(kThreads) rle_index_kernel(const __grid_constant__ RecvParams p) {
-  __shared__ int s_state;
+  __shared__ int s_state, s_first;
+  __shared__ int64_t s_nnz, s_nruns;
   __shared__ int s_bad;
   __shared__ long long s_sum[kWarps][2];
   cx::pdl_trigger();
   if (p.front_wait) cx::pdl_wait();
   if (threadIdx.x == 0) {
-    int st = 0;
+    int st = 0, first = 0;
+    int64_t nnz = 0, nruns = 0;
     if (!cx::wait_seq(&p.src.hdr->seq, p.expect_seq, p.timeout_ns)) st = CX_ST_TIMEOUT;
-    else if (__ldcg(&p.src.hdr->kind) != CX_KIND_RLE || (int64_t)__ldcg(&p.src.hdr->n) != p.n) st = CX_ST_BAD_HEADER;
+    if (!st) {
+      // one round trip for the header and the first words of the payload (there is room for them in any slot)
+      const int32_t* pay = reinterpret_cast<const int32_t*>(p.src.pairs);
+      const uint32_t kind = __ldcg(&p.src.hdr->kind), hn = __ldcg(&p.src.hdr->n);
+      const int32_t pn = __ldcg(pay);
+      nnz = __ldcg(pay + 1);
+      if (kind != CX_KIND_RLE || (int64_t)hn != p.n) st = CX_ST_BAD_HEADER;
+      else if ((int64_t)pn != p.n || nnz < 0 || nnz > p.n || 16 + 4 * nnz > p.slot_bytes) st = CX_ST_BAD_HEADER;
+      if (!st) {
+        const int32_t* rh = reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(p.src.pairs) + 8 + 4 * nnz);
+        nruns = __ldcg(rh);
+        first = __ldcg(rh + 1) != 0;
+        if (nruns < 0 || nruns > p.n + 1 || 16 + 4 * nnz + 4 * nruns > p.slot_bytes) st = CX_ST_BAD_HEADER;
+      }
+    }
     s_state = st;
+    s_first = first;
+    s_nnz = nnz;
+    s_nruns = nruns;
     s_bad = 0;
   }
   __syncthreads();
-  int st = s_state;
-  const int32_t* pay = reinterpret_cast<const int32_t*>(p.src.pairs);
-  int64_t nnz = 0, nruns = 0;
-  int first = 0;
-  if (!st) {
-    nnz = __ldcg(pay + 1);
-    if ((int64_t)__ldcg(pay) != p.n || nnz < 0 || nnz > p.n || 16 + 4 * nnz > p.slot_bytes) st = CX_ST_BAD_HEADER;
-  }
-  const int32_t* rh = nullptr;
-  if (!st) {
-    rh = reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(p.src.pairs) + 8 + 4 * nnz);
-    nruns = __ldcg(rh);
-    first = __ldcg(rh + 1) != 0;
-    if (nruns < 0 || nruns > p.n + 1 || 16 + 4 * nnz + 4 * nruns > p.slot_bytes) st = CX_ST_BAD_HEADER;
-  }
+  const int st = s_state, first = s_first;
+  const int64_t nnz = s_nnz, nruns = s_nruns;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (st && p.status) atomicOr(p.status, (uint32_t)st);
     p.meta->nnz = (int32_t)nnz;
@@ -387,7 +382,7 @@ __global__ void __launch_bounds__(kThreads) rle_index_kernel(const __grid_consta
   if (threadIdx.x == 0) p.group_bad[blockIdx.x] = st ? 1 : 0;
   if (!st) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t* runs = rh + 2;
+    const int32_t* runs = reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(p.src.pairs) + 16 + 4 * nnz);
     const int64_t nblocks = (nruns + kRunBlock - 1) / kRunBlock;
     const int64_t bpg = blocks_per_group(nruns, p.groups);
     const int64_t b0 = (int64_t)blockIdx.x * bpg, b1 = min(b0 + bpg, nblocks);
@@ -461,20 +456,29 @@ __device__ __forceinline__ V block_prefix(V x, V& tot, V* sm) {
   return pre + inc - x;
 }
 
-// Bound by the output (read and written for `add`).  Looking every output's run up by bisection in
-// the scanned block took 40 us for 2^22 elements at top-k 10 %; the mask needs one shared-memory
-// atomic per run and two shared-memory reads per four outputs.
+// Bound by the chain of dependent loads in front of the output, then by the output (read and written for
+// `add`).  Looking every output's run up by bisection in the scanned block took 40 us for 2^22 elements at
+// top-k 10 %, a mask with one shared-memory atomic per run and four outputs per thread 17 us.  Here two
+// blocks of runs are taken at a time (a window of 8192 outputs mostly needs no more), a thread's starts go
+// to the mask word by word, and a lane writes one bit of every word, which it gets by shuffles.
 __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_constant__ RecvParams p) {
   __shared__ long long s_l[kWarps];
   __shared__ int s_a[kWarps], s_b[kWarps];
   __shared__ int s_pick[3];
-  __shared__ uint32_t s_mask[kThreads];    // run starts of the window, then its selected outputs
-  __shared__ int s_base[kThreads];         // index of the word's first value
+  __shared__ uint32_t s_mask[kThreads];    // run starts of the window
+  // the window of `out` starts its way to L2 while the index is made
+  if (p.add) {
+    const int64_t i = (int64_t)blockIdx.x * p.per_cta + 32 * threadIdx.x;
+    if (i < p.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.out + i));
+  }
   cx::pdl_wait();
   cx::pdl_trigger();
-  if (!p.meta->ok) return;
-  const int nnz = p.meta->nnz, nruns = p.meta->nruns, first = p.meta->first_yes;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const bool have = tid < p.groups;
+  const int ok = p.meta->ok, nnz = p.meta->nnz, nruns = p.meta->nruns, first = p.meta->first_yes;
+  const RunSums g = have ? p.group[tid] : RunSums{0, 0};
+  const int gbad = have ? p.group_bad[tid] : 0;
+  if (!ok) return;
   const int64_t e0 = (int64_t)blockIdx.x * p.per_cta;
   const int64_t e1 = min(e0 + p.per_cta, p.n);
   // every CTA checks the whole payload before any of them writes; group g belongs to thread g
@@ -482,9 +486,6 @@ __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_co
   int at = 0, at_yes = 0;                  // elements and selected elements before block `blk`
   const int64_t nblocks = ((int64_t)nruns + kRunBlock - 1) / kRunBlock;
   {
-    const bool have = tid < p.groups;
-    const RunSums g = have ? p.group[tid] : RunSums{0, 0};
-    const int gbad = have ? p.group_bad[tid] : 0;
     long long total;
     int total_yes;
     const long long gstart = block_prefix<long long>(g.len, total, s_l);
@@ -515,46 +516,51 @@ __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_co
   }
   const int32_t* runs = reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(p.src.pairs) + 16 + 4 * (int64_t)nnz);
   const float* vals = reinterpret_cast<const float*>(reinterpret_cast<const char*>(p.src.pairs) + 8);
-  const bool vec = (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
   int vbase = -1;                          // index of the first value at or behind the window's start
   for (int64_t w0 = e0; w0 < e1; w0 += kWindow) {
     const int64_t w1 = min(w0 + kWindow, e1);
     s_mask[tid] = 0;
-    // blocks of runs that reach into the window; a run that began earlier counts at its first bit
+    // runs that reach into the window, two blocks at a time; a run that began earlier counts at its first bit
     for (;;) {
-      int len[4], mine = 0, part = 0;
+      int len[kRunsEach], mine = 0, part = 0;
+      const int64_t q0 = blk * kRunBlock + kRunsEach * tid;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int64_t q = blk * kRunBlock + 4 * tid + k;
-        len[k] = q < nruns ? runs[q] : 0;
+      for (int k = 0; k < kRunsEach; ++k) {
+        len[k] = q0 + k < nruns ? runs[q0 + k] : 0;
         mine += len[k];
       }
       int tot;
       int pos = at + block_prefix<int>(mine, tot, s_a);
+      uint32_t to = 0, flips = 0;          // starts of one word of the mask, before they go there together
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (blk * kRunBlock + 4 * tid + k < nruns && pos < w1) {
-          const int bit = pos > w0 ? (int)(pos - w0) : 0;
-          atomicXor(&s_mask[bit >> 5], 1u << (bit & 31));
+      for (int k = 0; k < kRunsEach; ++k) {
+        if (q0 + k < nruns && pos < w1) {
+          const uint32_t bit = pos > w0 ? (uint32_t)(pos - w0) : 0u;
+          if (bit >> 5 != to) {
+            if (flips) atomicXor(&s_mask[to], flips);
+            to = bit >> 5;
+            flips = 0;
+          }
+          flips ^= 1u << (bit & 31);
           const bool yes = ((k & 1) == 0) == (first != 0);
           if (yes && pos < w0) part += (int)(min((int64_t)pos + len[k], w0) - pos);
         }
         pos += len[k];
       }
-      if (vbase < 0) {                     // once per CTA: values of this block in front of the window
+      if (flips) atomicXor(&s_mask[to], flips);
+      if (vbase < 0) {                     // once per CTA: values of these runs in front of the window
         int before;
         block_prefix<int>(part, before, s_b);
         vbase = at_yes + before;
       }
-      if ((int64_t)at + tot >= w1 || blk + 1 >= nblocks) break;
+      if ((int64_t)at + tot >= w1 || blk + 2 >= nblocks) break;
       at += tot;
-      ++blk;
+      blk += 2;
       __syncthreads();                     // s_a is written again
     }
     __syncthreads();
     // word by word: parity of the starts up to every bit, the selected bits, and their number before
-    const uint32_t flips = s_mask[tid];
-    uint32_t x = flips;
+    uint32_t x = s_mask[tid];
     x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16;
     const uint32_t odd = __ballot_sync(0xffffffffu, x >> 31);
     if (lane == 0) s_b[w] = __popc(odd) & 1;
@@ -567,40 +573,30 @@ __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_co
     if (left < 32) x &= left <= 0 ? 0u : (1u << left) - 1u;
     int total;
     const int mybase = vbase + block_prefix<int>(__popc(x), total, s_a);
-    s_mask[tid] = x;
-    s_base[tid] = mybase;
     vbase += total;
-    __syncthreads();
-#pragma unroll 4
-    for (int it = 0; it < kWindow / (4 * kThreads); ++it) {
-      const int o = it * 4 * kThreads + 4 * tid;
-      const int64_t i0 = w0 + o;
-      if (i0 >= w1) continue;
-      const uint32_t word = s_mask[o >> 5];
-      const uint32_t yes = (word >> (o & 31)) & 0xfu;
-      if (p.add && yes == 0) continue;
-      int k = s_base[o >> 5] + __popc(word & ((1u << (o & 31)) - 1u));
-      float y[4] = {0.f, 0.f, 0.f, 0.f};
+    // lane l writes bit l of every word of its warp
+    const int64_t i0 = w0 + 32 * (tid & ~31) + lane;
+    const uint32_t below = (1u << lane) - 1u;
+#pragma unroll 1
+    for (int j0 = 0; j0 < 32; j0 += kRowsOut) {
+      float y[kRowsOut], z[kRowsOut];
+      uint32_t yes = 0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) if ((yes >> e) & 1u) y[e] = vals[k++];
-      if (vec && i0 + 4 <= w1) {
-        if (p.add) {
-          float z[4];
-          cx::load4(p.out + i0, z);
+      for (int j = 0; j < kRowsOut; ++j) {
+        const uint32_t word = __shfl_sync(0xffffffffu, x, j0 + j);
+        const int k = __shfl_sync(0xffffffffu, mybase, j0 + j) + __popc(word & below);
+        const bool sel = (word >> lane) & 1u;
+        yes |= (sel ? 1u : 0u) << j;
+        y[j] = sel ? vals[k] : 0.f;
+        z[j] = sel && p.add ? p.out[i0 + 32 * (j0 + j)] : 0.f;
+      }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] = (yes >> e) & 1u ? z[e] + y[e] : z[e];
-        }
-        cx::store4(p.out + i0, y);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (i0 + e >= w1) continue;
-          if ((yes >> e) & 1u) p.out[i0 + e] = p.add ? p.out[i0 + e] + y[e] : y[e];
-          else if (!p.add) p.out[i0 + e] = 0.f;
-        }
+      for (int j = 0; j < kRowsOut; ++j) {
+        const int64_t i = i0 + 32 * (j0 + j);
+        if (p.add ? ((yes >> j) & 1u) != 0 : i < w1) p.out[i] = p.add ? z[j] + y[j] : y[j];
       }
     }
-    __syncthreads();
+    if (w0 + kWindow < e1) __syncthreads();          // s_a is written again
   }
 }
 
@@ -608,12 +604,29 @@ __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_co
 
 int64_t cx_rle_slot_bytes(int64_t n) { return (16 + 8 * n + 15) / 16 * 16; }
 
-int64_t cx_rle_workspace_bytes(int64_t n) {
-  const int64_t send = 256 + kMaxSend * (1 + kWarps) * (int64_t)sizeof(ChunkTotals);
+static int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+static int64_t sub_tiles(int64_t n) { return (n + CX_SUBTILE - 1) / CX_SUBTILE; }
+constexpr int64_t kSendFixed = 256 + kMaxSend * (1 + kWarps) * (int64_t)sizeof(ChunkTotals);
+static_assert(kSendFixed % 256 == 0, "the words behind the totals are aligned");
+
+int64_t cx_rle_recv_workspace_bytes(int64_t n) {
   const int64_t blocks = (n + 1 + kRunBlock - 1) / kRunBlock;
-  const int64_t recv = 256 + kGroups * (int64_t)(sizeof(RunSums) + sizeof(int32_t)) + blocks * (int64_t)sizeof(RunSums);
-  return ((send > recv ? send : recv) + 255) / 256 * 256;
+  return align256(256 + kGroups * (int64_t)(sizeof(RunSums) + sizeof(int32_t)) + blocks * (int64_t)sizeof(RunSums));
 }
+int64_t cx_rle_workspace_bytes(int64_t n) {
+  const int64_t send = align256(kSendFixed + sub_tiles(n) * 128 + 4 * n), recv = cx_rle_recv_workspace_bytes(n);
+  return send > recv ? send : recv;
+}
+
+namespace {
+template <typename T>
+void launch_send(const SendParams& p, int grid, cudaStream_t s) {
+  if (p.g && p.r) cx_launch_pdl(rle_scan_kernel<T, true, true>, grid, kThreads, 0, s, p, false);
+  else if (p.r) cx_launch_pdl(rle_scan_kernel<T, false, true>, grid, kThreads, 0, s, p, false);
+  else cx_launch_pdl(rle_scan_kernel<T, true, false>, grid, kThreads, 0, s, p, false);
+  cx_launch_pdl(rle_emit_kernel, grid, kThreads, 0, s, p, false);
+}
+}  // namespace
 
 int cx_rle_send_cuda(int gdtype, const void* g, float* r, int64_t n, const float* thr,
                      int64_t slot_bytes, uint64_t seq, const CxTargets* tg, void* workspace,
@@ -625,30 +638,23 @@ int cx_rle_send_cuda(int gdtype, const void* g, float* r, int64_t n, const float
   if (ws_bytes < cx_rle_workspace_bytes(n)) return cx_set_error("cx_rle_send: workspace too small", 0);
   SendParams p;
   p.g = g; p.r = r; p.n = n; p.thr = thr; p.seq = seq; p.tg = *tg; p.src_rank = src_rank;
-  // one chunk of whole segments per warp, at most one wave of CTAs
-  const int64_t nsegs = n > 0 ? (n + kSeg - 1) / kSeg : 1;
+  // one chunk of whole sub-tiles per warp, at most one wave of CTAs
+  const int64_t nsub = n > 0 ? sub_tiles(n) : 1;
   int64_t wave = (int64_t)cx_sm_count() * kSendPerSm;
   if (wave > kMaxSend) wave = kMaxSend;
-  p.segs = (int)((nsegs + wave * kWarps - 1) / (wave * kWarps));
-  const int grid = (int)((nsegs + (int64_t)p.segs * kWarps - 1) / ((int64_t)p.segs * kWarps));
+  p.subs = (int)((nsub + wave * kWarps - 1) / (wave * kWarps));
+  const int grid = (int)((nsub + (int64_t)p.subs * kWarps - 1) / ((int64_t)p.subs * kWarps));
   char* ws = reinterpret_cast<char*>(workspace);
   p.meta = reinterpret_cast<RleMeta*>(ws);
   p.cta = reinterpret_cast<ChunkTotals*>(ws + 256);
   p.chunk = p.cta + kMaxSend;
+  p.bits = reinterpret_cast<uint32_t*>(ws + kSendFixed);
+  p.vals = reinterpret_cast<float*>(p.bits + 32 * sub_tiles(n));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   switch (gdtype) {
-    case CX_F32:
-      cx_launch_pdl(rle_count_kernel<float>, grid, kThreads, 0, s, p, false);
-      cx_launch_pdl(rle_emit_kernel<float>, grid, kThreads, 0, s, p, false);
-      break;
-    case CX_BF16:
-      cx_launch_pdl(rle_count_kernel<__nv_bfloat16>, grid, kThreads, 0, s, p, false);
-      cx_launch_pdl(rle_emit_kernel<__nv_bfloat16>, grid, kThreads, 0, s, p, false);
-      break;
-    case CX_F16:
-      cx_launch_pdl(rle_count_kernel<__half>, grid, kThreads, 0, s, p, false);
-      cx_launch_pdl(rle_emit_kernel<__half>, grid, kThreads, 0, s, p, false);
-      break;
+    case CX_F32: launch_send<float>(p, grid, s); break;
+    case CX_BF16: launch_send<__nv_bfloat16>(p, grid, s); break;
+    case CX_F16: launch_send<__half>(p, grid, s); break;
     default: return cx_set_error("cx_rle_send: unsupported dtype on CUDA", 0);
   }
   cx_note_stream(stream, false);
@@ -661,7 +667,7 @@ int cx_rle_recv_cuda(const CxEndpoint* src, uint64_t expect_seq, float* out, int
                      int64_t slot_bytes, void* workspace, int64_t ws_bytes, uint32_t* status,
                      uint64_t timeout_ns, void* stream) {
   if (n < 0 || n > 0x7fffffffLL) return cx_set_error("cx_rle_recv: n out of range", 0);
-  if (ws_bytes < cx_rle_workspace_bytes(n)) return cx_set_error("cx_rle_recv: workspace too small", 0);
+  if (ws_bytes < cx_rle_recv_workspace_bytes(n)) return cx_set_error("cx_rle_recv: workspace too small", 0);
   RecvParams p;
   p.src = *src; p.expect_seq = expect_seq; p.out = out; p.n = n; p.slot_bytes = slot_bytes;
   p.add = add; p.status = status; p.timeout_ns = timeout_ns;

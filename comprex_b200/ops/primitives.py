@@ -266,7 +266,8 @@ class RleCodec:
         self.ws_bytes = int(env.lib.cx_rle_workspace_bytes(n))
         self.slots = [DenseSlot.create(env, self.slot_bytes) for _ in range(2)]
         self.tx_ws = env.scratch(self.ws_bytes)
-        self.rx_ws = env.scratch(self.ws_bytes)
+        self.rx_ws_bytes = int(env.lib.cx_rle_recv_workspace_bytes(n))
+        self.rx_ws = env.scratch(self.rx_ws_bytes)
 
     def send(self, g, r, thr_cell: torch.Tensor, seq: int, dest: int) -> None:
         """Encode ``r + g`` at the threshold in ``thr_cell`` into rank ``dest``'s slot."""
@@ -284,7 +285,7 @@ class RleCodec:
             raise ComprexError("RLE decode needs a float32 vector of the connection's size")
         ep = self.slots[seq & 1].endpoint(env)
         _lib.check(env.lib.cx_rle_recv(env.dev, C.byref(ep), seq, out.data_ptr(), self.n, int(add), self.slot_bytes,
-                                       self.rx_ws.data_ptr(), self.ws_bytes, status.dev_ptr, env.timeout_ns,
+                                       self.rx_ws.data_ptr(), self.rx_ws_bytes, status.dev_ptr, env.timeout_ns,
                                        _lib.stream_ptr(env.device)), "cx_rle_recv")
 
 

@@ -811,6 +811,42 @@ def test_rle_chunks_and_run_blocks(n, kind):
     world.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1023, 1024, 1025, 8 * 1024 - 1, 8 * 1024 + 1, 4736 * 1024 + 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", ["edges", "runs", "none"])
+def test_rle_run_starts_at_chunk_edges(n, dtype, shape):
+    """Runs that begin, end or go on where a row, a sub-tile, a warp's chunk or a CTA's chunks meet (the
+    element in front decides), views at odd addresses, with and without a residual: payload bytes of the
+    host codec."""
+    world = cx.LoopbackWorld(2, device="cuda", timeout_ms=2000)
+    e0, e1 = world.envs
+    codecs = [P.RleCodec(e, n) for e in world.envs]
+    at = torch.arange(n)
+    keep = {"edges": (at % 32 == 31) | (at % 1024 == 0) | (at % 8192 == 8191), "runs": (at // 1024) % 2 == 1,
+            "none": torch.zeros(n, dtype=torch.bool)}[shape]
+    g = torch.where(keep, torch.full((n,), 2.0), torch.full((n,), 0.25)).to(dtype)
+    cell = torch.full((1,), 1.0, dtype=torch.float32, device="cuda")
+    status = e1.new_status("t")
+    for seq, with_r in ((1, True), (2, False)):
+        gd = torch.zeros(n + 1, dtype=dtype, device="cuda")[1:].copy_(g)
+        r = torch.zeros(n + 1, device="cuda")[1:].fill_(0.125) if with_r else None
+        codecs[0].send(gd, r, cell, seq, 1)
+        out = torch.full((n + 1,), 9.0, device="cuda")[1:]
+        codecs[1].recv(out, seq, False, status)
+        e1.flush()
+        assert status.value == 0
+        rh = torch.full((n,), 0.125) if with_r else None
+        expect = cx.CompressorRLE.encode(g.float(), rh, 1.0)
+        ep = codecs[1].slots[seq & 1].endpoint(e1)
+        assert e1.read_header(ep.hdr).bytes == len(expect) and e1.read_bytes(ep.pairs, len(expect)) == expect
+        v = g.float() + (0.125 if with_r else 0.0)
+        assert torch.equal(out.cpu(), torch.where(keep, v, torch.zeros(n)))
+        if with_r:
+            assert torch.equal(r.cpu(), rh)
+    world.close()
+
+
 def test_rle_fused_receive_rejects_corrupt_runs(world):
     """Host-side fault injection: run lengths that do not add up to n set BAD_HEADER and leave
     the output untouched; a payload that never arrives times out with a status."""
