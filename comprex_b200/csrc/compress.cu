@@ -144,10 +144,32 @@ __device__ __forceinline__ void load_subtile(const T* __restrict__ gl, const flo
   }
 }
 
+// The threshold where it is first needed: behind the wait for the kernel in front, which so covers the loads
+// ahead of it (that kernel only reads).  Nothing may be stored before get().
+struct LateThreshold {
+  const float* cell;
+  uint32_t chain;
+  bool have;
+  float thr;
+  __device__ __forceinline__ float get() {
+    if (!have) {
+      if (!(chain & CX_CHAINED)) cx::pdl_wait();
+      if (chain & CX_CHAIN_NEXT) cx::pdl_trigger();
+      thr = *reinterpret_cast<const volatile float*>(cell);
+      have = true;
+    }
+    return thr;
+  }
+};
+struct KnownThreshold {
+  float thr;
+  __device__ __forceinline__ float get() const { return thr; }
+};
+
 // The same for a folded input: up, mu, coef are the sub-tile's momentum and factors.
-template <typename T, Input IN>
+template <typename T, Input IN, typename Thr>
 __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, const float* __restrict__ rl, float* __restrict__ up,
-                                                  const float mu, const float coef, const int lane, float (&v)[kChunks][4]) {
+                                                  const float mu, const float coef, const int lane, float (&v)[kChunks][4], Thr& late) {
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) cx::load4(rl + lane * 4 + c * 128, v[c]);
   // all loads of a group are issued before its first store: the compiler must not move them across
@@ -161,6 +183,7 @@ __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, cons
       x[c] = cx::Raw4<T>::load(gl + lane * 4 + (c0 + c) * 128);
       if (IN == kFoldMom) cx::load4(up + lane * 4 + (c0 + c) * 128, y[c]);
     }
+    if (IN != kFold && c0 == 0) late.get();      // loads only before, stores from here on
 #pragma unroll
     for (int c = 0; c < kGroup; ++c) {
       float t[4];
@@ -297,9 +320,9 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
 // odd offsets) or folded from several tensors: element 32 j + lane is lane's j-th, kept in a register
 // from the load to the write-back, survivors ranked with warp ballots.  No assumption about alignment
 // or length.  (Two passes of dependent single loads made a vector of 44 k elements take 13 us.)
-template <typename T, bool HAS_G, bool HAS_R, bool MC, Input IN = kPlain>
+template <typename T, bool HAS_G, bool HAS_R, bool MC, Input IN = kPlain, typename Thr = KnownThreshold>
 __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, const uint32_t sub,
-                                                      const int lane, const float thr,
+                                                      const int lane, Thr&& late,
                                                       const T* __restrict__ g, float* __restrict__ r,
                                                       Tally& tally, const CxFold* f = nullptr) {
   constexpr int kEach = CX_SUBTILE / 32;
@@ -315,7 +338,7 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
   }
   if (IN != kPlain) {
     const cx::FoldBlock<T> blk = cx::fold_blocks<T>(*f, sub, lane);
-    constexpr int kGroup = 16;     // loads in flight: none of them moves across a store of the momentum
+    constexpr int kGroup = IN == kFoldMom ? 16 : 32;     // loads in flight: none of them moves across a store of the momentum
 #pragma unroll
     for (int j0 = 0; j0 < kEach; j0 += kGroup) {
       float x[kGroup], y[kGroup];
@@ -326,6 +349,7 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
         in |= (t ? 1u : 0u) << j;
         y[j] = IN == kFoldMom && t ? f->u[at + 32 * (j0 + j)] : 0.f;
       }
+      if (IN != kFold && j0 == 0) late.get();
 #pragma unroll
       for (int j = 0; j < kGroup; ++j) {
         const float t = f->mu * y[j] + __shfl_sync(0xffffffffu, blk.coef, (j0 + j) >> 1) * x[j];
@@ -334,6 +358,7 @@ __device__ __forceinline__ void compress_subtile_edge(const CompressParams& p, c
       }
     }
   }
+  const float thr = late.get();
   uint32_t mask = 0, count = 0;
 #pragma unroll
   for (int j = 0; j < kEach; ++j) {
@@ -525,7 +550,7 @@ compress_kernel(const __grid_constant__ CompressParams p) {
       loaded = false;
       emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage, v, tally);
     }
-    else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r, tally);
+    else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, KnownThreshold{thr}, g, r, tally);
   }
 
 #ifdef CX_COMPRESS_TRACE
@@ -548,13 +573,15 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   const CompressParams& p = q.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* __restrict__ r = p.r;
-  if (!(q.chain & CX_CHAINED)) cx::pdl_wait();
-  if (q.chain & CX_CHAIN_NEXT) cx::pdl_trigger();
-  const float thr = *p.thr;
+  LateThreshold late = {p.thr, q.chain, false, 0.f};
+  // In the small CTAs of a short vector, whose first sub-tiles are all there are, the loads go ahead of the wait
+  // for the threshold: descriptors, gradients and residual were complete before that kernel began (LeNet-5 step
+  // 20.2 -> 18.7 us).  Longer vectors gain nothing by it.
+  if (THREADS != kThreads || !p.early) late.get();
   Tally tally = {0, false};
   if (blockIdx.x < q.nborder_ctas) {
     for (uint32_t b = warp * q.nborder_ctas + blockIdx.x; b < (uint32_t)q.f.nborder; b += q.nborder_ctas * WARPS)
-      compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, thr, nullptr, r, tally, &q.f);
+      compress_subtile_edge<T, true, true, MC, IN>(p, (uint32_t)(q.f.border[b] - q.f.base / CX_SUBTILE), lane, late, nullptr, r, tally, &q.f);
   } else {
     const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * WARPS;
     uint32_t sub = (blockIdx.x - q.nborder_ctas) * WARPS + warp;
@@ -566,18 +593,18 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
       cx::FoldWhole<T> ahead = {nullptr, 0.f, 0};
       if (cur.kind == 2) {
         float v[kChunks][4];
-        load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v);
+        load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v, late);
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);     // on its way while this one is stored
-        emit_subtile<true, true, MC>(p, sub, lane, thr, r + off, s_stage[warp], v, tally);
+        emit_subtile<true, true, MC>(p, sub, lane, late.get(), r + off, s_stage[warp], v, tally);
       } else {
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);
-        if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, thr, nullptr, r, tally, &q.f);
+        if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, late, nullptr, r, tally, &q.f);
       }
       cur = ahead;
       sub = next;
     }
   }
-  compress_finish<WARPS>(p, tid, thr, false, tally);
+  compress_finish<WARPS>(p, tid, late.get(), false, tally);
   if (q.chain & CX_CHAINED) cx::pdl_wait();
 }
 
@@ -670,7 +697,7 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
     } else {
-      compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, thr, g, r, tally);
+      compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, KnownThreshold{thr}, g, r, tally);
     }
   }
   compress_finish<kBulkMaxWarps>(p, tid, thr, failed, tally);
