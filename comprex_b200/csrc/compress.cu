@@ -9,9 +9,9 @@
 //
 // Work is warp-granular and free of block-wide barriers: a warp owns one
 // 1024-element sub-tile at a time, loads it with 16-byte accesses (32
-// elements per lane, all loads in flight together), ranks the survivors with one warp scan, reserves room
-// for them in the pair list with ONE atomicAdd on a counter in this GPU's
-// memory, and stores them through a small shared staging buffer as coalesced
+// elements per lane, all loads in flight together), puts the sums into shared memory, ranks the survivors with
+// one warp scan, reserves room for them in the pair list with ONE atomicAdd on a counter in this GPU's
+// memory, and stores them, picked from shared memory by a list of their places, as coalesced
 // 8-byte (index, value) pairs straight into the receive
 // slots of up to CX_MAX_PEERS targets (peer GPUs' memory mapped over NVLink,
 // or local slots), or once through the switch's multicast mapping.  No warp
@@ -39,29 +39,24 @@ namespace {
 
 // 16 warps per SM: each lane keeps a whole sub-tile share of 32 values in registers with all its loads in
 // flight, which takes the 128 registers that leaves a thread (no spills without multicast; the folding
-// kernel spills 126 bytes a thread with fp32 momentum and 78 to 198 with 16-bit gradients).  Squeezing more warps onto an SM makes it spill and measured slower at every size (2^24 elements, 1 %: 55 us with 16 warps, 69 us
-// with 24), and so did an L2 prefetch of the warp's next sub-tile.
-#ifndef CX_COMPRESS_MIN_BLOCKS
-#define CX_COMPRESS_MIN_BLOCKS 2
-#endif
-#ifndef CX_COMPRESS_PREFETCH
-#define CX_COMPRESS_PREFETCH 0
-#endif
+// kernel spills 82 to 114 bytes a thread with fp32 momentum, 98 to 226 with 16-bit gradients, most of them at
+// tensor borders).  Squeezing more warps onto an SM makes it spill and measured slower at every size (2^24
+// elements, 1 %: 55 us with 16 warps, 69 us with 24), and so did an L2 prefetch of the warp's next sub-tile, and
+// loads of the next sub-tile issued while this one is stored (2^28 elements 633 -> 650 us).
 #ifndef CX_COMPRESS_BULK_DEFAULT
 #define CX_COMPRESS_BULK_DEFAULT 0
 #endif
 
 // Warps of one CTA wait for one another only at its end, so small CTAs spread a short vector over more
 // SMs and let each go as soon as it is done: 65 536 elements 12.3 us with 256 threads, 12.0 with 128 and
-// 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference, and the kernel that
-// folds (below) is slower with them.
-constexpr int kThreads = 64;
+// 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference.  The kernel that folds
+// (below) takes 128, whose staging leaves more of the SM's memory to the loads than that of 256.
+constexpr int kThreads = 64, kWarpsPerSm = 16;
 constexpr int kWarps = kThreads / 32;
-constexpr int kFoldThreads = 256;
-constexpr int kPerSm = CX_COMPRESS_MIN_BLOCKS * kFoldThreads / kThreads;
+constexpr int kFoldThreads = 128;
+constexpr int kPerSm = kWarpsPerSm / kWarps;
 constexpr int kFoldWarps = kFoldThreads / 32;
 constexpr int kChunks = CX_SUBTILE / 128;  // 128 elements = 32 lanes x 4
-constexpr int kStage = 128;                // pairs staged per warp and pass
 
 // -DCX_COMPRESS_TRACE: thread 0 of every CTA stamps %globaltimer at up to eight points of
 // compress_kernel (entry, before the loop, after the loop, after the arrival, and in the CTA that
@@ -197,23 +192,36 @@ __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, cons
   }
 }
 
+// A warp's survivors on their way out: the sub-tile's values, and the places of those that go, in order (more
+// than the list holds: one part of them after the other).
+constexpr uint32_t kList = 512;
+struct Stage {
+  float v[CX_SUBTILE];
+  uint16_t at[kList];
+};
+
 // Selection, compaction and write-back of a loaded sub-tile.  rs: the residual's sub-tile in global
 // memory, where the new residual goes.
+// A vector of one to three sub-tiles per warp is bound by this chain, not by memory: all warps walk through it
+// in step.  So the values go to shared memory first; a lane's survivors are then found by their bits (0.3 of 32 at
+// 1 %) instead of by 32 tests with a branch each, and the residual leaves before the reservation is back.
+// 2^16 / 2^20 elements 11.9 / 14.9 -> 11.4 / 14.3 us per exchange, 8 x 6.5 M 260 -> 250, 2^28 638 -> 633.
 template <bool HAS_G, bool HAS_R, bool MC>
 __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint32_t sub, const int lane, const float thr,
-                                             float* __restrict__ rs, CxPair* stage, float (&v)[kChunks][4],
+                                             float* __restrict__ rs, float* sv, uint16_t* sat, float (&v)[kChunks][4],
                                              Tally& tally) {
-  const int64_t sub_base = (int64_t)sub * CX_SUBTILE;
-  float* wp = rs + lane * 4;
-
-  // ---- classify: bit c*4+e of mask, strict '>' like the reference --------------
+  // ---- classify: bit c*4+e of mask, strict '>' like the reference; v becomes the new residual -------
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) cx::store4(sv + c * 128 + lane * 4, v[c]);
   uint32_t mask = 0;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const bool sel = fabsf(v[c][e]) > thr;
-      mask |= (sel ? 1u : 0u) << (4 * c + e);
+      if (fabsf(v[c][e]) > thr) {
+        mask |= 1u << (4 * c + e);
+        v[c][e] = 0.f;
+      }
     }
   }
 
@@ -226,17 +234,34 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
     if (lane >= d) incl += t;
   }
   const uint32_t count = __shfl_sync(0xffffffffu, incl, 31);
-  const uint32_t first = incl - mine;  // position of my first survivor inside the sub-tile
 
   // ---- reserve room in the pair list ----------------------------------------------
   // The list is cut into nregions equal regions with one counter each, neighbouring
   // sub-tiles use different regions: atomics on one address are serialised by the L2.
   const uint32_t region = sub & (p.nregions - 1);
   uint32_t base = 0;
-  if (count) {
-    if (lane == 0) base = atomicAdd(&p.ctr->region[region][0], count);
-    base = __shfl_sync(0xffffffffu, base, 0);
+  if (count && lane == 0) base = atomicAdd(&p.ctr->region[region][0], count);   // under way until it is asked for
+
+  // ---- residual: zero for every survivor; those that turn out not to fit are put back below ---------
+  if (HAS_R) {
+    float* wp = rs + lane * 4;
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      if (!HAS_G && ((mask >> (4 * c)) & 0xfu) == 0) continue;  // nothing changed in this vector
+      cx::store4(wp + c * 128, v[c]);
+    }
   }
+
+  // my survivors among the list's entries [w0, w0 + kList)
+  auto fill = [&](const uint32_t w0) {
+    uint32_t pos = incl - mine - w0;        // wraps below the window: fails the test
+    for (uint32_t bits = mask; bits; bits &= bits - 1, ++pos) {
+      const uint32_t b = __ffs(bits) - 1;
+      if (pos < kList) sat[pos] = (uint16_t)((b >> 2) * 128 + lane * 4 + (b & 3));
+    }
+  };
+  fill(0);
+  base = __shfl_sync(0xffffffffu, base, 0);
   const uint32_t emit = base >= p.region_size ? 0u : min(count, p.region_size - base);  // pairs that fit
   base += region * p.region_size;
   tally.found += count;
@@ -251,68 +276,32 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
       reinterpret_cast<uint2*>(p.tg.ep[lane].table)[sub] = entry;
     }
   }
+  __syncwarp();
 
-  // ---- stage in shared memory, store coalesced to every target ------------------------
-  const int32_t idx0 = (int32_t)sub_base + lane * 4;
-  for (uint32_t w0 = 0; w0 < emit; w0 += kStage) {   // one pass unless the sub-tile is dense
-    uint32_t pos = first - w0;                        // wraps below the window: fails the test
-#pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (mask & (1u << (4 * c + e))) {
-          if (pos < (uint32_t)kStage) {
-            CxPair pr;
-            pr.idx = idx0 + c * 128 + e;
-            pr.val = __float_as_uint(v[c][e]);
-            stage[pos] = pr;
-          }
-          ++pos;
-        }
-      }
-    }
-    __syncwarp();
-    const uint32_t lim = min((uint32_t)kStage, emit - w0);
-    if (MC) {
-      // one store per pair into the multicast mapping: the switch writes every target's slot
-      CxPair* mc = p.tg.ep[p.tg.count].pairs + base + w0;
-      for (uint32_t i = lane; i < lim; i += 32) {
-        const CxPair pr = stage[i];
-        cx::mm_st_b64(mc + i, make_uint2((uint32_t)pr.idx, pr.val));
-      }
-    } else {
-      for (uint32_t i = lane; i < lim; i += 32) {
-        const CxPair pr = stage[i];
+  // ---- coalesced to every target; what does not fit stays in the residual (the barrier above orders that
+  //      behind the other lanes' zeros) ------------------------
+  const int32_t sub_base = (int32_t)sub * CX_SUBTILE;
+  for (uint32_t w0 = 0;;) {
+    const uint32_t lim = min(count - w0, kList);
+    for (uint32_t i = lane; i < lim; i += 32) {
+      const uint32_t e = sat[i];
+      CxPair pr;
+      pr.idx = sub_base + (int32_t)e;
+      pr.val = __float_as_uint(sv[e]);
+      if (w0 + i >= emit) {
+        if (HAS_R) rs[e] = sv[e];
+      } else if (MC) {
+        // one store per pair into the multicast mapping: the switch writes every target's slot
+        cx::mm_st_b64(p.tg.ep[p.tg.count].pairs + base + w0 + i, make_uint2((uint32_t)pr.idx, pr.val));
+      } else {
         for (int k = 0; k < p.tg.count; ++k) p.tg.ep[k].pairs[base + w0 + i] = pr;
       }
     }
     __syncwarp();
-  }
-
-  // ---- residual: zero what was emitted, keep the rest ---------------------------------------
-  if (HAS_R) {
-    if (emit < count) {  // the slot is full: survivors from position emit on stay in the residual
-      uint32_t pos = first;
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (mask & (1u << (4 * c + e))) {
-            if (pos >= emit) mask &= ~(1u << (4 * c + e));
-            ++pos;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-      const uint32_t m = (mask >> (4 * c)) & 0xfu;
-      if (!HAS_G && m == 0) continue;  // nothing changed in this vector
-      float out[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) out[e] = (m & (1u << e)) ? 0.f : v[c][e];
-      cx::store4(wp + c * 128, out);
-    }
+    w0 += kList;
+    if (w0 >= count) break;                 // all of it, unless the sub-tile is dense
+    fill(w0);
+    __syncwarp();
   }
 }
 
@@ -497,7 +486,7 @@ __device__ __forceinline__ void compress_finish(const CompressParams& p, const i
 template <typename T, bool HAS_G, bool HAS_R, bool MC>
 __global__ void __launch_bounds__(kThreads, kPerSm)
 compress_kernel(const __grid_constant__ CompressParams p) {
-  __shared__ CxPair s_stage[kWarps][kStage];
+  __shared__ __align__(16) Stage s_stage[kWarps];
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -530,25 +519,15 @@ compress_kernel(const __grid_constant__ CompressParams p) {
   const float thr = *p.thr;
   Tally tally = {0, false};
   CX_TRACE(1);
-  CxPair* stage = s_stage[warp];
+  Stage& stage = s_stage[warp];
   const uint32_t nwarps = gridDim.x * kWarps;
 
   for (uint32_t sub = blockIdx.x * kWarps + warp; sub < p.nsub; sub += nwarps) {
-#if CX_COMPRESS_PREFETCH
-    // the warp's next sub-tile starts its way from DRAM to L2 now (one 128-byte line per lane
-    // and vector): its loads then find it there, without holding a register in the meantime
-    if ((uint64_t)sub + nwarps < nfull) {
-      const int64_t e0 = ((int64_t)sub + nwarps) * CX_SUBTILE;
-      if (HAS_R) asm volatile("prefetch.global.L2 [%0];" ::"l"(r + e0 + lane * 32));
-      if (HAS_G && lane * (128 / (int)sizeof(T)) < CX_SUBTILE)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(g + e0 + lane * (128 / (int)sizeof(T))));
-    }
-#endif
     if (sub < nfull) {
       const int64_t off = (int64_t)sub * CX_SUBTILE;
       if (!loaded) load_subtile<T, HAS_G, HAS_R>(g + off, r + off, lane, v);
       loaded = false;
-      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage, v, tally);
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage.v, stage.at, v, tally);
     }
     else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, KnownThreshold{thr}, g, r, tally);
   }
@@ -566,10 +545,10 @@ compress_kernel(const __grid_constant__ CompressParams p) {
 // 13.1 M bf16 gradients with momentum: 44 us for the fold and 34 us for the compression as two
 // kernels.
 template <typename T, bool MC, Input IN, int THREADS>
-__global__ void __launch_bounds__(THREADS, CX_COMPRESS_MIN_BLOCKS * kFoldThreads / THREADS)
+__global__ void __launch_bounds__(THREADS, kWarpsPerSm * 32 / THREADS)
 compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
   constexpr int WARPS = THREADS / 32;
-  __shared__ CxPair s_stage[WARPS][kStage];
+  __shared__ __align__(16) Stage s_stage[WARPS];
   const CompressParams& p = q.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* __restrict__ r = p.r;
@@ -595,7 +574,7 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
         float v[kChunks][4];
         load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v, late);
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);     // on its way while this one is stored
-        emit_subtile<true, true, MC>(p, sub, lane, late.get(), r + off, s_stage[warp], v, tally);
+        emit_subtile<true, true, MC>(p, sub, lane, late.get(), r + off, s_stage[warp].v, s_stage[warp].at, v, tally);
       } else {
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);
         if (cur.kind == 1) compress_subtile_edge<T, true, true, MC, IN>(p, sub, lane, late, nullptr, r, tally, &q.f);
@@ -623,6 +602,9 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
 #define CX_COMPRESS_BULK_STAGES 2
 #endif
 constexpr int kBulkMaxWarps = 16;
+// bytes per warp beside the stages: the list of survivors, and the sums where no stage holds 32-bit values
+template <typename T, bool HAS_R>
+__host__ __device__ constexpr uint32_t bulk_extra() { return 2 * kList + (HAS_R || sizeof(T) == 4 ? 0 : 4 * CX_SUBTILE); }
 
 template <typename T, bool HAS_G, bool HAS_R, bool MC, int STAGES>
 __global__ void __launch_bounds__(kBulkMaxWarps * 32, 1)
@@ -631,14 +613,14 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
   constexpr uint32_t kRB = HAS_R ? (uint32_t)(CX_SUBTILE * sizeof(float)) : 0u;
   constexpr uint32_t kGB = HAS_G ? (uint32_t)(CX_SUBTILE * sizeof(T)) : 0u;
   constexpr uint32_t kStageB = kRB + kGB;
-  constexpr uint32_t kWarpB = STAGES * kStageB + kStage * (uint32_t)sizeof(CxPair);
+  constexpr uint32_t kWarpB = STAGES * kStageB + bulk_extra<T, HAS_R>();
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const uint32_t nw = blockDim.x >> 5;
   unsigned char* mine = s_dyn + (size_t)warp * kWarpB;
-  CxPair* stage = reinterpret_cast<CxPair*>(mine + STAGES * kStageB);
+  uint16_t* list = reinterpret_cast<uint16_t*>(mine + STAGES * kStageB);
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_dyn + (size_t)nw * kWarpB) + warp * STAGES;
   if (lane == 0) {
 #pragma unroll
@@ -692,7 +674,9 @@ compress_bulk_kernel(const __grid_constant__ CompressParams p) {
       const unsigned char* src = mine + s * kStageB;
       float v[kChunks][4];
       load_subtile<T, HAS_G, HAS_R>(reinterpret_cast<const T*>(src + kRB), reinterpret_cast<const float*>(src), lane, v);
-      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + (size_t)sub * CX_SUBTILE, stage, v, tally);
+      // the sums go where the copy engine put the residual (or fp32 gradient), each lane's over its own
+      float* sums = reinterpret_cast<float*>(HAS_R || sizeof(T) == 4 ? mine + s * kStageB : mine + STAGES * kStageB + 2 * kList);
+      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + (size_t)sub * CX_SUBTILE, sums, list, v, tally);
       // this stage is handed back to the copy engine by a later issue()
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -749,7 +733,7 @@ template <typename T, bool HAS_G, bool HAS_R, bool MC>
 int launch_bulk_one(const CompressParams& p, cudaStream_t s) {
   constexpr int STAGES = CX_COMPRESS_BULK_STAGES;
   constexpr size_t kStageB = (HAS_R ? CX_SUBTILE * sizeof(float) : 0) + (HAS_G ? CX_SUBTILE * sizeof(T) : 0);
-  constexpr size_t kWarpB = STAGES * kStageB + kStage * sizeof(CxPair) + 8 * STAGES;
+  constexpr size_t kWarpB = STAGES * kStageB + bulk_extra<T, HAS_R>() + 8 * STAGES;
   constexpr size_t kBudget = 227 * 1024 - 1024;   // per SM, minus the static part and slack
   int nw = (int)(kBudget / kWarpB);
   if (nw > kBulkMaxWarps) nw = kBulkMaxWarps;
@@ -838,14 +822,13 @@ template <typename T, Input IN, int THREADS>
 void launch_fold_threads(const FoldCompressParams& q, cudaStream_t s) {
   FoldCompressParams p = q;
   int grid;
-  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, THREADS / 32, wave(CX_COMPRESS_MIN_BLOCKS * (kFoldThreads / THREADS)), &grid);
+  p.nborder_ctas = (uint32_t)cx_border_ctas(q.f, q.c.nsub, THREADS / 32, wave(kWarpsPerSm * 32 / THREADS), &grid);
   const bool capturing = q.c.seq_cell != nullptr;
   if (q.c.tg.pad & CX_TG_MULTICAST) cx_launch_pdl(compress_fold_kernel<T, true, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
   else cx_launch_pdl(compress_fold_kernel<T, false, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
 }
 
-// small CTAs for a vector too short for a large one on every SM (LeNet step 22.1 -> 21.8 us; the 13 M
-// element buckets of a ResNet-50 step are 0.6 us faster with the large ones)
+// small CTAs for a vector too short for a large one on every SM (LeNet step 22.1 -> 21.8 us)
 template <typename T, Input IN>
 void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
   if (q.c.nsub <= (uint32_t)(cx_sm_count() * kFoldWarps)) launch_fold_threads<T, IN, kThreads>(q, s);

@@ -882,6 +882,39 @@ def test_rle_fused_receive_rejects_corrupt_runs(world):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("count", [0, 1, 33, 511, 512, 513, 1023, 1024])
+@pytest.mark.parametrize("room", [1, 32, 511, 512, 513, 700, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_dense_subtiles_and_full_slots(count, room, dtype):
+    """One sub-tile with `count` survivors into a slot with room for `room`: around the length of the warp's
+    list, and cut off inside each of its parts.  What is stored and what stays add up to the vector, with
+    and without a gradient, and nothing else is touched."""
+    n = 1024
+    world = cx.LoopbackWorld(1, device="cuda", timeout_ms=2000)
+    e0 = world.envs[0]
+    cap, gen = room, torch.Generator().manual_seed(count)
+    big = torch.zeros(n, dtype=torch.bool)
+    big[torch.randperm(n, generator=gen)[:count]] = True
+    g = torch.where(big, 2.0 + torch.rand(n, generator=gen), 0.25 * torch.rand(n, generator=gen)).to(dtype)
+    comp = P.Compressor(e0, n)
+    for seq, with_g in ((1, True), (2, False)):
+        slot = P.SparseSlot.create(e0, n, cap)
+        r0 = 0.125 * torch.ones(n) if with_g else g.float()
+        v = g.float() + r0 if with_g else r0
+        r = r0.cuda()
+        comp.set_threshold(1.0)
+        comp.compress(g.cuda() if with_g else None, r, n, cap, seq, P.make_targets([slot.endpoint(e0)]))
+        e0.flush()
+        hdr, idx, val = read_pairs(e0, slot)[:3]
+        assert (hdr.nnz, hdr.nnz_found) == (min(count, cap), count)
+        sent = torch.zeros(n)
+        sent[idx.long()] = val
+        assert idx.unique().numel() == min(count, cap) and bool(big[idx.long()].all())
+        assert torch.equal(sent + r.cpu(), v) and bool((sent * r.cpu() == 0).all())
+    world.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 31, 1000, 1023, 8 * 1024, 8 * 1024 + 1, 100003, 296 * 8 * 1024, 296 * 8 * 1024 + 1])
 @pytest.mark.parametrize("ratio", [0.001, 0.01, 0.1, 0.7])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
