@@ -18,7 +18,8 @@
 // eighth of the sample and stores the keys through distributed shared memory into
 // the first CTA, which then selects alone.
 //
-// The selection is a chain of dependent block-wide steps, so it takes as few as the rank
+// Samples of up to 2048 elements have a kernel of their own (threshold_small_kernel).  The selection is a chain
+// of dependent block-wide steps, so it takes as few as the rank
 // allows (see select_cached).  Sampling rules ask for rank 9 unless the fraction is above 1 %.
 //
 // Several vectors (the buckets of an optimizer step) share one launch, one cluster each: the
@@ -306,6 +307,180 @@ __global__ void __launch_bounds__(kThreads) threshold_kernel(const __grid_consta
     __syncthreads();
   }
   if (tid == 0) *p.thr_out = __uint_as_float(prefix);
+}
+
+// ---- samples of up to 2048 elements ------------------------------------------------------------
+// All latency: the chain is the gather, then steps of the whole CTA.  256 threads hold the keys in registers,
+// up to eight each, with all their loads in flight: a barrier of 8 warps and a handful of them, where 32 warps
+// that keep the keys in shared memory spent half of the kernel in barriers (exchange of 2^16 / 2^20 elements
+// 11.4 / 14.1 -> 10.7 / 13.1 us, LeNet-5 step 18.7 -> 18.4).  A folded vector's dependent look-ups go side by side.
+constexpr int kSmallThreads = 256, kSmallEach = 8, kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallSample = kSmallThreads * kSmallEach;
+constexpr int kSmallRound = 4;       // samples of a thread whose loads go together
+
+// keys of samples tid, tid + 256, ... (kSmallRound of them from `first` on)
+template <typename T, bool FOLD>
+__device__ __forceinline__ void gather_small(const ThreshParams& p, int first, uint32_t (&k)[kSmallRound]) {
+  int64_t pos[kSmallRound];
+  float x[kSmallRound], y[kSmallRound];
+  bool in[kSmallRound];
+#pragma unroll
+  for (int u = 0; u < kSmallRound; ++u) {
+    const int i = first + u * kSmallThreads;
+    in[u] = i < p.samples;
+    pos[u] = in[u] ? sample_position(i, p.n, p.use_all, p.stepsize) : 0;
+    x[u] = p.r && in[u] ? p.r[pos[u]] : 0.f;
+    y[u] = 0.f;
+  }
+  if (FOLD) {
+    // cx::fold_at for all of them step by step, so that the steps' loads are in flight together
+    const CxFold& f = p.fold;
+    int seg[kSmallRound];
+    int64_t end[kSmallRound], off[kSmallRound];
+    float m[kSmallRound], coef[kSmallRound];
+    const T* g[kSmallRound];
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u) {
+      seg[u] = in[u] ? f.sub_seg[pos[u] / CX_SUBTILE] : f.nseg;
+      m[u] = in[u] && f.mu != 0.f ? f.u[pos[u]] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u) end[u] = seg[u] < f.nseg ? f.seg_end[seg[u]] : INT64_MAX;
+    for (bool again = true; again;) {
+      again = false;
+#pragma unroll
+      for (int u = 0; u < kSmallRound; ++u) {
+        if (end[u] <= f.base + pos[u]) {
+          ++seg[u];
+          end[u] = seg[u] < f.nseg ? f.seg_end[seg[u]] : INT64_MAX;
+          again = true;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u) {
+      const bool t = seg[u] < f.nseg;
+      off[u] = t ? f.seg_off[seg[u]] : INT64_MAX;
+      g[u] = t ? reinterpret_cast<const T*>(f.seg_ptr[seg[u]]) : nullptr;
+      coef[u] = t ? f.coef[seg[u]] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u)       // (a gap between tensors: 0)
+      if (off[u] <= f.base + pos[u]) y[u] = f.mu * m[u] + coef[u] * cx::Elem<T>::to_f(g[u][f.base + pos[u] - off[u]]);
+  } else if (p.g) {
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u) if (in[u]) y[u] = cx::Elem<T>::to_f(reinterpret_cast<const T*>(p.g)[pos[u]]);
+  }
+#pragma unroll
+  for (int u = 0; u < kSmallRound; ++u) k[u] = in[u] ? __float_as_uint(fabsf(FOLD || p.g ? x[u] + y[u] : x[u])) : 0u;
+}
+
+template <typename T, bool FOLD, int NV>
+__global__ void __launch_bounds__(kSmallThreads) threshold_small_kernel(const __grid_constant__ ThreshBatch<NV> batch) {
+  __shared__ __align__(16) uint32_t s_max[kSmallRound * kSmallWarps];     // 32 disjoint parts of the sample
+  __shared__ uint32_t s_sum[2][kSmallWarps];
+  __shared__ uint32_t s_few[kSmallThreads];
+  __shared__ uint32_t s_left;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const ThreshParams& p = batch.v[NV == 1 ? 0 : blockIdx.x];
+  const int s = p.samples;
+  if (tid == 0) s_left = 0;
+  cx::pdl_wait();     // resident early: what the kernel in front wrote may be read from here on
+  uint32_t k[kSmallEach];
+  {
+    uint32_t a[kSmallRound], b[kSmallRound] = {0u, 0u, 0u, 0u};
+    gather_small<T, FOLD>(p, tid, a);
+    if (s > kSmallRound * kSmallThreads) gather_small<T, FOLD>(p, tid + kSmallRound * kSmallThreads, b);
+#pragma unroll
+    for (int u = 0; u < kSmallRound; ++u) {
+      k[u] = a[u];
+      k[kSmallRound + u] = b[u];
+      const uint32_t m = __reduce_max_sync(0xffffffffu, max(a[u], b[u]));
+      if (lane == 0) s_max[kSmallRound * w + u] = m;
+    }
+  }
+  // the compress kernel queued behind this one may start now: it loads what both only read, and waits
+  // for this grid to finish before it reads the threshold or writes the residual.  (Let in before the
+  // gather, its 20 MB of loads were in front of the sample's.)
+  cx::pdl_trigger();
+  __syncthreads();
+  const uint32_t mine = s_max[lane];
+  if (p.topk_pos <= 0) {
+    const uint32_t m = __reduce_max_sync(0xffffffffu, mine);
+    if (tid == 0) *p.thr_out = __uint_as_float(m) + 1.0f;
+    return;
+  }
+  const uint32_t rank = (uint32_t)p.topk_pos;
+  // keys in [lo, hi] are candidates, `above` keys are larger than those
+  uint32_t lo = 0, hi = 0x7fffffffu, above = 0;
+  bool few = false;
+  if (rank < 32) {
+    // the (rank + 1)-th largest of the parts' maxima: at least rank + 1 keys are as large.  Every warp for itself.
+    uint32_t gt = 0, ge = 0;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(s_max + j);
+      gt += (q.x > mine) + (q.y > mine) + (q.z > mine) + (q.w > mine);
+      ge += (q.x >= mine) + (q.y >= mine) + (q.z >= mine) + (q.w >= mine);
+    }
+    const uint32_t who = __ballot_sync(0xffffffffu, gt <= rank && rank < ge);
+    lo = __shfl_sync(0xffffffffu, mine, __ffs(who) - 1);
+    few = lo > 0;            // (0: fewer than rank + 1 parts hold anything)
+  }
+  for (int attempt = 0;; ++attempt) {
+    if (!few) {
+      // bisection over the bits: t is the largest value so far with more than `rank` keys at or above it
+      uint32_t t = 0, at_t = (uint32_t)s;
+      above = 0;
+      int bit = 30;
+      do {
+        const uint32_t c = t | (1u << bit);
+        uint32_t n = 0;
+#pragma unroll
+        for (int u = 0; u < kSmallEach; ++u) n += k[u] >= c ? 1u : 0u;
+        n = __reduce_add_sync(0xffffffffu, n);
+        uint32_t* sum = s_sum[bit & 1];           // (written again two rounds on, behind the other's barrier)
+        if (lane == 0) sum[w] = n;
+        __syncthreads();
+        n = 0;
+#pragma unroll
+        for (int j = 0; j < kSmallWarps; ++j) n += sum[j];
+        if (n > rank) { t = c; at_t = n; } else above = n;
+        --bit;
+      } while (bit >= 0 && at_t - above > 64);
+      if (bit < 0) {                              // all candidates are equal
+        if (tid == 0) *p.thr_out = __uint_as_float(t);
+        return;
+      }
+      lo = t;
+      hi = t | ((2u << bit) - 1u);
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallEach; ++u) {
+      if (k[u] >= lo && k[u] <= hi && (u * kSmallThreads + tid) < s) {
+        const uint32_t at = atomicAdd(&s_left, 1u);
+        if (at < (uint32_t)kSmallThreads) s_few[at] = k[u];
+      }
+    }
+    __syncthreads();
+    const uint32_t left = s_left;
+    if (left <= (uint32_t)kSmallThreads) {
+      if (tid < (int)left) {                      // every candidate counts the ones above it; equal ones write the same
+        const uint32_t key = s_few[tid];
+        uint32_t gt = above, ge = above;
+        for (uint32_t j = 0; j < left; ++j) {
+          gt += s_few[j] > key ? 1u : 0u;
+          ge += s_few[j] >= key ? 1u : 0u;
+        }
+        if (gt <= rank && rank < ge) *p.thr_out = __uint_as_float(key);
+      }
+      return;
+    }
+    __syncthreads();                              // many ties: bisect (at most 64 candidates, or all equal)
+    if (tid == 0) s_left = 0;
+    few = false;
+    __syncthreads();
+  }
 }
 
 // ---- exact selection over the whole vector, grid-wide ----------------------------------------
@@ -801,8 +976,10 @@ template <typename T, bool FOLD>
 int launch_sampled(const ThreshParams* v, int count, unsigned ncta, bool capturing, cudaStream_t s) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
+  bool small = true;
+  for (int i = 0; i < count; ++i) small &= v[i].samples <= kSmallSample;
   cfg.gridDim = dim3(ncta * (unsigned)count, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.blockDim = dim3(small ? kSmallThreads : kThreads, 1, 1);
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   unsigned na = 0;
@@ -824,11 +1001,11 @@ int launch_sampled(const ThreshParams* v, int count, unsigned ncta, bool capturi
   if (count == 1) {
     ThreshBatch<1> b;
     b.v[0] = v[0];
-    e = cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, 1>, b);
+    e = small ? cudaLaunchKernelEx(&cfg, threshold_small_kernel<T, FOLD, 1>, b) : cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, 1>, b);
   } else {
     ThreshBatch<kVectors> b;
     memcpy(b.v, v, sizeof(ThreshParams) * (size_t)count);
-    e = cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, kVectors>, b);
+    e = small ? cudaLaunchKernelEx(&cfg, threshold_small_kernel<T, FOLD, kVectors>, b) : cudaLaunchKernelEx(&cfg, threshold_kernel<T, FOLD, kVectors>, b);
   }
   if (e != cudaSuccess) return cx_set_error("threshold_kernel launch", (int)e);
   cx_note_stream(s, true);       // a sample larger than the cache is gathered again behind the trigger
@@ -855,7 +1032,7 @@ void sampled_params(ThreshParams& p, const void* g, const float* r, int64_t n, f
 }
 
 // a cluster of 8 CTAs gathers large samples (their keys must fit the first CTA's shared memory)
-unsigned cluster_for(const ThreshParams& p) { return (p.samples > 2048 && p.samples <= kSmemKeys) ? 8u : 1u; }
+unsigned cluster_for(const ThreshParams& p) { return (p.samples > kSmallSample && p.samples <= kSmemKeys) ? 8u : 1u; }
 
 bool whole_vector(const ThreshParams& p) { return p.use_all && p.topk_pos > 0 && p.n > kSmemKeys; }
 

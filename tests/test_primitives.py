@@ -882,6 +882,31 @@ def test_rle_fused_receive_rejects_corrupt_runs(world):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("samples", [1, 2, 31, 33, 255, 256, 257, 1000, 1024, 1025, 2047, 2048, 2049])
+@pytest.mark.parametrize("ratio", [0.001, 0.01, 0.03, 0.1, 0.999])
+@pytest.mark.parametrize("kind", ["gauss", "ties", "equal", "zeros"])
+def test_threshold_of_small_samples(samples, ratio, kind):
+    """The sampled threshold for samples on both sides of the kernel's rounds and of its limit, ranks on both
+    sides of its two selections, and keys with so many ties that the candidates do not fit: the reference's
+    value, from a vector of exactly that many elements and from a longer one."""
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    for n in (samples, 7 * samples + 3):
+        gen = torch.Generator().manual_seed(samples)
+        x = torch.randn(n, generator=gen)
+        if kind == "ties":
+            x = torch.randint(-3, 4, (n,), generator=gen).float()
+        elif kind == "equal":
+            x = torch.full((n,), -1.5)
+        elif kind == "zeros":
+            x = torch.where(torch.rand(n, generator=gen) < 0.99, torch.zeros(n), x)
+        comp = P.Compressor(env, n)
+        comp.threshold_topk(x.cuda(), None, n, ratio, samples, 0.0)
+        env.flush()
+        assert float(comp.thr) == ref_threshold_topk(x, ratio, samples, 0.0)
+    env.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("count", [0, 1, 33, 511, 512, 513, 1023, 1024])
 @pytest.mark.parametrize("room", [1, 32, 511, 512, 513, 700, 1024])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
