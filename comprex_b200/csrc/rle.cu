@@ -35,6 +35,8 @@
 //
 // The expansion used to be prepared by one CTA that scanned all runs of the payload in sequence:
 // 2540 us for the 750 k runs of 2^22 elements at top-k 10 %.
+#include <type_traits>
+
 #include "cx_device.cuh"
 
 namespace {
@@ -48,7 +50,7 @@ constexpr int kGroups = 256;             // groups of run blocks, one per thread
 constexpr int kRunBlock = 1024;          // runs per block: one warp sums it, one CTA scans it
 constexpr int kWindow = 32 * kThreads;   // outputs per window: one mask word per thread
 constexpr int kRunsEach = 2 * kRunBlock / kThreads;   // runs a thread takes at a time
-constexpr int kRowsOut = 8;              // rows of 32 outputs in flight together
+constexpr int kBitsOut = 4;             // values of a lane in flight together
 
 struct ChunkTotals {       // of one warp's chunk, or of a CTA's eight.  Whether the first element starts a run is
   int32_t nnz;             // selected elements                        the element's in front to say: not counted
@@ -118,42 +120,40 @@ __global__ void __launch_bounds__(kThreads, kSendPerSm) rle_scan_kernel(const __
   cx::pdl_wait();
   cx::pdl_trigger();
   const float cut = cut_of(*p.thr);
-  float* vals = p.vals + lo;
+  float* to = p.vals + lo;             // where the next selected value goes (the same in all lanes)
   const uint32_t below = (1u << lane) - 1u;
-  uint32_t nnz = 0, tail = 0;          // selected so far (the same in all lanes), bit of the element in front
+  uint32_t tail = 0;                   // bit of the element in front
   int st = 0, last = -1, ends = lo < hi ? 0 : kEmpty;
   for (int64_t sub = lo; sub < hi; sub += CX_SUBTILE) {
     const int left = (int)min((int64_t)CX_SUBTILE, hi - sub);
     uint32_t word = 0;                 // elements 32 lane ... of the sub-tile
 #pragma unroll 1
     for (int j0 = 0; j0 < CX_SUBTILE / 32; j0 += kRows) {
-      const int64_t at = sub + 32 * j0 + lane;
       const int here = left - 32 * j0 - lane;          // my elements: 32 j < here
-      float v[kRows], b[kRows];
-      if (here > 32 * (kRows - 1)) {
+      const float* rp = p.r + (sub + 32 * j0 + lane);
+      const T* gp = g + (sub + 32 * j0 + lane);
+      auto rows = [&](auto whole) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        float v[kRows], b[kRows];
 #pragma unroll
         for (int j = 0; j < kRows; ++j) {
-          v[j] = HAS_R ? p.r[at + 32 * j] : 0.f;
-          b[j] = HAS_G ? cx::Elem<T>::to_f(g[at + 32 * j]) : 0.f;
+          v[j] = HAS_R && (WHOLE || 32 * j < here) ? rp[32 * j] : 0.f;
+          b[j] = HAS_G && (WHOLE || 32 * j < here) ? cx::Elem<T>::to_f(gp[32 * j]) : 0.f;
         }
-      } else {
 #pragma unroll
         for (int j = 0; j < kRows; ++j) {
-          v[j] = HAS_R && 32 * j < here ? p.r[at + 32 * j] : 0.f;
-          b[j] = HAS_G && 32 * j < here ? cx::Elem<T>::to_f(g[at + 32 * j]) : 0.f;
+          if (HAS_R && HAS_G) v[j] = b[j] + v[j];
+          else if (HAS_G) v[j] = b[j];
+          const bool yes = (WHOLE || 32 * j < here) && fabsf(v[j]) >= cut;
+          const uint32_t row = __ballot_sync(0xffffffffu, yes);
+          if (lane == j0 + j) word = row;
+          if (yes) to[__popc(row & below)] = v[j];
+          to += __popc(row);
+          if (HAS_R && (WHOLE || 32 * j < here)) const_cast<float*>(rp)[32 * j] = yes ? 0.f : v[j];
         }
-      }
-#pragma unroll
-      for (int j = 0; j < kRows; ++j) {
-        if (HAS_R && HAS_G) v[j] = b[j] + v[j];
-        else if (HAS_G) v[j] = b[j];
-        const bool yes = 32 * j < here && fabsf(v[j]) >= cut;
-        const uint32_t row = __ballot_sync(0xffffffffu, yes);
-        if (lane == j0 + j) word = row;
-        if (yes) vals[nnz + __popc(row & below)] = v[j];
-        nnz += __popc(row);
-        if (HAS_R && 32 * j < here) p.r[at + 32 * j] = yes ? 0.f : v[j];
-      }
+      };
+      if (left >= 32 * (j0 + kRows)) rows(std::true_type());         // (warp-uniform)
+      else rows(std::false_type());
     }
     p.bits[(sub >> 5) + lane] = word;
     uint32_t prev = __shfl_up_sync(0xffffffffu, word >> 31, 1);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, kSendPerSm) rle_scan_kernel(const __
   st = __reduce_add_sync(0xffffffffu, st);
   last = __reduce_max_sync(0xffffffffu, last);
   if (lane == 0) {
-    s_chunk[w] = ChunkTotals{(int32_t)nnz, st, last, ends};
+    s_chunk[w] = ChunkTotals{(int32_t)(to - (p.vals + lo)), st, last, ends};
     p.chunk[chunk] = s_chunk[w];
   }
   __syncthreads();
@@ -460,7 +460,7 @@ __device__ __forceinline__ V block_prefix(V x, V& tot, V* sm) {
 // `add`).  Looking every output's run up by bisection in the scanned block took 40 us for 2^22 elements at
 // top-k 10 %, a mask with one shared-memory atomic per run and four outputs per thread 17 us.  Here two
 // blocks of runs are taken at a time (a window of 8192 outputs mostly needs no more), a thread's starts go
-// to the mask word by word, and a lane writes one bit of every word, which it gets by shuffles.
+// to the mask word by word, and every lane walks the set bits of its own word.
 __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_constant__ RecvParams p) {
   __shared__ long long s_l[kWarps];
   __shared__ int s_a[kWarps], s_b[kWarps];
@@ -574,27 +574,30 @@ __global__ void __launch_bounds__(kThreads, 4) rle_expand_kernel(const __grid_co
     int total;
     const int mybase = vbase + block_prefix<int>(__popc(x), total, s_a);
     vbase += total;
-    // lane l writes bit l of every word of its warp
-    const int64_t i0 = w0 + 32 * (tid & ~31) + lane;
-    const uint32_t below = (1u << lane) - 1u;
-#pragma unroll 1
-    for (int j0 = 0; j0 < 32; j0 += kRowsOut) {
-      float y[kRowsOut], z[kRowsOut];
-      uint32_t yes = 0;
+    if (!p.add) {                          // zeros first, a row of 32 outputs at a time
+      float* row = p.out + (w0 + 32 * (tid & ~31) + lane);
+      const int64_t here = w1 - (w0 + 32 * (tid & ~31) + lane);
 #pragma unroll
-      for (int j = 0; j < kRowsOut; ++j) {
-        const uint32_t word = __shfl_sync(0xffffffffu, x, j0 + j);
-        const int k = __shfl_sync(0xffffffffu, mybase, j0 + j) + __popc(word & below);
-        const bool sel = (word >> lane) & 1u;
-        yes |= (sel ? 1u : 0u) << j;
-        y[j] = sel ? vals[k] : 0.f;
-        z[j] = sel && p.add ? p.out[i0 + 32 * (j0 + j)] : 0.f;
+      for (int j = 0; j < 32; ++j) if (32 * j < here) row[32 * j] = 0.f;
+      __syncwarp();                        // the other lanes' zeros are in front of this lane's values
+    }
+    // then every lane the selected outputs of its own word, kBitsOut of them in flight
+    float* mine32 = p.out + (w0 + 32 * tid);
+    const float* val = vals + mybase;
+    while (x) {
+      int at32[kBitsOut];
+      float y[kBitsOut], z[kBitsOut];
+#pragma unroll
+      for (int k = 0; k < kBitsOut; ++k) {
+        at32[k] = __ffs(x) - 1;            // -1: no more
+        x &= x - 1;
+        y[k] = at32[k] >= 0 ? val[k] : 0.f;
+        z[k] = at32[k] >= 0 && p.add ? mine32[at32[k]] : 0.f;
       }
 #pragma unroll
-      for (int j = 0; j < kRowsOut; ++j) {
-        const int64_t i = i0 + 32 * (j0 + j);
-        if (p.add ? ((yes >> j) & 1u) != 0 : i < w1) p.out[i] = p.add ? z[j] + y[j] : y[j];
-      }
+      for (int k = 0; k < kBitsOut; ++k)
+        if (at32[k] >= 0) mine32[at32[k]] = p.add ? z[k] + y[k] : y[k];
+      val += kBitsOut;
     }
     if (w0 + kWindow < e1) __syncthreads();          // s_a is written again
   }
