@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, 4) fold_update_kernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < kGroup; ++k) {
           const int e0 = (c0 + k) * 128 + lane * 4;
-          cx::load4(cur.g + e0, x[k]);
+          cx::load4_last(cur.g + e0, x[k]);
 #pragma unroll
           for (int e = 0; e < 4; ++e) y[k][e] = 0.f;
           if (KEEP == 2) cx::load4(q.f.u + lo + e0, y[k]);

@@ -175,7 +175,7 @@ __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, cons
     float y[kGroup][4];
 #pragma unroll
     for (int c = 0; c < kGroup; ++c) {
-      x[c] = cx::Raw4<T>::load(gl + lane * 4 + (c0 + c) * 128);
+      x[c] = cx::load_last(reinterpret_cast<const typename cx::Raw4<T>::type*>(gl + lane * 4 + (c0 + c) * 128));
       if (IN == kFoldMom) cx::load4(up + lane * 4 + (c0 + c) * 128, y[c]);
     }
     if (IN != kFold && c0 == 0) late.get();      // loads only before, stores from here on

@@ -136,6 +136,43 @@ __device__ __forceinline__ void store4(__half* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = t;
 }
 
+// L2 priorities of loads: data that another kernel reads soon, and everything else
+__device__ __forceinline__ uint64_t keep_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t plain_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint4 load_keep(const uint4* p, uint64_t keep) {
+  uint4 v;
+  asm("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(keep));
+  return v;
+}
+// The last read of data that an earlier kernel asked L2 to keep (keep_policy): its lines may go.
+__device__ __forceinline__ uint64_t last_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ float4 load_last(const float4* p) {
+  float4 v;
+  asm("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(last_policy()));
+  return v;
+}
+__device__ __forceinline__ uint2 load_last(const uint2* p) {
+  uint2 t;
+  asm("ld.global.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(t.x), "=r"(t.y) : "l"(p), "l"(last_policy()));
+  return t;
+}
+template <typename T>
+__device__ __forceinline__ void load4_last(const T* p, float (&v)[4]) {
+  Raw4<T>::to_f(load_last(reinterpret_cast<const typename Raw4<T>::type*>(p)), v);
+}
+
 }  // namespace cx
 
 // A launch that is part of a captured graph takes its sequence number from a device cell
