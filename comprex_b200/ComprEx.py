@@ -395,21 +395,23 @@ class Comprex(AbstractExchange):
         self._env.maybe_check()
 
     def _write_prepared(self, vector) -> bool:
-        """``writeRemote`` of a plain vector with a sampled or exact top-k threshold: one call for the
-        whole launch list.  False: take the general path."""
+        """``writeRemote`` of a plain vector with a sampled or exact top-k threshold, as pairs or run lengths:
+        one call for the whole launch list.  False: take the general path."""
         thr, comp = self.threshold, self._comp
-        if (self.compressor.kind != "pairs" or type(thr) is not ThresholdTopK or self.restsVect is None
+        kind = self.compressor.kind
+        if (kind not in ("pairs", "rle") or type(thr) is not ThresholdTopK or self.restsVect is None
                 or getattr(self._env, "_rec", None) is not None):
             return False
         dest = self._dest
         seq = self._tx_seq.get(dest, 0) + 1
-        cfg = (dest, thr.topK, thr.default_subsamples, thr.subsample_factor, self.restsVect)
+        cfg = (dest, thr.topK, thr.default_subsamples, thr.subsample_factor, kind, self.restsVect)
         got = self._tx_ops.get(seq & 1)
-        if got is None or got[0] != cfg[:4] or got[1] is not cfg[4]:
+        if got is None or got[0] != cfg[:5] or got[1] is not cfg[5]:
             ep = self._slots[seq & 1].endpoint(self._env, dest)
-            got = self._tx_ops[seq & 1] = (cfg[:4], cfg[4], _lib.VectorOps(
-                _lib.VectorOps.SEND, comp.send_ops(self.restsVect, self.size, self.cap, P.make_targets([ep]), *cfg[1:4]),
-                self._env.device, self.size))
+            ops = comp.send_ops(self.restsVect, self.size, self.cap, P.make_targets([ep]), *cfg[1:4])
+            if kind == "rle":
+                ops = [ops[0], self._rle.send_op(self.restsVect, comp.thr, seq & 1, dest)]
+            got = self._tx_ops[seq & 1] = (cfg[:5], cfg[5], _lib.VectorOps(_lib.VectorOps.SEND, ops, self._env.device, self.size))
         if not got[2].run(vector, seq):
             return False
         self._tx_seq[dest] = seq
@@ -419,18 +421,23 @@ class Comprex(AbstractExchange):
 
     def _read_prepared(self, vector, op: int) -> bool:
         """``readRemote(vector)`` / ``readRemote_add`` of a plain vector.  False: take the general path."""
-        if self.compressor.kind != "pairs" or self._rx_current is not None or self._src is None:
+        kind = self.compressor.kind
+        if kind not in ("pairs", "rle") or self._rx_current is not None or self._src is None:
             return False
         src = self._src
         seq = self._rx_seq.get(src, 0) + 1
-        got = self._rx_ops.get((seq & 1, op, self._env.timeout_ns))
-        if got is None:
+        key = (seq & 1, op, self._env.timeout_ns, kind)
+        got = self._rx_ops.get(key)
+        if got is None and kind == "rle":
+            o = self._rle.recv_op(seq & 1, op == _lib.OP_ADD, self._status, key[2])
+            got = self._rx_ops[key] = _lib.VectorOps(_lib.VectorOps.RLE_READ, [o], self._env.device, self.size)
+        elif got is None:
             o = _lib.Op()
             o.kind, o.dev, o.n = _lib.OPK_APPLY, self._env.dev, self.size
             o.src = P.make_sources([self._slots[seq & 1].endpoint(self._env)], [seq])
             o.apply.op, o.apply.scale = op, 1.0
             o.status, o.timeout_ns = self._status.dev_ptr, self._env.timeout_ns
-            got = self._rx_ops[(seq & 1, op, o.timeout_ns)] = _lib.VectorOps(_lib.VectorOps.APPLY, [o], self._env.device, self.size)
+            got = self._rx_ops[key] = _lib.VectorOps(_lib.VectorOps.APPLY, [o], self._env.device, self.size)
         if not got.run(vector, seq):
             return False
         self._rx_seq[src] = seq

@@ -63,7 +63,7 @@ class ApplyArgs(C.Structure):
 
 
 OPK_THRESHOLD, OPK_COMPRESS, OPK_APPLY, OPK_DENSE_SEND, OPK_DENSE_REDUCE, OPK_UPDATE, OPK_MM_ALLREDUCE = 1, 2, 3, 4, 5, 6, 7
-OPK_FOLD_COEF, OPK_FOLD_UPDATE = 8, 9
+OPK_FOLD_COEF, OPK_FOLD_UPDATE, OPK_RLE_SEND, OPK_RLE_RECV = 8, 9, 10, 11
 
 
 class Fold(C.Structure):
@@ -229,7 +229,7 @@ class VectorOps:
     returns False, with nothing launched, when the vector needs the caller's general path (another
     type or device, a NumPy array, a non-contiguous tensor, another size)."""
 
-    SEND, APPLY, DENSE_SEND, DENSE_READ, DENSE_ADD = range(5)      # roles of the vector
+    SEND, APPLY, DENSE_SEND, DENSE_READ, DENSE_ADD, RLE_READ = range(6)      # roles of the vector
 
     def __init__(self, role: int, ops, device: torch.device, n: int):
         self.ops = (Op * len(ops))(*ops)

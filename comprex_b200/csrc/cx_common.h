@@ -344,6 +344,9 @@ int cx_host_free(void* p);
 #define CX_OPK_UPDATE 6        /* cx_update_dense: g, n, apply */
 #define CX_OPK_FOLD_COEF 8     /* cx_fold_coef (CUDA): dtype, fold = address of a CxFoldCoef */
 #define CX_OPK_FOLD_UPDATE 9   /* cx_fold_update (CUDA): dtype, fold, n, apply */
+#define CX_OPK_RLE_SEND 10     /* cx_rle_send: dtype, g, r, n, thr, starts[0] = slot bytes, tg, workspace, ws_bytes, src_rank */
+#define CX_OPK_RLE_RECV 11     /* cx_rle_recv: src.ep[0], out, n, has_push = add, starts[0] = slot bytes, workspace, ws_bytes,
+                                  status, timeout_ns */
 #define CX_OPK_MM_ALLREDUCE 7  /* cx_mm_allreduce: out, own (= in), g (= stage), r (= stage_mc), starts[0] = stride,
                                   starts[1] = one_shot, starts[2] = slab bytes, lens[r] = rank r's flag block,
                                   src_rank, cap (= ranks), workspace (= counters), scale, status */

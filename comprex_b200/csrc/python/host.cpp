@@ -71,13 +71,14 @@ int element_code(const at::Tensor& t) {
 }
 
 typedef int (*RunOps)(CxOp*, int, uint64_t, void*);
-enum Role { kSend = 0, kApply = 1, kDenseSend = 2, kDenseRead = 3, kDenseAdd = 4 };
+enum Role { kSend = 0, kApply = 1, kDenseSend = 2, kDenseRead = 3, kDenseAdd = 4, kRleRead = 5 };
 
 // run_vector(role, run_ops, ops, count, seq, stream, vector, device, n) -> what cx_run_ops returns, or
 // None when the vector is not the plain case (a contiguous CUDA tensor of the right size and type on
 // `device`): nothing has happened then, the caller takes its general path.
-//   kSend: input of a threshold + compress list, n elements.  kApply: destination of an apply op, n
-//   elements.  kDense*: a dense message of the vector's length, at most n, of the op's element type.
+//   kSend: input of a threshold + compress (or run-length send) list, n elements.  kApply: destination of an
+//   apply op, n elements.  kDense*: a dense message of the vector's length, at most n, of the op's element type.
+//   kRleRead: destination of a run-length receive, n fp32 elements.
 PyObject* run_vector(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 9) {
     PyErr_SetString(PyExc_TypeError, "run_vector: nine arguments");
@@ -116,6 +117,9 @@ PyObject* run_vector(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (len < n) Py_RETURN_NONE;
     ops[0].apply.out = ptr;
     ops[0].apply.out_dtype = code;
+  } else if (role == kRleRead) {
+    if (len != n || code != CX_F32) Py_RETURN_NONE;
+    ops[0].out = ptr;
   } else {
     if (len > n || code != ops[0].dtype) Py_RETURN_NONE;
     ops[0].n = len;

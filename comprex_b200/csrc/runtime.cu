@@ -317,6 +317,12 @@ int run_one(CxOp& o, uint64_t seq, void* stream) {
                              (int)o.cap, o.scale, (int)o.starts[1], o.starts[2], seq, flags, o.workspace, o.status,
                              o.timeout_ns, stream);
     }
+    case CX_OPK_RLE_SEND:
+      return cx_rle_send(o.dev, o.dtype, o.g, o.r, o.n, o.thr, o.starts[0], seq, &o.tg, o.workspace, o.ws_bytes,
+                         o.src_rank, stream);
+    case CX_OPK_RLE_RECV:
+      return cx_rle_recv(o.dev, &o.src.ep[0], seq, reinterpret_cast<float*>(o.out), o.n, o.has_push, o.starts[0], o.workspace,
+                         o.ws_bytes, o.status, o.timeout_ns, stream);
     case CX_OPK_FOLD_COEF:
       return cx_fold_coef(o.dtype, reinterpret_cast<const CxFoldCoef*>(o.fold), stream);
     case CX_OPK_FOLD_UPDATE:
@@ -440,6 +446,8 @@ int cx_graph_build(CxOp* ops, int count, void** out) {
   if (count <= 0) return cx_set_error("cx_graph_build: empty sequence", 0);
   for (int i = 0; i < count; ++i)
     if (ops[i].dev != CX_DEV_CUDA) return cx_set_error("cx_graph_build: host ops cannot be captured", 0);
+    else if (ops[i].kind == CX_OPK_RLE_SEND || ops[i].kind == CX_OPK_RLE_RECV)   // their sequence number is a parameter
+      return cx_set_error("cx_graph_build: run-length messages cannot be captured", 0);
   CxGraph* g = new CxGraph();
   g->graph = nullptr; g->exec = nullptr; g->cell = nullptr; g->kernels = 0; g->device = 0;
   cudaStream_t cap = nullptr;

@@ -278,6 +278,23 @@ class RleCodec:
                                        seq, C.byref(tg), self.tx_ws.data_ptr(), self.ws_bytes, env.rank,
                                        _lib.stream_ptr(env.device)), "cx_rle_send")
 
+    def send_op(self, r, thr_cell: torch.Tensor, par: int, dest: int) -> _lib.Op:
+        """``send`` with residual ``r`` as an op of a launch list (the vector is filled in per call)."""
+        o = _lib.Op()
+        o.kind, o.dev, o.n, o.r, o.thr = _lib.OPK_RLE_SEND, self.env.dev, self.n, _ptr(r), thr_cell.data_ptr()
+        o.starts[0], o.workspace, o.ws_bytes, o.src_rank = self.slot_bytes, self.tx_ws.data_ptr(), self.ws_bytes, self.env.rank
+        o.tg = make_targets([self.slots[par].endpoint(self.env, dest)])
+        return o
+
+    def recv_op(self, par: int, add: bool, status, timeout_ns: int) -> _lib.Op:
+        """``recv`` the same way."""
+        o = _lib.Op()
+        o.kind, o.dev, o.n, o.has_push = _lib.OPK_RLE_RECV, self.env.dev, self.n, int(add)
+        o.starts[0], o.workspace, o.ws_bytes = self.slot_bytes, self.rx_ws.data_ptr(), self.rx_ws_bytes
+        o.src = make_sources([self.slots[par].endpoint(self.env)], [0])
+        o.status, o.timeout_ns = status.dev_ptr, timeout_ns
+        return o
+
     def recv(self, out: torch.Tensor, seq: int, add: bool, status) -> None:
         """Wait for payload ``seq`` in the local slot and expand it into the float32 ``out``."""
         env = self.env
