@@ -254,10 +254,22 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
 
   // my survivors among the list's entries [w0, w0 + kList)
   auto fill = [&](const uint32_t w0) {
-    uint32_t pos = incl - mine - w0;        // wraps below the window: fails the test
-    for (uint32_t bits = mask; bits; bits &= bits - 1, ++pos) {
-      const uint32_t b = __ffs(bits) - 1;
-      if (pos < kList) sat[pos] = (uint16_t)((b >> 2) * 128 + lane * 4 + (b & 3));
+    // two halves of the mask side by side: half the steps of a chain of dependent instructions
+    uint32_t low = mask & 0xffffu, high = mask >> 16;
+    uint32_t pos = incl - mine - w0, hpos = pos + __popc(low);   // wrap below the window: fail the test
+    while (low | high) {
+      if (low) {
+        const uint32_t b = __ffs(low) - 1;
+        if (pos < kList) sat[pos] = (uint16_t)((b >> 2) * 128 + lane * 4 + (b & 3));
+        low &= low - 1;
+        ++pos;
+      }
+      if (high) {
+        const uint32_t b = __ffs(high) - 1;
+        if (hpos < kList) sat[hpos] = (uint16_t)((b >> 2) * 128 + 512 + lane * 4 + (b & 3));
+        high &= high - 1;
+        ++hpos;
+      }
     }
   };
   fill(0);
