@@ -582,7 +582,8 @@ constexpr int kBins = 2048;          // 11 bits per radix pass of the finish
 constexpr int kCollectThreads = 256;
 constexpr int kCollectEach = 8;      // elements per thread and round
 constexpr int kBuffer = 3072;        // candidates a CTA keeps before it appends them to the list
-constexpr int kCollectPerSm = 6;
+constexpr int kCollectRounds = 16;   // rounds between two looks at how full that buffer is
+constexpr int kCollectPerSm = 5;     // registers
 
 struct ExactState {                  // in the workspace behind the histograms; zero between calls
   uint32_t lo, hi;
@@ -709,37 +710,45 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_kernel(const __grid_c
   }
 }
 
+// Bound by instructions, then by the read of the vector.  A thread compares its eight elements with the bracket
+// and keeps two bits of each; only those inside the bracket (1 %) are looked at one by one, and nobody waits for
+// the other warps: the CTA's buffer is emptied every 16 rounds, and what finds it full goes to the list at once.
+// With a vote for every element and two barriers a round 10 M fp32 elements took 23.5 us by itself, now 19.6; an
+// exchange of 1 M elements 30.9 -> 29.4 us (10 M: 63.4 -> 63.0).
 template <typename T>
 __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel(const __grid_constant__ OnePassParams p) {
   __shared__ uint32_t s_buf[kBuffer];
   __shared__ uint32_t s_hist[kBins];
-  __shared__ uint32_t s_fill, s_base;
+  __shared__ uint32_t s_fill, s_kept, s_base;    // s_kept: where the buffer's entries end once it was full
   __shared__ uint32_t s_cnt[3];
   const int tid = threadIdx.x, lane = tid & 31;
-  if (tid == 0) s_fill = 0;
+  if (tid == 0) { s_fill = 0; s_kept = kBuffer; }
   for (int i = tid; i < kBins; i += kCollectThreads) s_hist[i] = 0;
   if (tid < 3) s_cnt[tid] = 0;
   cx::pdl_wait();
   cx::pdl_trigger();
   const uint32_t lo = p.st->lo, hi = p.st->hi;
+  const float lof = __uint_as_float(lo), hif = __uint_as_float(hi);      // (no upper bound: a NaN)
   const int shift = max(bracket_bits(lo, hi) - 11, 0);
   const T* g = reinterpret_cast<const T*>(p.g);
   uint32_t above = 0, at_hi = 0, at_lo = 0;
   __syncthreads();
   const int64_t round = (int64_t)kCollectThreads * kCollectEach;
   auto flush = [&]() {                // all threads
-    const uint32_t fill = s_fill;
+    const uint32_t fill = min(s_fill, s_kept);
     if (tid == 0) s_base = atomicAdd(&p.st->found, fill);
     __syncthreads();
     for (uint32_t i = tid; i < fill; i += kCollectThreads)
       if (s_base + i < p.cap) p.list[s_base + i] = s_buf[i];
     __syncthreads();
-    if (tid == 0) s_fill = 0;
+    if (tid == 0) { s_fill = 0; s_kept = kBuffer; }
     __syncthreads();
   };
+  int rounds = 0;
   for (int64_t b = (int64_t)blockIdx.x * round; b < p.n; b += (int64_t)gridDim.x * round) {
     float v[kCollectEach];
     const bool whole = p.vec && b + round <= p.n;
+    uint32_t valid = (1u << kCollectEach) - 1u;
     if (whole) {
       constexpr int kQ = kCollectEach / 4;
       float y[kQ][4];
@@ -758,6 +767,7 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
         for (int e = 0; e < 4; ++e) v[4 * k + e] = p.r ? (g ? y[k][e] + t[e] : y[k][e]) : t[e];
       }
     } else {
+      valid = 0;
 #pragma unroll
       for (int k = 0; k < kCollectEach; ++k) {
         const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
@@ -765,33 +775,62 @@ __global__ void __launch_bounds__(kCollectThreads, kCollectPerSm) collect_kernel
         if (i < p.n) {
           if (p.r) v[k] = p.r[i];
           if (g) v[k] = v[k] + cx::Elem<T>::to_f(g[i]);
+          valid |= 1u << k;
         }
       }
     }
+    // keys are compared as integers below; as floats, every key that is not plainly below or above the bracket
+    // (a NaN never is) counts as inside
+    uint32_t from_lo = 0, over = 0;
 #pragma unroll
     for (int k = 0; k < kCollectEach; ++k) {
-      const int64_t i = b + (int64_t)(k / 4) * kCollectThreads * 4 + tid * 4 + (k & 3);
-      const uint32_t key = __float_as_uint(fabsf(v[k]));
-      const bool near = (whole || i < p.n) && key >= lo;       // few are
-      if (!__any_sync(0xffffffffu, near)) continue;
+      if (!(fabsf(v[k]) < lof)) from_lo |= 1u << k;
+      if (fabsf(v[k]) > hif) over |= 1u << k;
+    }
+    above += __popc(over & valid);
+    uint32_t mid = from_lo & ~over & valid;
+    while (__any_sync(0xffffffffu, mid != 0)) {
+      const bool have = mid != 0;
+      const int k = have ? __ffs(mid) - 1 : 0;
+      mid &= mid - 1;
+      float x[kCollectEach / 2];
+#pragma unroll
+      for (int j = 0; j < kCollectEach / 2; ++j) x[j] = k & 1 ? v[2 * j + 1] : v[2 * j];
+#pragma unroll
+      for (int j = 0; j < kCollectEach / 4; ++j) x[j] = k & 2 ? x[2 * j + 1] : x[2 * j];
+      static_assert(kCollectEach == 8, "three levels");
+      const uint32_t key = __float_as_uint(fabsf(k & 4 ? x[1] : x[0]));
+      const bool near = have && key >= lo;
       above += near && key > hi;
       at_hi += near && key == hi;
       at_lo += near && key == lo && lo != hi;
       const bool cand = near && key > lo && key < hi;
       const uint32_t who = __ballot_sync(0xffffffffu, cand);
       if (who) {
+        const uint32_t number = __popc(who);
+        const int first = __ffs(who) - 1;
         uint32_t at = 0;
-        if (lane == __ffs(who) - 1) at = atomicAdd(&s_fill, (uint32_t)__popc(who));
-        at = __shfl_sync(0xffffffffu, at, __ffs(who) - 1);
+        if (lane == first) at = atomicAdd(&s_fill, number);
+        at = __shfl_sync(0xffffffffu, at, first);
+        const bool room = at + number <= kBuffer;       // once it is false it stays so until the buffer is emptied
+        uint32_t to = at;
+        if (!room) {
+          if (lane == first) { atomicMin(&s_kept, at); to = atomicAdd(&p.st->found, number); }
+          to = __shfl_sync(0xffffffffu, to, first);
+        }
         if (cand) {
-          s_buf[at + __popc(who & ((1u << lane) - 1u))] = key;
+          to += __popc(who & ((1u << lane) - 1u));
+          if (room) s_buf[to] = key;
+          else if (to < p.cap) p.list[to] = key;
           atomicAdd(&s_hist[(key - bracket_base(lo)) >> shift], 1u);
         }
       }
     }
-    __syncthreads();
-    if (s_fill > kBuffer - kCollectThreads * kCollectEach) flush();      // uniform: the next round might not fit
-    else __syncthreads();
+    if (++rounds % kCollectRounds == 0) {
+      __syncthreads();
+      if (s_fill > kBuffer / 2) flush();                // uniform
+      else __syncthreads();
+    }
   }
   if (above) atomicAdd(&s_cnt[0], above);
   if (at_hi) atomicAdd(&s_cnt[1], at_hi);

@@ -131,6 +131,60 @@ def test_exact_topk_one_pass(n, dtype, data):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_exact_topk_candidates_in_few_ctas(dtype):
+    """The elements around the wanted rank lie where the same few CTAs come by, round after round: their
+    buffers fill up, are emptied between rounds, and what they have no room for goes to the list at once."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for per_sm in (4, 5, 6):                   # resident CTAs of the collecting kernel
+        grid, chunk, rounds = sms * per_sm, 2048, 20
+        n = grid * chunk * rounds
+        gen = torch.Generator(device="cuda").manual_seed(per_sm)
+        values = (0.5 + torch.rand(n, device="cuda", generator=gen)).to(dtype).float().sort().values
+        hot = max(1, round(0.04 * grid))       # CTAs that meet the middle 4 % of the values
+        mid0 = n // 2 - hot * rounds * chunk // 2
+        mid, rest = values[mid0:mid0 + hot * rounds * chunk], torch.cat((values[:mid0], values[mid0 + hot * rounds * chunk:]))
+        g = torch.empty(rounds, grid, chunk, device="cuda")
+        g[:, :hot] = mid.view(rounds, hot, chunk)
+        g[:, hot:] = rest[torch.randperm(rest.numel(), device="cuda", generator=gen)].view(rounds, grid - hot, chunk)
+        env = cx.GaspiEnvironment(1 << 16, device="cuda")
+        comp = P.Compressor(env, n)
+        comp.threshold_topk(g.view(-1).to(dtype), None, n, 0.5, cx.ThresholdTopK.EXACT)
+        k = int(torch.ceil(torch.tensor(float(n)) * torch.tensor(0.5)).item()) - 1
+        assert float(comp.thr) == float(values[n - 1 - k])
+        env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [0, 1, 31, 128, 129, 255, 256, 257, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_set_of_one_source(count, dtype, shift):
+    """Sub-tiles on both sides of the count up to which values go straight to their places, a partial one at
+    the end, and a destination that takes no wide accesses: every other element is overwritten with zero."""
+    n = 3 * 1024 + 500
+    world = cx.LoopbackWorld(1, device="cuda", timeout_ms=2000)
+    e0 = world.envs[0]
+    gen = torch.Generator().manual_seed(count)
+    keep = torch.zeros(n, dtype=torch.bool)
+    for sub in range(0, n, 1024):
+        room = min(1024, n - sub)
+        keep[sub + torch.randperm(room, generator=gen)[:count]] = True
+    x = torch.where(keep, torch.randn(n, generator=gen).abs() + 0.5, torch.zeros(n))
+    comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, n)
+    comp.set_threshold(0.25)
+    comp.compress(x.cuda(), None, n, n, 1, P.make_targets([slot.endpoint(e0)]))
+    out = torch.full((n + 1,), 9.0, dtype=dtype, device="cuda")
+    status = e0.new_status("t")
+    P.apply_sparse(e0, P.make_sources([slot.endpoint(e0)], [1]), n, P.args_set(out[shift:shift + n], 0.5), status)
+    e0.flush()
+    assert status.value == 0
+    assert torch.equal(out[shift:shift + n].cpu(), (0.5 * x).to(dtype))
+    assert float(out[n if shift == 0 else 0]) == 9.0
+    world.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("data", ["normal", "ties", "constant", "ends"])
 @pytest.mark.parametrize("n", [33, 1000, 1024, 1025, 2049, 11008])
 def test_threshold_selection_ranks(n, data):
