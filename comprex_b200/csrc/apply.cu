@@ -23,6 +23,8 @@
 // word and the kernel returns without touching the output.
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "cx_fold.cuh"
 
 namespace {
@@ -649,6 +651,45 @@ __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(co
   if (bad && p.status) atomicOr(p.status, bad);
 }
 
+// SET of one source: nothing is summed, so the pairs need not meet in shared memory.  Zeros go straight to the
+// sub-tile, then the values to their places (the warp's barrier orders the two); a sub-tile with more than
+// kDirect pairs (a store each, and the lines written twice; the line was not swept) takes shared memory.  Only
+// for sub-tiles whose 16-byte accesses all work.  Exchange of 2^20 elements, overwritten: 12.7 -> 12.2 us.
+constexpr uint32_t kDirect = 256;
+template <typename TO>
+__device__ __forceinline__ uint32_t set_subtile(const ApplyParams& p, uint32_t sub, int lane, uint32_t a, uint32_t b) {
+  const uint32_t lo = sub * CX_SUBTILE;
+  TO* out = reinterpret_cast<TO*>(p.a.out) + lo;
+  const CxPair* pairs = p.src.ep[0].pairs;
+  constexpr int kAt = 4;
+  uint32_t bad = 0;
+  CxPair pr[kAt];
+#pragma unroll
+  for (int k = 0; k < kAt; ++k) {
+    pr[k].idx = -1;
+    pr[k].val = 0;
+    if (a + 32 * k + lane < b) pr[k] = ld_pair(pairs + a + 32 * k + lane);
+  }
+  const float zero[4] = {p.a.scale * 0.f, p.a.scale * 0.f, p.a.scale * 0.f, p.a.scale * 0.f};
+#pragma unroll
+  for (int q = 0; q < CX_SUBTILE / 128; ++q) cx::store4(out + q * 128 + lane * 4, zero);
+  __syncwarp();
+  while (a < b) {                              // (warp-uniform)
+#pragma unroll
+    for (int k = 0; k < kAt; ++k) {
+      const uint32_t d = (uint32_t)pr[k].idx - lo;
+      if (a + 32 * k + lane < b) {
+        if (d < CX_SUBTILE) out[d] = cx::Elem<TO>::from_f(p.a.scale * (0.f + __uint_as_float(pr[k].val)));
+        else bad = CX_ST_BAD_INDEX;
+      }
+    }
+    a += 32 * kAt;
+#pragma unroll
+    for (int k = 0; k < kAt; ++k) if (a + 32 * k + lane < b) pr[k] = ld_pair(pairs + a + 32 * k + lane);
+  }
+  return bad;
+}
+
 // CTAs of apply_dense_kernel per SM (registers)
 constexpr int dense_per_sm(int op) { return op == CX_OP_MOMENTUM || op == CX_OP_ADAMW ? 5 : 6; }
 
@@ -670,18 +711,33 @@ __global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel
     uint32_t na, nb;                          // the next sub-tile's table entries, in flight meanwhile
     const uint64_t next = (uint64_t)sub + nwarps;
     table_entry(p, next < p.nsub ? (uint32_t)next : p.nsub, lane, na, nb);
+    const bool whole = p.vec && (int64_t)lo + CX_SUBTILE <= p.n;
+    if (OP == CX_OP_SET && whole && p.src.count == 1) {
+      const uint32_t a0 = __shfl_sync(0xffffffffu, a, 0), b0 = __shfl_sync(0xffffffffu, b, 0);
+      if (b0 - a0 <= kDirect) {
+        bad |= set_subtile<TO>(p, sub, lane, a0, b0);
+        a = na;
+        b = nb;
+        continue;
+      }
+    }
     bad |= accumulate_subtile(p, sub, lane, a, b, acc);
     a = na;
     b = nb;
-#pragma unroll
-    for (int q = 0; q < CX_SUBTILE / 128; ++q) {
-      const int e0 = q * 128 + lane * 4;
-      const int64_t i = (int64_t)lo + e0;
-      if (i >= p.n) continue;
-      const float4 t = *reinterpret_cast<const float4*>(acc + e0);
-      const float av[4] = {t.x, t.y, t.z, t.w};
-      update4<OP, TO>(p.a, p.n, i, av, p.vec && i + 3 < p.n);
-    }
+    auto walk = [&](auto all) {
+      constexpr int kUnroll = decltype(all)::value ? CX_SUBTILE / 128 : 1;
+#pragma unroll kUnroll
+      for (int q = 0; q < CX_SUBTILE / 128; ++q) {
+        const int e0 = q * 128 + lane * 4;
+        const int64_t i = (int64_t)lo + e0;
+        if (!decltype(all)::value && i >= p.n) continue;
+        const float4 t = *reinterpret_cast<const float4*>(acc + e0);
+        const float av[4] = {t.x, t.y, t.z, t.w};
+        update4<OP, TO>(p.a, p.n, i, av, decltype(all)::value || (p.vec && i + 3 < p.n));
+      }
+    };
+    if (whole) walk(std::true_type());         // without a test per access
+    else walk(std::false_type());
     __syncwarp();
   }
   if (bad && p.status) atomicOr(p.status, bad);
