@@ -41,7 +41,7 @@ struct ApplyParams {
   uint32_t* status;
   uint64_t timeout_ns;
   const uint64_t* seq_cell;  // non-NULL inside a captured graph: the waits use its value
-  uint32_t front_wait;       // the kernel in front may be at work on the same vectors
+  uint32_t front_wait;       // CX_WAIT_*: the kernel in front may be at work on the same vectors
   uint32_t early;            // dense ops: let the kernel behind in at the start
   uint32_t group;            // sparse ops: sub-tiles a warp takes at a time
 };
@@ -52,6 +52,14 @@ __device__ __forceinline__ CxPair ld_pair(const CxPair* p) {
   r.idx = (int32_t)t.x;
   r.val = t.y;
   return r;
+}
+
+// At the start of a receive kernel: lets the kernel behind in (`early`) and waits for the one in front as far as
+// that has to happen here.
+__device__ __forceinline__ void begin_apply(const ApplyParams& p, bool early) {
+  if (p.front_wait == CX_WAIT_CHAIN) cx::pdl_wait();
+  if (early) cx::pdl_trigger();
+  if (p.front_wait == CX_WAIT_START) cx::pdl_wait();
 }
 
 // Waits for all sources and validates their headers: the first warp does, lane j for source j.  (Every
@@ -139,8 +147,7 @@ __device__ __forceinline__ uint32_t group_of_several(const ApplyParams& p, uint6
 
 template <typename TO, int AHEAD, bool SEVERAL>
 __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_constant__ ApplyParams p) {
-  cx::pdl_trigger();
-  if (p.front_wait) cx::pdl_wait();
+  begin_apply(p, true);
   const int lane = threadIdx.x & 31;
   uint64_t all = 0;
   if (!wait_sources<SEVERAL>(p, &all)) { cx::pdl_wait(); return; }
@@ -148,6 +155,7 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
   const uint32_t nwarps = gridDim.x * kWarps;
   const bool sgd = p.a.op == CX_OP_SGD;
   const float scale = sgd ? -p.a.scale : p.a.scale;
+  bool wait = p.front_wait == CX_WAIT_VECTORS;
   uint32_t bad = 0;
   for (uint64_t s0 = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * group; s0 < p.nsub;
        s0 += (uint64_t)nwarps * group) {
@@ -188,6 +196,7 @@ __global__ void __launch_bounds__(kThreads) apply_sparse_kernel(const __grid_con
         for (int k = 0; k < AHEAD; ++k) {
           if (in[k] && !((uint32_t)pr[k].idx - lo[k] < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { in[k] = false; bad = CX_ST_BAD_INDEX; }
         }
+        if (wait) { cx::pdl_wait(); wait = false; }
         // indices are unique inside one payload: the loads may all go first
         float cur[AHEAD];
         if (sgd) {
@@ -232,8 +241,7 @@ template <typename TO>
 __global__ void __launch_bounds__(kThreads, 6) apply_sparse_batch_kernel(const __grid_constant__ ApplyParams p) {
   __shared__ uint8_t s_slot[kWarps][CX_SUBTILE];
   __shared__ float s_acc[kWarps][kBatchPairs];
-  cx::pdl_trigger();
-  if (p.front_wait) cx::pdl_wait();
+  begin_apply(p, true);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (!wait_sources(p)) { cx::pdl_wait(); return; }
   const uint32_t nwarps = gridDim.x * kWarps;
@@ -241,6 +249,7 @@ __global__ void __launch_bounds__(kThreads, 6) apply_sparse_batch_kernel(const _
   const float scale = sgd ? -p.a.scale : p.a.scale;
   uint8_t* slot = s_slot[warp];
   float* acc = s_acc[warp];
+  bool wait = p.front_wait == CX_WAIT_VECTORS;
   uint32_t bad = 0;
   uint32_t sub = blockIdx.x * kWarps + warp, a, b;
   table_entry(p, sub, lane, a, b);
@@ -282,6 +291,7 @@ __global__ void __launch_bounds__(kThreads, 6) apply_sparse_batch_kernel(const _
         if (src[k] >= 0 && !(d[k] < CX_SUBTILE && (int64_t)pr[k].idx < p.n)) { bad = CX_ST_BAD_INDEX; src[k] = -1; }
         if (src[k] >= 0) slot[d[k]] = (uint8_t)(32 * k + lane);
       }
+      if (wait) { cx::pdl_wait(); wait = false; }
       float cur[kBatch];
       if (sgd) {
         const float* w = reinterpret_cast<const float*>(p.a.out);
@@ -657,7 +667,7 @@ __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(co
 // for sub-tiles whose 16-byte accesses all work.  Exchange of 2^20 elements, overwritten: 12.7 -> 12.2 us.
 constexpr uint32_t kDirect = 256;
 template <typename TO>
-__device__ __forceinline__ uint32_t set_subtile(const ApplyParams& p, uint32_t sub, int lane, uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t set_subtile(const ApplyParams& p, uint32_t sub, int lane, uint32_t a, uint32_t b, bool& wait) {
   const uint32_t lo = sub * CX_SUBTILE;
   TO* out = reinterpret_cast<TO*>(p.a.out) + lo;
   const CxPair* pairs = p.src.ep[0].pairs;
@@ -670,6 +680,7 @@ __device__ __forceinline__ uint32_t set_subtile(const ApplyParams& p, uint32_t s
     pr[k].val = 0;
     if (a + 32 * k + lane < b) pr[k] = ld_pair(pairs + a + 32 * k + lane);
   }
+  if (wait) { cx::pdl_wait(); wait = false; }
   const float zero[4] = {p.a.scale * 0.f, p.a.scale * 0.f, p.a.scale * 0.f, p.a.scale * 0.f};
 #pragma unroll
   for (int q = 0; q < CX_SUBTILE / 128; ++q) cx::store4(out + q * 128 + lane * 4, zero);
@@ -696,13 +707,13 @@ constexpr int dense_per_sm(int op) { return op == CX_OP_MOMENTUM || op == CX_OP_
 template <int OP, typename TO>
 __global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel(const __grid_constant__ ApplyParams p) {
   __shared__ __align__(16) float s_acc[kWarps][CX_SUBTILE];
-  if (p.early) cx::pdl_trigger();
-  if (p.front_wait) cx::pdl_wait();
+  begin_apply(p, p.early);
   const int lane = threadIdx.x & 31;
   if (!wait_sources(p)) { cx::pdl_wait(); return; }
   const int warp = threadIdx.x >> 5;
   const uint32_t nwarps = gridDim.x * kWarps;
   float* acc = s_acc[warp];
+  bool wait = p.front_wait == CX_WAIT_VECTORS;
   uint32_t bad = 0;
   uint32_t sub = blockIdx.x * kWarps + warp, a, b;
   table_entry(p, sub, lane, a, b);
@@ -715,13 +726,14 @@ __global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel
     if (OP == CX_OP_SET && whole && p.src.count == 1) {
       const uint32_t a0 = __shfl_sync(0xffffffffu, a, 0), b0 = __shfl_sync(0xffffffffu, b, 0);
       if (b0 - a0 <= kDirect) {
-        bad |= set_subtile<TO>(p, sub, lane, a0, b0);
+        bad |= set_subtile<TO>(p, sub, lane, a0, b0, wait);
         a = na;
         b = nb;
         continue;
       }
     }
     bad |= accumulate_subtile(p, sub, lane, a, b, acc);
+    if (wait) { cx::pdl_wait(); wait = false; }
     a = na;
     b = nb;
     auto walk = [&](auto all) {
@@ -1043,7 +1055,9 @@ int cx_apply_cuda(const CxSources* src, int64_t n, const CxApplyArgs* a, uint32_
   if (a->op == CX_OP_ADAMW && !a->v) return cx_set_error("cx_apply: second-moment buffer missing", 0);
   p.vec = aligned16(a->out) && (!a->shadow || aligned16(a->shadow)) && (!a->m || aligned16(a->m)) &&
           (!a->v || aligned16(a->v));
-  p.front_wait = !(cx_chain_bits() & CX_CHAINED) && cx_front_wait(stream) ? 1u : 0u;
+  p.front_wait = cx_chain_bits() & CX_CHAINED ? CX_WAIT_NONE : cx_front_wait(stream);
+  // what the first of a chain waits for has to be complete for the others, too
+  if (p.front_wait != CX_WAIT_NONE && cx_chain_bits() & CX_CHAIN_NEXT) p.front_wait = CX_WAIT_CHAIN;
   const int dt = update ? (a->shadow ? a->shadow_dtype : CX_F32) : a->out_dtype;
   int grid = cx_sm_count() * dense_per_sm(a->op);      // the sparse ops: as many as for SET
   p.group = 1;
@@ -1153,7 +1167,7 @@ int cx_forward_cuda(const CxEndpoint* from, uint64_t expect_seq, const CxTargets
   // every CTA waits on the same notification, so keep the grid co-resident
   const int grid = cx_sm_count() * 2;
   forward_kernel<<<grid, kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
-  cx_note_stream(stream, false);
+  cx_note_sender(stream);
   cx_note_launch();
   return cx_check_launch("forward_kernel");
 }

@@ -891,7 +891,7 @@ int cx_compress_fold_cuda(int gdtype, const CxFold* fold, float* r, int64_t n, c
     case CX_F16: launch_fold_input<__half>(q, s); break;
     default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
   }
-  cx_note_stream(stream, false);
+  cx_note_sender(stream);
   cx_note_launch();
   return cx_check_launch("compress_fold_kernel");
 }
@@ -910,7 +910,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (n == 0) {
     compress_empty_kernel<<<1, 32, 0, s>>>(p);
-    cx_note_stream(stream, false);
+    cx_note_sender(stream);
     cx_note_launch();
     return cx_check_launch("compress_empty_kernel");
   }
@@ -928,7 +928,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
       default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
     }
     if (rc) return rc;
-    cx_note_stream(stream, false);
+    cx_note_sender(stream);
     cx_note_launch();
     return cx_check_launch("compress_bulk_kernel");
   }
@@ -939,7 +939,7 @@ int cx_compress_cuda(int gdtype, const void* g, float* r, int64_t n, const float
     case CX_F16: launch_mode<__half>(p, grid, s); break;
     default: return cx_set_error("cx_compress: unsupported dtype on CUDA", 0);
   }
-  cx_note_stream(stream, false);
+  cx_note_sender(stream);
   cx_note_launch();
   return cx_check_launch("compress_kernel");
 }

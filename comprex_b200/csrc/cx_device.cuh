@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "cx_common.h"
+#include "cx_notes.h"
 
 namespace cx {
 
@@ -287,9 +288,13 @@ bool cx_pdl_enabled();   // COMPREX_PDL != 0 (read once)
 // is over when it may go on.  A receive kernel, however, does not wait at its start when its sender is
 // in front of it, so it has to know what is: senders note "not early"; every other kernel that triggers
 // before it is done with its operands notes "early" (receive kernels, thresholds, norms, dense updates),
-// and cx_front_wait says whether the kernel about to be launched must wait first.
+// and cx_front_wait says how the kernel about to be launched must wait.  The notes know this library's
+// kernels alone: a kernel of the program's own that was queued behind the sender may be at work on the
+// receiver's vectors (and let the receiver in early), so without waiting the receiver may only poll and
+// read its slots, unless the sender was launched by the same native call.
 void cx_note_stream(const void* stream, bool early);
-bool cx_front_wait(const void* stream);
+void cx_note_sender(const void* stream);
+uint32_t cx_front_wait(const void* stream);
 
 // Launches of one op list that may overlap (CxOp::chain), for the op this thread issues right now.
 // A chained kernel does not wait for the one in front before it starts, only before it ends, so that

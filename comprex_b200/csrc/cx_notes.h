@@ -6,6 +6,12 @@
 #include <atomic>
 #include <mutex>
 
+/* how a receive kernel waits for the kernel in front */
+#define CX_WAIT_NONE 0u     /* the sender is in front, of the same native call: it touches none of the vectors */
+#define CX_WAIT_START 1u    /* a kernel that was let in early may be in front: wait first */
+#define CX_WAIT_VECTORS 2u  /* wait before the vectors are touched */
+#define CX_WAIT_CHAIN 3u    /* like CX_WAIT_START, and the kernel behind (chained) is let in after that */
+
 class CxStreamNotes {
  public:
   static constexpr int kDevices = 64, kSlots = 64;
@@ -44,4 +50,26 @@ class CxStreamNotes {
   }
   mutable std::atomic<uint64_t> last_[kDevices][kSlots] = {};
   std::mutex order_[kDevices][kSlots], order_of_others_;
+};
+
+// What a thread's native call has launched so far, for the op it launches next.  Between two calls the program
+// may queue kernels of its own on the stream, which the notes do not know: only a sender that the op in front,
+// in the same call, has launched on the same stream is known to be the kernel in front.
+class CxCallFront {
+ public:
+  void begin_call() { sent_ = behind_ = false; }
+  void begin_op(const void* stream) {
+    behind_ = sent_ && stream_ == stream;
+    sent_ = false;
+  }
+  void sender(const void* stream) {
+    sent_ = true;
+    stream_ = stream;
+  }
+  void end_call() { sent_ = behind_ = false; }
+  bool behind_sender() const { return behind_; }
+
+ private:
+  const void* stream_ = nullptr;
+  bool sent_ = false, behind_ = false;
 };

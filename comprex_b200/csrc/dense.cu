@@ -218,7 +218,7 @@ struct ReduceParams {
   uint64_t timeout_ns;
   Ranges rg;           // gather mode: source j lands at out[start_j .. start_j+len_j)
   int32_t gather;
-  int32_t front_wait;  // the kernel in front may be at work on the same vectors
+  uint32_t front_wait; // CX_WAIT_*: the kernel in front may be at work on the same vectors
   int32_t vec16;       // every operand and target takes 16-byte accesses
 };
 
@@ -298,6 +298,7 @@ __device__ __forceinline__ void dense_reduce_body(const ReduceParams& p) {
     if (s_last && threadIdx.x == 0) { p.ctr->pad[0] = 0; p.ctr->pad[2] = 0; }
     return;
   }
+  if (p.front_wait == CX_WAIT_VECTORS) cx::pdl_wait();
   T* out = reinterpret_cast<T*>(p.out);
   const T* own = reinterpret_cast<const T*>(p.own);
   const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -442,7 +443,7 @@ __device__ __forceinline__ void dense_reduce_body(const ReduceParams& p) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 4) dense_reduce_kernel(const __grid_constant__ ReduceParams p) {
   if (!p.has_push) cx::pdl_trigger();      // (a pushing reduce is a sender too: receivers behind it do not wait)
-  if (p.front_wait) cx::pdl_wait();
+  if (p.front_wait == CX_WAIT_START) cx::pdl_wait();
   dense_reduce_body<T>(p);
   cx::pdl_wait();   // launched early behind the sending kernel: do not complete before that grid has
 }
@@ -508,7 +509,7 @@ int cx_dense_send_cuda(int dtype, const void* g, float* r, int64_t n, uint64_t s
   const int grid = grid_for(work, starts || r ? 8 : 4);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const bool capturing = p.seq_cell != nullptr;
-  cx_note_stream(stream, false);
+  cx_note_sender(stream);
   switch (dtype) {
     case CX_F32:
       if (r) cx_launch_pdl(dense_send_kernel<float, true>, grid, kThreads, 0, s, p, capturing);
@@ -542,8 +543,9 @@ int cx_dense_reduce_cuda(int dtype, void* out, const void* own, int64_t n, const
   p.ctr = reinterpret_cast<CxWorkCounters*>(counters);
   p.status = status; p.timeout_ns = timeout_ns;
   p.gather = starts != nullptr;
-  p.front_wait = cx_front_wait(stream) ? 1 : 0;
-  cx_note_stream(stream, !p.has_push);
+  p.front_wait = cx_front_wait(stream);
+  if (p.has_push) cx_note_sender(stream);
+  else cx_note_stream(stream, true);
   {
     uintptr_t bits = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(own);
     for (int j = 0; j < src->count; ++j) bits |= reinterpret_cast<uintptr_t>(src->ep[j].pairs);

@@ -327,7 +327,7 @@ struct RecvParams {
   RunSums* block;      // [blocks of runs]: sums of the blocks before it in its group
   int32_t groups;      // CTAs of the index kernel
   int64_t per_cta;     // outputs per CTA of the expand kernel, a multiple of kWindow
-  uint32_t front_wait;  // the kernel in front may be an expansion that still reads the index
+  uint32_t front_wait;  // CX_WAIT_*: the kernel in front may be an expansion that still reads the index
   uint32_t* status;
   uint64_t timeout_ns;
 };
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads) rle_index_kernel(const __grid_consta
   __shared__ int s_bad;
   __shared__ long long s_sum[kWarps][2];
   cx::pdl_trigger();
-  if (p.front_wait) cx::pdl_wait();
+  if (p.front_wait == CX_WAIT_START) cx::pdl_wait();   // (the vector is touched by the kernel behind, which waits for this one)
   if (threadIdx.x == 0) {
     int st = 0, first = 0;
     int64_t nnz = 0, nruns = 0;
@@ -660,7 +660,7 @@ int cx_rle_send_cuda(int gdtype, const void* g, float* r, int64_t n, const float
     case CX_F16: launch_send<__half>(p, grid, s); break;
     default: return cx_set_error("cx_rle_send: unsupported dtype on CUDA", 0);
   }
-  cx_note_stream(stream, false);
+  cx_note_sender(stream);
   cx_note_launch();
   cx_note_launch();
   return cx_check_launch("rle send kernels");
@@ -689,7 +689,7 @@ int cx_rle_recv_cuda(const CxEndpoint* src, uint64_t expect_seq, float* out, int
   p.group_bad = reinterpret_cast<int32_t*>(p.group + kGroups);
   p.block = reinterpret_cast<RunSums*>(p.group_bad + kGroups);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  p.front_wait = cx_front_wait(stream) ? 1u : 0u;
+  p.front_wait = cx_front_wait(stream);
   cx_note_stream(stream, true);
   cx_launch_pdl(rle_index_kernel, p.groups, kThreads, 0, s, p, false);
   cx_note_launch();

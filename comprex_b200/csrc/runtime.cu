@@ -93,7 +93,15 @@ static int current_device() {
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
 void cx_note_stream(const void* stream, bool early) { g_notes.note(current_device(), stream, early); }
-bool cx_front_wait(const void* stream) { return g_notes.front_wait(current_device(), stream); }
+static thread_local CxCallFront g_call_front;
+void cx_note_sender(const void* stream) {
+  cx_note_stream(stream, false);
+  g_call_front.sender(stream);
+}
+uint32_t cx_front_wait(const void* stream) {
+  if (g_notes.front_wait(current_device(), stream)) return CX_WAIT_START;
+  return g_call_front.behind_sender() ? CX_WAIT_NONE : CX_WAIT_VECTORS;
+}
 namespace {
 // A thread's turn on a stream: launches that take part in the notes are made inside one.  (Ops of a list on
 // a side stream need none of their own, one list at a time uses those.)
@@ -367,6 +375,10 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
   bool cuda = false;           // (host ops wait for other threads' messages: no turn)
   for (int i = 0; i < count; ++i) cuda |= ops[i].dev == CX_DEV_CUDA;
   Turn turn(cuda ? CX_DEV_CUDA : CX_DEV_HOST, stream);
+  struct Call {
+    Call() { g_call_front.begin_call(); }
+    ~Call() { g_call_front.end_call(); }
+  } call;
   cudaStream_t main_stream = reinterpret_cast<cudaStream_t>(stream);
   Lanes* lanes = nullptr;
   std::unique_lock<std::mutex> lanes_held;   // taken with the first side-stream op, released on return
@@ -385,6 +397,7 @@ int cx_run_ops(CxOp* ops, int count, uint64_t seq, void* stream) {
   };
   // thresholds that follow one another on one lane share launches
   auto run_some = [&](int i, void* on) -> int {      // ops taken, or a negative error
+    g_call_front.begin_op(on);
     if (ops[i].kind == CX_OPK_THRESHOLD && ops[i].dev == CX_DEV_CUDA) return cx_threshold_batch_cuda(ops + i, count - i, on);
     auto chained = [&](int k) {
       return k > 0 && k < count && ops[k].chain && ops[k].kind == ops[k - 1].kind && ops[k].lane == ops[k - 1].lane;

@@ -290,6 +290,31 @@ static void notes_threads_case() {
   CHECK(wrong[0] == 0 && wrong[1] == 0 && free_to_go > 0);
 }
 
+// Only a sender that the op in front launched, in the same call and on the same stream, is known to be in front.
+static void call_front_case() {
+  CxCallFront f;
+  const void *a = nullptr, *b = (const void*)0x5000;
+  f.begin_op(a);
+  CHECK(!f.behind_sender());
+  f.sender(a);                                         // a call of its own: no op was begun behind it
+  CHECK(!f.behind_sender());
+  f.begin_call();                                      // the next call: the program may have launched in between
+  f.begin_op(a);
+  CHECK(!f.behind_sender());
+  f.sender(a);
+  f.begin_op(a);
+  CHECK(f.behind_sender());
+  f.begin_op(a);                                       // the op in front sent nothing
+  CHECK(!f.behind_sender());
+  f.sender(b);
+  f.begin_op(a);                                       // a sender on another stream
+  CHECK(!f.behind_sender());
+  f.sender(a);
+  f.begin_op(a);
+  f.end_call();
+  CHECK(!f.behind_sender());
+}
+
 int main(int argc, char** argv) {
   const bool only_protocol = argc > 1 && !strcmp(argv[1], "--protocol");
   if (!only_protocol) {
@@ -317,6 +342,7 @@ int main(int argc, char** argv) {
     }
   }
   notes_case();
+  call_front_case();
   notes_threads_case();
   protocol_case();
   if (g_fail) { fprintf(stderr, "%d checks failed (%s)\n", g_fail, g_err); return 1; }

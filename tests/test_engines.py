@@ -467,3 +467,42 @@ def test_prepared_sends_survive_a_change_to_exact_and_back():
         assert all(bool((t == 7).all()) for t in others), k
     env.check()
     env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["pairs", "rle", "dense"])
+@pytest.mark.parametrize("read", ["add", "set"])
+@pytest.mark.parametrize("side", [64, 256, 1024])
+def test_program_work_between_send_and_receive(kind, read, side):
+    """A matrix product of the program's own writes the receiver's vector between the two halves of a message: the
+    receive kernel may be resident early, but touches the vector only behind that."""
+    n = side * side
+    env = cx.GaspiEnvironment(1 << 20, device="cuda")
+    ex = cx.GaspiEx(env, n) if kind == "dense" else cx.Comprex(env, n)
+    if kind != "dense":
+        ex.setThreshold(cx.ThresholdTopK(0.05))
+        ex.setCompressor(cx.CompressorRLE() if kind == "rle" else cx.CompressorIndexPairs())
+    ex.connectTo(0, 0)
+    gen = torch.Generator(device="cuda").manual_seed(side)
+    out, held = torch.empty(n, device="cuda"), torch.zeros(n, device="cuda")
+    for _ in range(8):
+        v = torch.randint(-9, 10, (n,), device="cuda", generator=gen).float()
+        a, b = (torch.randint(-2, 3, (side, side), device="cuda", generator=gen).float() for _ in range(2))
+        product = (a @ b).view(n)
+        out.fill_(1e6)
+        ex.writeRemote(v)
+        torch.mm(a, b, out=out.view(side, side))
+        if read == "add":
+            ex.readRemote_add(out)
+        elif kind == "dense":
+            ex.readRemote_vec(out, n)
+        else:
+            ex.readRemote(out)
+        held += v
+        if kind != "dense":
+            sent, held = held - ex.getRests(), ex.getRests()
+        else:
+            sent = v
+        assert torch.equal(out, (product if read == "add" else 0) + sent)
+    env.check()
+    env.close()
