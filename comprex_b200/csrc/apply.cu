@@ -662,10 +662,17 @@ __global__ void __launch_bounds__(kBulkMaxThreads, 1) apply_dense_bulk_kernel(co
 }
 
 // SET of one source: nothing is summed, so the pairs need not meet in shared memory.  Zeros go straight to the
-// sub-tile, then the values to their places (the warp's barrier orders the two); a sub-tile with more than
-// kDirect pairs (a store each, and the lines written twice; the line was not swept) takes shared memory.  Only
-// for sub-tiles whose 16-byte accesses all work.  Exchange of 2^20 elements, overwritten: 12.7 -> 12.2 us.
-constexpr uint32_t kDirect = 256;
+// sub-tile, then the values to their places (the warp's barrier orders the two).  Only for sub-tiles whose 16-byte
+// accesses all work.  A value costs a store of its own and dirties its sector a second time, so a sub-tile with
+// more pairs than the limit takes shared memory.  Where a warp has one sub-tile (7.2 M elements) the shorter chain
+// counts; behind that the stores do.  us with the sums in shared memory / direct, fp32 destination:
+//   pairs per sub-tile     10            31            61            102           154
+//   2^20 elements      4.48 / 3.97   4.48 / 3.99   4.48 / 4.22   4.74 / 4.48   4.74 / 4.99
+//   2^24               13.4 / 13.2   13.7 / 14.5   14.7 / 16.3   15.2 / 18.3   16.3 / 21.1
+//   2^26               52.9 / 53.0   54.7 / 56.2   57.0 / 58.0   57.1 / 64.4   62.6 / 74.4
+// bf16 destination, 2^20: 3.97 / 3.71 with 10 pairs, 4.22 / 4.22 with 102; 2^24: 9.60 / 9.09 with 10, 9.60 / 9.85
+// with 20; 2^26: 28.6 / 27.5 and 29.8 / 31.0.
+constexpr uint32_t kDirectShort = 102, kDirect = 15;
 template <typename TO>
 __device__ __forceinline__ uint32_t set_subtile(const ApplyParams& p, uint32_t sub, int lane, uint32_t a, uint32_t b, bool& wait) {
   const uint32_t lo = sub * CX_SUBTILE;
@@ -714,6 +721,7 @@ __global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel
   const uint32_t nwarps = gridDim.x * kWarps;
   float* acc = s_acc[warp];
   bool wait = p.front_wait == CX_WAIT_VECTORS;
+  const uint32_t direct = p.nsub <= nwarps ? kDirectShort : kDirect;
   uint32_t bad = 0;
   uint32_t sub = blockIdx.x * kWarps + warp, a, b;
   table_entry(p, sub, lane, a, b);
@@ -725,7 +733,7 @@ __global__ void __launch_bounds__(kThreads, dense_per_sm(OP)) apply_dense_kernel
     const bool whole = p.vec && (int64_t)lo + CX_SUBTILE <= p.n;
     if (OP == CX_OP_SET && whole && p.src.count == 1) {
       const uint32_t a0 = __shfl_sync(0xffffffffu, a, 0), b0 = __shfl_sync(0xffffffffu, b, 0);
-      if (b0 - a0 <= kDirect) {
+      if (b0 - a0 <= direct) {
         bad |= set_subtile<TO>(p, sub, lane, a0, b0, wait);
         a = na;
         b = nb;
