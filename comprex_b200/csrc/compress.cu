@@ -205,8 +205,14 @@ struct Stage {
 // A vector of one to three sub-tiles per warp is bound by this chain, not by memory: all warps walk through it
 // in step.  So the values go to shared memory first; a lane's survivors are then found by their bits (0.3 of 32 at
 // 1 %) instead of by 32 tests with a branch each, and the residual leaves before the reservation is back.
-// 2^16 / 2^20 elements 11.9 / 14.9 -> 11.4 / 14.3 us per exchange, 8 x 6.5 M 260 -> 250, 2^28 638 -> 633.
-template <bool HAS_G, bool HAS_R, bool MC>
+// 2^16 / 2^20 elements 11.9 / 14.9 -> 11.4 / 14.3 us per exchange, 8 x 6.5 M 260 -> 250.
+// LONG: many sub-tiles per warp and fp32 gradients.  What counts there is how long the list of a sub-tile with many
+// survivors takes: the fullest lane has five or six of them at 10 %, and as many steps; eight steps of four tests,
+// with the lanes side by side, are faster then.  fp32, 10 %, added, us per exchange with the bits walked / with tests:
+// 30 M 111.2 / 112.1, 50 M 180.7 / 178.5, 100 M 355.5 / 345.6, 128 Mi 475 / 461 (a shorter vector waits for the code:
+// 1 Mi 15.4 / 16.0); bf16, 128 Mi 421 / 431.  At 3 % (31 of 1024, few sub-tiles above kMany) there is no difference.
+constexpr uint32_t kMany = 48;
+template <bool HAS_G, bool HAS_R, bool MC, bool LONG = false>
 __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint32_t sub, const int lane, const float thr,
                                              float* __restrict__ rs, float* sv, uint16_t* sat, float (&v)[kChunks][4],
                                              Tally& tally) {
@@ -254,6 +260,20 @@ __device__ __forceinline__ void emit_subtile(const CompressParams& p, const uint
 
   // my survivors among the list's entries [w0, w0 + kList)
   auto fill = [&](const uint32_t w0) {
+    if (LONG && count > kMany) {
+      uint32_t pos = incl - mine - w0;
+#pragma unroll 1
+      for (uint32_t m = mask, at = lane * 4; m; m >>= 4, at += 128) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (m >> e & 1u) {
+            if (pos < kList) sat[pos] = (uint16_t)(at + e);
+            ++pos;
+          }
+        }
+      }
+      return;
+    }
     // two halves of the mask side by side: half the steps of a chain of dependent instructions
     uint32_t low = mask & 0xffffu, high = mask >> 16;
     uint32_t pos = incl - mine - w0, hpos = pos + __popc(low);   // wrap below the window: fail the test
@@ -503,7 +523,7 @@ __device__ __forceinline__ void pull_subtile(const T* __restrict__ g, const floa
 // compress_update (r only) and compress (g only).  MC: table and pairs go out once through
 // the multicast endpoint tg.ep[tg.count] (multimem.st) instead of once per target; headers and
 // notifications are still written target by target.
-template <typename T, bool HAS_G, bool HAS_R, bool MC>
+template <typename T, bool HAS_G, bool HAS_R, bool MC, bool LONG = false>
 __global__ void __launch_bounds__(kThreads, kPerSm)
 compress_kernel(const __grid_constant__ CompressParams p) {
   __shared__ __align__(16) Stage s_stage[kWarps];
@@ -551,7 +571,7 @@ compress_kernel(const __grid_constant__ CompressParams p) {
       const int64_t off = (int64_t)sub * CX_SUBTILE;
       if (!loaded) load_subtile<T, HAS_G, HAS_R>(g + off, r + off, lane, v);
       loaded = false;
-      emit_subtile<HAS_G, HAS_R, MC>(p, sub, lane, thr, r + off, stage.v, stage.at, v, tally);
+      emit_subtile<HAS_G, HAS_R, MC, LONG>(p, sub, lane, thr, r + off, stage.v, stage.at, v, tally);
     }
     else compress_subtile_edge<T, HAS_G, HAS_R, MC>(p, sub, lane, KnownThreshold{thr}, g, r, tally);
   }
@@ -732,9 +752,14 @@ void launch_pdl(K kernel, const CompressParams& p, int grid, cudaStream_t s) {
   cx_launch_pdl(kernel, grid, kThreads, 0, s, p, p.seq_cell != nullptr);
 }
 
+// from so many sub-tiles per warp on LONG is the faster one (between 12 and 20)
+constexpr uint32_t kLongRounds = 16;
+
 template <typename T, bool MC>
 void launch_mode_mc(const CompressParams& p, int grid, cudaStream_t s) {
-  if (p.g && p.r) launch_pdl(compress_kernel<T, true, true, MC>, p, grid, s);
+  if (p.g && p.r && sizeof(T) == 4 && p.nsub > kLongRounds * kWarps * (uint32_t)grid)
+    launch_pdl(compress_kernel<T, true, true, MC, sizeof(T) == 4>, p, grid, s);
+  else if (p.g && p.r) launch_pdl(compress_kernel<T, true, true, MC>, p, grid, s);
   else if (p.r) launch_pdl(compress_kernel<T, false, true, MC>, p, grid, s);
   else launch_pdl(compress_kernel<T, true, false, MC>, p, grid, s);
 }

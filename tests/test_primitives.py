@@ -997,6 +997,44 @@ def test_dense_subtiles_and_full_slots(count, room, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("extra", [0, 1024, 1024 + 500])
+@pytest.mark.parametrize("counts", [(0, 47, 48, 49), (1024, 500, 10, 0), (511, 512, 513, 48)])
+@pytest.mark.parametrize("room", [1.0, 0.7])
+def test_dense_subtiles_of_long_vectors(extra, counts, room):
+    """fp32 vectors on both sides of the length from which sub-tiles with many survivors are listed another way: all
+    of them, none, numbers around the line and around the length of the warp's list, and slots that are too small."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    subs = 16 * 16 * sms                       # 16 sub-tiles for each of 16 warps per SM
+    n = 1024 * subs + extra
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    e0 = env.get()
+    gen = torch.Generator(device="cuda").manual_seed(extra)
+    score = torch.rand(subs, 1024, device="cuda", generator=gen)
+    want = torch.tensor(counts, device="cuda").repeat(subs)[:subs]
+    kth = score.sort(dim=1).values
+    big = score <= torch.where(want > 0, kth.gather(1, (want - 1).clamp(min=0)[:, None])[:, 0], -1.0)[:, None]
+    big = torch.cat((big.view(-1), torch.ones(extra, dtype=torch.bool, device="cuda")))
+    del score, kth
+    g = torch.where(big, 2.0, 0.25) + 0.125 * torch.rand(n, device="cuda", generator=gen)
+    r = torch.rand(n, device="cuda", generator=gen) * 0.125
+    v = r + g
+    cap = n if room == 1.0 else int(room * int(big.sum()))      # (the regions of a slot fill unevenly here)
+    comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, cap)
+    comp.set_threshold(1.0)
+    comp.compress(g, r, n, cap, 1, P.make_targets([slot.endpoint(e0)]))
+    out, status = torch.full((n,), 9.0, device="cuda"), e0.new_status("t")
+    P.apply_sparse(e0, P.make_sources([slot.endpoint(e0)], [1]), n, P.args_set(out), status)
+    e0.flush()
+    hdr = e0.read_header(slot.endpoint(e0).hdr)
+    sent = out != 0
+    assert status.value == 0 and hdr.nnz_found == int(big.sum()) and hdr.nnz == int(sent.sum())
+    assert bool((sent <= big).all()) and torch.equal(out + r, v) and not bool(r[sent].any())
+    if room == 1.0:
+        assert torch.equal(sent, big)
+    env.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 31, 1000, 1023, 8 * 1024, 8 * 1024 + 1, 100003, 296 * 8 * 1024, 296 * 8 * 1024 + 1])
 @pytest.mark.parametrize("ratio", [0.001, 0.01, 0.1, 0.7])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
