@@ -49,13 +49,10 @@ namespace {
 
 // Warps of one CTA wait for one another only at its end, so small CTAs spread a short vector over more
 // SMs and let each go as soon as it is done: 65 536 elements 12.3 us with 256 threads, 12.0 with 128 and
-// 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference.  The kernel that folds
-// (below) takes 128, whose staging leaves more of the SM's memory to the loads than that of 256.
+// 64; 2^20 elements 15.8, 15.3 and 15.1.  From 6 M elements on it makes no difference.
 constexpr int kThreads = 64, kWarpsPerSm = 16;
 constexpr int kWarps = kThreads / 32;
-constexpr int kFoldThreads = 128;
 constexpr int kPerSm = kWarpsPerSm / kWarps;
-constexpr int kFoldWarps = kFoldThreads / 32;
 constexpr int kChunks = CX_SUBTILE / 128;  // 128 elements = 32 lanes x 4
 
 // -DCX_COMPRESS_TRACE: thread 0 of every CTA stamps %globaltimer at up to eight points of
@@ -877,10 +874,17 @@ void launch_fold_threads(const FoldCompressParams& q, cudaStream_t s) {
   else cx_launch_pdl(compress_fold_kernel<T, false, IN, THREADS>, grid, THREADS, 0, s, p, capturing);
 }
 
-// small CTAs for a vector too short for a large one on every SM (LeNet step 22.1 -> 21.8 us)
+// Small CTAs for a vector of at most eight sub-tiles per SM (LeNet step 22.1 -> 21.8 us; 1.0 M parameters, us per step
+// with 64 / 128 threads: 22.6 / 24.2 fp32, 22.4 / 24.0 bf16).  Then 256 threads, but 128 for fp32 gradients that are
+// folded into a momentum; us per step with 128 / 256, 25 MB buckets:
+//   bf16, AdamW:     GPT-2 of 30 / 36 / 61 / 124 M parameters 210.0 / 206.0, 250.7 / 242.8, 410 / 399, 803 / 786
+//   bf16, momentum:  ResNet of 3.0 / 4.5 / 25.6 M parameters 30.4 / 29.1, 35.9 / 35.3, 118.5 / 117.9
+//   fp32, momentum:  ResNet of 10 / 16 / 25.6 / 27.9 M parameters 68.2 / 69.0, 91.0 / 92.1, 133.3 / 135.2, 142.4 / 144.6,
+//                    but 6.9 M, whose second bucket is small, 57.2 / 55.3
 template <typename T, Input IN>
 void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
-  if (q.c.nsub <= (uint32_t)(cx_sm_count() * kFoldWarps)) launch_fold_threads<T, IN, kThreads>(q, s);
+  constexpr int kFoldThreads = IN == kFoldMom && sizeof(T) == 4 ? 128 : 256;
+  if (q.c.nsub <= (uint32_t)cx_sm_count() * 8) launch_fold_threads<T, IN, kThreads>(q, s);
   else launch_fold_threads<T, IN, kFoldThreads>(q, s);
 }
 
