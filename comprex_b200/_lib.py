@@ -70,14 +70,14 @@ class Fold(C.Structure):
     """A vector folded from gradient tensors (CxFold in csrc/cx_common.h)."""
     _fields_ = [("seg_ptr", C.c_void_p), ("seg_off", C.c_void_p), ("seg_end", C.c_void_p), ("coef", C.c_void_p),
                 ("sub_seg", C.c_void_p), ("border", C.c_void_p), ("u", C.c_void_p), ("base", C.c_int64), ("nseg", C.c_int32),
-                ("nborder", C.c_int32), ("mu", C.c_float), ("pad", C.c_int32)]
+                ("nborder", C.c_int32), ("mu", C.c_float), ("keep", C.c_int32)]
 
 
 class FoldCoef(C.Structure):
     """Arguments of cx_fold_coef (CxFoldCoef in csrc/cx_common.h)."""
     _fields_ = [("seg_ptr", C.c_void_p), ("item_rel", C.c_void_p), ("item_len", C.c_void_p), ("item_seg", C.c_void_p),
                 ("seg_first", C.c_void_p), ("partial", C.c_void_p), ("coef", C.c_void_p), ("count", C.c_void_p), ("items", C.c_int32),
-                ("segs", C.c_int32), ("clip", C.c_float), ("lr", C.c_float)]
+                ("segs", C.c_int32), ("clip", C.c_float), ("lr", C.c_float), ("keep", C.c_int32), ("pad", C.c_int32)]
 
 
 class Op(C.Structure):

@@ -852,6 +852,7 @@ __global__ void __launch_bounds__(kThreads, 4) fold_update_kernel(const __grid_c
   }
   const uint32_t nwarps = (gridDim.x - q.nborder_ctas) * kWarps;
   uint32_t sub = (blockIdx.x - q.nborder_ctas) * kWarps + warp;
+  const uint64_t last = q.f.keep ? cx::drop_policy() : cx::plain_policy();
   cx::FoldWhole<T> cur = {nullptr, 0.f, 0};
   if (sub < q.nsub) cur = cx::fold_whole<T>(q.f, sub);
   while (sub < q.nsub) {
@@ -867,7 +868,7 @@ __global__ void __launch_bounds__(kThreads, 4) fold_update_kernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < kGroup; ++k) {
           const int e0 = (c0 + k) * 128 + lane * 4;
-          cx::load4_last(cur.g + e0, x[k]);
+          cx::Raw4<T>::to_f(cx::load_hint(reinterpret_cast<const typename cx::Raw4<T>::type*>(cur.g + e0), last), x[k]);
 #pragma unroll
           for (int e = 0; e < 4; ++e) y[k][e] = 0.f;
           if (KEEP == 2) cx::load4(q.f.u + lo + e0, y[k]);

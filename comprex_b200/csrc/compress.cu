@@ -161,7 +161,8 @@ struct KnownThreshold {
 // The same for a folded input: up, mu, coef are the sub-tile's momentum and factors.
 template <typename T, Input IN, typename Thr>
 __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, const float* __restrict__ rl, float* __restrict__ up,
-                                                  const float mu, const float coef, const int lane, float (&v)[kChunks][4], Thr& late) {
+                                                  const float mu, const float coef, const uint64_t last, const int lane,
+                                                  float (&v)[kChunks][4], Thr& late) {
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) cx::load4(rl + lane * 4 + c * 128, v[c]);
   // all loads of a group are issued before its first store: the compiler must not move them across
@@ -172,7 +173,7 @@ __device__ __forceinline__ void load_fold_subtile(const T* __restrict__ gl, cons
     float y[kGroup][4];
 #pragma unroll
     for (int c = 0; c < kGroup; ++c) {
-      x[c] = cx::load_last(reinterpret_cast<const typename cx::Raw4<T>::type*>(gl + lane * 4 + (c0 + c) * 128));
+      x[c] = cx::load_hint(reinterpret_cast<const typename cx::Raw4<T>::type*>(gl + lane * 4 + (c0 + c) * 128), last);
       if (IN == kFoldMom) cx::load4(up + lane * 4 + (c0 + c) * 128, y[c]);
     }
     if (IN != kFold && c0 == 0) late.get();      // loads only before, stores from here on
@@ -613,7 +614,7 @@ compress_fold_kernel(const __grid_constant__ FoldCompressParams q) {
       cx::FoldWhole<T> ahead = {nullptr, 0.f, 0};
       if (cur.kind == 2) {
         float v[kChunks][4];
-        load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, lane, v, late);
+        load_fold_subtile<T, IN>(cur.g, r + off, IN == kFold ? nullptr : q.f.u + off, q.f.mu, cur.coef, q.f.keep ? cx::drop_policy() : cx::plain_policy(), lane, v, late);
         if (next < p.nsub) ahead = cx::fold_whole<T>(q.f, next);     // on its way while this one is stored
         emit_subtile<true, true, MC>(p, sub, lane, late.get(), r + off, s_stage[warp].v, s_stage[warp].at, v, tally);
       } else {

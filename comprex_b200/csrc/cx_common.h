@@ -157,7 +157,7 @@ typedef struct CxFold {
   int32_t nseg;
   int32_t nborder;
   float mu;
-  int32_t pad;
+  int32_t keep;                /* as in CxFoldCoef: the gradients' lines in L2 may go when they are read */
 } CxFold;
 
 /* arguments of cx_fold_coef; the item arrays as for cx_fold, every tensor with at least one item */
@@ -172,6 +172,9 @@ typedef struct CxFoldCoef {
   uint32_t* count;             /* scratch: one counter per tensor, zeroed once, left zeroed           */
   int32_t items, segs;
   float clip, lr;
+  int32_t keep;                /* the gradients are asked to stay in L2 until a kernel that takes the CxFold reads them
+                                  once more                                                           */
+  int32_t pad;
 } CxFoldCoef;
 
 /* ---- exported C ABI ------------------------------------------------- */

@@ -50,14 +50,6 @@ constexpr int kSpread = 128;
 constexpr int kSumWarps = kSum / 32;
 constexpr int kAhead = 8;
 
-// The gradients are read twice in a step: here, and by the kernel that folds them.  If they fit in L2 (126 MB)
-// they are read with the priority to stay there, against the weights, moments and residuals that stream past in
-// between, and the second reader gives the lines up again (cx::load_last).  25.6 M parameters, us per step with
-// bf16 gradients (51 MB): local 98.6 -> 96.3, exchange 119.3 -> 116.6; fp32 (102 MB): 101.1 -> 98.7, 132.9 -> 131.7.
-// With 710 MB of gradients it would cost 6 of 2168.  Their size is known by the items, of at most 65 536
-// elements: an upper bound, a third above the size in those models.
-constexpr int64_t kItem = 65536, kKeep = 160ll << 20;
-
 // lr times the clip factor of tensor `seg`, by the first kSpread threads of a CTA; valid in all of them.
 // W: floats per item.  Thread t adds the items t, t + kSpread, ..., then the threads' sums are added in a
 // fixed order.
@@ -97,14 +89,14 @@ __global__ void __launch_bounds__(kStrands) fold_sumsq_kernel(const __grid_const
   const T* g = reinterpret_cast<const T*>(p.seg_ptr[seg]) + p.item_rel[item];
   constexpr int kGroup = 16 / sizeof(T);
   float acc = 0.f;
-  const uint64_t keep = p.keep ? cx::keep_policy() : cx::plain_policy();
+  const uint64_t first = p.keep ? cx::keep_policy() : cx::plain_policy();
   if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
     const uint4* g16 = reinterpret_cast<const uint4*>(g);
     const int nv = len / kGroup;
     for (int q = strand; q < nv; q += kAhead * kSum) {
       uint4 x[kAhead];
 #pragma unroll
-      for (int k = 0; k < kAhead; ++k) x[k] = q + k * kSum < nv ? cx::load_keep(g16 + q + k * kSum, keep) : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < kAhead; ++k) x[k] = q + k * kSum < nv ? cx::load_hint(g16 + q + k * kSum, first) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int k = 0; k < kAhead; ++k) {
         const T* e16 = reinterpret_cast<const T*>(&x[k]);
@@ -207,7 +199,7 @@ int cx_fold_coef_cuda(int gdtype, const CxFoldCoef* f, void* stream) {
   p.seg_ptr = f->seg_ptr; p.item_rel = f->item_rel; p.item_len = f->item_len; p.item_seg = f->item_seg;
   p.seg_first = f->seg_first; p.partial = f->partial; p.coef = f->coef; p.count = f->count; p.segs = f->segs;
   p.clip = f->clip; p.lr = f->lr;
-  p.keep = (int64_t)f->items * kItem * (gdtype == CX_F32 ? 4 : 2) <= kKeep;
+  p.keep = f->keep;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (f->clip > 0.f) {
     if (const int rc = sumsq<kSpread>(gdtype, p, f->items, s)) return rc;

@@ -938,3 +938,20 @@ def test_local_step_of_more_than_2_31_parameters():
             # fp32 sums rounded to bf16 once
             assert ((p.detach()[k:k + (1 << 28)].float() - want).abs() <= want.abs() * 2.0 ** -8 * 1.001).all()
     env.close()
+
+
+def test_gradients_kept_in_l2_by_the_bytes_of_the_model(monkeypatch):
+    """The rule looks at all gradients of the model and the device's L2; every table of the model has its answer,
+    the buckets' own ones too, whatever the size of the items that the norms cut the tensors into."""
+    import types
+    from comprex_b200 import optim as O
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: types.SimpleNamespace(L2_cache_size=1000))
+    assert O._kept_in_l2(torch.device("cuda", 0), 2500) and not O._kept_in_l2(torch.device("cuda", 0), 2501)
+    assert not O._kept_in_l2(torch.device("cpu"), 4)
+    for answer in (True, False):
+        asked = []
+        monkeypatch.setattr(O, "_kept_in_l2", lambda d, n: asked.append(n) or answer)
+        params = [torch.nn.Parameter(torch.zeros(k, dtype=torch.bfloat16)) for k in (3000, 7, 20000, 64)]
+        opt = ComprexOptimizer(params, cx.GaspiEnvironment(1 << 20, device="cpu"), bucket_cap_mb=0.01)
+        assert asked == [2 * 23071] and len(opt._buckets) > 1
+        assert all(opt._table(b).keep == answer for b in opt._buckets)
