@@ -273,6 +273,8 @@ class Comprex(AbstractExchange):
                 self._dense.connectRx(self._src)
         if comp.kind == "rle" and self._rle is None:
             self._rle = P.RleCodec(self._env, self.size)     # worst-case sized slots (collective allocation)
+            if self._dest is not None:
+                self._rle.connect_tx()
         self.compressor = comp
 
     def getSize(self) -> int:
@@ -330,6 +332,8 @@ class Comprex(AbstractExchange):
         self._alloc_rests()
         if self._dense is not None:
             self._dense.connectTx(Rank, tag)
+        if self._rle is not None:
+            self._rle.connect_tx()
 
     def connectRx(self, Rank: int, tag: int = 0) -> None:
         self._check_rank(Rank)

@@ -300,8 +300,8 @@ int cx_rle_decode_host(const void* in, int64_t in_bytes, float* out, int64_t n,
 /* RLE fused with the transfer: the payload (same byte layout as the host codec) is stored
  * into every target's slot and released with `seq`; the receiver waits (bounded), checks the
  * runs and expands.  thr points to device memory on CUDA.  slot_bytes is the payload room of
- * a slot (>= cx_rle_slot_bytes(n)); the workspace (>= cx_rle_workspace_bytes(n), zeroed once)
- * is rank-local scratch.  A payload that fails a check sets CX_ST_BAD_HEADER and leaves `out`
+ * a slot (>= cx_rle_slot_bytes(n)); the workspace (>= cx_rle_workspace_bytes(n), 4.1 bytes an
+ * element, its first 256 bytes zeroed once) is rank-local scratch.  A payload that fails a check sets CX_ST_BAD_HEADER and leaves `out`
  * as it was. */
 int64_t cx_rle_slot_bytes(int64_t n);
 int64_t cx_rle_workspace_bytes(int64_t n);

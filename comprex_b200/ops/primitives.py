@@ -258,16 +258,30 @@ class Compressor:
 
 class RleCodec:
     """Slots and scratch of one run-length coded connection (csrc/rle.cu): two receive slots
-    sized for the worst case (collective allocation) plus one workspace per direction."""
+    sized for the worst case (collective allocation) plus one workspace per direction.  The sender's
+    (4.1 bytes an element) comes with :meth:`connect_tx`: a connection that only receives has none."""
+
+    TX_ZEROED = 256      # counters at the start of that; a message writes all else that it reads
 
     def __init__(self, env: GaspiEnvironment, n: int):
         self.env, self.n = env, n
         self.slot_bytes = int(env.lib.cx_rle_slot_bytes(n))
         self.ws_bytes = int(env.lib.cx_rle_workspace_bytes(n))
         self.slots = [DenseSlot.create(env, self.slot_bytes) for _ in range(2)]
-        self.tx_ws = env.scratch(self.ws_bytes)
+        self.tx_ws = None
         self.rx_ws_bytes = int(env.lib.cx_rle_recv_workspace_bytes(n))
         self.rx_ws = env.scratch(self.rx_ws_bytes)
+
+    def connect_tx(self) -> torch.Tensor:
+        """The sender's workspace, made when it is first asked for."""
+        if self.tx_ws is None:
+            if self.env.dev == _lib.DEV_CUDA:
+                ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=self.env.device)
+                ws[:self.TX_ZEROED].zero_()
+            else:
+                ws = self.env.scratch(0)          # the host codec needs none
+            self.tx_ws = ws
+        return self.tx_ws
 
     def send(self, g, r, thr_cell: torch.Tensor, seq: int, dest: int) -> None:
         """Encode ``r + g`` at the threshold in ``thr_cell`` into rank ``dest``'s slot."""
@@ -275,14 +289,14 @@ class RleCodec:
         gd = _lib.dtype_code(g.dtype) if g is not None else _lib.F32
         tg = make_targets([self.slots[seq & 1].endpoint(env, dest)])
         _lib.check(env.lib.cx_rle_send(env.dev, gd, _ptr(g), _ptr(r), self.n, thr_cell.data_ptr(), self.slot_bytes,
-                                       seq, C.byref(tg), self.tx_ws.data_ptr(), self.ws_bytes, env.rank,
+                                       seq, C.byref(tg), self.connect_tx().data_ptr(), self.ws_bytes, env.rank,
                                        _lib.stream_ptr(env.device)), "cx_rle_send")
 
     def send_op(self, r, thr_cell: torch.Tensor, par: int, dest: int) -> _lib.Op:
         """``send`` with residual ``r`` as an op of a launch list (the vector is filled in per call)."""
         o = _lib.Op()
         o.kind, o.dev, o.n, o.r, o.thr = _lib.OPK_RLE_SEND, self.env.dev, self.n, _ptr(r), thr_cell.data_ptr()
-        o.starts[0], o.workspace, o.ws_bytes, o.src_rank = self.slot_bytes, self.tx_ws.data_ptr(), self.ws_bytes, self.env.rank
+        o.starts[0], o.workspace, o.ws_bytes, o.src_rank = self.slot_bytes, self.connect_tx().data_ptr(), self.ws_bytes, self.env.rank
         o.tg = make_targets([self.slots[par].endpoint(self.env, dest)])
         return o
 

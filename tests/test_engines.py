@@ -506,3 +506,34 @@ def test_program_work_between_send_and_receive(kind, read, side):
         assert torch.equal(out, (product if read == "add" else 0) + sent)
     env.check()
     env.close()
+
+
+@pytest.mark.parametrize("codec_first", [False, True])
+def test_run_length_scratch_comes_with_the_sending_side(world, codec_first):
+    """The sender's workspace (4.1 bytes an element) is made when an engine connects to send, in either order with
+    the codec; an engine that only receives has none, and messages arrive whatever the memory held before."""
+    n, dev = 70001, world.device
+    junk = [torch.full((n,), 7, dtype=torch.int32, device=dev) for _ in range(8)]
+    del junk
+    ex = make(world, cx.Comprex, n)
+    for e in ex:
+        e.setThreshold(cx.ThresholdTopK(0.1))
+    if not codec_first:
+        ex[0].connectTx(1)
+        ex[1].connectRx(0)
+    for e in ex:
+        e.setCompressor(cx.CompressorRLE())
+    if codec_first:
+        ex[0].connectTx(1)
+        ex[1].connectRx(0)
+    assert ex[0]._rle.tx_ws is not None and ex[1]._rle.tx_ws is None and ex[2]._rle.tx_ws is None
+    held = torch.zeros(n, device=dev)
+    for _ in range(3):
+        v = torch.randint(-50, 50, (n,), device=dev).float()
+        ex[0].writeRemote(v)
+        out = torch.ones(n, device=dev)
+        ex[1].readRemote_add(out)
+        held += v
+        assert torch.equal(out - 1 + ex[0].getRests(), held)
+        held = ex[0].getRests()
+    assert ex[1]._rle.tx_ws is None
