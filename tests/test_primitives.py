@@ -174,9 +174,10 @@ def test_set_of_one_source(subs, count, dtype, shift):
         at = (place + 7 * (sub // 1024)) % 1024
         keep[sub + at[at < n - sub][:count]] = True
     x = torch.where(keep, torch.randn(n, generator=gen).abs() + 0.5, torch.zeros(n))
-    comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, n)
+    cap = n + 32 * 1024                        # every region has room for its sub-tiles
+    comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, cap)
     comp.set_threshold(0.25)
-    comp.compress(x.cuda(), None, n, n, 1, P.make_targets([slot.endpoint(e0)]))
+    comp.compress(x.cuda(), None, n, cap, 1, P.make_targets([slot.endpoint(e0)]))
     out = torch.full((n + 1,), 9.0, dtype=dtype, device="cuda")
     status = e0.new_status("t")
     P.apply_sparse(e0, P.make_sources([slot.endpoint(e0)], [1]), n, P.args_set(out[shift:shift + n], 0.5), status)
@@ -1018,7 +1019,7 @@ def test_dense_subtiles_of_long_vectors(extra, counts, room):
     g = torch.where(big, 2.0, 0.25) + 0.125 * torch.rand(n, device="cuda", generator=gen)
     r = torch.rand(n, device="cuda", generator=gen) * 0.125
     v = r + g
-    cap = n if room == 1.0 else int(room * int(big.sum()))      # (the regions of a slot fill unevenly here)
+    cap = n + 32 * 1024 if room == 1.0 else int(room * int(big.sum()))      # (the regions of a slot fill unevenly)
     comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, cap)
     comp.set_threshold(1.0)
     comp.compress(g, r, n, cap, 1, P.make_targets([slot.endpoint(e0)]))
