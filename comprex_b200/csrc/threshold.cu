@@ -140,19 +140,12 @@ __device__ __forceinline__ uint32_t block_rank(uint32_t key, int count, uint32_t
 //  * A lower bound with at least rank + 1 keys at or above it leaves few keys to rank.  Up to rank 31
 //    it is the (rank + 1)-th largest of 32 parts' maxima, and the warps rank what is left together;
 //    up to rank 767 it is that of the threads' maxima.
-//  * Up to one key per thread: bisection over the bits, no bound needed.
-//  * What is left (a large sample and a large rank, or many ties): four radix passes of 8 bits.
-// One warp ranking by shuffles and one count per bit to the last one: the 64 Ki exchange (1000 samples,
-// rank 9) took 12.7 us instead of 12.3, 25 M elements (10 000 samples) 57.7 for 57.2, 4 M at 10 %
-// (rank 99) 57.0 for 56.7.
+//  * What is left (a large rank, or many ties): four radix passes of 8 bits.
+// With one warp that ranks by shuffles 25 M elements (10 000 samples) took 57.7 us instead of 57.2.
+// (Samples of up to 2048 come here only beside a larger one in the same launch.)
 __device__ __forceinline__ void select_cached(uint32_t* s_keys, int s, uint32_t rank, const uint32_t* s_max, int maxima,
                                               uint32_t* s_hist, uint32_t* s_sel, float* out) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (rank >= 32 && s <= kThreads) {
-    const uint32_t key = block_rank(tid < s ? s_keys[tid] : 0u, s, rank, s_hist, s_sel + 2);
-    if (tid == 0) *out = __uint_as_float(key);
-    return;
-  }
   if (rank < 768) {
     uint32_t bound;
     if (tid == 0) s_sel[0] = 0;

@@ -955,3 +955,32 @@ def test_gradients_kept_in_l2_by_the_bytes_of_the_model(monkeypatch):
         opt = ComprexOptimizer(params, cx.GaspiEnvironment(1 << 20, device="cpu"), bucket_cap_mb=0.01)
         assert asked == [2 * 23071] and len(opt._buckets) > 1
         assert all(opt._table(b).keep == answer for b in opt._buckets)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("ratio", [0.01, 0.2])
+def test_thresholds_of_short_folded_buckets(dtype, ratio):
+    """Buckets of a few short tensors, sampled whole and in part, borders and gaps between the samples: every
+    bucket's threshold is the reference's for residual plus folded vector (which is stored as the momentum)."""
+    from helpers import ref_threshold_topk
+    torch.manual_seed(1)
+    sizes = [3, 64, 65, 700, 1, 900, 2048, 130, 1500, 40, 5000, 77]
+    params = [torch.nn.Parameter(torch.randn(k, device="cuda").to(dtype)) for k in sizes]
+    env = cx.GaspiEnvironment(1 << 20, device="cuda")
+    cap = 2048 * params[0].element_size() / 2 ** 20
+    opt = ComprexOptimizer(params, env, lr=0.1, momentum=0.9, compression_ratio=ratio, bucket_cap_mb=cap,
+                           single_rank_bypass=False)
+    assert len(opt._buckets) >= 5
+    for step in range(3):
+        for p in params:
+            p.grad = torch.randn_like(p) * 3.0
+        before = [None if b.ar is None else b.ar.rests.clone() for b in opt._buckets]
+        opt.step()
+        env.flush()
+        for b, rests in zip(opt._buckets, before):
+            folded = opt._update[b.start:b.end]
+            if rests is not None:
+                folded = folded + rests[:b.end - b.start]
+            assert float(b.ar._comp.thr) == ref_threshold_topk(folded, ratio), (step, b.start)
+    env.close()

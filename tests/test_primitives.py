@@ -192,8 +192,8 @@ def test_set_of_one_source(subs, count, dtype, shift):
 @pytest.mark.parametrize("data", ["normal", "ties", "constant", "ends"])
 @pytest.mark.parametrize("n", [33, 1000, 1024, 1025, 2049, 11008])
 def test_threshold_selection_ranks(n, data):
-    """The block-wide selection at the edges of its ranges: ranks around 32 and 768, samples around one
-    key per thread and the cluster's first size, few distinct keys."""
+    """Both selections at the edges of their ranges: ranks around 32 and 768, samples around 1024 (the kernel for up
+    to 2048 samples) and at the cluster's first and last size, few distinct keys."""
     torch.manual_seed(n)
     g = torch.randn(n)
     if data == "ties":
@@ -210,6 +210,33 @@ def test_threshold_selection_ranks(n, data):
         if rank < n and ratio < 1.0:
             comp.threshold_topk(dev, None, n, ratio, n, 1.0)
             assert comp.thr.item() == float(keys[rank]), rank
+    env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("large", [0, 12000, 30000])
+@pytest.mark.parametrize("data", ["normal", "ties"])
+def test_thresholds_that_share_a_launch(large, data):
+    """Several vectors in one list: samples of up to 2048 alone, and beside one that is larger than the cluster's
+    (they then take the large kernel, with every rank): each the reference's value."""
+    env = cx.GaspiEnvironment(1 << 16, device="cuda")
+    gen = torch.Generator().manual_seed(large)
+    todo = [(5, 0.5, 1000), (700, 0.1, 1000), (1000, 0.9, 1024), (1024, 0.01, 1024), (2048, 0.3, 2048), (3000, 0.02, 1500)]
+    if large:
+        todo.insert(3, (large + 17, 0.01, large))
+    ops, keep = (_lib.Op * len(todo))(), []
+    for o, (n, ratio, samples) in zip(ops, todo):
+        x = torch.randn(n, generator=gen)
+        if data == "ties":
+            x = x.mul(2.0).round()
+        comp, dev = P.Compressor(env, n), x.cuda()
+        o.kind, o.dev, o.n, o.dtype, o.g, o.thr = _lib.OPK_THRESHOLD, env.dev, n, _lib.F32, dev.data_ptr(), comp.thr.data_ptr()
+        o.ratio, o.default_subsamples, o.subsample_factor = ratio, samples, 0.0
+        keep.append((comp, dev, x))
+    _lib.check(env.lib.cx_run_ops(ops, len(todo), 1, _lib.stream_ptr(env.device)))
+    env.flush()
+    for (comp, _, x), (n, ratio, samples) in zip(keep, todo):
+        assert float(comp.thr) == ref_threshold_topk(x, ratio, samples, 0.0), (n, ratio)
     env.close()
 
 
