@@ -57,7 +57,7 @@ def _compile(src: Path, verbose: bool, ptxas_v: bool) -> Path:
     if not _stale(obj, [src] + headers):
         return obj
     if src.suffix == ".cu":
-        extra = os.environ.get("COMPREX_NVCC_EXTRA", "").split()   # e.g. -DCX_COMPRESS_MIN_BLOCKS=3
+        extra = os.environ.get("COMPREX_NVCC_EXTRA", "").split()   # e.g. -DCX_COMPRESS_TRACE
         cmd = ([_nvcc()] + NVCC_FLAGS + extra + (["-Xptxas", "-v"] if ptxas_v else [])
                + ["-c", str(src), "-o", str(obj)])
     else:

@@ -876,17 +876,19 @@ void launch_fold_threads(const FoldCompressParams& q, cudaStream_t s) {
 }
 
 // Small CTAs for a vector of at most eight sub-tiles per SM (LeNet step 22.1 -> 21.8 us; 1.0 M parameters, us per step
-// with 64 / 128 threads: 22.6 / 24.2 fp32, 22.4 / 24.0 bf16).  Then 256 threads, but 128 for fp32 gradients that are
-// folded into a momentum; us per step with 128 / 256, 25 MB buckets:
+// with 64 / 128 threads: 22.6 / 24.2 fp32, 22.4 / 24.0 bf16).  Then 256 threads, but 128 for gradients that are folded
+// into a momentum if they are fp32 or the vector is long; us per step with 128 / 256, 25 MB buckets:
 //   bf16, AdamW:     GPT-2 of 30 / 36 / 61 / 124 M parameters 210.0 / 206.0, 250.7 / 242.8, 410 / 399, 803 / 786
-//   bf16, momentum:  ResNet of 3.0 / 4.5 / 25.6 M parameters 30.4 / 29.1, 35.9 / 35.3, 118.5 / 117.9
+//   bf16, momentum:  ResNet of 3.0 / 4.5 / 6.9 M parameters 30.4 / 29.1, 35.9 / 35.3, 41.7 / 41.4,
+//                    9.4 / 16 / 25.6 M 47.4 / 47.5, 76.7 / 77.4, 116.5 / 117.2
 //   fp32, momentum:  ResNet of 10 / 16 / 25.6 / 27.9 M parameters 68.2 / 69.0, 91.0 / 92.1, 133.3 / 135.2, 142.4 / 144.6,
 //                    but 6.9 M, whose second bucket is small, 57.2 / 55.3
+constexpr uint32_t kLongFold = 8192;       // sub-tiles
 template <typename T, Input IN>
 void launch_fold(const FoldCompressParams& q, cudaStream_t s) {
-  constexpr int kFoldThreads = IN == kFoldMom && sizeof(T) == 4 ? 128 : 256;
   if (q.c.nsub <= (uint32_t)cx_sm_count() * 8) launch_fold_threads<T, IN, kThreads>(q, s);
-  else launch_fold_threads<T, IN, kFoldThreads>(q, s);
+  else if (IN == kFoldMom && (sizeof(T) == 4 || q.c.nsub > kLongFold)) launch_fold_threads<T, IN, IN == kFoldMom ? 128 : 256>(q, s);
+  else launch_fold_threads<T, IN, IN == kFoldMom && sizeof(T) == 4 ? 128 : 256>(q, s);
 }
 
 template <typename T>

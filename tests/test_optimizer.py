@@ -660,15 +660,15 @@ def test_no_sync_accumulates_like_plain_accumulation():
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["sgd", "sgd_no_momentum", "receive_momentum", "adamw"])
 @pytest.mark.parametrize("exchange", [True, False])
-@pytest.mark.parametrize("large", [False, True])      # a bucket with more sub-tiles than the small CTAs take
+@pytest.mark.parametrize("large", [False, True, "long"])   # a bucket with more sub-tiles than the small CTAs take, a long one
 def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange, large):
     """Folding inside the compress and update kernels (register path, tensor borders, gaps, a missing
     and an unaligned gradient, several buckets) against the vector built in memory first."""
-    sizes = [1, 63, 64, 65, 1023, 1024, 1025, 4096, 70001, 1500000 if large else 200000, 7, 2048]
+    sizes = [1, 63, 64, 65, 1023, 1024, 1025, 4096, 9000001 if large == "long" else 70001, 1500000 if large else 200000, 7, 2048]
     arms = []
     for fused in (True, False):
         torch.manual_seed(5)
-        env = cx.GaspiEnvironment((64 if large else 8) << 20, device="cuda")
+        env = cx.GaspiEnvironment((256 if large == "long" else 64 if large else 8) << 20, device="cuda")
         params = [torch.nn.Parameter(torch.randn(s, device="cuda").to(dtype)) for s in sizes]
         opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.0 if kind == "sgd_no_momentum" else 0.9,
                                compression_ratio=0.05, rule="adamw" if kind == "adamw" else "sgd", pre_clipnorm=20.0,
