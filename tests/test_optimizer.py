@@ -660,15 +660,15 @@ def test_no_sync_accumulates_like_plain_accumulation():
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["sgd", "sgd_no_momentum", "receive_momentum", "adamw"])
 @pytest.mark.parametrize("exchange", [True, False])
-@pytest.mark.parametrize("large", [False, True, "long"])   # a bucket with more sub-tiles than the small CTAs take, a long one
+@pytest.mark.parametrize("large", [False, True])      # a bucket with more sub-tiles than the small CTAs take
 def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange, large):
     """Folding inside the compress and update kernels (register path, tensor borders, gaps, a missing
     and an unaligned gradient, several buckets) against the vector built in memory first."""
-    sizes = [1, 63, 64, 65, 1023, 1024, 1025, 4096, 9000001 if large == "long" else 70001, 1500000 if large else 200000, 7, 2048]
+    sizes = [1, 63, 64, 65, 1023, 1024, 1025, 4096, 70001, 1500000 if large else 200000, 7, 2048]
     arms = []
     for fused in (True, False):
         torch.manual_seed(5)
-        env = cx.GaspiEnvironment((256 if large == "long" else 64 if large else 8) << 20, device="cuda")
+        env = cx.GaspiEnvironment((64 if large else 8) << 20, device="cuda")
         params = [torch.nn.Parameter(torch.randn(s, device="cuda").to(dtype)) for s in sizes]
         opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.0 if kind == "sgd_no_momentum" else 0.9,
                                compression_ratio=0.05, rule="adamw" if kind == "adamw" else "sgd", pre_clipnorm=20.0,
@@ -683,6 +683,42 @@ def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange, l
             for i, p in enumerate(params):
                 g = torch.randn(sizes[i] + 1, device="cuda", generator=gen).to(dtype)
                 p.grad = None if (step == 1 and i == 7) else g[1:] if i == 9 else g[:-1]     # i == 9: odd address
+            opt.step()
+        env.flush()
+        arms.append([opt._master.clone(), opt._shadow if dtype != torch.float32 else opt._master]
+                    + [t for t in (opt._m, opt._v) if t is not None] + ([opt._update] if opt._keeps_u else [])
+                    + [ar.rests for ar in opt.comprex_allreducers.values()])
+    assert len(arms[0]) == len(arms[1])
+    for a, b in zip(*arms):
+        assert torch.equal(a, b)
+    env.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["sgd", "sgd_no_momentum", "receive_momentum", "adamw"])
+@pytest.mark.parametrize("exchange", [True, False])
+def test_fused_step_of_a_long_bucket(dtype, kind, exchange):
+    """The same where a bucket is on the other side of the length from which 16-bit gradients with momentum are
+    folded in smaller CTAs."""
+    sizes = [65, 9000001, 1023, 70001, 7]
+    arms = []
+    for fused in (True, False):
+        torch.manual_seed(5)
+        env = cx.GaspiEnvironment(256 << 20, device="cuda")
+        params = [torch.nn.Parameter(torch.randn(s, device="cuda").to(dtype)) for s in sizes]
+        opt = ComprexOptimizer(params, env, lr=0.05, momentum=0.0 if kind == "sgd_no_momentum" else 0.9,
+                               compression_ratio=0.05, rule="adamw" if kind == "adamw" else "sgd", pre_clipnorm=20.0,
+                               local_momentum=kind != "receive_momentum", weight_decay=0.01, bucket_cap_mb=0.2,
+                               single_rank_bypass=not exchange)
+        assert len(opt._buckets) > 1
+        if not fused:
+            opt._fusable = lambda b: False
+            opt._cuda = False
+        for step in range(3):
+            gen = torch.Generator(device="cuda").manual_seed(step)
+            for p in params:
+                p.grad = torch.randn(p.numel(), device="cuda", generator=gen).to(dtype)
             opt.step()
         env.flush()
         arms.append([opt._master.clone(), opt._shadow if dtype != torch.float32 else opt._master]

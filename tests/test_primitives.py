@@ -156,11 +156,39 @@ def test_exact_topk_candidates_in_few_ctas(dtype):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("subs,count", [(3, c) for c in (0, 1, 31, 101, 102, 103, 128, 129, 255, 256, 257, 1024)]
-                         + [(8000, c) for c in (0, 14, 15, 16, 129, 1024)])
+@pytest.mark.parametrize("count", [0, 1, 31, 128, 129, 255, 256, 257, 1024])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shift", [0, 1])
-def test_set_of_one_source(subs, count, dtype, shift):
+def test_set_of_one_source(count, dtype, shift):
+    """Sub-tiles on both sides of the count up to which values go straight to their places, a partial one at
+    the end, and a destination that takes no wide accesses: every other element is overwritten with zero."""
+    n = 3 * 1024 + 500
+    world = cx.LoopbackWorld(1, device="cuda", timeout_ms=2000)
+    e0 = world.envs[0]
+    gen = torch.Generator().manual_seed(count)
+    keep = torch.zeros(n, dtype=torch.bool)
+    for sub in range(0, n, 1024):
+        room = min(1024, n - sub)
+        keep[sub + torch.randperm(room, generator=gen)[:count]] = True
+    x = torch.where(keep, torch.randn(n, generator=gen).abs() + 0.5, torch.zeros(n))
+    comp, slot = P.Compressor(e0, n), P.SparseSlot.create(e0, n, n)
+    comp.set_threshold(0.25)
+    comp.compress(x.cuda(), None, n, n, 1, P.make_targets([slot.endpoint(e0)]))
+    out = torch.full((n + 1,), 9.0, dtype=dtype, device="cuda")
+    status = e0.new_status("t")
+    P.apply_sparse(e0, P.make_sources([slot.endpoint(e0)], [1]), n, P.args_set(out[shift:shift + n], 0.5), status)
+    e0.flush()
+    assert status.value == 0
+    assert torch.equal(out[shift:shift + n].cpu(), (0.5 * x).to(dtype))
+    assert float(out[n if shift == 0 else 0]) == 9.0
+    world.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("subs,count", [(3, c) for c in (101, 102, 103)] + [(8000, c) for c in (0, 14, 15, 16, 129, 1024)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_set_of_one_source_by_length(subs, count, dtype, shift):
     """Sub-tiles on both sides of the counts up to which values go straight to their places, in a vector of one
     sub-tile per warp and in a longer one, a partial one at the end, and a destination that takes no wide
     accesses: every other element is overwritten with zero."""
