@@ -700,7 +700,8 @@ def test_fused_step_gives_the_bits_of_the_stored_vector(dtype, kind, exchange, l
 @pytest.mark.parametrize("exchange", [True, False])
 def test_fused_step_of_a_long_bucket(dtype, kind, exchange):
     """The same where a bucket is on the other side of the length from which 16-bit gradients with momentum are
-    folded in smaller CTAs."""
+    folded in smaller CTAs.  (The model stays below 9.7 M elements: there the norms of one bucket and of all of
+    them are summed over items of another length.)"""
     sizes = [65, 9000001, 1023, 70001, 7]
     arms = []
     for fused in (True, False):
